@@ -192,8 +192,9 @@ int pjx_attn_bwd_band(const void* q, const void* k, const void* v, const void* o
                       int band_lo, int band_hi, float sm_scale, int impl, void* workspace,
                       size_t workspace_bytes, int32_t* status, void* stream);
 size_t pjx_attn_bwd_workspace_bytes(int B, int Lq, int Hq);
-/* pjx_attn_bwd_band with score modifiers (mod may be NULL).  With modifiers the CUDA-core kernels
- * run; `dbias` cannot be combined with head_scale / softcap. */
+/* pjx_attn_bwd_band with score modifiers (mod may be NULL).  16-bit calls with modifiers run on the
+ * tensor cores as well (head shapes (64, 64), (128, 128), (192, 128)) unless `impl` forces a kernel;
+ * `dbias` cannot be combined with head_scale / softcap. */
 int pjx_attn_bwd_mod(const void* q, const void* k, const void* v, const void* o, const float* lse,
                      const void* d_o, void* dq, void* dk, void* dv, const int32_t* kv_lengths,
                      const float* bias, int64_t bias_batch_stride, int64_t bias_head_stride,

@@ -30,6 +30,7 @@ SOURCES = [
     "attn_fwd_generic.cu",
     "attn_bwd_generic.cu",
     "attn_bwd_sm100.cu",
+    "attn_bwd_sm100_exact.cu",
     "attn_fwd_sm100.cu",
     "attn_decode.cu",
     "attn_decode_latent.cu",

@@ -53,7 +53,8 @@ __global__ void bwd_delta_kernel(const BwdParams p) {
   for (int off = 16; off >= 1; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
   if (lane == 0) {
     p.delta[at] = acc;
-    p.lse2[at] = p.lse[((int64_t)b * p.Hq + h) * p.Lq + i] * kLog2e;  // +inf (row without keys) stays +inf
+    // +inf (row without keys) stays +inf
+    p.lse2[at] = p.lse[((int64_t)b * p.Hq + h) * p.Lq + i] * (p.lse_natural ? 1.f : kLog2e);
   }
 }
 
@@ -314,11 +315,6 @@ template <typename T_, int NCK, int NCV>
 int launch_widths(const BwdParams& p, cudaStream_t stream) {
   const size_t smem = bwd_smem_bytes(p.D, p.Dv);
   int rc;
-  const int64_t rows = (int64_t)p.B * p.Lq_pad * p.Hq;
-  bwd_delta_kernel<T_><<<(unsigned)((rows + 7) / 8), 256, 0, stream>>>(p);
-  count_launch();
-  if ((rc = check_cuda(cudaGetLastError(), "backward delta launch"))) return rc;
-  if (p.use_sm100) return launch_bwd_sm100(p, stream);
   auto kq = bwd_dq_kernel<T_, NCK>;
   if ((rc = set_smem(kq, smem, "cudaFuncSetAttribute(backward dq)"))) return rc;
   kq<<<dim3((p.Lq + T - 1) / T, p.Hq, p.B), NT, smem, stream>>>(p);
@@ -332,8 +328,18 @@ int launch_widths(const BwdParams& p, cudaStream_t stream) {
   return check_cuda(cudaGetLastError(), "backward dk/dv launch");
 }
 
+// The kernels behind one backward call, picked by pjx_attn_bwd_mod.
+enum class BwdRoute { CudaCores, Sm100, Sm100Exact };
+
 template <typename T_>
-int launch_dtype(const BwdParams& p, cudaStream_t stream) {
+int launch_dtype(const BwdParams& p, BwdRoute route, void* scratch, cudaStream_t stream) {
+  const int64_t rows = (int64_t)p.B * p.Lq_pad * p.Hq;
+  bwd_delta_kernel<T_><<<(unsigned)((rows + 7) / 8), 256, 0, stream>>>(p);
+  count_launch();
+  const int rc = check_cuda(cudaGetLastError(), "backward delta launch");
+  if (rc) return rc;
+  if (route == BwdRoute::Sm100) return launch_bwd_sm100(p, stream);
+  if (route == BwdRoute::Sm100Exact) return launch_bwd_exact_sm100(p, scratch, stream);
   const int nk = p.D <= 64 ? 4 : (p.D <= 128 ? 8 : 16);
   const int nv = p.Dv <= 64 ? 4 : (p.Dv <= 128 ? 8 : 16);
   switch (nk * 100 + nv) {
@@ -599,34 +605,58 @@ int pjx_attn_bwd_mod(const void* q, const void* k, const void* v, const void* o,
   p.status = status;
   p.mod = smod;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  size_t dbias_bytes = 0;
   if (dbias) {
     if (!bias) return fail(PJX_ERR_BAD_ARG, "backward: dbias given without a bias");
     if (bias_batch_stride < 0 || bias_head_stride < 0) return fail(PJX_ERR_BAD_ARG, "bias strides must be non-negative");
     // the bias is [Bb, Hb, Lq, Lkv] with Bb in {1, B}, Hb in {1, Hq}: its extent follows from the strides
     const int64_t hb = bias_head_stride ? Hq : 1, bbn = bias_batch_stride ? B : 1;
-    int rc0 = check_cuda(cudaMemsetAsync(dbias, 0, (size_t)bbn * hb * Lq * Lkv * sizeof(float), st), "clear dbias");
-    if (rc0) return rc0;
+    dbias_bytes = (size_t)bbn * hb * Lq * Lkv * sizeof(float);
     p.dbias = dbias;
     p.dbias_atomic = (bias_batch_stride == 0 && B > 1) || (bias_head_stride == 0 && Hq > 1);
+  }
+  // 16-bit calls that the plain tcgen05 kernels do not take (score modifiers, dense bias, the latent head shape) run
+  // on the tensor cores with P and dS as 16 + 16 bits; what is left there (fp32 inputs, other head widths) and calls
+  // whose scratch cannot be had run on the CUDA cores.  A forced tcgen05 backward means the plain kernels.
+  const char* why = nullptr;
+  bool tc_ok = bwd_sm100_supported(p, &why);
+  if (tc_ok && smod.on) {
+    tc_ok = false;
+    why = "score modifiers are not evaluated by the plain tcgen05 kernels";
+  }
+  if (impl == PJX_IMPL_SM100 && !tc_ok && Lq > 0) return fail(PJX_ERR_UNSUPPORTED, "tcgen05 backward: %s", why);
+  BwdRoute route = impl != PJX_IMPL_GENERIC && tc_ok ? BwdRoute::Sm100 : BwdRoute::CudaCores;
+  void* scratch = nullptr;
+  if (impl == PJX_IMPL_AUTO && !tc_ok && bwd_exact_sm100_supported(p)) {
+    route = BwdRoute::Sm100Exact;
+    const size_t bytes = bwd_exact_scratch_bytes(p);
+    if (bytes > 0) {
+      keep_pool_memory();
+      if (cudaMallocAsync(&scratch, bytes, st) != cudaSuccess) {
+        (void)cudaGetLastError();
+        scratch = nullptr;
+        route = BwdRoute::CudaCores;
+      }
+    }
+  }
+  p.lse_natural = route == BwdRoute::Sm100Exact && (smod.on || bias);
+  if (dbias_bytes > 0 && route == BwdRoute::CudaCores) {  // (the tcgen05 kernel writes every entry)
+    const int rc0 = check_cuda(cudaMemsetAsync(dbias, 0, dbias_bytes, st), "clear dbias");
+    if (rc0) return rc0;
   }
   if (Lq == 0) {  // no queries: the key-side gradients are zero
     int rc = check_cuda(cudaMemsetAsync(dk, 0, (size_t)B * Lkv * Hkv * D * dtype_size(dtype), st), "clear dk");
     if (rc) return rc;
     return check_cuda(cudaMemsetAsync(dv, 0, (size_t)B * Lkv * Hkv * Dv * dtype_size(dtype), st), "clear dv");
   }
-  const char* why = nullptr;
-  bool tc_ok = bwd_sm100_supported(p, &why);
-  if (tc_ok && smod.on) {
-    tc_ok = false;
-    why = "score modifiers are evaluated by the CUDA-core backward only";
-  }
-  if (impl == PJX_IMPL_SM100 && !tc_ok) return fail(PJX_ERR_UNSUPPORTED, "tcgen05 backward: %s", why);
-  p.use_sm100 = impl != PJX_IMPL_GENERIC && tc_ok;
+  int rc;
   switch (dtype) {
-    case PJX_F32: return launch_dtype<float>(p, st);
-    case PJX_BF16: return launch_dtype<__nv_bfloat16>(p, st);
-    default: return launch_dtype<__half>(p, st);
+    case PJX_F32: rc = launch_dtype<float>(p, route, scratch, st); break;
+    case PJX_BF16: rc = launch_dtype<__nv_bfloat16>(p, route, scratch, st); break;
+    default: rc = launch_dtype<__half>(p, route, scratch, st);
   }
+  if (scratch) cudaFreeAsync(scratch, st);
+  return rc;
 }
 
 int pjx_attn_bwd(const void* q, const void* k, const void* v, const void* o, const float* lse, const void* d_o,

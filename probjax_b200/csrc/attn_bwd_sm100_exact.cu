@@ -1,0 +1,1188 @@
+// Flash-attention backward for sm_100a with P and dS carried at 32-bit grade: score modifiers
+// (segments, ALiBi, relative tables, soft cap, dropout, ...), a dense fp32 bias and its gradient, and the
+// latent head shape (192, 128).  Same two-kernel split, warp roles and half-step issue order as
+// attn_bwd_sm100.cu (dQ owns query tiles, dK/dV owns key tiles, no atomics); what differs:
+//
+// * P and dS enter the accumulating products as a sum of two 16-bit numbers, x = hi + lo with
+//   hi = round16(x) and lo = round16(x - hi): two MMAs against the same B descriptor instead of one.  The
+//   calls that arrive here ran on CUDA cores with P and dS in fp32 before, and 16 + 16 bits keep what that
+//   gave (2^-17 relative in bf16 against the 2^-9 of the stored gradients).  Per 128 x 128 tile that is 10
+//   products of 128 x 128 x D for both kernels instead of 7.  A 16-column chunk of scores (16 columns of
+//   tensor memory) is overwritten by its own 8 columns of hi and 8 of lo pairs, so the split costs no
+//   tensor memory.
+// * fp16 has no exponent range to spare for lo: P is packed scaled by a power of two (`p_scale`), dS by one
+//   derived from max|dO| and max|V| (`bwd_amax_kernel`), and the accumulators are scaled back when they
+//   leave tensor memory.
+// * head shape (192, 128): dV and dK take 320 columns of tensor memory, so the dK/dV kernel walks query
+//   tiles of 96 rows (two halves of 48: 2 x 96 + 320 = 512 columns) instead of 128.
+// * a segment mask cuts the tile loops to the ranges that can match (one range per 128 rows, both ways).
+// * a dense bias is read with keys on the lanes (coalesced) in the dK/dV and dbias kernels; the dQ kernel,
+//   whose threads own query rows, transposes it through a per-warp window in shared memory.
+// * the gradient of the bias is a kernel of its own: one CTA per 128 x 128 tile of the bias, walking the
+//   (batch, head) pairs that share it and summing dS in registers in a fixed order (no atomics).
+//
+// FEAT: bit 0 = score modifiers, bit 1 = dense bias; band and key-length masks always.
+// With FEAT 0 the row vector `lse2` is base 2; otherwise it is the natural log-sum-exp, subtracted before
+// the change of base, so that a bias of the type's lowest value cannot overflow to inf - inf.
+//
+// Bound by the MMA issue stream at D = 128 and by the element work of the compute warps at D = 64.
+// Measured (forward + backward, against the CUDA-core kernels these calls ran on before; B200):
+//   packed documents + ALiBi, B1 S4096 Hq32 Hkv8 D128 bf16     41.9 ms -> 0.90 ms
+//   dense bias with gradient, B8 S1024 H16 D64 bf16            6.26 ms -> 0.89 ms
+//   latent training step, B2 S2048 H16 (192,128) bf16          16.6 ms -> 0.67 ms
+#include "attn_bwd_sm100.cuh"
+
+namespace pjx {
+
+int make_tmap_blhd(CUtensorMap* m, const void* base, int dtype, int B, int L, int H, int Dim, int rows);
+bool bwd_exact_uses_ranges(const BwdParams& p);
+
+namespace {
+
+using namespace sm100;
+
+constexpr int BM = 128;        // query rows per tile of the dQ and dbias kernels
+constexpr int BN = 128;        // keys per tile
+constexpr int NTHREADS = 320;  // 10 warps: TMA producer, MMA issuer, two compute groups of four
+constexpr int CH = 16;         // score columns a thread works on at a time
+
+// What the kernels need beside BwdParams.
+struct ExactArgs {
+  int order_w;
+  const int32_t* q_range;  // [nb, ceil(Lq/128), 2]: keys a query tile can see (segments), or null
+  const int32_t* k_range;  // [nb, ceil(Lkv/128), 2]: query rows a key tile is seen by, or null
+  int64_t q_range_bs, k_range_bs;  // batch strides in tiles (0 = shared)
+  const uint32_t* amax;    // fp16: bit patterns of max|dO|, max|V|, max|head_scale|
+  float p_scale;           // fp16: factor P is packed with (a power of two); 1 for bf16
+};
+
+// fp16: the power of two dS is packed with.  |dS| <= P (|dP| + |delta|) |ds'/ds| and both |dP| and |delta| are at
+// most keep * Dv * max|dO| * max|V|, so the packed values stay below 2^15.
+template <int DV, bool BF16>
+__device__ __forceinline__ float ds_pack_scale(const ExactArgs& a, const ScoreMod& m) {
+  if constexpr (BF16) return 1.f;
+  const float keep = m.dropout_rate > 0.f ? 1.f / (1.f - m.dropout_rate) : 1.f;
+  const float bound = 2.f * keep * DV * __uint_as_float(a.amax[0]) * __uint_as_float(a.amax[1]) *
+                      (1.f + __uint_as_float(a.amax[2]));
+  if (!(bound > 0.f)) return 1.f;
+  const int e = (int)((__float_as_uint(bound) >> 23) & 255u) - 127;  // bound in [2^e, 2^(e+1))
+  return exp2f((float)max(-100, min(100, 14 - e)));
+}
+
+// A chunk of CH fp32 values as hi pairs (8 registers) and lo pairs (8 registers).
+template <bool BF16>
+__device__ __forceinline__ void split_pack(const float (&x)[CH], float scale, uint32_t (&r)[CH]) {
+#pragma unroll
+  for (int i = 0; i < CH / 2; ++i) {
+    float a = x[2 * i], b = x[2 * i + 1];
+    if constexpr (!BF16) {
+      a *= scale;
+      b *= scale;
+    }
+    const uint32_t hi = pack16<BF16>(a, b);
+    float ha, hb;
+    if constexpr (BF16) {
+      ha = __uint_as_float(hi << 16);
+      hb = __uint_as_float(hi & 0xffff0000u);
+    } else {
+      const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&hi));
+      ha = h.x;
+      hb = h.y;
+    }
+    r[i] = hi;
+    r[CH / 2 + i] = pack16<BF16>(a - ha, b - hb);
+  }
+}
+
+// CH bias values of one key: rows i0 .. i0 + CH - 1 of a plane with `Lkv` entries per row (`src` is at the key's
+// column), rows past Lq clamped.  The opaque index and the volatile loads keep the compiler from computing the 64-bit
+// addresses of a whole tile ahead of its loop and from hoisting the tile's loads to its start (both spill).
+__device__ __forceinline__ void load_bias_column(const float* src, int i0, int Lq, int Lkv, float* out) {
+  asm volatile("" : "+r"(i0));
+  const float* ptr = src + (int64_t)min(i0, Lq - 1) * Lkv;
+#pragma unroll
+  for (int e = 0; e < CH; ++e) {
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(out[e]) : "l"(ptr));
+    if (i0 + e + 1 < Lq) ptr += Lkv;
+  }
+}
+
+// The element (i, j) a column e of a chunk stands for.  ROWS: the thread owns query row i0 and the columns are
+// keys j0 + e; otherwise it owns key j0 and the columns are query rows i0 + e.
+struct Place {
+  int kv_len, Lq, Lkv, band_lo, band_hi;
+};
+
+// Bit e of the result: column e is visible.
+template <int FEAT, bool ROWS>
+__device__ __forceinline__ uint32_t keep_bits(const Place& pl, const ScoreModView& mv, bool seg_mixed, int own_seg, int i0, int j0) {
+  constexpr uint32_t ALL = (1u << CH) - 1;
+  const int i_last = ROWS ? i0 : i0 + CH - 1, j_last = ROWS ? j0 + CH - 1 : j0;
+  bool inside = j_last < pl.kv_len && i_last < pl.Lq && j_last <= i0 + pl.band_hi && j0 >= i_last + pl.band_lo;
+  if constexpr ((FEAT & 1) != 0) {
+    if (mv.row_limit) inside = inside && ROWS && j_last < mv.row_limit[min(i0, pl.Lq - 1)];
+    inside = inside && !seg_mixed;
+  }
+  if (inside) return ALL;
+  uint32_t bits = 0;
+#pragma unroll
+  for (int e = 0; e < CH; ++e) {
+    const int i = ROWS ? i0 : i0 + e, j = ROWS ? j0 + e : j0;
+    bool keep = j <= i + pl.band_hi && j >= i + pl.band_lo;
+    if constexpr ((FEAT & 1) != 0) {
+      keep = keep || j < mv.prefix;
+      if (mv.row_limit) keep = keep && j < mv.row_limit[min(i, pl.Lq - 1)];
+      if (seg_mixed) keep = keep && (ROWS ? mv.seg_k[min(j, pl.Lkv - 1)] : mv.seg_q[min(i, pl.Lq - 1)]) == own_seg;
+    }
+    keep = keep && j < pl.kv_len && i < pl.Lq;
+    bits |= keep ? (1u << e) : 0u;
+  }
+  return bits;
+}
+
+// P (dropped and rescaled under dropout) and dS of one chunk.  `lse` and `delta` hold one value (ROWS) or one per column.
+// NL = false: no head_scale / softcap (refused together with a bias gradient).
+template <int FEAT, bool ROWS, bool NL = true>
+__device__ __forceinline__ void chunk_p_ds(const float (&s)[CH], const float (&dp)[CH], float c, const Place& pl,
+                                           const ScoreModView& mv, uint32_t keep, int i0, int j0, const float* lse,
+                                           const float* delta, const float* bias, float (&pr)[CH], float (&ds)[CH]) {
+  if constexpr (FEAT == 0) {
+#pragma unroll
+    for (int e = 0; e < CH; ++e) {
+      pr[e] = ex2_approx(fmaf(s[e], c, -lse[ROWS ? 0 : e]));
+      ds[e] = pr[e] * (dp[e] - delta[ROWS ? 0 : e]);
+    }
+  } else {
+    float x[CH];
+#pragma unroll
+    for (int e = 0; e < CH; ++e) x[e] = s[e] * c;
+    const bool nonlinear = NL && (FEAT & 1) && (mv.hscale_m1 != 0.f || mv.softcap > 0.f);
+    float g[CH];
+    if (nonlinear) {
+      const float inv_cap = mv.softcap > 0.f ? 1.f / mv.softcap : 0.f;
+#pragma unroll
+      for (int e = 0; e < CH; ++e) {
+        const float sx = x[e];
+        float out = fmaf(sx, mv.hscale_m1, sx), d = 1.f + mv.hscale_m1;
+        if (mv.softcap > 0.f) {
+          const float t = tanhf(sx * inv_cap);
+          out += mv.softcap * t - sx;
+          d -= t * t;
+        }
+        x[e] = out;
+        g[e] = d;
+      }
+    }
+    if ((FEAT & 1) && mv.alibi_mode) {
+      const float base = (float)(i0 - j0);
+#pragma unroll
+      for (int e = 0; e < CH; ++e) {
+        const float dist = ROWS ? base - (float)e : base + (float)e;  // i - j, exact
+        x[e] = fmaf(-mv.slope, mv.alibi_mode == 1 ? fmaxf(dist, 0.f) : fabsf(dist), x[e]);
+      }
+    }
+    if ((FEAT & 1) && mv.rel) {
+#pragma unroll
+      for (int e = 0; e < CH; ++e) {
+        const int t = ROWS ? j0 + e - i0 : j0 - i0 - e;
+        x[e] += __ldg(mv.rel + max(1 - pl.Lq, min(pl.Lkv - 1, t)));  // clamped: rows and keys past the tensors
+      }
+    }
+    if constexpr ((FEAT & 2) != 0) {
+#pragma unroll
+      for (int e = 0; e < CH; ++e) x[e] += bias[e];
+    }
+    if ((FEAT & 1) && mv.drop_rate > 0.f) {
+      // dV sees the dropped, rescaled probabilities and dP is dropped the same way; delta includes it already
+#pragma unroll
+      for (int e = 0; e < CH; ++e) {
+        const float p = ex2_approx((x[e] - lse[ROWS ? 0 : e]) * kLog2e);
+        const float dm = mod_dropout(mv, ROWS ? i0 : i0 + e, ROWS ? j0 + e : j0);
+        pr[e] = p * dm;
+        ds[e] = p * fmaf(dp[e], dm, -delta[ROWS ? 0 : e]);
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < CH; ++e) {
+        pr[e] = ex2_approx((x[e] - lse[ROWS ? 0 : e]) * kLog2e);
+        ds[e] = pr[e] * (dp[e] - delta[ROWS ? 0 : e]);
+      }
+    }
+    if (nonlinear) {
+#pragma unroll
+      for (int e = 0; e < CH; ++e) ds[e] *= g[e];
+    }
+  }
+  if (keep != (1u << CH) - 1) {  // selects, not products: masked scores may be anything
+#pragma unroll
+    for (int e = 0; e < CH; ++e) {
+      const bool k = (keep >> e) & 1u;
+      pr[e] = k ? pr[e] : 0.f;
+      ds[e] = k ? ds[e] : 0.f;
+    }
+  }
+}
+
+// Whether the ids of a warp's 32 own rows (or keys) and of `n` columns from c0 on are not all the same.
+__device__ __forceinline__ bool segments_mixed(const int32_t* col_seg, int c0, int n, int limit, int own, int lane) {
+  const int ref = __shfl_sync(0xffffffffu, own, 0);
+  const int a = col_seg[min(c0 + lane, limit - 1)];
+  const int b = col_seg[min(c0 + min(32 + lane, n - 1), limit - 1)];
+  return !__all_sync(0xffffffffu, own == ref && a == ref && b == ref);
+}
+
+// Rows [kv_len, tile end) of a K or V tile hold anything (a cache tail that was never written) and 0 x NaN inside
+// an accumulating product is not 0: one warp zeroes them in shared memory.
+template <int SUB>
+__device__ __forceinline__ void clear_rows(uint32_t tile, int first, int lane) {
+  for (int r = first + lane; r < BN; r += 32) {
+    const uint32_t row = tile + r * 128;
+#pragma unroll
+    for (int sub = 0; sub < SUB; ++sub)
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};\n" ::"r"(row + sub * BN * 128 + u * 16), "r"(0) : "memory");
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// dQ kernel
+// ---------------------------------------------------------------------------------------------
+template <int D, int DV, int FEAT>
+struct DqCfg {
+  static constexpr int SUBQ = D / 64, SUBV = DV / 64;  // 64-element (128-byte) column blocks of a row
+  static constexpr int TQ = SUBQ * 128 * 128, TV = SUBV * 128 * 128;  // bytes of a 128-row tile
+  static constexpr int KST = 2, VST = D > 128 ? 1 : 2;
+  static constexpr int OFF_Q = 0;
+  static constexpr int OFF_DO = TQ;
+  static constexpr int OFF_K = OFF_DO + TV;
+  static constexpr int OFF_V = OFF_K + KST * TQ;
+  static constexpr int OFF_BIAS = OFF_V + VST * TV;                    // Dense bias: 8 warps x 32 rows x 33 floats
+  static constexpr int OFF_BAR = OFF_BIAS + ((FEAT & 2) ? 8 * 32 * 33 * 4 : 0);
+  // barriers: QDO_FULL, K_FULL[2], K_EMPTY[2], V_FULL[2], V_EMPTY[2], SP_FULL[2], DS_FULL[2], DQ_FULL, K_CLEAN
+  static constexpr int N_BAR = 15;
+  static constexpr int SMEM_BYTES = OFF_BAR + N_BAR * 8 + 16 + 1024;
+  static constexpr int TMEM_COLS = 512;  // S 128 | dP 128 | dQ D
+  static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
+};
+
+template <int D, int DV, bool BF16, int FEAT>
+__global__ void __launch_bounds__(NTHREADS, 1)
+bwd_dq_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
+                          const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
+                          const __grid_constant__ BwdParams p, const __grid_constant__ ExactArgs a) {
+  using C = DqCfg<D, DV, FEAT>;
+  extern __shared__ unsigned char smem_unaligned[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~uintptr_t(1023));
+  const uint32_t sbase = smem_u32(smem);
+  const uint32_t bar0 = sbase + C::OFF_BAR;
+  auto BAR = [&](int i) { return bar0 + 8u * i; };
+  const int QDO_FULL = 0, K_FULL = 1, K_EMPTY = 3, V_FULL = 5, V_EMPTY = 7, SP_FULL = 9, DS_FULL = 11, DQ_FULL = 13,
+            K_CLEAN = 14;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::OFF_BAR + C::N_BAR * 8);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n_qt = (p.Lq + BM - 1) / BM;
+  int tile, pair;
+  work_item(blockIdx.x, n_qt, p.Hq * p.B, a.order_w, tile, pair);
+  const int qt = n_qt - 1 - tile;  // the last query tiles see the most keys under a causal band
+  const int h = pair % p.Hq, b = pair / p.Hq;
+  const int hk = h / (p.Hq / p.Hkv);
+  const int q0 = qt * BM;
+
+  int kv_len = p.Lkv;
+  if (p.kv_lengths) kv_len = max(0, min(kv_len, p.kv_lengths[b]));
+  // KV tiles any row of this query tile can see
+  int kv_end = max(0, min(kv_len, min(q0 + BM, p.Lq) + p.band_hi));
+  int kv_begin = max(0, q0 + p.band_lo);
+  if constexpr ((FEAT & 1) != 0) {
+    if (a.q_range) {
+      const int32_t* r = a.q_range + ((int64_t)b * a.q_range_bs + qt) * 2;
+      kv_begin = max(kv_begin, r[0]);
+      kv_end = min(kv_end, r[1]);
+    }
+    if (p.mod.prefix_len) {  // prefix keys are visible to every row
+      const int pre = min(kv_len, p.mod.prefix_len[b]);
+      if (pre > 0) {
+        kv_end = max(kv_end, pre);
+        kv_begin = 0;
+      }
+    }
+  }
+  const int j_lo = kv_begin / BN;
+  const int n = kv_begin < kv_end ? (kv_end + BN - 1) / BN - j_lo : 0;
+  const int clean_j = (n > 0 && (j_lo + n) * BN > kv_len) ? n - 1 : -1;  // a last tile with rows past the valid length
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < C::N_BAR; ++i)
+      mbar_init(BAR(i), i == K_CLEAN ? 32u : ((i == DS_FULL || i == DS_FULL + 1) ? 128u : 1u));
+    *abort_flag = 0;
+    fence_barrier_init();
+  }
+  if (warp == 0) {
+    tmem_alloc(smem_u32(tmem_slot), C::TMEM_COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  const uint32_t T_S = tmem, T_DP = tmem + BN, T_DQ = tmem + 2 * BN;
+
+  if (warp == 0) {
+    // ---------------------------------------------------------------- TMA producer
+    if (lane == 0 && n > 0) {
+      prefetch_tmap(&tm_q);
+      prefetch_tmap(&tm_do);
+      prefetch_tmap(&tm_k);
+      prefetch_tmap(&tm_v);
+      mbar_arrive_expect_tx(BAR(QDO_FULL), C::TQ + C::TV);
+#pragma unroll
+      for (int s = 0; s < C::SUBQ; ++s) tma_load_4d(sbase + C::OFF_Q + s * BM * 128, &tm_q, BAR(QDO_FULL), s * 64, h, q0, b);
+#pragma unroll
+      for (int s = 0; s < C::SUBV; ++s) tma_load_4d(sbase + C::OFF_DO + s * BM * 128, &tm_do, BAR(QDO_FULL), s * 64, h, q0, b);
+      for (int j = 0; j < n; ++j) {
+        const int ks = j % C::KST, vs = j % C::VST;
+        if (!mbar_wait(BAR(K_EMPTY + ks), ((j / C::KST) & 1) ^ 1, abort_flag)) break;
+        mbar_arrive_expect_tx(BAR(K_FULL + ks), C::TQ);
+#pragma unroll
+        for (int s = 0; s < C::SUBQ; ++s)
+          tma_load_4d(sbase + C::OFF_K + ks * C::TQ + s * BN * 128, &tm_k, BAR(K_FULL + ks), s * 64, hk, (j_lo + j) * BN, b);
+        if (!mbar_wait(BAR(V_EMPTY + vs), ((j / C::VST) & 1) ^ 1, abort_flag)) break;
+        mbar_arrive_expect_tx(BAR(V_FULL + vs), C::TV);
+#pragma unroll
+        for (int s = 0; s < C::SUBV; ++s)
+          tma_load_4d(sbase + C::OFF_V + vs * C::TV + s * BN * 128, &tm_v, BAR(V_FULL + vs), s * 64, hk, (j_lo + j) * BN, b);
+      }
+    }
+    __syncwarp();
+    if (clean_j >= 0) {
+      const int ks = clean_j % C::KST;
+      if (mbar_wait(BAR(K_FULL + ks), (clean_j / C::KST) & 1, abort_flag)) {
+        clear_rows<C::SUBQ>(sbase + C::OFF_K + ks * C::TQ, kv_len - (j_lo + clean_j) * BN, lane);
+        fence_proxy_async();
+      }
+      mbar_arrive(BAR(K_CLEAN));
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer
+    if (lane == 0 && n > 0) {
+      constexpr uint32_t idesc_s = make_idesc(BM, BN / 2, BF16, false, false);
+      constexpr uint32_t idesc_q = make_idesc(BM, D, BF16, false, true);
+      const uint32_t qa = sbase + C::OFF_Q, doa = sbase + C::OFF_DO;
+      // S and dP of one half (64 keys) of KV tile j
+      auto issue_sdp = [&](int half, int j) {
+        const uint32_t ka = sbase + C::OFF_K + (j % C::KST) * C::TQ + half * 64 * 128;
+        const uint32_t va = sbase + C::OFF_V + (j % C::VST) * C::TV + half * 64 * 128;
+#pragma unroll
+        for (int s = 0; s < C::SUBQ; ++s)
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk)
+            mma_ss(T_S + half * 64, make_smem_desc(qa + s * BM * 128 + kk * 32, 16, 1024),
+                   make_smem_desc(ka + s * BN * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0);
+#pragma unroll
+        for (int s = 0; s < C::SUBV; ++s)
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk)
+            mma_ss(T_DP + half * 64, make_smem_desc(doa + s * BM * 128 + kk * 32, 16, 1024),
+                   make_smem_desc(va + s * BN * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0);
+        mma_commit(BAR(SP_FULL + half));
+      };
+      // dQ += (hi + lo of dS).K over one half, the K tile read MN-major
+      auto issue_acc = [&](int half, int j) {
+        const uint32_t ka = sbase + C::OFF_K + (j % C::KST) * C::TQ;
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+          const uint64_t kd = make_smem_desc(ka + (half * 4 + kk) * 2048, BN * 128, 1024);
+          mma_ts(T_DQ, T_S + half * 64 + kk * CH, kd, idesc_q, (j | half | kk) != 0);
+          mma_ts(T_DQ, T_S + half * 64 + kk * CH + CH / 2, kd, idesc_q, true);
+        }
+      };
+      bool ok = mbar_wait(BAR(QDO_FULL), 0, abort_flag);
+      if (ok) ok = mbar_wait(BAR(K_FULL), 0, abort_flag);
+      if (ok && clean_j == 0) ok = mbar_wait(BAR(K_CLEAN), 0, abort_flag);
+      if (ok) ok = mbar_wait(BAR(V_FULL), 0, abort_flag);
+      if (ok) {
+        tc_fence_after();
+        issue_sdp(0, 0);
+        issue_sdp(1, 0);
+        mma_commit(BAR(V_EMPTY));
+      }
+      for (int j = 0; ok && j < n; ++j) {
+        const bool next = j + 1 < n;
+        ok = mbar_wait(BAR(DS_FULL + 0), j & 1, abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        issue_acc(0, j);
+        if (next) {
+          ok = mbar_wait(BAR(K_FULL + (j + 1) % C::KST), ((j + 1) / C::KST) & 1, abort_flag);
+          if (ok && j + 1 == clean_j) ok = mbar_wait(BAR(K_CLEAN), 0, abort_flag);
+          if (ok) ok = mbar_wait(BAR(V_FULL + (j + 1) % C::VST), ((j + 1) / C::VST) & 1, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          issue_sdp(0, j + 1);  // over dS of half 0, which the MMAs just issued consume first
+        }
+        ok = mbar_wait(BAR(DS_FULL + 1), j & 1, abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        issue_acc(1, j);
+        mma_commit(BAR(K_EMPTY + j % C::KST));
+        if (next) {
+          issue_sdp(1, j + 1);
+          mma_commit(BAR(V_EMPTY + (j + 1) % C::VST));
+        }
+      }
+      if (ok) mma_commit(BAR(DQ_FULL));
+    }
+  } else {
+    // --------------------------------------------------------------- compute warps
+    const int grp = (warp - 2) >> 2;  // which half of the score columns
+    const int quarter = warp & 3;
+    const int r_in = quarter * 32 + lane;
+    const int row = q0 + r_in;
+    const bool row_ok = row < p.Lq;
+    const uint32_t lane_sel = static_cast<uint32_t>(quarter * 32) << 16;
+    const float c = FEAT == 0 ? p.sm_scale * kLog2e : p.sm_scale;
+    const float pack = ds_pack_scale<DV, BF16>(a, p.mod);
+    // padded per-row vectors: +inf / 0 for rows past Lq and +inf for rows without keys, so P = 0 there
+    const int64_t at = ((int64_t)b * p.Hq + h) * p.Lq_pad + row;
+    const float lse = p.lse2[at], delta = p.delta[at];
+    const uint32_t s_addr = T_S + lane_sel + grp * 64, dp_addr = T_DP + lane_sel + grp * 64;
+    const Place pl = {kv_len, p.Lq, p.Lkv, p.band_lo, p.band_hi};
+    ScoreModView mv = {};
+    int own_seg = 0;
+    if constexpr ((FEAT & 1) != 0) {
+      mv = view_of(p.mod, b, h, p.Lq);
+      if (mv.seg_q) own_seg = mv.seg_q[min(row, p.Lq - 1)];
+    }
+    // Dense bias: the warp's 32 rows of the bias, 32 keys at a time, through its window in shared memory
+    [[maybe_unused]] float breg[(FEAT & 2) ? 32 : 1];
+    [[maybe_unused]] float* bwin = reinterpret_cast<float*>(smem + C::OFF_BIAS) + (warp - 2) * 32 * 33;
+    [[maybe_unused]] const float* bsrc = (FEAT & 2) ? p.bias + (int64_t)b * p.bias_bs + (int64_t)h * p.bias_hs : nullptr;
+    auto fetch_bias = [&](int key0) {
+      if constexpr ((FEAT & 2) != 0) {
+        const int key = min(key0 + lane, p.Lkv - 1);
+        int r0 = q0 + quarter * 32;
+        asm volatile("" : "+r"(r0));  // as in load_bias_column
+        const float* ptr = bsrc + (int64_t)min(r0, p.Lq - 1) * p.Lkv + key;
+#pragma unroll
+        for (int r = 0; r < 32; ++r) {
+          asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(breg[r]) : "l"(ptr));
+          if (r0 + r + 1 < p.Lq) ptr += p.Lkv;
+        }
+      }
+    };
+    if (n > 0) fetch_bias(j_lo * BN + grp * 64);
+    bool ok = true;
+    for (int j = 0; j < n; ++j) {
+      const int k0 = (j_lo + j) * BN + grp * 64;  // first key of this group's columns
+      bool mixed = false;
+      if constexpr ((FEAT & 1) != 0) {
+        if (mv.seg_q) mixed = segments_mixed(mv.seg_k, k0, 64, p.Lkv, own_seg, lane);
+      }
+      ok = mbar_wait(BAR(SP_FULL + grp), j & 1, abort_flag);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+      float s[2][CH], dp[2][CH];
+      tmem_ld16f(s_addr, s[0]);
+      tmem_ld16f(dp_addr, dp[0]);
+#pragma unroll
+      for (int cc = 0; cc < 64 / CH; ++cc) {
+        if constexpr ((FEAT & 2) != 0) {
+          if (cc % 2 == 0) {
+            __syncwarp();
+#pragma unroll
+            for (int r = 0; r < 32; ++r) bwin[r * 33 + lane] = breg[r];
+            __syncwarp();
+            fetch_bias(cc == 0 ? k0 + 32 : k0 + BN);
+          }
+        }
+        tmem_wait_ld();
+        if (cc + 1 < 64 / CH) {
+          tmem_ld16f(s_addr + (cc + 1) * CH, s[(cc + 1) & 1]);
+          tmem_ld16f(dp_addr + (cc + 1) * CH, dp[(cc + 1) & 1]);
+        }
+        float bias[CH], pr[CH], ds[CH];
+        if constexpr ((FEAT & 2) != 0) {
+#pragma unroll
+          for (int e = 0; e < CH; ++e) bias[e] = bwin[lane * 33 + (cc & 1) * CH + e];
+        }
+        const int j0 = k0 + cc * CH;
+        const uint32_t keep = keep_bits<FEAT, true>(pl, mv, mixed, own_seg, row, j0);
+        chunk_p_ds<FEAT, true>(s[cc & 1], dp[cc & 1], c, pl, mv, keep, row, j0, &lse, &delta, bias, pr, ds);
+        uint32_t pk[CH];
+        split_pack<BF16>(ds, pack, pk);
+        tmem_st16(s_addr + cc * CH, pk);  // over the chunk's own scores, which were read already
+      }
+      tmem_wait_st();
+      tc_fence_before();
+      mbar_arrive(BAR(DS_FULL + grp));
+    }
+    if (ok && q0 < p.Lq) {
+      if (n > 0) {
+        ok = mbar_wait(BAR(DQ_FULL), 0, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
+      }
+      if (ok) {
+        tc_fence_after();
+        // each group stores one half of the row's D columns
+        unsigned char* dst = static_cast<unsigned char*>(p.dq) + ((((int64_t)b * p.Lq + row) * p.Hq + h) * D) * 2;
+        store_row<D / 2, BF16>(T_DQ + lane_sel + grp * (D / 2), dst + grp * D, p.sm_scale / pack, n > 0, row_ok);
+      }
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    __syncwarp();
+    tmem_dealloc(tmem, C::TMEM_COLS);
+    if (lane == 0 && *abort_flag && p.status) atomicExch(p.status, (int)PJX_ERR_DEVICE_TIMEOUT);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// dK/dV kernel
+// ---------------------------------------------------------------------------------------------
+template <int D, int DV>
+struct DkvCfg {
+  static constexpr int SUBQ = D / 64, SUBV = DV / 64;
+  static constexpr int QT = D > 128 ? 96 : 128;      // query rows per step: S^T | dP^T | dV | dK fill tensor memory
+  static constexpr int HALF = QT / 2;
+  static constexpr int TK = SUBQ * BN * 128, TV = SUBV * BN * 128;
+  static constexpr int TQ = SUBQ * QT * 128, TDO = SUBV * QT * 128;
+  static constexpr int OFF_K = 0;
+  static constexpr int OFF_V = TK;
+  static constexpr int OFF_Q = OFF_V + TV;           // 2 stages
+  static constexpr int OFF_DO = OFF_Q + 2 * TQ;      // 2 stages
+  static constexpr int OFF_ROW = OFF_DO + 2 * TDO;   // 2 stages x { float lse[QT]; float delta[QT]; }
+  static constexpr int OFF_BAR = OFF_ROW + 2 * 2 * QT * 4;
+  // barriers: KV_FULL, QDO_FULL[2], QDO_EMPTY[2], SP_FULL[2], PDS_FULL[2], ACC_FULL
+  static constexpr int N_BAR = 10;
+  static constexpr int SMEM_BYTES = OFF_BAR + N_BAR * 8 + 16 + 1024;
+  static constexpr int TMEM_COLS = 512;              // S^T QT | dP^T QT | dV DV | dK D
+  static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
+  static_assert(2 * QT + DV + D <= 512, "tensor memory has 512 columns");
+  static_assert(HALF % CH == 0 && (HALF * 128) % 1024 == 0, "halves are whole chunks and whole swizzle groups");
+};
+
+template <int D, int DV, bool BF16, int FEAT>
+__global__ void __launch_bounds__(NTHREADS, 1)
+bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
+                            const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
+                            const __grid_constant__ BwdParams p, const __grid_constant__ ExactArgs a) {
+  using C = DkvCfg<D, DV>;
+  constexpr int QT = C::QT, HALF = C::HALF, NCH = HALF / CH;
+  extern __shared__ unsigned char smem_unaligned[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~uintptr_t(1023));
+  const uint32_t sbase = smem_u32(smem);
+  const uint32_t bar0 = sbase + C::OFF_BAR;
+  auto BAR = [&](int i) { return bar0 + 8u * i; };
+  const int KV_FULL = 0, QDO_FULL = 1, QDO_EMPTY = 3, SP_FULL = 5, PDS_FULL = 7, ACC_FULL = 9;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::OFF_BAR + C::N_BAR * 8);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  float* row_s = reinterpret_cast<float*>(smem + C::OFF_ROW);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int kt, pair;  // the first key tiles are seen by the most queries under a causal band
+  work_item(blockIdx.x, (p.Lkv + BN - 1) / BN, p.Hkv * p.B, a.order_w, kt, pair);
+  const int hk = pair % p.Hkv, b = pair / p.Hkv;
+  const int G = p.Hq / p.Hkv;
+  const int k0 = kt * BN;
+
+  int kv_len = p.Lkv;
+  if (p.kv_lengths) kv_len = max(0, min(kv_len, p.kv_lengths[b]));
+  // query rows that see a key of this tile: [first key - band_hi, last valid key - band_lo]
+  int q_begin = max(0, k0 - p.band_hi);
+  int q_end = min(p.Lq, min(k0 + BN, kv_len) - p.band_lo);
+  if constexpr ((FEAT & 1) != 0) {
+    if (a.k_range) {
+      const int32_t* r = a.k_range + ((int64_t)b * a.k_range_bs + kt) * 2;
+      q_begin = max(q_begin, r[0]);
+      q_end = min(q_end, r[1]);
+    }
+    if (p.mod.prefix_len && k0 < p.mod.prefix_len[b]) {  // a prefix key is seen by every row
+      q_begin = 0;
+      q_end = p.Lq;
+    }
+  }
+  const int t_lo = q_begin / QT;
+  const int n_t = (k0 < kv_len && q_begin < q_end) ? (q_end + QT - 1) / QT - t_lo : 0;
+  const int n = n_t * G;  // steps: query heads of the group outer, query tiles inner
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < C::N_BAR; ++i)
+      mbar_init(BAR(i), (i == PDS_FULL || i == PDS_FULL + 1) ? 128u : 1u);
+    *abort_flag = 0;
+    fence_barrier_init();
+  }
+  if (warp == 0) {
+    tmem_alloc(smem_u32(tmem_slot), C::TMEM_COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  const uint32_t T_S = tmem, T_DP = tmem + QT, T_DV = tmem + 2 * QT, T_DK = tmem + 2 * QT + DV;
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------- TMA producer
+    if (lane == 0 && n > 0) {
+      prefetch_tmap(&tm_q);
+      prefetch_tmap(&tm_do);
+      prefetch_tmap(&tm_k);
+      prefetch_tmap(&tm_v);
+      mbar_arrive_expect_tx(BAR(KV_FULL), C::TK + C::TV);
+#pragma unroll
+      for (int s = 0; s < C::SUBQ; ++s) tma_load_4d(sbase + C::OFF_K + s * BN * 128, &tm_k, BAR(KV_FULL), s * 64, hk, k0, b);
+#pragma unroll
+      for (int s = 0; s < C::SUBV; ++s) tma_load_4d(sbase + C::OFF_V + s * BN * 128, &tm_v, BAR(KV_FULL), s * 64, hk, k0, b);
+      for (int it = 0; it < n; ++it) {
+        const int st = it & 1;
+        const int h = hk * G + it / n_t;
+        const int q0 = (t_lo + it % n_t) * QT;
+        // the rows' log-sum-exp and delta out of the padded workspace arrays (a 96-row tile may reach past their
+        // padding: a multiple of 4 floats either way)
+        const int rows = QT == 128 ? 128 : min(QT, p.Lq_pad - q0);
+        if (!mbar_wait(BAR(QDO_EMPTY + st), ((it >> 1) & 1) ^ 1, abort_flag)) break;
+        mbar_arrive_expect_tx(BAR(QDO_FULL + st), C::TQ + C::TDO + 2 * rows * 4);
+#pragma unroll
+        for (int s = 0; s < C::SUBQ; ++s)
+          tma_load_4d(sbase + C::OFF_Q + st * C::TQ + s * QT * 128, &tm_q, BAR(QDO_FULL + st), s * 64, h, q0, b);
+#pragma unroll
+        for (int s = 0; s < C::SUBV; ++s)
+          tma_load_4d(sbase + C::OFF_DO + st * C::TDO + s * QT * 128, &tm_do, BAR(QDO_FULL + st), s * 64, h, q0, b);
+        const int64_t at = ((int64_t)b * p.Hq + h) * p.Lq_pad + q0;
+        bulk_load(sbase + C::OFF_ROW + st * 2 * QT * 4, p.lse2 + at, rows * 4, BAR(QDO_FULL + st));
+        bulk_load(sbase + C::OFF_ROW + st * 2 * QT * 4 + QT * 4, p.delta + at, rows * 4, BAR(QDO_FULL + st));
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer
+    if (lane == 0 && n > 0) {
+      constexpr uint32_t idesc_s = make_idesc(BN, HALF, BF16, false, false);
+      constexpr uint32_t idesc_v = make_idesc(BN, DV, BF16, false, true);
+      constexpr uint32_t idesc_k = make_idesc(BN, D, BF16, false, true);
+      const uint32_t ka = sbase + C::OFF_K, va = sbase + C::OFF_V;
+      // S^T and dP^T of one half of step `it`: keys on the lanes, query rows on the columns
+      auto issue_sdp = [&](int half, int it) {
+        const uint32_t qa = sbase + C::OFF_Q + (it & 1) * C::TQ + half * HALF * 128;
+        const uint32_t doa = sbase + C::OFF_DO + (it & 1) * C::TDO + half * HALF * 128;
+#pragma unroll
+        for (int s = 0; s < C::SUBQ; ++s)
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk)
+            mma_ss(T_S + half * HALF, make_smem_desc(ka + s * BN * 128 + kk * 32, 16, 1024),
+                   make_smem_desc(qa + s * QT * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0);
+#pragma unroll
+        for (int s = 0; s < C::SUBV; ++s)
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk)
+            mma_ss(T_DP + half * HALF, make_smem_desc(va + s * BN * 128 + kk * 32, 16, 1024),
+                   make_smem_desc(doa + s * QT * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0);
+        mma_commit(BAR(SP_FULL + half));
+      };
+      // dV += (hi + lo of P^T).dO and dK += (hi + lo of dS^T).Q over one half, dO / Q tiles read MN-major
+      auto issue_acc = [&](int half, int it) {
+        const uint32_t qa = sbase + C::OFF_Q + (it & 1) * C::TQ, doa = sbase + C::OFF_DO + (it & 1) * C::TDO;
+#pragma unroll
+        for (int kk = 0; kk < NCH; ++kk) {
+          const uint64_t dd = make_smem_desc(doa + (half * NCH + kk) * 2048, QT * 128, 1024);
+          mma_ts(T_DV, T_S + half * HALF + kk * CH, dd, idesc_v, (it | half | kk) != 0);
+          mma_ts(T_DV, T_S + half * HALF + kk * CH + CH / 2, dd, idesc_v, true);
+        }
+#pragma unroll
+        for (int kk = 0; kk < NCH; ++kk) {
+          const uint64_t qd = make_smem_desc(qa + (half * NCH + kk) * 2048, QT * 128, 1024);
+          mma_ts(T_DK, T_DP + half * HALF + kk * CH, qd, idesc_k, (it | half | kk) != 0);
+          mma_ts(T_DK, T_DP + half * HALF + kk * CH + CH / 2, qd, idesc_k, true);
+        }
+      };
+      bool ok = mbar_wait(BAR(KV_FULL), 0, abort_flag);
+      if (ok) ok = mbar_wait(BAR(QDO_FULL), 0, abort_flag);
+      if (ok) {
+        tc_fence_after();
+        issue_sdp(0, 0);
+        issue_sdp(1, 0);
+      }
+      for (int it = 0; ok && it < n; ++it) {
+        const int st = it & 1;
+        const bool next = it + 1 < n;
+        ok = mbar_wait(BAR(PDS_FULL + 0), it & 1, abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        issue_acc(0, it);
+        if (next) {
+          ok = mbar_wait(BAR(QDO_FULL + (st ^ 1)), ((it + 1) >> 1) & 1, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          issue_sdp(0, it + 1);  // over P^T / dS^T of half 0, which the MMAs just issued consume first
+        }
+        ok = mbar_wait(BAR(PDS_FULL + 1), it & 1, abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        issue_acc(1, it);
+        mma_commit(BAR(QDO_EMPTY + st));
+        if (next) issue_sdp(1, it + 1);
+      }
+      if (ok) mma_commit(BAR(ACC_FULL));
+    }
+  } else {
+    // --------------------------------------------------------------- compute warps
+    const int grp = (warp - 2) >> 2;  // which half of the query columns
+    const int quarter = warp & 3;
+    const int r_in = quarter * 32 + lane;
+    const int key = k0 + r_in;
+    const uint32_t lane_sel = static_cast<uint32_t>(quarter * 32) << 16;
+    const float c = FEAT == 0 ? p.sm_scale * kLog2e : p.sm_scale;
+    const float pack = ds_pack_scale<DV, BF16>(a, p.mod);
+    const uint32_t s_addr = T_S + lane_sel + grp * HALF, dp_addr = T_DP + lane_sel + grp * HALF;
+    const Place pl = {kv_len, p.Lq, p.Lkv, p.band_lo, p.band_hi};
+    ScoreModView mv = {};
+    int own_seg = 0;
+    [[maybe_unused]] const float* bsrc = nullptr;  // Dense bias: this thread's column of the bias of head h
+    [[maybe_unused]] float bnext[(FEAT & 2) ? CH : 1];
+    auto fetch_bias = [&](int i0) {  // keys on the lanes: 128 contiguous bytes per row
+      if constexpr ((FEAT & 2) != 0) load_bias_column(bsrc, i0, p.Lq, p.Lkv, bnext);
+    };
+    bool ok = true;
+    for (int it = 0; it < n; ++it) {
+      const int st = it & 1;
+      const int q0 = (t_lo + it % n_t) * QT + grp * HALF;  // first query row of this group's columns
+      bool mixed = false;
+      if (it % n_t == 0) {  // the next query head of the group
+        const int h = hk * G + it / n_t;
+        if constexpr ((FEAT & 1) != 0) {
+          mv = view_of(p.mod, b, h, p.Lq);
+          if (mv.seg_q) own_seg = mv.seg_k[min(key, p.Lkv - 1)];
+        }
+        if constexpr ((FEAT & 2) != 0) bsrc = p.bias + (int64_t)b * p.bias_bs + (int64_t)h * p.bias_hs + min(key, p.Lkv - 1);
+      }
+      if constexpr ((FEAT & 1) != 0) {
+        if (mv.seg_q) mixed = segments_mixed(mv.seg_q, q0, HALF, p.Lq, own_seg, lane);
+      }
+      fetch_bias(q0);
+      ok = mbar_wait(BAR(SP_FULL + grp), it & 1, abort_flag);
+      if (ok) ok = mbar_wait(BAR(QDO_FULL + st), (it >> 1) & 1, abort_flag);  // the row vectors landed with Q and dO
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+      const float* lse_s = row_s + st * 2 * QT + grp * HALF;
+      const float* delta_s = lse_s + QT;
+      float s[2][CH], dp[2][CH];
+      tmem_ld16f(s_addr, s[0]);
+      tmem_ld16f(dp_addr, dp[0]);
+#pragma unroll
+      for (int cc = 0; cc < NCH; ++cc) {
+        float lse[CH], delta[CH], bias[CH], pr[CH], ds[CH];
+#pragma unroll
+        for (int e = 0; e < CH; e += 4) {
+          *reinterpret_cast<float4*>(lse + e) = *reinterpret_cast<const float4*>(lse_s + cc * CH + e);
+          *reinterpret_cast<float4*>(delta + e) = *reinterpret_cast<const float4*>(delta_s + cc * CH + e);
+        }
+        if constexpr ((FEAT & 2) != 0) {
+#pragma unroll
+          for (int e = 0; e < CH; ++e) bias[e] = bnext[e];
+          if (cc + 1 < NCH) fetch_bias(q0 + (cc + 1) * CH);
+        }
+        tmem_wait_ld();
+        if (cc + 1 < NCH) {
+          tmem_ld16f(s_addr + (cc + 1) * CH, s[(cc + 1) & 1]);
+          tmem_ld16f(dp_addr + (cc + 1) * CH, dp[(cc + 1) & 1]);
+        }
+        const int i0 = q0 + cc * CH;
+        const uint32_t keep = keep_bits<FEAT, false>(pl, mv, mixed, own_seg, i0, key);
+        chunk_p_ds<FEAT, false>(s[cc & 1], dp[cc & 1], c, pl, mv, keep, i0, key, lse, delta, bias, pr, ds);
+        uint32_t pk[CH];
+        split_pack<BF16>(pr, a.p_scale, pk);
+        tmem_st16(s_addr + cc * CH, pk);  // over the chunk's own scores, which were read already
+        split_pack<BF16>(ds, pack, pk);
+        tmem_st16(dp_addr + cc * CH, pk);
+      }
+      tmem_wait_st();
+      tc_fence_before();
+      mbar_arrive(BAR(PDS_FULL + grp));
+    }
+    if (ok && k0 < p.Lkv) {
+      if (n > 0) {
+        ok = mbar_wait(BAR(ACC_FULL), 0, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
+      }
+      if (ok) {
+        tc_fence_after();
+        const bool row_ok = key < p.Lkv;
+        const int64_t at = ((int64_t)b * p.Lkv + key) * p.Hkv + hk;
+        // group 0 stores the dV row, group 1 the dK row
+        if (grp == 0) store_row<DV, BF16>(T_DV + lane_sel, static_cast<unsigned char*>(p.dv) + at * DV * 2, 1.f / a.p_scale, n > 0, row_ok);
+        else store_row<D, BF16>(T_DK + lane_sel, static_cast<unsigned char*>(p.dk) + at * D * 2, p.sm_scale / pack, n > 0, row_ok);
+      }
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    __syncwarp();
+    tmem_dealloc(tmem, C::TMEM_COLS);
+    if (lane == 0 && *abort_flag && p.status) atomicExch(p.status, (int)PJX_ERR_DEVICE_TIMEOUT);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// Gradient of the dense bias: dbias = sum of dS over the (batch, head) pairs that share an entry
+// ---------------------------------------------------------------------------------------------
+// One CTA per 128 x 128 tile of the bias.  S^T and dP^T of successive pairs alternate between the two halves of
+// tensor memory, so that the products of the next pair run while the threads (one key, 64 query rows each) add dS
+// of this one to their 64 registers; the tile is written once, coalesced over the keys.  Summing in registers
+// costs two products per pair and no memory traffic; adding dS into memory from the dQ kernel instead would move
+// 4 bytes per score through the L2's atomic units (537 MB at B8 S1024 H16) in an order that changes per run.
+template <int D, int DV>
+struct DbCfg {
+  static constexpr int SUBQ = D / 64, SUBV = DV / 64;
+  static constexpr int TQ = SUBQ * 128 * 128, TV = SUBV * 128 * 128;
+  static constexpr int STAGE = 2 * TQ + 2 * TV;                  // Q | K | dO | V
+  static constexpr int NST = STAGE <= 72 * 1024 ? 3 : 1;
+  static constexpr int OFF_ROW = NST * STAGE;                    // 2 x { float lse[128]; float delta[128]; }
+  static constexpr int OFF_BAR = OFF_ROW + 2 * 2 * BM * 4;
+  // barriers: FULL[NST], EMPTY[NST], ROW_FULL[2], SP_FULL[2], T_FREE[2]
+  static constexpr int N_BAR = 2 * NST + 6;
+  static constexpr int SMEM_BYTES = OFF_BAR + N_BAR * 8 + 16 + 1024;
+  static constexpr int TMEM_COLS = 512;                          // 2 x { S^T 128 | dP^T 128 }
+  static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
+};
+
+template <int D, int DV, bool BF16, int FEAT>
+__global__ void __launch_bounds__(NTHREADS, 1)
+bwd_dbias_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
+                       const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
+                       const __grid_constant__ BwdParams p) {
+  using C = DbCfg<D, DV>;
+  extern __shared__ unsigned char smem_unaligned[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~uintptr_t(1023));
+  const uint32_t sbase = smem_u32(smem);
+  const uint32_t bar0 = sbase + C::OFF_BAR;
+  auto BAR = [&](int i) { return bar0 + 8u * i; };
+  const int FULL = 0, EMPTY = C::NST, ROW_FULL = 2 * C::NST, SP_FULL = ROW_FULL + 2, T_FREE = SP_FULL + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::OFF_BAR + C::N_BAR * 8);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  float* row_s = reinterpret_cast<float*>(smem + C::OFF_ROW);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n_kt = (p.Lkv + BN - 1) / BN, n_qt = (p.Lq + BM - 1) / BM;
+  const int k0 = (int)(blockIdx.x % n_kt) * BN, q0 = (int)(blockIdx.x / n_kt % n_qt) * BM;
+  const int plane = blockIdx.x / (n_kt * n_qt);  // (batch, head) plane of the bias
+  const int nhb = p.bias_hs ? p.Hq : 1;
+  // the pairs of this plane: b0 .. b0 + nb - 1 times h0 .. h0 + nh - 1
+  const int h0 = p.bias_hs ? plane % nhb : 0, nh = p.bias_hs ? 1 : p.Hq;
+  const int b0 = p.bias_bs ? plane / nhb : 0, nb = p.bias_bs ? 1 : p.B;
+  const bool in_band = p.mod.prefix_len || (k0 <= min(q0 + BM, p.Lq) - 1 + p.band_hi && min(k0 + BN, p.Lkv) - 1 >= q0 + p.band_lo);
+  const int n_pairs = in_band ? nb * nh : 0;
+  const int G = p.Hq / p.Hkv;
+  auto len_of = [&](int b) { return p.kv_lengths ? max(0, min(p.Lkv, p.kv_lengths[b])) : p.Lkv; };
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < C::N_BAR; ++i) mbar_init(BAR(i), i >= T_FREE ? 256u : 1u);
+    *abort_flag = 0;
+    fence_barrier_init();
+  }
+  if (warp == 0) {
+    tmem_alloc(smem_u32(tmem_slot), C::TMEM_COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  // every role walks the pairs the same way; `it` counts those with a valid key in the tile
+  if (warp == 0) {
+    if (lane == 0) {
+      int it = 0;
+      for (int pi = 0; pi < n_pairs; ++pi) {
+        const int b = b0 + pi / nh, h = h0 + pi % nh, hk = h / G;
+        if (k0 >= len_of(b)) continue;
+        const int st = it % C::NST, buf = it & 1;
+        const uint32_t sa = sbase + st * C::STAGE;
+        if (!mbar_wait(BAR(EMPTY + st), ((it / C::NST) & 1) ^ 1, abort_flag)) break;
+        mbar_arrive_expect_tx(BAR(FULL + st), C::STAGE);
+#pragma unroll
+        for (int s = 0; s < C::SUBQ; ++s) {
+          tma_load_4d(sa + s * BM * 128, &tm_q, BAR(FULL + st), s * 64, h, q0, b);
+          tma_load_4d(sa + C::TQ + s * BN * 128, &tm_k, BAR(FULL + st), s * 64, hk, k0, b);
+        }
+#pragma unroll
+        for (int s = 0; s < C::SUBV; ++s) {
+          tma_load_4d(sa + 2 * C::TQ + s * BM * 128, &tm_do, BAR(FULL + st), s * 64, h, q0, b);
+          tma_load_4d(sa + 2 * C::TQ + C::TV + s * BN * 128, &tm_v, BAR(FULL + st), s * 64, hk, k0, b);
+        }
+        if (!mbar_wait(BAR(T_FREE + buf), ((it >> 1) & 1) ^ 1, abort_flag)) break;  // row vectors of pair it - 2 were read
+        mbar_arrive_expect_tx(BAR(ROW_FULL + buf), 2 * BM * 4);
+        const int64_t at = ((int64_t)b * p.Hq + h) * p.Lq_pad + q0;
+        bulk_load(sbase + C::OFF_ROW + buf * 2 * BM * 4, p.lse2 + at, BM * 4, BAR(ROW_FULL + buf));
+        bulk_load(sbase + C::OFF_ROW + buf * 2 * BM * 4 + BM * 4, p.delta + at, BM * 4, BAR(ROW_FULL + buf));
+        ++it;
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = make_idesc(BN, BM, BF16, false, false);
+      int it = 0;
+      for (int pi = 0; pi < n_pairs; ++pi) {
+        if (k0 >= len_of(b0 + pi / nh)) continue;
+        const int st = it % C::NST, buf = it & 1;
+        const uint32_t sa = sbase + st * C::STAGE;
+        if (!mbar_wait(BAR(FULL + st), (it / C::NST) & 1, abort_flag)) break;
+        if (!mbar_wait(BAR(T_FREE + buf), ((it >> 1) & 1) ^ 1, abort_flag)) break;
+        tc_fence_after();
+#pragma unroll
+        for (int s = 0; s < C::SUBQ; ++s)
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk)
+            mma_ss(tmem + buf * 256, make_smem_desc(sa + C::TQ + s * BN * 128 + kk * 32, 16, 1024),
+                   make_smem_desc(sa + s * BM * 128 + kk * 32, 16, 1024), idesc, (s | kk) != 0);
+#pragma unroll
+        for (int s = 0; s < C::SUBV; ++s)
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk)
+            mma_ss(tmem + buf * 256 + 128, make_smem_desc(sa + 2 * C::TQ + C::TV + s * BN * 128 + kk * 32, 16, 1024),
+                   make_smem_desc(sa + 2 * C::TQ + s * BM * 128 + kk * 32, 16, 1024), idesc, (s | kk) != 0);
+        mma_commit(BAR(EMPTY + st));
+        mma_commit(BAR(SP_FULL + buf));
+        ++it;
+      }
+    }
+  } else {
+    const int grp = (warp - 2) >> 2, quarter = warp & 3;
+    const int key = k0 + quarter * 32 + lane;
+    const int i_first = q0 + grp * 64;
+    const uint32_t lane_sel = static_cast<uint32_t>(quarter * 32) << 16;
+    const float* bsrc = p.bias + (int64_t)b0 * p.bias_bs + (int64_t)h0 * p.bias_hs + min(key, p.Lkv - 1);
+    float acc[64];
+#pragma unroll
+    for (int e = 0; e < 64; ++e) acc[e] = 0.f;
+    int it = 0;
+    bool ok = true;
+    for (int pi = 0; pi < n_pairs; ++pi) {
+      const int b = b0 + pi / nh, h = h0 + pi % nh;
+      const int kv_len = len_of(b);
+      if (k0 >= kv_len) continue;
+      const int buf = it & 1;
+      const Place pl = {kv_len, p.Lq, p.Lkv, p.band_lo, p.band_hi};
+      ScoreModView mv = {};
+      int own_seg = 0;
+      bool mixed = false;
+      if constexpr ((FEAT & 1) != 0) {
+        mv = view_of(p.mod, b, h, p.Lq);
+        if (mv.seg_q) {
+          own_seg = mv.seg_k[min(key, p.Lkv - 1)];
+          mixed = segments_mixed(mv.seg_q, i_first, 64, p.Lq, own_seg, lane);
+        }
+      }
+      const uint32_t s_addr = tmem + buf * 256 + lane_sel + grp * 64, dp_addr = s_addr + 128;
+      float bnext[CH];
+      load_bias_column(bsrc, i_first, p.Lq, p.Lkv, bnext);
+      ok = mbar_wait(BAR(SP_FULL + buf), (it >> 1) & 1, abort_flag);
+      if (ok) ok = mbar_wait(BAR(ROW_FULL + buf), (it >> 1) & 1, abort_flag);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+      const float* lse_s = row_s + buf * 2 * BM + grp * 64;
+      const float* delta_s = lse_s + BM;
+#pragma unroll
+      for (int cc = 0; cc < 64 / CH; ++cc) {
+        float s[CH], dp[CH], lse[CH], delta[CH], bias[CH], pr[CH], ds[CH];
+        tmem_ld16f(s_addr + cc * CH, s);
+        tmem_ld16f(dp_addr + cc * CH, dp);
+#pragma unroll
+        for (int e = 0; e < CH; e += 4) {
+          *reinterpret_cast<float4*>(lse + e) = *reinterpret_cast<const float4*>(lse_s + cc * CH + e);
+          *reinterpret_cast<float4*>(delta + e) = *reinterpret_cast<const float4*>(delta_s + cc * CH + e);
+        }
+#pragma unroll
+        for (int e = 0; e < CH; ++e) bias[e] = bnext[e];
+        if (cc + 1 < 64 / CH) load_bias_column(bsrc, i_first + (cc + 1) * CH, p.Lq, p.Lkv, bnext);
+        tmem_wait_ld();
+        int i0 = i_first + cc * CH;
+        asm volatile("" : "+r"(i0));  // the tests below do not change over the pairs: not all of them ahead of the loop
+        const uint32_t keep = keep_bits<FEAT, false>(pl, mv, mixed, own_seg, i0, key);
+        chunk_p_ds<FEAT, false, false>(s, dp, p.sm_scale, pl, mv, keep, i0, key, lse, delta, bias, pr, ds);
+#pragma unroll
+        for (int e = 0; e < CH; ++e) acc[cc * CH + e] += ds[e];
+      }
+      tc_fence_before();
+      mbar_arrive(BAR(T_FREE + buf));
+      ++it;
+    }
+    if (ok && key < p.Lkv) {
+      float* dst = p.dbias + (int64_t)b0 * p.bias_bs + (int64_t)h0 * p.bias_hs + key;
+#pragma unroll
+      for (int e = 0; e < 64; ++e)
+        if (i_first + e < p.Lq) dst[(int64_t)(i_first + e) * p.Lkv] = acc[e];
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    __syncwarp();
+    tmem_dealloc(tmem, C::TMEM_COLS);
+    if (lane == 0 && *abort_flag && p.status) atomicExch(p.status, (int)PJX_ERR_DEVICE_TIMEOUT);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// fp16: largest finite |dO|, |V| (valid keys only) and |head_scale|, as bit patterns (non-negative
+// floats order like their bits)
+// ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ float amax8(uint4 w, float m) {
+  const uint32_t r[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&r[i]));
+    const float x = fabsf(f.x), y = fabsf(f.y);
+    if (x < INFINITY) m = fmaxf(m, x);  // not for inf, nor for NaN
+    if (y < INFINITY) m = fmaxf(m, y);
+  }
+  return m;
+}
+
+__global__ void __launch_bounds__(256) bwd_amax_kernel(const BwdParams p, uint32_t* out) {
+  const int64_t step = (int64_t)gridDim.x * blockDim.x, first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t n_o = (int64_t)p.B * p.Lq * p.Hq * p.Dv / 8, row_v = (int64_t)p.Hkv * p.Dv / 8, n_v = (int64_t)p.B * p.Lkv * row_v;
+  float m[3] = {0.f, 0.f, 0.f};
+  for (int64_t i = first; i < n_o; i += step) m[0] = amax8(static_cast<const uint4*>(p.d_o)[i], m[0]);
+  for (int64_t i = first; i < n_v; i += step) {
+    const int64_t t = i / row_v;
+    if (p.kv_lengths && (int)(t % p.Lkv) >= p.kv_lengths[t / p.Lkv]) continue;
+    m[1] = amax8(static_cast<const uint4*>(p.v)[i], m[1]);
+  }
+  if (p.mod.head_scale && first < p.Hq && fabsf(p.mod.head_scale[first]) < INFINITY) m[2] = fabsf(p.mod.head_scale[first]);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m[k] = fmaxf(m[k], __shfl_xor_sync(0xffffffffu, m[k], o));
+    if ((threadIdx.x & 31) == 0 && m[k] > 0.f) atomicMax(out + k, __float_as_uint(m[k]));
+  }
+}
+
+template <typename K, typename... Args>
+int launch_kernel(K kern, int64_t grid, int smem, cudaStream_t stream, const char* what, const Args&... args) {
+  int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), what);
+  if (rc) return rc;
+  kern<<<dim3((unsigned)grid), NTHREADS, smem, stream>>>(args...);
+  count_launch();
+  return check_cuda(cudaGetLastError(), what);
+}
+
+template <int D, int DV, bool BF16, int FEAT>
+int launch_feat(const BwdParams& p, const ExactArgs& a, cudaStream_t stream) {
+  using Q = DqCfg<D, DV, FEAT>;
+  using KV = DkvCfg<D, DV>;
+  CUtensorMap tq, tdo, tk, tv, tq2, tdo2;
+  int rc;
+  if ((rc = make_tmap_blhd(&tq, p.q, p.dtype, p.B, p.Lq, p.Hq, D, BM))) return rc;
+  if ((rc = make_tmap_blhd(&tdo, p.d_o, p.dtype, p.B, p.Lq, p.Hq, DV, BM))) return rc;
+  if ((rc = make_tmap_blhd(&tk, p.k, p.dtype, p.B, p.Lkv, p.Hkv, D, BN))) return rc;
+  if ((rc = make_tmap_blhd(&tv, p.v, p.dtype, p.B, p.Lkv, p.Hkv, DV, BN))) return rc;
+  tq2 = tq;
+  tdo2 = tdo;
+  if constexpr (KV::QT != BM) {
+    if ((rc = make_tmap_blhd(&tq2, p.q, p.dtype, p.B, p.Lq, p.Hq, D, KV::QT))) return rc;
+    if ((rc = make_tmap_blhd(&tdo2, p.d_o, p.dtype, p.B, p.Lq, p.Hq, DV, KV::QT))) return rc;
+  }
+  const int64_t n_q = (p.Lq + BM - 1) / BM, n_k = (p.Lkv + BN - 1) / BN;
+  if ((rc = launch_kernel(bwd_dq_exact_sm100_kernel<D, DV, BF16, FEAT>, n_q * p.Hq * p.B, Q::SMEM_BYTES, stream,
+                          "sm100 exact dq launch", tq, tdo, tk, tv, p, a)))
+    return rc;
+  if ((rc = launch_kernel(bwd_dkdv_exact_sm100_kernel<D, DV, BF16, FEAT>, n_k * p.Hkv * p.B, KV::SMEM_BYTES, stream,
+                          "sm100 exact dk/dv launch", tq2, tdo2, tk, tv, p, a)))
+    return rc;
+  if constexpr ((FEAT & 2) != 0) {
+    if (p.dbias) {
+      const int64_t planes = (int64_t)(p.bias_bs ? p.B : 1) * (p.bias_hs ? p.Hq : 1);
+      return launch_kernel(bwd_dbias_sm100_kernel<D, DV, BF16, FEAT>, planes * n_q * n_k, DbCfg<D, DV>::SMEM_BYTES, stream,
+                           "sm100 dbias launch", tq, tdo, tk, tv, p);
+    }
+  }
+  return PJX_OK;
+}
+
+template <int D, bool BF16>
+int launch_square(const BwdParams& p, const ExactArgs& a, cudaStream_t stream) {
+  if (!p.bias) return launch_feat<D, D, BF16, 1>(p, a, stream);
+  return p.mod.on ? launch_feat<D, D, BF16, 3>(p, a, stream) : launch_feat<D, D, BF16, 2>(p, a, stream);
+}
+
+template <bool BF16>
+int launch_shape(const BwdParams& p, const ExactArgs& a, cudaStream_t stream) {
+  if (p.D == 192) return p.mod.on ? launch_feat<192, 128, BF16, 1>(p, a, stream) : launch_feat<192, 128, BF16, 0>(p, a, stream);
+  return p.D == 128 ? launch_square<128, BF16>(p, a, stream) : launch_square<64, BF16>(p, a, stream);
+}
+
+}  // namespace
+
+// 16-bit calls of the tensor-core head shapes that the two kernels of attn_bwd_sm100.cu do not take.  The dense bias
+// at (192, 128) stays on the CUDA cores: its staging window does not fit beside the tiles.
+bool bwd_exact_sm100_supported(const BwdParams& p) {
+  if (p.dtype != PJX_BF16 && p.dtype != PJX_F16) return false;
+  const bool square = p.D == p.Dv && (p.D == 64 || p.D == 128);
+  if (!square && !(p.D == 192 && p.Dv == 128 && !p.bias)) return false;
+  if (p.B < 1 || p.Lq < 1 || p.Lkv < 1) return false;
+  const int64_t n_q = (p.Lq + BM - 1) / BM, n_k = (p.Lkv + BN - 1) / BN, planes = (int64_t)p.Hq * p.B;
+  if (n_q * planes > 0x7fffffffLL || n_k * planes > 0x7fffffffLL || (p.dbias && n_q * n_k > 0x7fffffffLL / planes)) return false;
+  if ((reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v) |
+       reinterpret_cast<uintptr_t>(p.d_o) | reinterpret_cast<uintptr_t>(p.dq) | reinterpret_cast<uintptr_t>(p.dk) |
+       reinterpret_cast<uintptr_t>(p.dv) | reinterpret_cast<uintptr_t>(p.delta)) & 15)
+    return false;
+  return true;
+}
+
+// Bytes of stream-ordered scratch: segment ranges both ways and the three fp16 maxima.
+int launch_bwd_exact_sm100(const BwdParams& p, void* scratch, cudaStream_t stream) {
+  ExactArgs a = {};
+  a.order_w = (p.band_hi < PJX_BAND_NO_UPPER && p.band_lo == PJX_BAND_NO_LOWER) ? 16 : 1;
+  a.p_scale = 1.f;
+  uint32_t* amax = static_cast<uint32_t*>(scratch);
+  int rc;
+  if (p.dtype == PJX_F16) {
+    if ((rc = check_cuda(cudaMemsetAsync(amax, 0, 16, stream), "clear maxima"))) return rc;
+    const int64_t n = ((int64_t)p.B * p.Lq * p.Hq * p.Dv / 8 + 255) / 256;
+    bwd_amax_kernel<<<(unsigned)(n < 592 ? n : 592), 256, 0, stream>>>(p, amax);
+    count_launch();
+    if ((rc = check_cuda(cudaGetLastError(), "backward amax launch"))) return rc;
+    a.amax = amax;
+    a.p_scale = 16384.f;  // P <= 1 / (1 - rate): below 2^15 once scaled
+    for (float keep = 1.f / (1.f - p.mod.dropout_rate); keep > 1.f && a.p_scale > 0x1p-14f; keep *= 0.5f) a.p_scale *= 0.5f;
+  }
+  if (bwd_exact_uses_ranges(p)) {
+    const int n_q = (p.Lq + BM - 1) / BM, n_k = (p.Lkv + BN - 1) / BN;
+    const int nb = (p.mod.seg_q_bs == 0 && p.mod.seg_k_bs == 0) ? 1 : p.B;
+    int32_t* qr = static_cast<int32_t*>(scratch) + 4;
+    int32_t* kr = qr + (int64_t)nb * n_q * 2;
+    launch_seg_tile_range(p.mod.seg_q, p.mod.seg_k, p.mod.seg_q_bs, p.mod.seg_k_bs, p.Lq, p.Lkv, n_q, nb, qr, stream);
+    launch_seg_tile_range(p.mod.seg_k, p.mod.seg_q, p.mod.seg_k_bs, p.mod.seg_q_bs, p.Lkv, p.Lq, n_k, nb, kr, stream);
+    if ((rc = check_cuda(cudaGetLastError(), "segment ranges launch"))) return rc;
+    a.q_range = qr;
+    a.k_range = kr;
+    a.q_range_bs = nb == 1 ? 0 : n_q;
+    a.k_range_bs = nb == 1 ? 0 : n_k;
+  }
+  return p.dtype == PJX_BF16 ? launch_shape<true>(p, a, stream) : launch_shape<false>(p, a, stream);
+}
+
+// Segment masks cut the tile loops (prefix keys are visible to every row: no ranges then).
+bool bwd_exact_uses_ranges(const BwdParams& p) {
+  return p.mod.seg_q && p.mod.seg_k && !p.mod.prefix_len && p.B <= 65535;
+}
+
+size_t bwd_exact_scratch_bytes(const BwdParams& p) {
+  if (p.dtype != PJX_F16 && !bwd_exact_uses_ranges(p)) return 0;
+  size_t n = 16;
+  if (bwd_exact_uses_ranges(p)) n += (size_t)p.B * ((p.Lq + BM - 1) / BM + (p.Lkv + BN - 1) / BN) * 2 * sizeof(int32_t);
+  return n;
+}
+
+}  // namespace pjx

@@ -1008,6 +1008,21 @@ int make_tmap_blhd(CUtensorMap* m, const void* base, int dtype, int B, int L, in
   return PJX_OK;
 }
 
+// Scratch of a call (partials of the KV halves, segment ranges) comes from the stream-ordered allocator.  Its default pool hands freed memory
+// back to the driver at every synchronisation, which would make each call pay for a fresh mapping: keep it.
+void keep_pool_memory() {
+  static std::atomic<bool> done[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || done[dev].exchange(true)) return;
+  cudaMemPool_t pool;
+  if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
+    uint64_t keep = 256ull << 20;  // the partials are at most 74 items x 2 halves x 256 rows x Dv floats (< 40 MB)
+    uint64_t cur = 0;
+    if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &cur) == cudaSuccess && cur < keep)
+      cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  }
+}
+
 namespace {
 
 // fp32 bias [Bb, Hb, Lq, Lkv] (strides in elements, 0 = broadcast): box = 32 keys x 128 rows.
@@ -1031,21 +1046,6 @@ int make_tmap_bias(CUtensorMap* m, const FwdParams& p) {
 bool bias_can_be_staged(const FwdParams& p) {
   return p.bias && p.Lkv % 4 == 0 && (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0 && p.bias_hs % 4 == 0 &&
          p.bias_bs % 4 == 0;
-}
-
-// The partials of the KV halves come from the stream-ordered allocator.  Its default pool hands freed memory
-// back to the driver at every synchronisation, which would make each call pay for a fresh mapping: keep it.
-void keep_pool_memory() {
-  static std::atomic<bool> done[64];
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || done[dev].exchange(true)) return;
-  cudaMemPool_t pool;
-  if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
-    uint64_t keep = 256ull << 20;  // the partials are at most 74 items x 2 halves x 256 rows x Dv floats (< 40 MB)
-    uint64_t cur = 0;
-    if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &cur) == cudaSuccess && cur < keep)
-      cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-  }
 }
 
 // A second stream per device for the halves: they do not depend on the full-length CTAs, and launched beside
@@ -1124,6 +1124,16 @@ __global__ void __launch_bounds__(128) seg_tile_range_kernel(const int32_t* __re
     r[1] = last + 1;
   }
 }
+
+}  // namespace
+
+void launch_seg_tile_range(const int32_t* seg_q, const int32_t* seg_k, int64_t sq_bs, int64_t sk_bs, int Lq, int Lkv, int tiles,
+                           int nb, int32_t* out, cudaStream_t stream) {
+  seg_tile_range_kernel<<<dim3(tiles, nb), 128, 0, stream>>>(seg_q, seg_k, sq_bs, sk_bs, Lq, Lkv, out);
+  count_launch();
+}
+
+namespace {
 
 template <int DQK, int DV, int BN, int KST, int VST, bool BF16, int BIAS, bool BAND = false, int MOD = 0>
 int launch_one(const FwdParams& p, int dtype, cudaStream_t stream) {
@@ -1224,9 +1234,8 @@ int launch_one(const FwdParams& p, int dtype, cudaStream_t stream) {
       void* ranges = nullptr;
       keep_pool_memory();
       if (nb <= 65535 && cudaMallocAsync(&ranges, (size_t)nb * tiles * 2 * sizeof(int32_t), stream) == cudaSuccess) {
-        seg_tile_range_kernel<<<dim3(tiles, nb), 128, 0, stream>>>(p.mod.seg_q, p.mod.seg_k, p.mod.seg_q_bs, p.mod.seg_k_bs,
-                                                                   p.Lq, p.Lkv, static_cast<int32_t*>(ranges));
-        count_launch();
+        launch_seg_tile_range(p.mod.seg_q, p.mod.seg_k, p.mod.seg_q_bs, p.mod.seg_k_bs, p.Lq, p.Lkv, tiles, nb,
+                              static_cast<int32_t*>(ranges), stream);
         ScoreMod mod = p.mod;
         mod.q_tile_range = static_cast<const int32_t*>(ranges);
         mod.q_tile_range_bs = nb == 1 ? 0 : tiles;

@@ -173,8 +173,8 @@ struct BwdParams {
   float sm_scale;
   int dtype = PJX_F32;
   int32_t* status = nullptr;  // device status word or null
-  bool use_sm100 = false;     // dQ and dK/dV by the tcgen05 kernels instead of the CUDA-core ones
-  ScoreMod mod;               // structured masks / score modifiers (CUDA-core kernels only)
+  ScoreMod mod;               // structured masks / score modifiers
+  bool lse_natural = false;   // lse2 holds the natural log-sum-exp (tcgen05 kernels that add terms to the scores)
 };
 
 constexpr int kMaxExchangeRanks = 16;
@@ -212,6 +212,15 @@ int launch_fwd_sm100(const FwdParams& p, int dtype, cudaStream_t stream);
 // tcgen05 backward (dQ kernel and dK/dV kernel); expects p.delta filled.
 bool bwd_sm100_supported(const BwdParams& p, const char** why);
 int launch_bwd_sm100(const BwdParams& p, cudaStream_t stream);
+// tcgen05 backward with P and dS as 16 + 16 bits: score modifiers, dense bias, head shape (192, 128)
+// (attn_bwd_sm100_exact.cu); expects p.delta filled and `scratch` of bwd_exact_scratch_bytes (0: may be null).
+bool bwd_exact_sm100_supported(const BwdParams& p);
+size_t bwd_exact_scratch_bytes(const BwdParams& p);
+int launch_bwd_exact_sm100(const BwdParams& p, void* scratch, cudaStream_t stream);
+// Range of keys per tile of 128 query rows that can share a segment with the tile (attn_fwd_sm100.cu).
+void launch_seg_tile_range(const int32_t* seg_q, const int32_t* seg_k, int64_t sq_bs, int64_t sk_bs, int Lq, int Lkv, int tiles,
+                           int nb, int32_t* out, cudaStream_t stream);
+void keep_pool_memory();
 bool decode_fast_supported(const DecodeParams& p, int dtype);
 int launch_decode(const DecodeParams& p, int dtype, cudaStream_t stream);
 // Split length chosen for split_len = 0; `ragged`: per-sequence lengths are given (see pjx_api.cu).

@@ -21,14 +21,16 @@
 // * the gradient of the bias is a kernel of its own: one CTA per 128 x 128 tile of the bias, walking the
 //   (batch, head) pairs that share it and summing dS in registers in a fixed order (no atomics).
 //
-// FEAT: bit 0 = score modifiers, bit 1 = dense bias; band and key-length masks always.
+// FEAT: bit 0 = structured masks and terms added to the scores (ALiBi, relative table), bit 1 = dense bias, bit 2 =
+// head scale, soft cap and dropout (a hash and a tanhf per score: inlined for a whole tile they make the loop
+// miss the instruction cache, 45% of the time of the packed ALiBi step); band and key-length masks always.
 // With FEAT 0 the row vector `lse2` is base 2; otherwise it is the natural log-sum-exp, subtracted before
 // the change of base, so that a bias of the type's lowest value cannot overflow to inf - inf.
 //
 // Bound by the MMA issue stream at D = 128 and by the element work of the compute warps at D = 64.
 // Measured (forward + backward, against the CUDA-core kernels these calls ran on before; B200):
-//   packed documents + ALiBi, B1 S4096 Hq32 Hkv8 D128 bf16     41.9 ms -> 0.90 ms
-//   dense bias with gradient, B8 S1024 H16 D64 bf16            6.26 ms -> 0.89 ms
+//   packed documents + ALiBi, B1 S4096 Hq32 Hkv8 D128 bf16     41.9 ms -> 0.60 ms
+//   dense bias with gradient, B8 S1024 H16 D64 bf16            6.26 ms -> 0.66 ms
 //   latent training step, B2 S2048 H16 (192,128) bf16          16.6 ms -> 0.67 ms
 #include "attn_bwd_sm100.cuh"
 
@@ -94,18 +96,59 @@ __device__ __forceinline__ void split_pack(const float (&x)[CH], float scale, ui
   }
 }
 
-// CH bias values of one key: rows i0 .. i0 + CH - 1 of a plane with `Lkv` entries per row (`src` is at the key's
-// column), rows past Lq clamped.  The opaque index and the volatile loads keep the compiler from computing the 64-bit
-// addresses of a whole tile ahead of its loop and from hoisting the tile's loads to its start (both spill).
-__device__ __forceinline__ void load_bias_column(const float* src, int i0, int Lq, int Lkv, float* out) {
-  asm volatile("" : "+r"(i0));
+// Dense bias: a ring of CH-column chunks per compute warp (2 KB each: 32 lanes x 16 values), filled by 4-byte
+// asynchronous copies (rows of the bias may start at any element) a half step (D = 64) or two chunks (D = 128, where the
+// tiles leave no more room) ahead of their use.  Loads into registers one chunk ahead did not cover the L2 latency:
+// 600 to 1900 cycles per chunk against 350 without a bias.
+template <int D>
+constexpr int BIAS_RING = D > 64 ? 2 : 4;
+constexpr int BIAS_SLOT = 32 * CH * 4;
+
+__device__ __forceinline__ void copy4_async(uint32_t dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ float lds(uint32_t addr) {
+  float x;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x) : "r"(addr) : "memory");
+  return x;
+}
+
+// Keys on the lanes: this lane's key (`src` is at its column), rows i0 .. i0 + CH - 1, clamped to the tensor.
+__device__ __forceinline__ void fetch_bias_column(uint32_t slot, const float* src, int i0, int Lq, int Lkv, int lane) {
   const float* ptr = src + (int64_t)min(i0, Lq - 1) * Lkv;
 #pragma unroll
   for (int e = 0; e < CH; ++e) {
-    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(out[e]) : "l"(ptr));
-    if (i0 + e + 1 < Lq) ptr += Lkv;
+    copy4_async(slot + (e * 32 + lane) * 4, ptr);
+    ptr += i0 + e + 1 < Lq ? Lkv : 0;
   }
 }
+__device__ __forceinline__ void read_bias_column(uint32_t slot, int lane, float (&out)[CH]) {
+#pragma unroll
+  for (int e = 0; e < CH; ++e) out[e] = lds(slot + (e * 32 + lane) * 4);
+}
+// Rows on the lanes: rows r0 .. r0 + 31 of keys j0 .. j0 + CH - 1, copied two rows at a time (64 contiguous bytes each)
+// and read a row per lane; element (r, k) is stored at column k ^ (r / 2), which keeps both free of bank conflicts.
+__device__ __forceinline__ void fetch_bias_rows(uint32_t slot, const float* plane, int r0, int j0, int Lq, int Lkv, int lane) {
+  const int k = lane & 15, key = min(j0 + k, Lkv - 1);
+#pragma unroll
+  for (int e = 0; e < CH; ++e) {
+    const int r = 2 * e + (lane >> 4);
+    copy4_async(slot + (r * CH + (k ^ e)) * 4, plane + (int64_t)min(r0 + r, Lq - 1) * Lkv + key);
+  }
+}
+__device__ __forceinline__ void read_bias_row(uint32_t slot, int lane, float (&out)[CH]) {
+#pragma unroll
+  for (int e = 0; e < CH; ++e) out[e] = lds(slot + (lane * CH + (e ^ (lane >> 1))) * 4);
+}
+
+// Chunks of a half step in straight line; with modifiers as a loop, whose code stays in the instruction cache.
+template <int FEAT>
+constexpr int UNROLL = (FEAT & 1) ? 1 : 4;
 
 // The element (i, j) a column e of a chunk stands for.  ROWS: the thread owns query row i0 and the columns are
 // keys j0 + e; otherwise it owns key j0 and the columns are query rows i0 + e.
@@ -124,18 +167,38 @@ __device__ __forceinline__ uint32_t keep_bits(const Place& pl, const ScoreModVie
     inside = inside && !seg_mixed;
   }
   if (inside) return ALL;
+  // the columns' ids and limits first, all loads in flight together (one at a time they cost a latency per column)
+  [[maybe_unused]] int col_seg[CH], col_limit[CH];
+  if constexpr ((FEAT & 1) != 0) {
+    if (seg_mixed) {
+      const int32_t* src = ROWS ? mv.seg_k : mv.seg_q;
+      const int first = ROWS ? j0 : i0, last = (ROWS ? pl.Lkv : pl.Lq) - 1;
+#pragma unroll
+      for (int e = 0; e < CH; ++e) col_seg[e] = __ldg(src + min(first + e, last));
+    }
+    if (mv.row_limit) {
+#pragma unroll
+      for (int e = 0; e < CH; ++e) col_limit[e] = __ldg(mv.row_limit + min(ROWS ? i0 : i0 + e, pl.Lq - 1));
+    }
+  }
   uint32_t bits = 0;
 #pragma unroll
   for (int e = 0; e < CH; ++e) {
     const int i = ROWS ? i0 : i0 + e, j = ROWS ? j0 + e : j0;
-    bool keep = j <= i + pl.band_hi && j >= i + pl.band_lo;
-    if constexpr ((FEAT & 1) != 0) {
-      keep = keep || j < mv.prefix;
-      if (mv.row_limit) keep = keep && j < mv.row_limit[min(i, pl.Lq - 1)];
-      if (seg_mixed) keep = keep && (ROWS ? mv.seg_k[min(j, pl.Lkv - 1)] : mv.seg_q[min(i, pl.Lq - 1)]) == own_seg;
-    }
-    keep = keep && j < pl.kv_len && i < pl.Lq;
+    bool keep = (j <= i + pl.band_hi) & (j >= i + pl.band_lo);
+    if constexpr ((FEAT & 1) != 0) keep |= j < mv.prefix;
+    keep = keep & (j < pl.kv_len) & (i < pl.Lq);
     bits |= keep ? (1u << e) : 0u;
+  }
+  if constexpr ((FEAT & 1) != 0) {
+    if (seg_mixed) {
+#pragma unroll
+      for (int e = 0; e < CH; ++e) bits &= col_seg[e] == own_seg ? ALL : ALL ^ (1u << e);
+    }
+    if (mv.row_limit) {
+#pragma unroll
+      for (int e = 0; e < CH; ++e) bits &= (ROWS ? j0 + e : j0) < col_limit[e] ? ALL : ALL ^ (1u << e);
+    }
   }
   return bits;
 }
@@ -156,7 +219,7 @@ __device__ __forceinline__ void chunk_p_ds(const float (&s)[CH], const float (&d
     float x[CH];
 #pragma unroll
     for (int e = 0; e < CH; ++e) x[e] = s[e] * c;
-    const bool nonlinear = NL && (FEAT & 1) && (mv.hscale_m1 != 0.f || mv.softcap > 0.f);
+    const bool nonlinear = NL && (FEAT & 4) && (mv.hscale_m1 != 0.f || mv.softcap > 0.f);
     float g[CH];
     if (nonlinear) {
       const float inv_cap = mv.softcap > 0.f ? 1.f / mv.softcap : 0.f;
@@ -192,7 +255,7 @@ __device__ __forceinline__ void chunk_p_ds(const float (&s)[CH], const float (&d
 #pragma unroll
       for (int e = 0; e < CH; ++e) x[e] += bias[e];
     }
-    if ((FEAT & 1) && mv.drop_rate > 0.f) {
+    if ((FEAT & 4) && mv.drop_rate > 0.f) {
       // dV sees the dropped, rescaled probabilities and dP is dropped the same way; delta includes it already
 #pragma unroll
       for (int e = 0; e < CH; ++e) {
@@ -257,8 +320,8 @@ struct DqCfg {
   static constexpr int OFF_DO = TQ;
   static constexpr int OFF_K = OFF_DO + TV;
   static constexpr int OFF_V = OFF_K + KST * TQ;
-  static constexpr int OFF_BIAS = OFF_V + VST * TV;                    // Dense bias: 8 warps x 32 rows x 33 floats
-  static constexpr int OFF_BAR = OFF_BIAS + ((FEAT & 2) ? 8 * 32 * 33 * 4 : 0);
+  static constexpr int OFF_BIAS = OFF_V + VST * TV;                    // dense bias: a ring per compute warp
+  static constexpr int OFF_BAR = OFF_BIAS + ((FEAT & 2) ? 8 * BIAS_RING<D> * BIAS_SLOT : 0);
   // barriers: QDO_FULL, K_FULL[2], K_EMPTY[2], V_FULL[2], V_EMPTY[2], SP_FULL[2], DS_FULL[2], DQ_FULL, K_CLEAN
   static constexpr int N_BAR = 15;
   static constexpr int SMEM_BYTES = OFF_BAR + N_BAR * 8 + 16 + 1024;
@@ -456,24 +519,18 @@ bwd_dq_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
       mv = view_of(p.mod, b, h, p.Lq);
       if (mv.seg_q) own_seg = mv.seg_q[min(row, p.Lq - 1)];
     }
-    // Dense bias: the warp's 32 rows of the bias, 32 keys at a time, through its window in shared memory
-    [[maybe_unused]] float breg[(FEAT & 2) ? 32 : 1];
-    [[maybe_unused]] float* bwin = reinterpret_cast<float*>(smem + C::OFF_BIAS) + (warp - 2) * 32 * 33;
+    constexpr int NB = BIAS_RING<D>;
+    [[maybe_unused]] const uint32_t ring = sbase + C::OFF_BIAS + (warp - 2) * NB * BIAS_SLOT;
     [[maybe_unused]] const float* bsrc = (FEAT & 2) ? p.bias + (int64_t)b * p.bias_bs + (int64_t)h * p.bias_hs : nullptr;
-    auto fetch_bias = [&](int key0) {
-      if constexpr ((FEAT & 2) != 0) {
-        const int key = min(key0 + lane, p.Lkv - 1);
-        int r0 = q0 + quarter * 32;
-        asm volatile("" : "+r"(r0));  // as in load_bias_column
-        const float* ptr = bsrc + (int64_t)min(r0, p.Lq - 1) * p.Lkv + key;
-#pragma unroll
-        for (int r = 0; r < 32; ++r) {
-          asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(breg[r]) : "l"(ptr));
-          if (r0 + r + 1 < p.Lq) ptr += p.Lkv;
-        }
-      }
+    auto fetch_bias = [&](int t) {  // chunk t of this warp: CH keys, four chunks per tile
+      if (t < 4 * n)
+        fetch_bias_rows(ring + (t % NB) * BIAS_SLOT, bsrc, q0 + quarter * 32, (j_lo + t / 4) * BN + grp * 64 + (t % 4) * CH, p.Lq,
+                        p.Lkv, lane);
+      copy_commit();
     };
-    if (n > 0) fetch_bias(j_lo * BN + grp * 64);
+    if constexpr ((FEAT & 2) != 0) {
+      for (int t = 0; t < NB; ++t) fetch_bias(t);
+    }
     bool ok = true;
     for (int j = 0; j < n; ++j) {
       const int k0 = (j_lo + j) * BN + grp * 64;  // first key of this group's columns
@@ -485,33 +542,33 @@ bwd_dq_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      float s[2][CH], dp[2][CH];
-      tmem_ld16f(s_addr, s[0]);
-      tmem_ld16f(dp_addr, dp[0]);
-#pragma unroll
+      float s_next[CH], dp_next[CH];
+      tmem_ld16f(s_addr, s_next);
+      tmem_ld16f(dp_addr, dp_next);
+#pragma unroll(UNROLL<FEAT>)
       for (int cc = 0; cc < 64 / CH; ++cc) {
-        if constexpr ((FEAT & 2) != 0) {
-          if (cc % 2 == 0) {
-            __syncwarp();
-#pragma unroll
-            for (int r = 0; r < 32; ++r) bwin[r * 33 + lane] = breg[r];
-            __syncwarp();
-            fetch_bias(cc == 0 ? k0 + 32 : k0 + BN);
-          }
-        }
         tmem_wait_ld();
+        float s[CH], dp[CH];
+#pragma unroll
+        for (int e = 0; e < CH; ++e) {
+          s[e] = s_next[e];
+          dp[e] = dp_next[e];
+        }
         if (cc + 1 < 64 / CH) {
-          tmem_ld16f(s_addr + (cc + 1) * CH, s[(cc + 1) & 1]);
-          tmem_ld16f(dp_addr + (cc + 1) * CH, dp[(cc + 1) & 1]);
+          tmem_ld16f(s_addr + (cc + 1) * CH, s_next);
+          tmem_ld16f(dp_addr + (cc + 1) * CH, dp_next);
         }
         float bias[CH], pr[CH], ds[CH];
         if constexpr ((FEAT & 2) != 0) {
-#pragma unroll
-          for (int e = 0; e < CH; ++e) bias[e] = bwin[lane * 33 + (cc & 1) * CH + e];
+          copy_wait<NB - 1>();
+          __syncwarp();
+          read_bias_row(ring + (cc % NB) * BIAS_SLOT, lane, bias);
+          __syncwarp();  // the slot has been read by all lanes
+          fetch_bias(4 * j + cc + NB);
         }
         const int j0 = k0 + cc * CH;
         const uint32_t keep = keep_bits<FEAT, true>(pl, mv, mixed, own_seg, row, j0);
-        chunk_p_ds<FEAT, true>(s[cc & 1], dp[cc & 1], c, pl, mv, keep, row, j0, &lse, &delta, bias, pr, ds);
+        chunk_p_ds<FEAT, true>(s, dp, c, pl, mv, keep, row, j0, &lse, &delta, bias, pr, ds);
         uint32_t pk[CH];
         split_pack<BF16>(ds, pack, pk);
         tmem_st16(s_addr + cc * CH, pk);  // over the chunk's own scores, which were read already
@@ -520,6 +577,7 @@ bwd_dq_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
       tc_fence_before();
       mbar_arrive(BAR(DS_FULL + grp));
     }
+    if constexpr ((FEAT & 2) != 0) copy_wait<0>();  // none in flight at the exit, should a wait have expired
     if (ok && q0 < p.Lq) {
       if (n > 0) {
         ok = mbar_wait(BAR(DQ_FULL), 0, abort_flag);
@@ -546,7 +604,7 @@ bwd_dq_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
 // ---------------------------------------------------------------------------------------------
 // dK/dV kernel
 // ---------------------------------------------------------------------------------------------
-template <int D, int DV>
+template <int D, int DV, int FEAT>
 struct DkvCfg {
   static constexpr int SUBQ = D / 64, SUBV = DV / 64;
   static constexpr int QT = D > 128 ? 96 : 128;      // query rows per step: S^T | dP^T | dV | dK fill tensor memory
@@ -558,10 +616,11 @@ struct DkvCfg {
   static constexpr int OFF_Q = OFF_V + TV;           // 2 stages
   static constexpr int OFF_DO = OFF_Q + 2 * TQ;      // 2 stages
   static constexpr int OFF_ROW = OFF_DO + 2 * TDO;   // 2 stages x { float lse[QT]; float delta[QT]; }
-  static constexpr int OFF_BAR = OFF_ROW + 2 * 2 * QT * 4;
+  static constexpr int OFF_BIAS = OFF_ROW + 2 * 2 * QT * 4;
+  static constexpr int OFF_BAR = OFF_BIAS + ((FEAT & 2) ? 8 * BIAS_RING<D> * BIAS_SLOT : 0);
   // barriers: KV_FULL, QDO_FULL[2], QDO_EMPTY[2], SP_FULL[2], PDS_FULL[2], ACC_FULL
   static constexpr int N_BAR = 10;
-  static constexpr int SMEM_BYTES = OFF_BAR + N_BAR * 8 + 16 + 1024;
+  static constexpr int SMEM_BYTES = OFF_BAR + N_BAR * 8 + 16 + 896;  // 1024-byte alignment from a 128-byte one
   static constexpr int TMEM_COLS = 512;              // S^T QT | dP^T QT | dV DV | dK D
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
   static_assert(2 * QT + DV + D <= 512, "tensor memory has 512 columns");
@@ -573,9 +632,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                             const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                             const __grid_constant__ BwdParams p, const __grid_constant__ ExactArgs a) {
-  using C = DkvCfg<D, DV>;
+  using C = DkvCfg<D, DV, FEAT>;
   constexpr int QT = C::QT, HALF = C::HALF, NCH = HALF / CH;
-  extern __shared__ unsigned char smem_unaligned[];
+  extern __shared__ __align__(128) unsigned char smem_unaligned[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~uintptr_t(1023));
   const uint32_t sbase = smem_u32(smem);
   const uint32_t bar0 = sbase + C::OFF_BAR;
@@ -743,11 +802,29 @@ bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
     const Place pl = {kv_len, p.Lq, p.Lkv, p.band_lo, p.band_hi};
     ScoreModView mv = {};
     int own_seg = 0;
-    [[maybe_unused]] const float* bsrc = nullptr;  // Dense bias: this thread's column of the bias of head h
-    [[maybe_unused]] float bnext[(FEAT & 2) ? CH : 1];
-    auto fetch_bias = [&](int i0) {  // keys on the lanes: 128 contiguous bytes per row
-      if constexpr ((FEAT & 2) != 0) load_bias_column(bsrc, i0, p.Lq, p.Lkv, bnext);
+    constexpr int NB = BIAS_RING<D>;
+    [[maybe_unused]] const uint32_t ring = sbase + C::OFF_BIAS + (warp - 2) * NB * BIAS_SLOT;
+    // dense bias: position of the next chunk to fetch (chunk of the half, query tile, head of the group)
+    [[maybe_unused]] int f_cc = 0, f_t = 0, f_g = 0;
+    [[maybe_unused]] const float* bsrc =
+        (FEAT & 2) ? p.bias + (int64_t)b * p.bias_bs + (int64_t)hk * G * p.bias_hs + min(key, p.Lkv - 1) : nullptr;
+    auto fetch_bias = [&](int slot) {
+      if (f_g < G && n > 0)
+        fetch_bias_column(ring + slot * BIAS_SLOT, bsrc + (int64_t)f_g * p.bias_hs, (t_lo + f_t) * QT + grp * HALF + f_cc * CH, p.Lq,
+                          p.Lkv, lane);
+      copy_commit();
+      if (++f_cc == NCH) {
+        f_cc = 0;
+        if (++f_t == n_t) {
+          f_t = 0;
+          ++f_g;
+        }
+      }
     };
+    if constexpr ((FEAT & 2) != 0) {
+      static_assert(!(FEAT & 2) || NCH % NB == 0, "slots follow the chunk index");
+      for (int t = 0; t < NB; ++t) fetch_bias(t);
+    }
     bool ok = true;
     for (int it = 0; it < n; ++it) {
       const int st = it & 1;
@@ -759,12 +836,10 @@ bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
           mv = view_of(p.mod, b, h, p.Lq);
           if (mv.seg_q) own_seg = mv.seg_k[min(key, p.Lkv - 1)];
         }
-        if constexpr ((FEAT & 2) != 0) bsrc = p.bias + (int64_t)b * p.bias_bs + (int64_t)h * p.bias_hs + min(key, p.Lkv - 1);
       }
       if constexpr ((FEAT & 1) != 0) {
         if (mv.seg_q) mixed = segments_mixed(mv.seg_q, q0, HALF, p.Lq, own_seg, lane);
       }
-      fetch_bias(q0);
       ok = mbar_wait(BAR(SP_FULL + grp), it & 1, abort_flag);
       if (ok) ok = mbar_wait(BAR(QDO_FULL + st), (it >> 1) & 1, abort_flag);  // the row vectors landed with Q and dO
       ok = __all_sync(0xffffffffu, ok);
@@ -772,10 +847,10 @@ bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
       tc_fence_after();
       const float* lse_s = row_s + st * 2 * QT + grp * HALF;
       const float* delta_s = lse_s + QT;
-      float s[2][CH], dp[2][CH];
-      tmem_ld16f(s_addr, s[0]);
-      tmem_ld16f(dp_addr, dp[0]);
-#pragma unroll
+      float s_next[CH], dp_next[CH];
+      tmem_ld16f(s_addr, s_next);
+      tmem_ld16f(dp_addr, dp_next);
+#pragma unroll(UNROLL<FEAT>)
       for (int cc = 0; cc < NCH; ++cc) {
         float lse[CH], delta[CH], bias[CH], pr[CH], ds[CH];
 #pragma unroll
@@ -784,18 +859,24 @@ bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
           *reinterpret_cast<float4*>(delta + e) = *reinterpret_cast<const float4*>(delta_s + cc * CH + e);
         }
         if constexpr ((FEAT & 2) != 0) {
-#pragma unroll
-          for (int e = 0; e < CH; ++e) bias[e] = bnext[e];
-          if (cc + 1 < NCH) fetch_bias(q0 + (cc + 1) * CH);
+          copy_wait<NB - 1>();
+          read_bias_column(ring + (cc % NB) * BIAS_SLOT, lane, bias);  // this lane's own copies
+          fetch_bias(cc % NB);
         }
         tmem_wait_ld();
+        float s[CH], dp[CH];
+#pragma unroll
+        for (int e = 0; e < CH; ++e) {
+          s[e] = s_next[e];
+          dp[e] = dp_next[e];
+        }
         if (cc + 1 < NCH) {
-          tmem_ld16f(s_addr + (cc + 1) * CH, s[(cc + 1) & 1]);
-          tmem_ld16f(dp_addr + (cc + 1) * CH, dp[(cc + 1) & 1]);
+          tmem_ld16f(s_addr + (cc + 1) * CH, s_next);
+          tmem_ld16f(dp_addr + (cc + 1) * CH, dp_next);
         }
         const int i0 = q0 + cc * CH;
         const uint32_t keep = keep_bits<FEAT, false>(pl, mv, mixed, own_seg, i0, key);
-        chunk_p_ds<FEAT, false>(s[cc & 1], dp[cc & 1], c, pl, mv, keep, i0, key, lse, delta, bias, pr, ds);
+        chunk_p_ds<FEAT, false>(s, dp, c, pl, mv, keep, i0, key, lse, delta, bias, pr, ds);
         uint32_t pk[CH];
         split_pack<BF16>(pr, a.p_scale, pk);
         tmem_st16(s_addr + cc * CH, pk);  // over the chunk's own scores, which were read already
@@ -806,6 +887,7 @@ bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
       tc_fence_before();
       mbar_arrive(BAR(PDS_FULL + grp));
     }
+    if constexpr ((FEAT & 2) != 0) copy_wait<0>();
     if (ok && k0 < p.Lkv) {
       if (n > 0) {
         ok = mbar_wait(BAR(ACC_FULL), 0, abort_flag);
@@ -844,8 +926,9 @@ struct DbCfg {
   static constexpr int SUBQ = D / 64, SUBV = DV / 64;
   static constexpr int TQ = SUBQ * 128 * 128, TV = SUBV * 128 * 128;
   static constexpr int STAGE = 2 * TQ + 2 * TV;                  // Q | K | dO | V
-  static constexpr int NST = STAGE <= 72 * 1024 ? 3 : 1;
-  static constexpr int OFF_ROW = NST * STAGE;                    // 2 x { float lse[128]; float delta[128]; }
+  static constexpr int NST = STAGE <= 72 * 1024 ? 2 : 1;
+  static constexpr int OFF_BIAS = NST * STAGE;                   // the tile of the bias, 128 x 128 fp32
+  static constexpr int OFF_ROW = OFF_BIAS + BM * BN * 4;         // 2 x { float lse[128]; float delta[128]; }
   static constexpr int OFF_BAR = OFF_ROW + 2 * 2 * BM * 4;
   // barriers: FULL[NST], EMPTY[NST], ROW_FULL[2], SP_FULL[2], T_FREE[2]
   static constexpr int N_BAR = 2 * NST + 6;
@@ -960,6 +1043,17 @@ bwd_dbias_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     const int i_first = q0 + grp * 64;
     const uint32_t lane_sel = static_cast<uint32_t>(quarter * 32) << 16;
     const float* bsrc = p.bias + (int64_t)b0 * p.bias_bs + (int64_t)h0 * p.bias_hs + min(key, p.Lkv - 1);
+    // every pair adds the same tile of the bias: read from memory once, each thread keeps its values in shared memory
+    const uint32_t btile = sbase + C::OFF_BIAS + grp * 64 * BN * 4 + (quarter * 32 + lane) * 4;
+    if (n_pairs > 0) {
+      for (int e = 0; e < 64; e += 8) {
+        float t[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) t[u] = __ldg(bsrc + (int64_t)min(i_first + e + u, p.Lq - 1) * p.Lkv);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) asm volatile("st.shared.f32 [%0], %1;" ::"r"(btile + (e + u) * BN * 4), "f"(t[u]) : "memory");
+      }
+    }
     float acc[64];
 #pragma unroll
     for (int e = 0; e < 64; ++e) acc[e] = 0.f;
@@ -982,8 +1076,6 @@ bwd_dbias_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         }
       }
       const uint32_t s_addr = tmem + buf * 256 + lane_sel + grp * 64, dp_addr = s_addr + 128;
-      float bnext[CH];
-      load_bias_column(bsrc, i_first, p.Lq, p.Lkv, bnext);
       ok = mbar_wait(BAR(SP_FULL + buf), (it >> 1) & 1, abort_flag);
       if (ok) ok = mbar_wait(BAR(ROW_FULL + buf), (it >> 1) & 1, abort_flag);
       ok = __all_sync(0xffffffffu, ok);
@@ -1002,8 +1094,7 @@ bwd_dbias_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
           *reinterpret_cast<float4*>(delta + e) = *reinterpret_cast<const float4*>(delta_s + cc * CH + e);
         }
 #pragma unroll
-        for (int e = 0; e < CH; ++e) bias[e] = bnext[e];
-        if (cc + 1 < 64 / CH) load_bias_column(bsrc, i_first + (cc + 1) * CH, p.Lq, p.Lkv, bnext);
+        for (int e = 0; e < CH; ++e) bias[e] = lds(btile + (cc * CH + e) * BN * 4);
         tmem_wait_ld();
         int i0 = i_first + cc * CH;
         asm volatile("" : "+r"(i0));  // the tests below do not change over the pairs: not all of them ahead of the loop
@@ -1080,7 +1171,7 @@ int launch_kernel(K kern, int64_t grid, int smem, cudaStream_t stream, const cha
 template <int D, int DV, bool BF16, int FEAT>
 int launch_feat(const BwdParams& p, const ExactArgs& a, cudaStream_t stream) {
   using Q = DqCfg<D, DV, FEAT>;
-  using KV = DkvCfg<D, DV>;
+  using KV = DkvCfg<D, DV, FEAT>;
   CUtensorMap tq, tdo, tk, tv, tq2, tdo2;
   int rc;
   if ((rc = make_tmap_blhd(&tq, p.q, p.dtype, p.B, p.Lq, p.Hq, D, BM))) return rc;
@@ -1112,13 +1203,14 @@ int launch_feat(const BwdParams& p, const ExactArgs& a, cudaStream_t stream) {
 
 template <int D, bool BF16>
 int launch_square(const BwdParams& p, const ExactArgs& a, cudaStream_t stream) {
-  if (!p.bias) return launch_feat<D, D, BF16, 1>(p, a, stream);
-  return p.mod.on ? launch_feat<D, D, BF16, 3>(p, a, stream) : launch_feat<D, D, BF16, 2>(p, a, stream);
+  const bool heavy = p.mod.head_scale || p.mod.softcap > 0.f || p.mod.dropout_rate > 0.f;
+  if (!p.bias) return heavy ? launch_feat<D, D, BF16, 5>(p, a, stream) : launch_feat<D, D, BF16, 1>(p, a, stream);
+  return p.mod.on ? launch_feat<D, D, BF16, 7>(p, a, stream) : launch_feat<D, D, BF16, 2>(p, a, stream);
 }
 
 template <bool BF16>
 int launch_shape(const BwdParams& p, const ExactArgs& a, cudaStream_t stream) {
-  if (p.D == 192) return p.mod.on ? launch_feat<192, 128, BF16, 1>(p, a, stream) : launch_feat<192, 128, BF16, 0>(p, a, stream);
+  if (p.D == 192) return p.mod.on ? launch_feat<192, 128, BF16, 5>(p, a, stream) : launch_feat<192, 128, BF16, 0>(p, a, stream);
   return p.D == 128 ? launch_square<128, BF16>(p, a, stream) : launch_square<64, BF16>(p, a, stream);
 }
 

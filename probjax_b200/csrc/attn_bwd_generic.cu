@@ -693,7 +693,7 @@ int pjx_attn_bwd_mod(const void* q, const void* k, const void* v, const void* o,
       }
     }
   }
-  p.lse_natural = route == BwdRoute::Sm100Exact && (smod.on || bias);
+  p.lse_natural = route == BwdRoute::Sm100Exact && (smod.rel_bias || bias);
   if (dbias_bytes > 0 && route == BwdRoute::CudaCores) {  // (the tcgen05 kernel writes every entry)
     const int rc0 = check_cuda(cudaMemsetAsync(dbias, 0, dbias_bytes, st), "clear dbias");
     if (rc0) return rc0;

@@ -24,14 +24,15 @@
 // FEAT: bit 0 = structured masks and terms added to the scores (ALiBi, relative table), bit 1 = dense bias, bit 2 =
 // head scale, soft cap and dropout (a hash and a tanhf per score: inlined for a whole tile they make the loop
 // miss the instruction cache, 45% of the time of the packed ALiBi step); band and key-length masks always.
-// With FEAT 0 the row vector `lse2` is base 2; otherwise it is the natural log-sum-exp, subtracted before
-// the change of base, so that a bias of the type's lowest value cannot overflow to inf - inf.
+// The row vector `lse2` is base 2 unless a relative table or a dense bias is added to the scores: then it is
+// the natural log-sum-exp, subtracted before the change of base, so that an entry of the type's lowest value
+// cannot overflow to inf - inf.
 //
 // Bound by the MMA issue stream at D = 128 and by the element work of the compute warps at D = 64.
 // Measured (forward + backward, against the CUDA-core kernels these calls ran on before; B200):
-//   packed documents + ALiBi, B1 S4096 Hq32 Hkv8 D128 bf16     41.9 ms -> 0.60 ms
-//   dense bias with gradient, B8 S1024 H16 D64 bf16            6.26 ms -> 0.66 ms
-//   latent training step, B2 S2048 H16 (192,128) bf16          16.6 ms -> 0.67 ms
+//   packed documents + ALiBi, B1 S4096 Hq32 Hkv8 D128 bf16     41.9 ms -> 0.52 ms
+//   dense bias with gradient, B8 S1024 H16 D64 bf16            6.26 ms -> 0.59 ms
+//   latent training step, B2 S2048 H16 (192,128) bf16          16.6 ms -> 0.65 ms
 #include "attn_bwd_sm100.cuh"
 
 namespace pjx {
@@ -71,28 +72,24 @@ __device__ __forceinline__ float ds_pack_scale(const ExactArgs& a, const ScoreMo
   return exp2f((float)max(-100, min(100, 14 - e)));
 }
 
-// A chunk of CH fp32 values as hi pairs (8 registers) and lo pairs (8 registers).
+// A chunk of CH fp32 values as hi pairs (8 registers) and lo pairs (8 registers).  bf16 truncates hi (the upper half of
+// the fp32 word: one byte permute packs a pair, one AND gives its value back) and rounds lo: 2^-16 of x at most.
 template <bool BF16>
-__device__ __forceinline__ void split_pack(const float (&x)[CH], float scale, uint32_t (&r)[CH]) {
+__device__ __forceinline__ void split_pack(const float2 (&x)[CH / 2], float scale, uint32_t (&r)[CH]) {
 #pragma unroll
   for (int i = 0; i < CH / 2; ++i) {
-    float a = x[2 * i], b = x[2 * i + 1];
-    if constexpr (!BF16) {
-      a *= scale;
-      b *= scale;
-    }
-    const uint32_t hi = pack16<BF16>(a, b);
-    float ha, hb;
     if constexpr (BF16) {
-      ha = __uint_as_float(hi << 16);
-      hb = __uint_as_float(hi & 0xffff0000u);
+      const uint32_t u = __float_as_uint(x[i].x), v = __float_as_uint(x[i].y);
+      r[i] = __byte_perm(u, v, 0x7632);
+      const float2 lo = __fadd2_rn(x[i], make_float2(-__uint_as_float(u & 0xffff0000u), -__uint_as_float(v & 0xffff0000u)));
+      r[CH / 2 + i] = pack16<true>(lo.x, lo.y);
     } else {
+      const float2 y = __fmul2_rn(x[i], make_float2(scale, scale));
+      const uint32_t hi = pack16<false>(y.x, y.y);
       const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&hi));
-      ha = h.x;
-      hb = h.y;
+      r[i] = hi;
+      r[CH / 2 + i] = pack16<false>(y.x - h.x, y.y - h.y);
     }
-    r[i] = hi;
-    r[CH / 2 + i] = pack16<BF16>(a - ha, b - hb);
   }
 }
 
@@ -148,7 +145,7 @@ __device__ __forceinline__ void read_bias_row(uint32_t slot, int lane, float (&o
 
 // Chunks of a half step in straight line; with modifiers as a loop, whose code stays in the instruction cache.
 template <int FEAT>
-constexpr int UNROLL = (FEAT & 1) ? 1 : 4;
+constexpr int UNROLL = (FEAT & 1) ? 2 : 4;
 
 // The element (i, j) a column e of a chunk stands for.  ROWS: the thread owns query row i0 and the columns are
 // keys j0 + e; otherwise it owns key j0 and the columns are query rows i0 + e.
@@ -181,15 +178,13 @@ __device__ __forceinline__ uint32_t keep_bits(const Place& pl, const ScoreModVie
       for (int e = 0; e < CH; ++e) col_limit[e] = __ldg(mv.row_limit + min(ROWS ? i0 : i0 + e, pl.Lq - 1));
     }
   }
-  uint32_t bits = 0;
-#pragma unroll
-  for (int e = 0; e < CH; ++e) {
-    const int i = ROWS ? i0 : i0 + e, j = ROWS ? j0 + e : j0;
-    bool keep = (j <= i + pl.band_hi) & (j >= i + pl.band_lo);
-    if constexpr ((FEAT & 1) != 0) keep |= j < mv.prefix;
-    keep = keep & (j < pl.kv_len) & (i < pl.Lq);
-    bits |= keep ? (1u << e) : 0u;
-  }
+  // band, lengths and prefix are ranges of columns
+  auto below = [](int e) { return (1u << max(0, min(CH, e))) - 1u; };  // bits of the columns before e
+  uint32_t bits = ROWS ? below(i0 + pl.band_hi - j0 + 1) & ~below(i0 + pl.band_lo - j0)
+                       : below(j0 - pl.band_lo - i0 + 1) & ~below(j0 - pl.band_hi - i0);
+  if constexpr ((FEAT & 1) != 0) bits |= ROWS ? below(mv.prefix - j0) : (j0 < mv.prefix ? ALL : 0u);
+  bits &= ROWS ? below(pl.kv_len - j0) : below(pl.Lq - i0);
+  if (ROWS ? i0 >= pl.Lq : j0 >= pl.kv_len) bits = 0;
   if constexpr ((FEAT & 1) != 0) {
     if (seg_mixed) {
 #pragma unroll
@@ -204,84 +199,113 @@ __device__ __forceinline__ uint32_t keep_bits(const Place& pl, const ScoreModVie
 }
 
 // P (dropped and rescaled under dropout) and dS of one chunk.  `lse` and `delta` hold one value (ROWS) or one per column.
-// NL = false: no head_scale / softcap (refused together with a bias gradient).
+// NL = false: no head_scale / softcap (refused together with a bias gradient).  Packed arithmetic (two columns per
+// instruction) throughout: the issue slots of the compute warps are what bounds the modifier variants.
 template <int FEAT, bool ROWS, bool NL = true>
 __device__ __forceinline__ void chunk_p_ds(const float (&s)[CH], const float (&dp)[CH], float c, const Place& pl,
                                            const ScoreModView& mv, uint32_t keep, int i0, int j0, const float* lse,
-                                           const float* delta, const float* bias, float (&pr)[CH], float (&ds)[CH]) {
-  if constexpr (FEAT == 0) {
+                                           const float* delta, const float* bias, float2 (&pr)[CH / 2], float2 (&ds)[CH / 2]) {
+  auto two = [](float x) { return make_float2(x, x); };
+  auto at = [](const float* v, int e) { return ROWS ? make_float2(v[0], v[0]) : make_float2(v[e], v[e + 1]); };
+  auto neg = [](float2 v) { return make_float2(-v.x, -v.y); };
+  float2 y[CH / 2];  // exponents, base 2
+  float2 g[CH / 2];  // d(modified score) / d(scaled score)
+  const bool nonlinear = NL && (FEAT & 4) && (mv.hscale_m1 != 0.f || mv.softcap > 0.f);
+  if (!(FEAT & 2) && !((FEAT & 1) && mv.rel) && !nonlinear) {
+    // `lse` in base 2 here and below unless a table or a dense bias is added
+    const float2 c2 = two(c * kLog2e);
 #pragma unroll
-    for (int e = 0; e < CH; ++e) {
-      pr[e] = ex2_approx(fmaf(s[e], c, -lse[ROWS ? 0 : e]));
-      ds[e] = pr[e] * (dp[e] - delta[ROWS ? 0 : e]);
+    for (int i = 0; i < CH / 2; ++i) y[i] = __ffma2_rn(make_float2(s[2 * i], s[2 * i + 1]), c2, neg(at(lse, 2 * i)));
+    if ((FEAT & 1) && mv.alibi_mode) {
+      const float base = (float)(i0 - j0);
+      const float2 slope = two(-mv.slope * kLog2e);
+#pragma unroll
+      for (int i = 0; i < CH / 2; ++i) {
+        const float e = 2.f * i;
+        float2 d = __fadd2_rn(two(base), ROWS ? make_float2(-e, -e - 1.f) : make_float2(e, e + 1.f));  // i - j, exact
+        d = mv.alibi_mode == 1 ? make_float2(fmaxf(d.x, 0.f), fmaxf(d.y, 0.f)) : make_float2(fabsf(d.x), fabsf(d.y));
+        y[i] = __ffma2_rn(d, slope, y[i]);
+      }
     }
   } else {
-    float x[CH];
+    float2 x[CH / 2];
 #pragma unroll
-    for (int e = 0; e < CH; ++e) x[e] = s[e] * c;
-    const bool nonlinear = NL && (FEAT & 4) && (mv.hscale_m1 != 0.f || mv.softcap > 0.f);
-    float g[CH];
+    for (int i = 0; i < CH / 2; ++i) x[i] = __fmul2_rn(make_float2(s[2 * i], s[2 * i + 1]), two(c));
     if (nonlinear) {
       const float inv_cap = mv.softcap > 0.f ? 1.f / mv.softcap : 0.f;
-#pragma unroll
-      for (int e = 0; e < CH; ++e) {
-        const float sx = x[e];
-        float out = fmaf(sx, mv.hscale_m1, sx), d = 1.f + mv.hscale_m1;
+      auto modify = [&](float sx, float& out, float& d) {
+        out = fmaf(sx, mv.hscale_m1, sx);
+        d = 1.f + mv.hscale_m1;
         if (mv.softcap > 0.f) {
           const float t = tanhf(sx * inv_cap);
           out += mv.softcap * t - sx;
           d -= t * t;
         }
-        x[e] = out;
-        g[e] = d;
+      };
+#pragma unroll
+      for (int i = 0; i < CH / 2; ++i) {
+        float2 o;
+        modify(x[i].x, o.x, g[i].x);
+        modify(x[i].y, o.y, g[i].y);
+        x[i] = o;
       }
     }
     if ((FEAT & 1) && mv.alibi_mode) {
       const float base = (float)(i0 - j0);
 #pragma unroll
-      for (int e = 0; e < CH; ++e) {
-        const float dist = ROWS ? base - (float)e : base + (float)e;  // i - j, exact
-        x[e] = fmaf(-mv.slope, mv.alibi_mode == 1 ? fmaxf(dist, 0.f) : fabsf(dist), x[e]);
+      for (int i = 0; i < CH / 2; ++i) {
+        const float e = 2.f * i;
+        float2 d = __fadd2_rn(two(base), ROWS ? make_float2(-e, -e - 1.f) : make_float2(e, e + 1.f));
+        d = mv.alibi_mode == 1 ? make_float2(fmaxf(d.x, 0.f), fmaxf(d.y, 0.f)) : make_float2(fabsf(d.x), fabsf(d.y));
+        x[i] = __ffma2_rn(d, two(-mv.slope), x[i]);
       }
     }
     if ((FEAT & 1) && mv.rel) {
+      auto entry = [&](int e) {  // clamped: rows and keys past the tensors
+        return __ldg(mv.rel + max(1 - pl.Lq, min(pl.Lkv - 1, ROWS ? j0 + e - i0 : j0 - i0 - e)));
+      };
 #pragma unroll
-      for (int e = 0; e < CH; ++e) {
-        const int t = ROWS ? j0 + e - i0 : j0 - i0 - e;
-        x[e] += __ldg(mv.rel + max(1 - pl.Lq, min(pl.Lkv - 1, t)));  // clamped: rows and keys past the tensors
-      }
+      for (int i = 0; i < CH / 2; ++i) x[i] = __fadd2_rn(x[i], make_float2(entry(2 * i), entry(2 * i + 1)));
     }
     if constexpr ((FEAT & 2) != 0) {
 #pragma unroll
-      for (int e = 0; e < CH; ++e) x[e] += bias[e];
+      for (int i = 0; i < CH / 2; ++i) x[i] = __fadd2_rn(x[i], make_float2(bias[2 * i], bias[2 * i + 1]));
     }
-    if ((FEAT & 4) && mv.drop_rate > 0.f) {
-      // dV sees the dropped, rescaled probabilities and dP is dropped the same way; delta includes it already
+    if ((FEAT & 2) || ((FEAT & 1) && mv.rel)) {
 #pragma unroll
-      for (int e = 0; e < CH; ++e) {
-        const float p = ex2_approx((x[e] - lse[ROWS ? 0 : e]) * kLog2e);
-        const float dm = mod_dropout(mv, ROWS ? i0 : i0 + e, ROWS ? j0 + e : j0);
-        pr[e] = p * dm;
-        ds[e] = p * fmaf(dp[e], dm, -delta[ROWS ? 0 : e]);
-      }
+      for (int i = 0; i < CH / 2; ++i) y[i] = __fmul2_rn(__fadd2_rn(x[i], neg(at(lse, 2 * i))), two(kLog2e));
     } else {
 #pragma unroll
-      for (int e = 0; e < CH; ++e) {
-        pr[e] = ex2_approx((x[e] - lse[ROWS ? 0 : e]) * kLog2e);
-        ds[e] = pr[e] * (dp[e] - delta[ROWS ? 0 : e]);
-      }
+      for (int i = 0; i < CH / 2; ++i) y[i] = __ffma2_rn(x[i], two(kLog2e), neg(at(lse, 2 * i)));
     }
-    if (nonlinear) {
+  }
 #pragma unroll
-      for (int e = 0; e < CH; ++e) ds[e] *= g[e];
+  for (int i = 0; i < CH / 2; ++i) pr[i] = make_float2(ex2_approx(y[i].x), ex2_approx(y[i].y));
+  if ((FEAT & 4) && mv.drop_rate > 0.f) {
+    // dV sees the dropped, rescaled probabilities and dP is dropped the same way; delta includes it already
+#pragma unroll
+    for (int i = 0; i < CH / 2; ++i) {
+      const int e = 2 * i;
+      const float2 dm = make_float2(mod_dropout(mv, ROWS ? i0 : i0 + e, ROWS ? j0 + e : j0),
+                                    mod_dropout(mv, ROWS ? i0 : i0 + e + 1, ROWS ? j0 + e + 1 : j0));
+      ds[i] = __fmul2_rn(pr[i], __ffma2_rn(make_float2(dp[e], dp[e + 1]), dm, neg(at(delta, e))));
+      pr[i] = __fmul2_rn(pr[i], dm);
     }
+  } else {
+#pragma unroll
+    for (int i = 0; i < CH / 2; ++i)
+      ds[i] = __fmul2_rn(pr[i], __fadd2_rn(make_float2(dp[2 * i], dp[2 * i + 1]), neg(at(delta, 2 * i))));
+  }
+  if (nonlinear) {
+#pragma unroll
+    for (int i = 0; i < CH / 2; ++i) ds[i] = __fmul2_rn(ds[i], g[i]);
   }
   if (keep != (1u << CH) - 1) {  // selects, not products: masked scores may be anything
 #pragma unroll
-    for (int e = 0; e < CH; ++e) {
-      const bool k = (keep >> e) & 1u;
-      pr[e] = k ? pr[e] : 0.f;
-      ds[e] = k ? ds[e] : 0.f;
+    for (int i = 0; i < CH / 2; ++i) {
+      const bool k0 = (keep >> (2 * i)) & 1u, k1 = (keep >> (2 * i + 1)) & 1u;
+      pr[i] = make_float2(k0 ? pr[i].x : 0.f, k1 ? pr[i].y : 0.f);
+      ds[i] = make_float2(k0 ? ds[i].x : 0.f, k1 ? ds[i].y : 0.f);
     }
   }
 }
@@ -506,7 +530,7 @@ bwd_dq_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     const int row = q0 + r_in;
     const bool row_ok = row < p.Lq;
     const uint32_t lane_sel = static_cast<uint32_t>(quarter * 32) << 16;
-    const float c = FEAT == 0 ? p.sm_scale * kLog2e : p.sm_scale;
+    const float c = p.sm_scale;
     const float pack = ds_pack_scale<DV, BF16>(a, p.mod);
     // padded per-row vectors: +inf / 0 for rows past Lq and +inf for rows without keys, so P = 0 there
     const int64_t at = ((int64_t)b * p.Hq + h) * p.Lq_pad + row;
@@ -558,7 +582,8 @@ bwd_dq_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
           tmem_ld16f(s_addr + (cc + 1) * CH, s_next);
           tmem_ld16f(dp_addr + (cc + 1) * CH, dp_next);
         }
-        float bias[CH], pr[CH], ds[CH];
+        float bias[CH];
+        float2 pr[CH / 2], ds[CH / 2];
         if constexpr ((FEAT & 2) != 0) {
           copy_wait<NB - 1>();
           __syncwarp();
@@ -796,7 +821,7 @@ bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
     const int r_in = quarter * 32 + lane;
     const int key = k0 + r_in;
     const uint32_t lane_sel = static_cast<uint32_t>(quarter * 32) << 16;
-    const float c = FEAT == 0 ? p.sm_scale * kLog2e : p.sm_scale;
+    const float c = p.sm_scale;
     const float pack = ds_pack_scale<DV, BF16>(a, p.mod);
     const uint32_t s_addr = T_S + lane_sel + grp * HALF, dp_addr = T_DP + lane_sel + grp * HALF;
     const Place pl = {kv_len, p.Lq, p.Lkv, p.band_lo, p.band_hi};
@@ -852,7 +877,8 @@ bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
       tmem_ld16f(dp_addr, dp_next);
 #pragma unroll(UNROLL<FEAT>)
       for (int cc = 0; cc < NCH; ++cc) {
-        float lse[CH], delta[CH], bias[CH], pr[CH], ds[CH];
+        float lse[CH], delta[CH], bias[CH];
+        float2 pr[CH / 2], ds[CH / 2];
 #pragma unroll
         for (int e = 0; e < CH; e += 4) {
           *reinterpret_cast<float4*>(lse + e) = *reinterpret_cast<const float4*>(lse_s + cc * CH + e);
@@ -1054,9 +1080,9 @@ bwd_dbias_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         for (int u = 0; u < 8; ++u) asm volatile("st.shared.f32 [%0], %1;" ::"r"(btile + (e + u) * BN * 4), "f"(t[u]) : "memory");
       }
     }
-    float acc[64];
+    float2 acc[32];
 #pragma unroll
-    for (int e = 0; e < 64; ++e) acc[e] = 0.f;
+    for (int i = 0; i < 32; ++i) acc[i] = make_float2(0.f, 0.f);
     int it = 0;
     bool ok = true;
     for (int pi = 0; pi < n_pairs; ++pi) {
@@ -1085,7 +1111,8 @@ bwd_dbias_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
       const float* delta_s = lse_s + BM;
 #pragma unroll
       for (int cc = 0; cc < 64 / CH; ++cc) {
-        float s[CH], dp[CH], lse[CH], delta[CH], bias[CH], pr[CH], ds[CH];
+        float s[CH], dp[CH], lse[CH], delta[CH], bias[CH];
+        float2 pr[CH / 2], ds[CH / 2];
         tmem_ld16f(s_addr + cc * CH, s);
         tmem_ld16f(dp_addr + cc * CH, dp);
 #pragma unroll
@@ -1101,7 +1128,7 @@ bwd_dbias_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         const uint32_t keep = keep_bits<FEAT, false>(pl, mv, mixed, own_seg, i0, key);
         chunk_p_ds<FEAT, false, false>(s, dp, p.sm_scale, pl, mv, keep, i0, key, lse, delta, bias, pr, ds);
 #pragma unroll
-        for (int e = 0; e < CH; ++e) acc[cc * CH + e] += ds[e];
+        for (int i = 0; i < CH / 2; ++i) acc[cc * CH / 2 + i] = __fadd2_rn(acc[cc * CH / 2 + i], ds[i]);
       }
       tc_fence_before();
       mbar_arrive(BAR(T_FREE + buf));
@@ -1111,7 +1138,7 @@ bwd_dbias_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
       float* dst = p.dbias + (int64_t)b0 * p.bias_bs + (int64_t)h0 * p.bias_hs + key;
 #pragma unroll
       for (int e = 0; e < 64; ++e)
-        if (i_first + e < p.Lq) dst[(int64_t)(i_first + e) * p.Lkv] = acc[e];
+        if (i_first + e < p.Lq) dst[(int64_t)(i_first + e) * p.Lkv] = e % 2 ? acc[e / 2].y : acc[e / 2].x;
     }
   }
 

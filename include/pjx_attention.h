@@ -398,6 +398,19 @@ int pjx_kv_cache_append(void* k_cache, void* v_cache, const void* k_new, const v
 int pjx_linear(const void* x, const void* w, void* y, int64_t M, int N, int K, int dtype, int impl,
                int32_t* status, void* stream);
 
+/* Two layers that share their input, y0 = x . w0^T and y1 = x . w1^T, in one launch where the tensor cores
+ * take them (the key and value up-projections of latent attention, latent_attention.py:396-410). */
+int pjx_linear_pair(const void* x, const void* w0, const void* w1, void* y0, void* y1, int64_t M, int N0,
+                    int N1, int K, int dtype, int32_t* status, void* stream);
+/* Gradients of pjx_linear_pair (N1 = 0: of pjx_linear): dx [M, K] = dy0 . w0 + dy1 . w1 in one
+ * accumulation, dw_p [N_p, K] = dy_p^T . x; outputs that are NULL are not computed.  The operands are read
+ * as they are stored, without transposed copies.  16-bit operands, M, N0, N1, K at least 64, N0, N1, K
+ * multiples of 8 and 16-byte aligned addresses; anything else is PJX_ERR_UNSUPPORTED (compose pjx_linear
+ * calls over transposed operands instead). */
+int pjx_linear_pair_bwd(const void* x, const void* w0, const void* w1, const void* dy0, const void* dy1,
+                        void* dx, void* dw0, void* dw1, int64_t M, int N0, int N1, int K, int dtype,
+                        int32_t* status, void* stream);
+
 /* pjx_linear on a column block of wider matrices: row i of x starts at x + i * x_row_pitch and row i
  * of y at y + i * y_row_pitch (pitches in elements).  One call per head applies a per-head weight
  * to a [.., H, K] activation without gathering it, e.g. the value up-projection folded onto the

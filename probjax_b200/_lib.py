@@ -74,6 +74,8 @@ SIGNATURES = {
                                            _vp, _sz, _i, _i, _vp, C.c_uint32, _i, _vp, _vp]),
     "pjx_attn_decode_sharded_buffer_bytes": (_sz, [_i, _i, _i, _i, _i]),
     "pjx_linear": (_i, [_vp, _vp, _vp, _i64, _i, _i, _i, _i, _vp, _vp]),
+    "pjx_linear_pair": (_i, [_vp, _vp, _vp, _vp, _vp, _i64, _i, _i, _i, _i, _vp, _vp]),
+    "pjx_linear_pair_bwd": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i, _i, _i, _i, _vp, _vp]),
     "pjx_linear_strided": (_i, [_vp, _i64, _vp, _vp, _i64, _i64, _i, _i, _i, _i, _vp, _vp]),
     "pjx_rms_norm": (_i, [_vp, _vp, _vp, _i64, _i, _f, _i, _vp]),
     "pjx_rope_interleaved": (_i, [_vp, _vp, _vp, _f, _i64, _i, _i, _i, _i, _f, _i, _vp]),

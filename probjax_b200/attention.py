@@ -894,10 +894,10 @@ def mla(q, cache, wk=None, wv=None, *, mask=None, bias=None, rng=None, sm_scale:
         if lm.q_limit is not None:
             raise NotImplementedError("gradients under a query-length mask are not implemented")
         if wk is not None:
-            from .cache import linear_autograd
+            from .cache import linear_pair_autograd
 
-            kmat = linear_autograd(cache, wk.reshape(H * Dqk, R)).view(B, S, H, Dqk)
-            vmat = linear_autograd(cache, wv.reshape(H * Dv, R)).view(B, S, H, Dv)
+            kmat, vmat = linear_pair_autograd(cache, wk.reshape(H * Dqk, R), wv.reshape(H * Dv, R))
+            kmat, vmat = kmat.view(B, S, H, Dqk), vmat.view(B, S, H, Dv)
         else:
             kmat = vmat = cache[:, :, None, :]  # one shared KV head
         out, lse = _AttentionFunction.apply(q, kmat, vmat, lm.band, lm.kv_lengths, bt, float(sm_scale), implementation,

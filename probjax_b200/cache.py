@@ -132,9 +132,34 @@ def linear(x: torch.Tensor, weight: torch.Tensor, *, implementation: str | None 
     return y.view(*x.shape[:-1], w.shape[0])
 
 
+def _linear_grads(x, weights, dys, want_dx: bool, want_dw):
+    """``(dx, [dw, ..])`` of one or two layers ``y_p = x . w_p^T`` sharing ``x [M, K]``: one launch for ``dx`` (summed
+    over the layers in fp32) and one for the weight gradients, on the operands as they are stored.  Operands the
+    tensor-core kernel does not take go through :func:`linear` and transposed copies."""
+    M, K = x.shape
+    ns = [w.shape[0] for w in weights]
+    ptrs = [x, *weights, *dys]
+    if (x.dtype != torch.float32 and M >= 64 and K >= 64 and K % 8 == 0 and all(n >= 64 and n % 8 == 0 for n in ns)
+            and all(t.data_ptr() % 16 == 0 for t in ptrs)):
+        dx = torch.empty_like(x) if want_dx else None
+        dws = [torch.empty_like(w) if need else None for w, need in zip(weights, want_dw)]
+        w1, dy1, dw1 = (weights[1], dys[1], dws[1]) if len(ns) > 1 else (None, None, None)
+        with torch.cuda.device(x.device):
+            rc = _lib.lib().pjx_linear_pair_bwd(_ptr(x), _ptr(weights[0]), _ptr(w1), _ptr(dys[0]), _ptr(dy1), _ptr(dx),
+                                                _ptr(dws[0]), _ptr(dw1), M, ns[0], ns[1] if len(ns) > 1 else 0, K,
+                                                _DTYPES[x.dtype], _ptr(_status_word(x.device)), _stream(x.device))
+        _lib.check(rc)
+        return dx, dws
+    dx = None
+    if want_dx:
+        parts = [linear(dy, w.t().contiguous()) for dy, w in zip(dys, weights)]      # [M, n] . [K, n]^T
+        dx = parts[0] if len(parts) == 1 else parts[0] + parts[1]
+    dws = [linear(dy.t().contiguous(), x.t().contiguous()) if need else None for dy, need in zip(dys, want_dw)]
+    return dx, dws
+
+
 class _LinearFunction(torch.autograd.Function):
-    """``linear`` with its gradients computed by the same kernel: ``dx = dy . w`` and ``dw = dy^T . x`` are
-    again products of the ``A . B^T`` form once the second operand is transposed (a copy)."""
+    """``linear`` with its gradients: ``dx = dy . w`` and ``dw = dy^T . x``."""
 
     @staticmethod
     def forward(ctx, x, weight):
@@ -144,19 +169,48 @@ class _LinearFunction(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, weight = ctx.saved_tensors
-        dx = dw = None
-        dy2 = dy.reshape(-1, dy.shape[-1]).to(x.dtype)
-        if ctx.needs_input_grad[0]:
-            dx = linear(dy2, weight.t().contiguous()).reshape(x.shape)          # [M, N] . [K, N]^T
-        if ctx.needs_input_grad[1]:
-            x2 = x.reshape(-1, x.shape[-1])
-            dw = linear(dy2.t().contiguous(), x2.t().contiguous())              # [N, M] . [K, M]^T
-        return dx, dw
+        dy2 = dy.reshape(-1, dy.shape[-1]).to(x.dtype).contiguous()
+        x2 = x.reshape(-1, x.shape[-1]).contiguous()
+        dx, (dw,) = _linear_grads(x2, [weight.contiguous()], [dy2], ctx.needs_input_grad[0], [ctx.needs_input_grad[1]])
+        return None if dx is None else dx.view(x.shape), dw
 
 
 def linear_autograd(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
-    """:func:`linear` that records itself for reverse-mode differentiation (both gradients on ``pjx_linear``)."""
+    """:func:`linear` that records itself for reverse-mode differentiation."""
     return _LinearFunction.apply(x, weight)
+
+
+class _LinearPairFunction(torch.autograd.Function):
+    """Two layers that share their input (keys and values of latent attention): one launch forward, and backward one
+    for the gradient of the input and one for both weight gradients."""
+
+    @staticmethod
+    def forward(ctx, x, w0, w1):
+        ctx.save_for_backward(x, w0, w1)
+        x2, w0, w1 = x.contiguous().view(-1, x.shape[-1]), w0.contiguous(), w1.contiguous()
+        y0, y1 = (torch.empty((x2.shape[0], w.shape[0]), dtype=x.dtype, device=x.device) for w in (w0, w1))
+        with torch.cuda.device(x.device):
+            rc = _lib.lib().pjx_linear_pair(_ptr(x2), _ptr(w0), _ptr(w1), _ptr(y0), _ptr(y1), x2.shape[0], w0.shape[0],
+                                            w1.shape[0], x2.shape[1], _DTYPES[x.dtype], _ptr(_status_word(x.device)),
+                                            _stream(x.device))
+        _lib.check(rc)
+        return y0.view(*x.shape[:-1], w0.shape[0]), y1.view(*x.shape[:-1], w1.shape[0])
+
+    @staticmethod
+    def backward(ctx, dy0, dy1):
+        x, w0, w1 = ctx.saved_tensors
+        dys = [dy.reshape(-1, dy.shape[-1]).to(x.dtype).contiguous() for dy in (dy0, dy1)]
+        x2 = x.reshape(-1, x.shape[-1]).contiguous()
+        dx, (dw0, dw1) = _linear_grads(x2, [w0.contiguous(), w1.contiguous()], dys, ctx.needs_input_grad[0],
+                                       ctx.needs_input_grad[1:3])
+        return None if dx is None else dx.view(x.shape), dw0, dw1
+
+
+def linear_pair_autograd(x: torch.Tensor, w0: torch.Tensor, w1: torch.Tensor):
+    """``(linear(x, w0), linear(x, w1))``, recorded for reverse-mode differentiation."""
+    if not x.is_cuda or x.shape[-1] != w0.shape[-1] or x.shape[-1] != w1.shape[-1] or not x.dtype == w0.dtype == w1.dtype:
+        raise ValueError("linear takes CUDA tensors x [..., K] and weight [N, K] of one dtype")
+    return _LinearPairFunction.apply(x, w0, w1)
 
 
 def decode_paged(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, block_table: torch.Tensor, kv_lengths,

@@ -995,6 +995,8 @@ EncodeTiledFn encode_fn() {
 
 // [B, L, H, Dim] row-major 16-bit tensor, box = 64 elements x 1 head x `rows` tokens.
 int make_tmap_blhd(CUtensorMap* m, const void* base, int dtype, int B, int L, int H, int Dim, int rows) {
+  const int rcb = bind_context();
+  if (rcb) return rcb;
   EncodeTiledFn fn = encode_fn();
   if (!fn) return fail(PJX_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
   cuuint64_t dims[4] = {(cuuint64_t)Dim, (cuuint64_t)H, (cuuint64_t)L, (cuuint64_t)B};

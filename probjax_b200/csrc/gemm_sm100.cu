@@ -269,6 +269,181 @@ gemm_tn_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
   }
 }
 
+// ---------------------------------------------------------------------------------------------
+// Gradients of one or two linear layers y_p = x . w_p^T that share x (the key and value up-projections of latent
+// attention).  Both are products whose second operand is stored with the contraction along its rows ("MN-major" for
+// the MMA unit), which TMA and the shared-memory descriptors take as it is -- transposed copies of the operands cost
+// more than the products themselves (B2 S2048 H16 latent step: 140 us of copies, 107 us of products).
+//   CHAIN:  dx [M, K]   = sum_p dy_p [M, n_p] . w_p [n_p, K]    one accumulation over both contractions
+//   else:   dw_p [n_p, K] = dy_p [M, n_p]^T . x [M, K]          the tiles of both products in one launch
+// Persistent CTAs over 128 x TN output tiles, a TMA lane, an MMA lane and four epilogue warps with the accumulator
+// double buffered, as above.  Tiles of 192 columns where they cover the width with less padding (576 = 3 x 192).
+// Measured there (both layers): dx 51 -> @DX@ us, dw 61 -> @DW@ us, and no copies.
+// ---------------------------------------------------------------------------------------------
+struct GradArgs {
+  void* c[2];      // CHAIN: c[0] only
+  int64_t m[2];    // rows of the outputs
+  int64_t k[2];    // contraction lengths
+  int n;           // columns of the outputs
+  int pairs;       // layers
+  int32_t* status;
+};
+
+template <int TN_>
+struct GradCfg {
+  static constexpr int BBYTES = TN_ * TK * 2;
+  static constexpr int ST = TN_ == 256 ? 4 : 5;
+  static constexpr int OFF_BAR = ST * (A_BYTES + BBYTES);
+  static constexpr int NBAR = 2 * ST + 4;
+  static constexpr int SMEM = OFF_BAR + NBAR * 8 + 16 + 1024;
+  static_assert(SMEM <= 227 * 1024, "shared memory budget");
+};
+
+template <bool BF16, bool CHAIN, int TN_>
+__global__ void __launch_bounds__(G_THREADS, 1)
+linear_grad_sm100_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_constant__ CUtensorMap tm_a1,
+                         const __grid_constant__ CUtensorMap tm_b0, const __grid_constant__ CUtensorMap tm_b1, const GradArgs g) {
+  using GC = GradCfg<TN_>;
+  constexpr int ST = GC::ST, STAGE = A_BYTES + GC::BBYTES;
+  extern __shared__ unsigned char smem_unaligned[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~uintptr_t(1023));
+  const uint32_t sbase = smem_u32(smem);
+  auto BAR = [&](int i) { return sbase + GC::OFF_BAR + 8u * i; };
+  const int FULL = 0, EMPTY = ST, ACC_FULL = 2 * ST, ACC_EMPTY = 2 * ST + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + GC::OFF_BAR + GC::NBAR * 8);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nt = (g.n + TN_ - 1) / TN_;
+  const int mt0 = (int)((g.m[0] + TM - 1) / TM), mt1 = (!CHAIN && g.pairs > 1) ? (int)((g.m[1] + TM - 1) / TM) : 0;
+  const int ntiles = (mt0 + mt1) * nt;
+  const int nk0 = (int)((g.k[0] + TK - 1) / TK), nk1 = g.pairs > 1 ? (int)((g.k[1] + TK - 1) / TK) : 0;
+  // tile -> (pair, row tile, column tile), columns fastest: the CTAs in flight share the A rows
+  auto decode = [&](int tile, int& which, int& m_idx, int& n_idx) {
+    m_idx = tile / nt;
+    n_idx = tile - m_idx * nt;
+    which = m_idx >= mt0;
+    if (which) m_idx -= mt0;
+  };
+  auto steps = [&](int which) { return CHAIN ? nk0 + nk1 : (which ? nk1 : nk0); };
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < GC::NBAR; ++i) mbar_init(BAR(i), i >= ACC_EMPTY ? 128u : 1u);
+    *abort_flag = 0;
+    fence_barrier_init();
+  }
+  if (warp == 0) {
+    tmem_alloc(smem_u32(tmem_slot), 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int it = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x) {
+        int which, m_idx, n_idx;
+        decode(tile, which, m_idx, n_idx);
+        const int nk = steps(which);
+        for (int k = 0; k < nk; ++k, ++it) {
+          const int s = it % ST;
+          const int pair = CHAIN ? k >= nk0 : which;
+          const int kr = (CHAIN && pair ? k - nk0 : k) * TK;  // first row of the contraction
+          const CUtensorMap* ta = pair ? &tm_a1 : &tm_a0;
+          const CUtensorMap* tb = pair ? &tm_b1 : &tm_b0;
+          ok = mbar_wait(BAR(EMPTY + s), ((it / ST) & 1) ^ 1, abort_flag);
+          if (!ok) break;
+          mbar_arrive_expect_tx(BAR(FULL + s), STAGE);
+          const uint32_t a = sbase + s * STAGE;
+          if constexpr (CHAIN) {
+            tma_load_2d(a, ta, BAR(FULL + s), kr, m_idx * TM);  // 128 rows x 64 of the contraction
+          } else {
+#pragma unroll
+            for (int blk = 0; blk < TM / 64; ++blk)  // 64 rows of the contraction x 64 output rows each
+              tma_load_2d(a + blk * (TK * 128), ta, BAR(FULL + s), m_idx * TM + blk * 64, kr);
+          }
+#pragma unroll
+          for (int blk = 0; blk < TN_ / 64; ++blk)
+            tma_load_2d(a + A_BYTES + blk * (TK * 128), tb, BAR(FULL + s), n_idx * TN_ + blk * 64, kr);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = make_idesc(TM, TN_, BF16, !CHAIN, true);
+      int it = 0, local = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x, ++local) {
+        int which, m_idx, n_idx;
+        decode(tile, which, m_idx, n_idx);
+        const int nk = steps(which), acc = local & 1;
+        ok = mbar_wait(BAR(ACC_EMPTY + acc), ((local >> 1) & 1) ^ 1, abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        for (int k = 0; k < nk; ++k, ++it) {
+          const int s = it % ST;
+          ok = mbar_wait(BAR(FULL + s), (it / ST) & 1, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t a = sbase + s * STAGE, bb = a + A_BYTES;
+#pragma unroll
+          for (int kk = 0; kk < TK / 16; ++kk)
+            mma_ss(tmem + acc * 256, CHAIN ? make_smem_desc(a + kk * 32, 16, 1024) : make_smem_desc(a + kk * 2048, TK * 128, 1024),
+                   make_smem_desc(bb + kk * 2048, TK * 128, 1024), idesc, (k | kk) != 0);
+          mma_commit(BAR(EMPTY + s));
+        }
+        if (ok) mma_commit(BAR(ACC_FULL + acc));
+      }
+    }
+  } else {
+    const int quarter = warp & 3;
+    int local = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x, ++local) {
+      const int acc = local & 1;
+      int which, m_idx, n_idx;
+      decode(tile, which, m_idx, n_idx);
+      ok = mbar_wait(BAR(ACC_FULL + acc), (local >> 1) & 1, abort_flag);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+      const int64_t row = (int64_t)m_idx * TM + quarter * 32 + lane;
+      const uint32_t taddr = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + acc * 256;
+#pragma unroll 2
+      for (int c = 0; c < TN_ / 32; ++c) {
+        float accv[32];
+        tmem_ld32f(taddr + c * 32, accv);
+        tmem_wait_ld();
+        const int col0 = n_idx * TN_ + c * 32;
+        if (row < (which ? g.m[1] : g.m[0])) {
+          uint4* dst = reinterpret_cast<uint4*>(static_cast<unsigned char*>(which ? g.c[1] : g.c[0]) + (row * g.n + col0) * 2);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {  // (the width is a multiple of 8: whole 16-byte units)
+            uint4 w;
+            w.x = gpack<BF16>(accv[8 * i + 0], accv[8 * i + 1]);
+            w.y = gpack<BF16>(accv[8 * i + 2], accv[8 * i + 3]);
+            w.z = gpack<BF16>(accv[8 * i + 4], accv[8 * i + 5]);
+            w.w = gpack<BF16>(accv[8 * i + 6], accv[8 * i + 7]);
+            if (col0 + 8 * i < g.n) dst[i] = w;
+          }
+        }
+      }
+      tc_fence_before();
+      mbar_arrive(BAR(ACC_EMPTY + acc));
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    __syncwarp();
+    tmem_dealloc(tmem, 512);
+    if (lane == 0 && *abort_flag && g.status) atomicExch(g.status, (int)PJX_ERR_DEVICE_TIMEOUT);
+  }
+}
+
 // CUDA-core fallback: 64 x 64 tile, 16-wide K slices, 4 x 4 outputs per thread.
 template <typename T>
 __global__ void __launch_bounds__(256) gemm_tn_simt_kernel(const T* __restrict__ A, const T* __restrict__ Bm,
@@ -344,6 +519,8 @@ int launch_simt(const void* A, const void* Bm, void* C, int64_t M, int N, int K,
 // Row-major [rows, cols] 16-bit matrix with a row pitch of `pitch` elements (0 = cols),
 // box = 64 columns x box_rows rows.
 int make_tmap_2d(CUtensorMap* m, const void* base, int dtype, int64_t rows, int64_t cols, int box_rows, int64_t pitch) {
+  int rc = bind_context();
+  if (rc) return rc;
   EncodeTiledFn fn = encode_fn2();
   if (!fn) return fail(PJX_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
   cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
@@ -432,6 +609,85 @@ int launch_gemm_tn2(const void* A, const void* B0, void* C0, int N0, const void*
   int rc = simt_by_dtype(A, B0, C0, M, N0, K, lda, ldc, dtype, stream);
   if (rc || !N1) return rc;
   return simt_by_dtype(A, B1, C1, M, N1, K, lda, N1, dtype, stream);
+}
+
+// Both gradients of the layers y_p = x . w_p^T; outputs that are null are not computed.  False: the caller's general
+// path (unaligned operands, widths that are no multiple of 8 or below 64, fp32).
+bool linear_grad_supported(const LinearGrad& l, int dtype) {
+  if (dtype != PJX_BF16 && dtype != PJX_F16) return false;
+  uintptr_t al = reinterpret_cast<uintptr_t>(l.x) | reinterpret_cast<uintptr_t>(l.dx);
+  if (l.M < 64 || l.M > 2147483647LL - TM || l.K < 64 || l.K % 8) return false;
+  for (int p = 0; p < l.pairs; ++p) {
+    if (l.n[p] < 64 || l.n[p] % 8) return false;
+    al |= reinterpret_cast<uintptr_t>(l.dy[p]) | reinterpret_cast<uintptr_t>(l.w[p]) | reinterpret_cast<uintptr_t>(l.dw[p]);
+  }
+  return (al & 15) == 0;
+}
+
+namespace {
+
+template <bool BF16, bool CHAIN, int TN_>
+int launch_grad_tiles(const CUtensorMap (&ta)[2], const CUtensorMap (&tb)[2], const GradArgs& g, cudaStream_t stream) {
+  auto kern = linear_grad_sm100_kernel<BF16, CHAIN, TN_>;
+  int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GradCfg<TN_>::SMEM),
+                      "cudaFuncSetAttribute(linear gradient)");
+  if (rc) return rc;
+  const int64_t mt = (g.m[0] + TM - 1) / TM + (!CHAIN && g.pairs > 1 ? (g.m[1] + TM - 1) / TM : 0);
+  const int64_t tiles = mt * ((g.n + TN_ - 1) / TN_);
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  kern<<<(unsigned)(tiles < sms ? tiles : sms), G_THREADS, GradCfg<TN_>::SMEM, stream>>>(ta[0], ta[1], tb[0], tb[1], g);
+  count_launch();
+  return check_cuda(cudaGetLastError(), "linear gradient launch");
+}
+
+template <bool CHAIN>
+int launch_grad(const CUtensorMap (&ta)[2], const CUtensorMap (&tb)[2], const GradArgs& g, int dtype, cudaStream_t stream) {
+  const bool narrow = (g.n + 191) / 192 * 192 < (g.n + 255) / 256 * 256;
+  if (dtype == PJX_BF16)
+    return narrow ? launch_grad_tiles<true, CHAIN, 192>(ta, tb, g, stream) : launch_grad_tiles<true, CHAIN, 256>(ta, tb, g, stream);
+  return narrow ? launch_grad_tiles<false, CHAIN, 192>(ta, tb, g, stream) : launch_grad_tiles<false, CHAIN, 256>(ta, tb, g, stream);
+}
+
+}  // namespace
+
+int launch_linear_grad(const LinearGrad& l, int dtype, int32_t* status, cudaStream_t stream) {
+  int rc;
+  CUtensorMap ta[2], tb[2];
+  GradArgs g = {};
+  g.n = l.K;
+  g.status = status;
+  if (l.dx) {
+    g.pairs = l.pairs;
+    g.c[0] = l.dx;
+    g.m[0] = l.M;
+    for (int p = 0; p < l.pairs; ++p) {
+      g.k[p] = l.n[p];
+      if ((rc = make_tmap_2d(&ta[p], l.dy[p], dtype, l.M, l.n[p], TM))) return rc;
+      if ((rc = make_tmap_2d(&tb[p], l.w[p], dtype, l.n[p], l.K, TK))) return rc;
+    }
+    if (l.pairs == 1) {
+      ta[1] = ta[0];
+      tb[1] = tb[0];
+    }
+    if ((rc = launch_grad<true>(ta, tb, g, dtype, stream))) return rc;
+  }
+  g.pairs = 0;
+  for (int p = 0; p < l.pairs; ++p) {
+    if (!l.dw[p]) continue;
+    g.c[g.pairs] = l.dw[p];
+    g.m[g.pairs] = l.n[p];
+    g.k[g.pairs] = l.M;
+    if ((rc = make_tmap_2d(&ta[g.pairs], l.dy[p], dtype, l.M, l.n[p], TK))) return rc;
+    if ((rc = make_tmap_2d(&tb[g.pairs], l.x, dtype, l.M, l.K, TK))) return rc;
+    ++g.pairs;
+  }
+  if (g.pairs == 0) return PJX_OK;
+  if (g.pairs == 1) {
+    ta[1] = ta[0];
+    tb[1] = tb[0];
+  }
+  return launch_grad<false>(ta, tb, g, dtype, stream);
 }
 
 int launch_gemm_tn(const void* A, const void* Bm, void* C, int64_t M, int N, int K, int dtype, int impl,

@@ -47,6 +47,14 @@ int validate_common(const void* q, const void* k, const void* v, const void* o, 
 }  // namespace
 
 // Validates a caller's pjx_score_mod and converts it to the kernels' form (null: no modifiers).
+int bind_context() {
+  static thread_local bool bound = false;
+  if (bound) return PJX_OK;
+  const int rc = check_cuda(cudaFree(nullptr), "initialise the device context");
+  bound = rc == PJX_OK;
+  return rc;
+}
+
 int convert_score_mod(const pjx_score_mod* m, ScoreMod* out) {
   *out = ScoreMod();
   if (!m) return PJX_OK;
@@ -230,6 +238,36 @@ int pjx_linear(const void* x, const void* w, void* y, int64_t M, int N, int K, i
   if (M == 0 || N == 0) return PJX_OK;
   if (!x || !w || !y) return fail(PJX_ERR_BAD_ARG, "linear: null buffer");
   return launch_gemm_tn2(x, w, y, N, nullptr, nullptr, 0, M, K, dtype, impl, status, static_cast<cudaStream_t>(stream));
+}
+
+int pjx_linear_pair(const void* x, const void* w0, const void* w1, void* y0, void* y1, int64_t M, int N0, int N1, int K, int dtype,
+                    int32_t* status, void* stream) {
+  if (dtype != PJX_F32 && dtype != PJX_BF16 && dtype != PJX_F16)
+    return fail(PJX_ERR_BAD_ARG, "dtype must be float32, bfloat16 or float16 (got code %d)", dtype);
+  if (M < 0 || N0 < 1 || N1 < 1 || K < 1) return fail(PJX_ERR_BAD_ARG, "linear_pair: negative dimension or an empty layer");
+  if (M == 0) return PJX_OK;
+  if (!x || !w0 || !w1 || !y0 || !y1) return fail(PJX_ERR_BAD_ARG, "linear_pair: null buffer");
+  return launch_gemm_tn2(x, w0, y0, N0, w1, y1, N1, M, K, dtype, PJX_IMPL_AUTO, status, static_cast<cudaStream_t>(stream));
+}
+
+int pjx_linear_pair_bwd(const void* x, const void* w0, const void* w1, const void* dy0, const void* dy1, void* dx, void* dw0,
+                        void* dw1, int64_t M, int N0, int N1, int K, int dtype, int32_t* status, void* stream) {
+  if (M < 0 || N0 < 1 || N1 < 0 || K < 1) return fail(PJX_ERR_BAD_ARG, "linear_pair_bwd: negative dimension or an empty layer");
+  if (!x || !w0 || !dy0 || (N1 > 0 && (!w1 || !dy1))) return fail(PJX_ERR_BAD_ARG, "linear_pair_bwd: null buffer");
+  LinearGrad l = {};
+  l.x = x;
+  l.dy[0] = dy0; l.dy[1] = dy1;
+  l.w[0] = w0; l.w[1] = w1;
+  l.dx = dx;
+  l.dw[0] = dw0; l.dw[1] = dw1;
+  l.M = M;
+  l.n[0] = N0; l.n[1] = N1;
+  l.K = K;
+  l.pairs = N1 > 0 ? 2 : 1;
+  if (!linear_grad_supported(l, dtype))
+    return fail(PJX_ERR_UNSUPPORTED, "linear_pair_bwd needs 16-bit operands at 16-byte aligned addresses, widths of at least 64 that are "
+                                     "multiples of 8 and at least 64 rows");
+  return launch_linear_grad(l, dtype, status, static_cast<cudaStream_t>(stream));
 }
 
 int pjx_linear_strided(const void* x, int64_t x_row_pitch, const void* w, void* y, int64_t y_row_pitch, int64_t M, int N,

@@ -201,6 +201,9 @@ int fail(int status, const char* fmt, ...);
 int convert_score_mod(const pjx_score_mod* m, ScoreMod* out);
 int check_cuda(cudaError_t e, const char* what);
 void count_launch(int n = 1);
+// Makes the current device's context current on this thread: cuTensorMapEncodeTiled is a driver call and fails on a
+// thread that has made no runtime call yet (the first call of an autograd worker thread).
+int bind_context();
 
 // ---------------------------------------------------------------------------
 // Launchers implemented in the kernel translation units. Each returns a
@@ -244,5 +247,18 @@ int launch_gemm_tn(const void* A, const void* Bm, void* C, int64_t M, int N, int
 int launch_gemm_tn2(const void* A, const void* B0, void* C0, int N0, const void* B1, void* C1, int N1,
                     int64_t M, int K, int dtype, int impl, int32_t* status, cudaStream_t stream,
                     int64_t lda = 0, int64_t ldc = 0);
+
+// Gradients of the layers y_p = x . w_p^T (p < pairs <= 2) from dy_p; null outputs are skipped.
+struct LinearGrad {
+  const void* x;      // [M, K]
+  const void* dy[2];  // [M, n_p]
+  const void* w[2];   // [n_p, K]
+  void* dx;           // [M, K]: summed over the layers
+  void* dw[2];        // [n_p, K]
+  int64_t M;
+  int n[2], K, pairs;
+};
+bool linear_grad_supported(const LinearGrad& l, int dtype);
+int launch_linear_grad(const LinearGrad& l, int dtype, int32_t* status, cudaStream_t stream);
 
 }  // namespace pjx

@@ -107,7 +107,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   using C = DqCfg<D>;
   extern __shared__ unsigned char smem_unaligned[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~uintptr_t(1023));
-  const uint32_t sbase = smem_u32(smem);
+  const uint32_t sbase = uniform(smem_u32(smem));
   const uint32_t bar0 = sbase + C::OFF_BAR;
   auto BAR = [&](int i) { return bar0 + 8u * i; };
   const int QDO_FULL = 0, K_FULL = 1, K_EMPTY = 3, V_FULL = 5, V_EMPTY = 7, SP_FULL = 9, DS_FULL = 11, DQ_FULL = 13,
@@ -115,7 +115,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::OFF_BAR + C::N_BAR * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform(static_cast<int>(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   const int n_qt = (p.Lq + BM - 1) / BM;
   int tile, pair;
   work_item(blockIdx.x, n_qt, p.Hq * p.B, order_w, tile, pair);
@@ -130,11 +130,11 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   const int kv_end = max(0, min(kv_len, min(q0 + BM, p.Lq) + p.band_hi));
   const int kv_begin = max(0, q0 + p.band_lo);
   const int j_lo = kv_begin / BN;
-  const int n = kv_begin < kv_end ? (kv_end + BN - 1) / BN - j_lo : 0;
+  const int n = uniform(kv_begin < kv_end ? (kv_end + BN - 1) / BN - j_lo : 0);
   // The last KV tile may reach past the valid length: dS is exactly 0 there, but those K rows may
   // hold anything and 0 x NaN inside dQ += dS.K is not 0. The producer warp clears them in shared
   // memory once the tile has landed; the MMA issuer waits for that before it uses the tile.
-  const int clean_j = (n > 0 && (j_lo + n) * BN > kv_len) ? n - 1 : -1;
+  const int clean_j = uniform((n > 0 && (j_lo + n) * BN > kv_len) ? n - 1 : -1);
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < C::N_BAR; ++i)
@@ -149,7 +149,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = uniform(*tmem_slot);
   const uint32_t T_S = tmem, T_DP = tmem + BN, T_DQ = tmem + 2 * BN;
 
   if (warp == 0) {
@@ -199,7 +199,8 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && n > 0) {
+    if (n > 0) {
+      const uint32_t leader = elect_leader();
       constexpr uint32_t idesc_s = make_idesc(BM, BN / 2, BF16, false, false);
       constexpr uint32_t idesc_q = make_idesc(BM, D, BF16, false, true);
       const uint32_t qa = sbase + C::OFF_Q, doa = sbase + C::OFF_DO;
@@ -212,14 +213,14 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
             mma_ss(T_S + half * 64, make_smem_desc(qa + s * BM * 128 + kk * 32, 16, 1024),
-                   make_smem_desc(ka + s * BN * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0);
+                   make_smem_desc(ka + s * BN * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0, leader);
 #pragma unroll
         for (int s = 0; s < C::SUB; ++s)
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
             mma_ss(T_DP + half * 64, make_smem_desc(doa + s * BM * 128 + kk * 32, 16, 1024),
-                   make_smem_desc(va + s * BN * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0);
-        mma_commit(BAR(SP_FULL + half));
+                   make_smem_desc(va + s * BN * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0, leader);
+        mma_commit(BAR(SP_FULL + half), leader);
       };
       // dQ += dS.K over one half: A = dS (16-bit pairs at the first 32 columns of the half of S),
       // B = the K tile read MN-major
@@ -228,48 +229,48 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
           mma_ts(T_DQ, T_S + half * 64 + kk * 8, make_smem_desc(ka + (half * 4 + kk) * 2048, BN * 128, 1024), idesc_q,
-                 (j | half | kk) != 0);
+                 (j | half | kk) != 0, leader);
       };
-      bool ok = mbar_wait(BAR(QDO_FULL), 0, abort_flag);
-      if (ok) ok = mbar_wait(BAR(K_FULL), 0, abort_flag);
-      if (ok && clean_j == 0) ok = mbar_wait(BAR(K_CLEAN), 0, abort_flag);
-      if (ok) ok = mbar_wait(BAR(V_FULL), 0, abort_flag);
+      bool ok = mbar_wait_all(BAR(QDO_FULL), 0, abort_flag);
+      if (ok) ok = mbar_wait_all(BAR(K_FULL), 0, abort_flag);
+      if (ok && clean_j == 0) ok = mbar_wait_all(BAR(K_CLEAN), 0, abort_flag);
+      if (ok) ok = mbar_wait_all(BAR(V_FULL), 0, abort_flag);
       if (ok) {
         tc_fence_after();
         issue_sdp(0, 0);
         issue_sdp(1, 0);
-        mma_commit(BAR(V_EMPTY));
+        mma_commit(BAR(V_EMPTY), leader);
       }
       for (int j = 0; ok && j < n; ++j) {
         const int st = j & 1;
         const bool next = j + 1 < n;
         PJX_BTRACE(0, j, 0);
-        ok = mbar_wait(BAR(DS_FULL + 0), j & 1, abort_flag);
+        ok = mbar_wait_all(BAR(DS_FULL + 0), j & 1, abort_flag);
         if (!ok) break;
         tc_fence_after();
         PJX_BTRACE(0, j, 1);
         issue_acc(0, j);
         if (next) {
-          ok = mbar_wait(BAR(K_FULL + (st ^ 1)), ((j + 1) >> 1) & 1, abort_flag);
-          if (ok && j + 1 == clean_j) ok = mbar_wait(BAR(K_CLEAN), 0, abort_flag);
-          if (ok) ok = mbar_wait(BAR(V_FULL + (st ^ 1)), ((j + 1) >> 1) & 1, abort_flag);
+          ok = mbar_wait_all(BAR(K_FULL + (st ^ 1)), ((j + 1) >> 1) & 1, abort_flag);
+          if (ok && j + 1 == clean_j) ok = mbar_wait_all(BAR(K_CLEAN), 0, abort_flag);
+          if (ok) ok = mbar_wait_all(BAR(V_FULL + (st ^ 1)), ((j + 1) >> 1) & 1, abort_flag);
           if (!ok) break;
           tc_fence_after();
           issue_sdp(0, j + 1);  // over dS of half 0, which the MMAs just issued consume first
         }
         PJX_BTRACE(0, j, 2);
-        ok = mbar_wait(BAR(DS_FULL + 1), j & 1, abort_flag);
+        ok = mbar_wait_all(BAR(DS_FULL + 1), j & 1, abort_flag);
         if (!ok) break;
         tc_fence_after();
         issue_acc(1, j);
-        mma_commit(BAR(K_EMPTY + st));
+        mma_commit(BAR(K_EMPTY + st), leader);
         if (next) {
           issue_sdp(1, j + 1);
-          mma_commit(BAR(V_EMPTY + (st ^ 1)));
+          mma_commit(BAR(V_EMPTY + (st ^ 1)), leader);
         }
         PJX_BTRACE(0, j, 3);
       }
-      if (ok) mma_commit(BAR(DQ_FULL));
+      if (ok) mma_commit(BAR(DQ_FULL), leader);
     }
   } else {
     // --------------------------------------------------------------- compute warps
@@ -374,7 +375,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   using C = DkvCfg<D>;
   extern __shared__ unsigned char smem_unaligned[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~uintptr_t(1023));
-  const uint32_t sbase = smem_u32(smem);
+  const uint32_t sbase = uniform(smem_u32(smem));
   const uint32_t bar0 = sbase + C::OFF_BAR;
   auto BAR = [&](int i) { return bar0 + 8u * i; };
   const int KV_FULL = 0, QDO_FULL = 1, QDO_EMPTY = 3, SP_FULL = 5, PDS_FULL = 7, ACC_FULL = 9;
@@ -382,7 +383,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* row_s = reinterpret_cast<float*>(smem + C::OFF_ROW);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform(static_cast<int>(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   int kt, pair;  // the first key tiles are seen by the most queries under a causal band
   work_item(blockIdx.x, (p.Lkv + BN - 1) / BN, p.Hkv * p.B, order_w, kt, pair);
   const int hk = pair % p.Hkv, b = pair / p.Hkv;
@@ -396,7 +397,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   const int q_end = min(p.Lq, min(k0 + BN, kv_len) - p.band_lo);
   const int t_lo = q_begin / BM;
   const int n_t = (k0 < kv_len && q_begin < q_end) ? (q_end + BM - 1) / BM - t_lo : 0;
-  const int n = n_t * G;  // steps: query heads of the group outer, query tiles inner
+  const int n = uniform(n_t * G);  // steps: query heads of the group outer, query tiles inner
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < C::N_BAR; ++i)
@@ -411,7 +412,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = uniform(*tmem_slot);
   const uint32_t T_S = tmem, T_DP = tmem + BM, T_DV = tmem + 2 * BM, T_DK = tmem + 2 * BM + D;
 
   if (warp == 0) {
@@ -446,7 +447,8 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && n > 0) {
+    if (n > 0) {
+      const uint32_t leader = elect_leader();
       constexpr uint32_t idesc_s = make_idesc(BN, BM / 2, BF16, false, false);
       constexpr uint32_t idesc_acc = make_idesc(BN, D, BF16, false, true);
       const uint32_t ka = sbase + C::OFF_K, va = sbase + C::OFF_V;
@@ -460,14 +462,14 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
             mma_ss(T_S + half * 64, make_smem_desc(ka + s * BN * 128 + kk * 32, 16, 1024),
-                   make_smem_desc(qa + s * BM * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0);
+                   make_smem_desc(qa + s * BM * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0, leader);
 #pragma unroll
         for (int s = 0; s < C::SUB; ++s)
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
             mma_ss(T_DP + half * 64, make_smem_desc(va + s * BN * 128 + kk * 32, 16, 1024),
-                   make_smem_desc(doa + s * BM * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0);
-        mma_commit(BAR(SP_FULL + half));
+                   make_smem_desc(doa + s * BM * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0, leader);
+        mma_commit(BAR(SP_FULL + half), leader);
       };
       // dV += P^T.dO and dK += dS^T.Q over one half: A from tensor memory (16-bit pairs at the
       // first 32 columns of the half), dO / Q tiles read MN-major
@@ -476,14 +478,14 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
           mma_ts(T_DV, T_S + half * 64 + kk * 8, make_smem_desc(doa + (half * 4 + kk) * 2048, BM * 128, 1024), idesc_acc,
-                 (it | half | kk) != 0);
+                 (it | half | kk) != 0, leader);
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
           mma_ts(T_DK, T_DP + half * 64 + kk * 8, make_smem_desc(qa + (half * 4 + kk) * 2048, BM * 128, 1024), idesc_acc,
-                 (it | half | kk) != 0);
+                 (it | half | kk) != 0, leader);
       };
-      bool ok = mbar_wait(BAR(KV_FULL), 0, abort_flag);
-      if (ok) ok = mbar_wait(BAR(QDO_FULL), 0, abort_flag);
+      bool ok = mbar_wait_all(BAR(KV_FULL), 0, abort_flag);
+      if (ok) ok = mbar_wait_all(BAR(QDO_FULL), 0, abort_flag);
       if (ok) {
         tc_fence_after();
         issue_sdp(0, 0);
@@ -493,27 +495,27 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         const int st = it & 1;
         const bool next = it + 1 < n;
         PJX_KTRACE(0, it, 0);
-        ok = mbar_wait(BAR(PDS_FULL + 0), it & 1, abort_flag);
+        ok = mbar_wait_all(BAR(PDS_FULL + 0), it & 1, abort_flag);
         if (!ok) break;
         tc_fence_after();
         PJX_KTRACE(0, it, 1);
         issue_acc(0, it);
         if (next) {
-          ok = mbar_wait(BAR(QDO_FULL + (st ^ 1)), ((it + 1) >> 1) & 1, abort_flag);
+          ok = mbar_wait_all(BAR(QDO_FULL + (st ^ 1)), ((it + 1) >> 1) & 1, abort_flag);
           if (!ok) break;
           tc_fence_after();
           issue_sdp(0, it + 1);  // over P^T / dS^T of half 0, which the MMAs just issued consume first
         }
         PJX_KTRACE(0, it, 2);
-        ok = mbar_wait(BAR(PDS_FULL + 1), it & 1, abort_flag);
+        ok = mbar_wait_all(BAR(PDS_FULL + 1), it & 1, abort_flag);
         if (!ok) break;
         tc_fence_after();
         issue_acc(1, it);
-        mma_commit(BAR(QDO_EMPTY + st));
+        mma_commit(BAR(QDO_EMPTY + st), leader);
         if (next) issue_sdp(1, it + 1);
         PJX_KTRACE(0, it, 3);
       }
-      if (ok) mma_commit(BAR(ACC_FULL));
+      if (ok) mma_commit(BAR(ACC_FULL), leader);
     }
   } else {
     // --------------------------------------------------------------- compute warps

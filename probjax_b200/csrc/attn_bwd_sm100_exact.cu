@@ -361,7 +361,7 @@ bwd_dq_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
   using C = DqCfg<D, DV, FEAT>;
   extern __shared__ unsigned char smem_unaligned[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~uintptr_t(1023));
-  const uint32_t sbase = smem_u32(smem);
+  const uint32_t sbase = uniform(smem_u32(smem));
   const uint32_t bar0 = sbase + C::OFF_BAR;
   auto BAR = [&](int i) { return bar0 + 8u * i; };
   const int QDO_FULL = 0, K_FULL = 1, K_EMPTY = 3, V_FULL = 5, V_EMPTY = 7, SP_FULL = 9, DS_FULL = 11, DQ_FULL = 13,
@@ -369,7 +369,7 @@ bwd_dq_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::OFF_BAR + C::N_BAR * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform(static_cast<int>(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   const int n_qt = (p.Lq + BM - 1) / BM;
   int tile, pair;
   work_item(blockIdx.x, n_qt, p.Hq * p.B, a.order_w, tile, pair);
@@ -398,8 +398,8 @@ bwd_dq_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     }
   }
   const int j_lo = kv_begin / BN;
-  const int n = kv_begin < kv_end ? (kv_end + BN - 1) / BN - j_lo : 0;
-  const int clean_j = (n > 0 && (j_lo + n) * BN > kv_len) ? n - 1 : -1;  // a last tile with rows past the valid length
+  const int n = uniform(kv_begin < kv_end ? (kv_end + BN - 1) / BN - j_lo : 0);
+  const int clean_j = uniform((n > 0 && (j_lo + n) * BN > kv_len) ? n - 1 : -1);  // a last tile with rows past the valid length
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < C::N_BAR; ++i)
@@ -414,7 +414,7 @@ bwd_dq_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = uniform(*tmem_slot);
   const uint32_t T_S = tmem, T_DP = tmem + BN, T_DQ = tmem + 2 * BN;
 
   if (warp == 0) {
@@ -454,7 +454,8 @@ bwd_dq_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && n > 0) {
+    if (n > 0) {
+      const uint32_t leader = elect_leader();
       constexpr uint32_t idesc_s = make_idesc(BM, BN / 2, BF16, false, false);
       constexpr uint32_t idesc_q = make_idesc(BM, D, BF16, false, true);
       const uint32_t qa = sbase + C::OFF_Q, doa = sbase + C::OFF_DO;
@@ -467,14 +468,14 @@ bwd_dq_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
             mma_ss(T_S + half * 64, make_smem_desc(qa + s * BM * 128 + kk * 32, 16, 1024),
-                   make_smem_desc(ka + s * BN * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0);
+                   make_smem_desc(ka + s * BN * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0, leader);
 #pragma unroll
         for (int s = 0; s < C::SUBV; ++s)
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
             mma_ss(T_DP + half * 64, make_smem_desc(doa + s * BM * 128 + kk * 32, 16, 1024),
-                   make_smem_desc(va + s * BN * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0);
-        mma_commit(BAR(SP_FULL + half));
+                   make_smem_desc(va + s * BN * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0, leader);
+        mma_commit(BAR(SP_FULL + half), leader);
       };
       // dQ += (hi + lo of dS).K over one half, the K tile read MN-major
       auto issue_acc = [&](int half, int j) {
@@ -482,45 +483,45 @@ bwd_dq_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
           const uint64_t kd = make_smem_desc(ka + (half * 4 + kk) * 2048, BN * 128, 1024);
-          mma_ts(T_DQ, T_S + half * 64 + kk * CH, kd, idesc_q, (j | half | kk) != 0);
-          mma_ts(T_DQ, T_S + half * 64 + kk * CH + CH / 2, kd, idesc_q, true);
+          mma_ts(T_DQ, T_S + half * 64 + kk * CH, kd, idesc_q, (j | half | kk) != 0, leader);
+          mma_ts(T_DQ, T_S + half * 64 + kk * CH + CH / 2, kd, idesc_q, true, leader);
         }
       };
-      bool ok = mbar_wait(BAR(QDO_FULL), 0, abort_flag);
-      if (ok) ok = mbar_wait(BAR(K_FULL), 0, abort_flag);
-      if (ok && clean_j == 0) ok = mbar_wait(BAR(K_CLEAN), 0, abort_flag);
-      if (ok) ok = mbar_wait(BAR(V_FULL), 0, abort_flag);
+      bool ok = mbar_wait_all(BAR(QDO_FULL), 0, abort_flag);
+      if (ok) ok = mbar_wait_all(BAR(K_FULL), 0, abort_flag);
+      if (ok && clean_j == 0) ok = mbar_wait_all(BAR(K_CLEAN), 0, abort_flag);
+      if (ok) ok = mbar_wait_all(BAR(V_FULL), 0, abort_flag);
       if (ok) {
         tc_fence_after();
         issue_sdp(0, 0);
         issue_sdp(1, 0);
-        mma_commit(BAR(V_EMPTY));
+        mma_commit(BAR(V_EMPTY), leader);
       }
       for (int j = 0; ok && j < n; ++j) {
         const bool next = j + 1 < n;
-        ok = mbar_wait(BAR(DS_FULL + 0), j & 1, abort_flag);
+        ok = mbar_wait_all(BAR(DS_FULL + 0), j & 1, abort_flag);
         if (!ok) break;
         tc_fence_after();
         issue_acc(0, j);
         if (next) {
-          ok = mbar_wait(BAR(K_FULL + (j + 1) % C::KST), ((j + 1) / C::KST) & 1, abort_flag);
-          if (ok && j + 1 == clean_j) ok = mbar_wait(BAR(K_CLEAN), 0, abort_flag);
-          if (ok) ok = mbar_wait(BAR(V_FULL + (j + 1) % C::VST), ((j + 1) / C::VST) & 1, abort_flag);
+          ok = mbar_wait_all(BAR(K_FULL + (j + 1) % C::KST), ((j + 1) / C::KST) & 1, abort_flag);
+          if (ok && j + 1 == clean_j) ok = mbar_wait_all(BAR(K_CLEAN), 0, abort_flag);
+          if (ok) ok = mbar_wait_all(BAR(V_FULL + (j + 1) % C::VST), ((j + 1) / C::VST) & 1, abort_flag);
           if (!ok) break;
           tc_fence_after();
           issue_sdp(0, j + 1);  // over dS of half 0, which the MMAs just issued consume first
         }
-        ok = mbar_wait(BAR(DS_FULL + 1), j & 1, abort_flag);
+        ok = mbar_wait_all(BAR(DS_FULL + 1), j & 1, abort_flag);
         if (!ok) break;
         tc_fence_after();
         issue_acc(1, j);
-        mma_commit(BAR(K_EMPTY + j % C::KST));
+        mma_commit(BAR(K_EMPTY + j % C::KST), leader);
         if (next) {
           issue_sdp(1, j + 1);
-          mma_commit(BAR(V_EMPTY + (j + 1) % C::VST));
+          mma_commit(BAR(V_EMPTY + (j + 1) % C::VST), leader);
         }
       }
-      if (ok) mma_commit(BAR(DQ_FULL));
+      if (ok) mma_commit(BAR(DQ_FULL), leader);
     }
   } else {
     // --------------------------------------------------------------- compute warps
@@ -661,7 +662,7 @@ bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
   constexpr int QT = C::QT, HALF = C::HALF, NCH = HALF / CH;
   extern __shared__ __align__(128) unsigned char smem_unaligned[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~uintptr_t(1023));
-  const uint32_t sbase = smem_u32(smem);
+  const uint32_t sbase = uniform(smem_u32(smem));
   const uint32_t bar0 = sbase + C::OFF_BAR;
   auto BAR = [&](int i) { return bar0 + 8u * i; };
   const int KV_FULL = 0, QDO_FULL = 1, QDO_EMPTY = 3, SP_FULL = 5, PDS_FULL = 7, ACC_FULL = 9;
@@ -669,7 +670,7 @@ bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* row_s = reinterpret_cast<float*>(smem + C::OFF_ROW);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform(static_cast<int>(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   int kt, pair;  // the first key tiles are seen by the most queries under a causal band
   work_item(blockIdx.x, (p.Lkv + BN - 1) / BN, p.Hkv * p.B, a.order_w, kt, pair);
   const int hk = pair % p.Hkv, b = pair / p.Hkv;
@@ -694,7 +695,7 @@ bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
   }
   const int t_lo = q_begin / QT;
   const int n_t = (k0 < kv_len && q_begin < q_end) ? (q_end + QT - 1) / QT - t_lo : 0;
-  const int n = n_t * G;  // steps: query heads of the group outer, query tiles inner
+  const int n = uniform(n_t * G);  // steps: query heads of the group outer, query tiles inner
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < C::N_BAR; ++i)
@@ -709,7 +710,7 @@ bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = uniform(*tmem_slot);
   const uint32_t T_S = tmem, T_DP = tmem + QT, T_DV = tmem + 2 * QT, T_DK = tmem + 2 * QT + DV;
 
   if (warp == 0) {
@@ -746,7 +747,8 @@ bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && n > 0) {
+    if (n > 0) {
+      const uint32_t leader = elect_leader();
       constexpr uint32_t idesc_s = make_idesc(BN, HALF, BF16, false, false);
       constexpr uint32_t idesc_v = make_idesc(BN, DV, BF16, false, true);
       constexpr uint32_t idesc_k = make_idesc(BN, D, BF16, false, true);
@@ -760,14 +762,14 @@ bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
             mma_ss(T_S + half * HALF, make_smem_desc(ka + s * BN * 128 + kk * 32, 16, 1024),
-                   make_smem_desc(qa + s * QT * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0);
+                   make_smem_desc(qa + s * QT * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0, leader);
 #pragma unroll
         for (int s = 0; s < C::SUBV; ++s)
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
             mma_ss(T_DP + half * HALF, make_smem_desc(va + s * BN * 128 + kk * 32, 16, 1024),
-                   make_smem_desc(doa + s * QT * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0);
-        mma_commit(BAR(SP_FULL + half));
+                   make_smem_desc(doa + s * QT * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0, leader);
+        mma_commit(BAR(SP_FULL + half), leader);
       };
       // dV += (hi + lo of P^T).dO and dK += (hi + lo of dS^T).Q over one half, dO / Q tiles read MN-major
       auto issue_acc = [&](int half, int it) {
@@ -775,18 +777,18 @@ bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
 #pragma unroll
         for (int kk = 0; kk < NCH; ++kk) {
           const uint64_t dd = make_smem_desc(doa + (half * NCH + kk) * 2048, QT * 128, 1024);
-          mma_ts(T_DV, T_S + half * HALF + kk * CH, dd, idesc_v, (it | half | kk) != 0);
-          mma_ts(T_DV, T_S + half * HALF + kk * CH + CH / 2, dd, idesc_v, true);
+          mma_ts(T_DV, T_S + half * HALF + kk * CH, dd, idesc_v, (it | half | kk) != 0, leader);
+          mma_ts(T_DV, T_S + half * HALF + kk * CH + CH / 2, dd, idesc_v, true, leader);
         }
 #pragma unroll
         for (int kk = 0; kk < NCH; ++kk) {
           const uint64_t qd = make_smem_desc(qa + (half * NCH + kk) * 2048, QT * 128, 1024);
-          mma_ts(T_DK, T_DP + half * HALF + kk * CH, qd, idesc_k, (it | half | kk) != 0);
-          mma_ts(T_DK, T_DP + half * HALF + kk * CH + CH / 2, qd, idesc_k, true);
+          mma_ts(T_DK, T_DP + half * HALF + kk * CH, qd, idesc_k, (it | half | kk) != 0, leader);
+          mma_ts(T_DK, T_DP + half * HALF + kk * CH + CH / 2, qd, idesc_k, true, leader);
         }
       };
-      bool ok = mbar_wait(BAR(KV_FULL), 0, abort_flag);
-      if (ok) ok = mbar_wait(BAR(QDO_FULL), 0, abort_flag);
+      bool ok = mbar_wait_all(BAR(KV_FULL), 0, abort_flag);
+      if (ok) ok = mbar_wait_all(BAR(QDO_FULL), 0, abort_flag);
       if (ok) {
         tc_fence_after();
         issue_sdp(0, 0);
@@ -795,24 +797,24 @@ bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
       for (int it = 0; ok && it < n; ++it) {
         const int st = it & 1;
         const bool next = it + 1 < n;
-        ok = mbar_wait(BAR(PDS_FULL + 0), it & 1, abort_flag);
+        ok = mbar_wait_all(BAR(PDS_FULL + 0), it & 1, abort_flag);
         if (!ok) break;
         tc_fence_after();
         issue_acc(0, it);
         if (next) {
-          ok = mbar_wait(BAR(QDO_FULL + (st ^ 1)), ((it + 1) >> 1) & 1, abort_flag);
+          ok = mbar_wait_all(BAR(QDO_FULL + (st ^ 1)), ((it + 1) >> 1) & 1, abort_flag);
           if (!ok) break;
           tc_fence_after();
           issue_sdp(0, it + 1);  // over P^T / dS^T of half 0, which the MMAs just issued consume first
         }
-        ok = mbar_wait(BAR(PDS_FULL + 1), it & 1, abort_flag);
+        ok = mbar_wait_all(BAR(PDS_FULL + 1), it & 1, abort_flag);
         if (!ok) break;
         tc_fence_after();
         issue_acc(1, it);
-        mma_commit(BAR(QDO_EMPTY + st));
+        mma_commit(BAR(QDO_EMPTY + st), leader);
         if (next) issue_sdp(1, it + 1);
       }
-      if (ok) mma_commit(BAR(ACC_FULL));
+      if (ok) mma_commit(BAR(ACC_FULL), leader);
     }
   } else {
     // --------------------------------------------------------------- compute warps
@@ -971,7 +973,7 @@ bwd_dbias_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
   using C = DbCfg<D, DV>;
   extern __shared__ unsigned char smem_unaligned[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~uintptr_t(1023));
-  const uint32_t sbase = smem_u32(smem);
+  const uint32_t sbase = uniform(smem_u32(smem));
   const uint32_t bar0 = sbase + C::OFF_BAR;
   auto BAR = [&](int i) { return bar0 + 8u * i; };
   const int FULL = 0, EMPTY = C::NST, ROW_FULL = 2 * C::NST, SP_FULL = ROW_FULL + 2, T_FREE = SP_FULL + 2;
@@ -979,7 +981,7 @@ bwd_dbias_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* row_s = reinterpret_cast<float*>(smem + C::OFF_ROW);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform(static_cast<int>(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   const int n_kt = (p.Lkv + BN - 1) / BN, n_qt = (p.Lq + BM - 1) / BM;
   const int k0 = (int)(blockIdx.x % n_kt) * BN, q0 = (int)(blockIdx.x / n_kt % n_qt) * BM;
   const int plane = blockIdx.x / (n_kt * n_qt);  // (batch, head) plane of the bias
@@ -1004,7 +1006,7 @@ bwd_dbias_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = uniform(*tmem_slot);
 
   // every role walks the pairs the same way; `it` counts those with a valid key in the tile
   if (warp == 0) {
@@ -1036,30 +1038,31 @@ bwd_dbias_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      const uint32_t leader = elect_leader();
       constexpr uint32_t idesc = make_idesc(BN, BM, BF16, false, false);
       int it = 0;
       for (int pi = 0; pi < n_pairs; ++pi) {
-        if (k0 >= len_of(b0 + pi / nh)) continue;
+        if (uniform(static_cast<int>(k0 >= len_of(b0 + pi / nh)))) continue;
         const int st = it % C::NST, buf = it & 1;
         const uint32_t sa = sbase + st * C::STAGE;
-        if (!mbar_wait(BAR(FULL + st), (it / C::NST) & 1, abort_flag)) break;
-        if (!mbar_wait(BAR(T_FREE + buf), ((it >> 1) & 1) ^ 1, abort_flag)) break;
+        if (!mbar_wait_all(BAR(FULL + st), (it / C::NST) & 1, abort_flag)) break;
+        if (!mbar_wait_all(BAR(T_FREE + buf), ((it >> 1) & 1) ^ 1, abort_flag)) break;
         tc_fence_after();
 #pragma unroll
         for (int s = 0; s < C::SUBQ; ++s)
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
             mma_ss(tmem + buf * 256, make_smem_desc(sa + C::TQ + s * BN * 128 + kk * 32, 16, 1024),
-                   make_smem_desc(sa + s * BM * 128 + kk * 32, 16, 1024), idesc, (s | kk) != 0);
+                   make_smem_desc(sa + s * BM * 128 + kk * 32, 16, 1024), idesc, (s | kk) != 0, leader);
 #pragma unroll
         for (int s = 0; s < C::SUBV; ++s)
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
             mma_ss(tmem + buf * 256 + 128, make_smem_desc(sa + 2 * C::TQ + C::TV + s * BN * 128 + kk * 32, 16, 1024),
-                   make_smem_desc(sa + 2 * C::TQ + s * BM * 128 + kk * 32, 16, 1024), idesc, (s | kk) != 0);
-        mma_commit(BAR(EMPTY + st));
-        mma_commit(BAR(SP_FULL + buf));
+                   make_smem_desc(sa + 2 * C::TQ + s * BM * 128 + kk * 32, 16, 1024), idesc, (s | kk) != 0, leader);
+        mma_commit(BAR(EMPTY + st), leader);
+        mma_commit(BAR(SP_FULL + buf), leader);
         ++it;
       }
     }

@@ -80,14 +80,6 @@ struct TCfg {
   static_assert(SMEM <= 227 * 1024, "shared memory budget");
 };
 
-__device__ __forceinline__ void tmem_ld16f(uint32_t taddr, float* r) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-      : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7]), "=f"(r[8]),
-        "=f"(r[9]), "=f"(r[10]), "=f"(r[11]), "=f"(r[12]), "=f"(r[13]), "=f"(r[14]), "=f"(r[15])
-      : "r"(taddr)
-      : "memory");
-}
 __device__ __forceinline__ void tmem_st16f(uint32_t taddr, const float* r) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(taddr),
@@ -141,7 +133,7 @@ decode_latent_tc_kernel(const __grid_constant__ CUtensorMap tm_c, const DecodePa
   constexpr int NSUB = C::NSUB, NBLK = C::NBLK;
   extern __shared__ unsigned char smem_unaligned[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~uintptr_t(1023));
-  const uint32_t sbase = smem_u32(smem);
+  const uint32_t sbase = uniform(smem_u32(smem));
   const uint32_t bar0 = sbase + C::OFF_BAR;
   auto BAR = [&](int i) { return bar0 + 8u * i; };
   // barrier indices
@@ -171,9 +163,9 @@ decode_latent_tc_kernel(const __grid_constant__ CUtensorMap tm_c, const DecodePa
   // the combine of the splits, next on the stream, may become resident as SM slots free up (it waits
   // for this grid before it reads a partial)
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-  const int n_tiles = (end - start + TK - 1) / TK;
+  const int n_tiles = uniform((end - start + TK - 1) / TK);
   const int last_rows = end - start - (n_tiles - 1) * TK;  // valid rows of the last tile, 1 .. 128
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   const int G = p.Hq / p.Hkv;  // heads per row group
 
   if (tid == 0) {
@@ -205,7 +197,7 @@ decode_latent_tc_kernel(const __grid_constant__ CUtensorMap tm_c, const DecodePa
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = uniform(*tmem_slot);
   const int row0 = (int)((int64_t)b * p.capacity + start);  // row of the 2-D view [B * capacity, R]
 
   if (warp == 0) {
@@ -260,7 +252,8 @@ decode_latent_tc_kernel(const __grid_constant__ CUtensorMap tm_c, const DecodePa
     }
   } else if (warp == 1) {
     // ------------------------------------------------------ MMA issuer, scores
-    if (lane == 0) {
+    {
+      const uint32_t leader = elect_leader();
       constexpr uint32_t idesc_s = make_idesc(TK, NROW, BF16, false, false);
       // descriptors differ only in the address field (bits 0-13, address >> 4): add to a base.  The address is
       // masked to the 18 bits of the field (bits above them would spill into the leading-offset field)
@@ -269,50 +262,51 @@ decode_latent_tc_kernel(const __grid_constant__ CUtensorMap tm_c, const DecodePa
       bool ok = true;
       for (int t = 0, n = 0; t < n_tiles && ok; ++t) {
         if (t >= 2) {  // S^T[t % 2] is free once every softmax thread has written P(t - 2)
-          ok = mbar_wait(BAR(P_FULL + (t & 1)), ((t - 2) >> 1) & 1, abort_flag);
+          ok = mbar_wait_all(BAR(P_FULL + (t & 1)), ((t - 2) >> 1) & 1, abort_flag);
           if (!ok) break;
           tc_fence_after();
         }
         for (int i = 0; i < NSUB; ++i, ++n) {
           const int s = n % NQ;
-          ok = mbar_wait(BAR(QF + s), (n / NQ) & 1, abort_flag);
+          ok = mbar_wait_all(BAR(QF + s), (n / NQ) & 1, abort_flag);
           if (!ok) break;
           tc_fence_after();
           const uint64_t ca = kdesc + (ring16 + s * (SUB_BYTES >> 4)), qa = kdesc + (q16 + i * (2048 >> 4));
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk) mma_ss(tmem + (t & 1) * 16, ca + kk * 2, qa + kk * 2, idesc_s, (i | kk) != 0);
-          mma_commit(BAR(QE + s));  // the slot is free again after its four MMAs
+          for (int kk = 0; kk < 4; ++kk) mma_ss(tmem + (t & 1) * 16, ca + kk * 2, qa + kk * 2, idesc_s, (i | kk) != 0, leader);
+          mma_commit(BAR(QE + s), leader);  // the slot is free again after its four MMAs
         }
-        if (ok) mma_commit(BAR(S_FULL + (t & 1)));
+        if (ok) mma_commit(BAR(S_FULL + (t & 1)), leader);
       }
     }
   } else if (warp == 7) {
     // ------------------------------------------------------ MMA issuer, output
-    if (lane == 0) {
+    {
+      const uint32_t leader = elect_leader();
       constexpr uint32_t idesc_o = make_idesc(128, NROW, BF16, true, false);
       const uint64_t adesc = make_smem_desc(0, SUB_BYTES, 1024), bdesc = make_smem_desc(0, 16, 1024);
       const uint32_t ring16 = ((sbase + C::OFF_PRING) & 0x3FFFF) >> 4, p16 = ((sbase + C::OFF_P) & 0x3FFFF) >> 4;
       bool ok = true;
       for (int t = 0, n = 0; t < n_tiles && ok; ++t) {
-        ok = mbar_wait(BAR(P_FULL + (t & 1)), (t >> 1) & 1, abort_flag);
+        ok = mbar_wait_all(BAR(P_FULL + (t & 1)), (t >> 1) & 1, abort_flag);
         if (!ok) break;
         const bool dirty = (t == n_tiles - 1) && last_rows < TK;
         const uint64_t pa = bdesc + (p16 + (t & 1) * (4096 >> 4));
         // O^T block m += C(t)^T [128 latent columns x 128 keys] . P^T
         for (int m = 0; m < NBLK; ++m, ++n) {
           const int s = n % NP;
-          ok = mbar_wait(BAR(PF + s), (n / NP) & 1, abort_flag);
-          if (ok && dirty) ok = mbar_wait(BAR(CLEAN + s), (m / NP) & 1, abort_flag);
+          ok = mbar_wait_all(BAR(PF + s), (n / NP) & 1, abort_flag);
+          if (ok && dirty) ok = mbar_wait_all(BAR(CLEAN + s), (m / NP) & 1, abort_flag);
           if (!ok) break;
           tc_fence_after();
           const uint64_t ca = adesc + (ring16 + s * (2 * SUB_BYTES >> 4));
 #pragma unroll
           for (int kk = 0; kk < TK / 16; ++kk)
             mma_ss(tmem + C::O_COL + m * 16, ca + kk * (2048 >> 4), pa + (kk >> 2) * (2048 >> 4) + (kk & 3) * 2, idesc_o,
-                   (t | kk) != 0);
-          mma_commit(BAR(PE + s));
+                   (t | kk) != 0, leader);
+          mma_commit(BAR(PE + s), leader);
         }
-        if (ok) mma_commit(BAR(PV_DONE + (t & 1)));
+        if (ok) mma_commit(BAR(PV_DONE + (t & 1)), leader);
       }
     }
   } else {

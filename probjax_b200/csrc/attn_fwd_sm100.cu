@@ -249,7 +249,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   using C = Cfg<DQK, DV, BN, KST, VST, BIAS == 2, MOD == 3>;
   extern __shared__ unsigned char smem_unaligned[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~uintptr_t(1023));
-  const uint32_t sbase = smem_u32(smem);
+  const uint32_t sbase = uniform(smem_u32(smem));
   const uint32_t bar0 = sbase + C::OFF_BAR;
   auto BAR = [&](int i) { return bar0 + 8u * i; };
   // barrier indices
@@ -269,7 +269,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::OFF_BAR + C::N_BAR * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform(static_cast<int>(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   // Work order: the (batch, head) pairs are taken in blocks of `order_w`; inside a block the
   // query-tile index is the slow, descending axis. Under a causal mask the long CTAs of a
   // block therefore start first and its short ones fill the gaps; unmasked grids use blocks
@@ -344,6 +344,8 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       for (int t = 0; t < 2; ++t) n_t[t] = n_t[t] > 0 ? mine : 0;
     }
   }
+  n_t[0] = uniform(n_t[0]);
+  n_t[1] = uniform(n_t[1]);
   const int n = max(n_t[0], n_t[1]);
   // The last KV tile of the loop may reach past the valid length. Probabilities are exactly 0
   // there, but those rows may hold anything (a cache tail that was never written) and 0 x NaN
@@ -375,7 +377,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = uniform(*tmem_slot);
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -442,7 +444,8 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issuer
-    if (lane == 0 && n > 0) {
+    if (n > 0) {
+      const uint32_t leader = elect_leader();
       constexpr uint32_t idesc_s = make_idesc(BM, BN, BF16, false, false);
       constexpr uint32_t idesc_o = make_idesc(BM, DV, BF16, false, true);
       auto issue_s = [&](int t, int j) {
@@ -453,58 +456,58 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
             mma_ss(tmem + t * BN, make_smem_desc(qa + s * BM * 128 + kk * 32, 16, 1024),
-                   make_smem_desc(ka + s * BN * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0);
+                   make_smem_desc(ka + s * BN * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0, leader);
       };
       auto issue_pv = [&](int t, int j) {
         const uint32_t va = sbase + C::OFF_V + (j % VST) * C::V_TILE_BYTES;
 #pragma unroll
         for (int kk = 0; kk < BN / 16; ++kk)
           mma_ts(tmem + 2 * BN + t * DV, tmem + t * BN + kk * 8, make_smem_desc(va + kk * 2048, BN * 128, 1024),
-                 idesc_o, (j | kk) != 0);
+                 idesc_o, (j | kk) != 0, leader);
       };
       bool ok = true;
 #pragma unroll
       for (int t = 0; t < 2; ++t)
-        if (ok && n_t[t] > 0) ok = mbar_wait(BAR(Q_FULL + t), 0, abort_flag);
-      if (ok) ok = mbar_wait(BAR(K_FULL + 0), 0, abort_flag);
+        if (ok && n_t[t] > 0) ok = mbar_wait_all(BAR(Q_FULL + t), 0, abort_flag);
+      if (ok) ok = mbar_wait_all(BAR(K_FULL + 0), 0, abort_flag);
       if (ok) {
         tc_fence_after();
 #pragma unroll
         for (int t = 0; t < 2; ++t)
           if (n_t[t] > 0) {
             issue_s(t, 0);
-            mma_commit(BAR(S_FULL + t));
+            mma_commit(BAR(S_FULL + t), leader);
           }
-        mma_commit(BAR(K_EMPTY + 0));
+        mma_commit(BAR(K_EMPTY + 0), leader);
         PJX_CTA_AT(2);
       }
       for (int j = 0; ok && j < n; ++j) {
         const bool have_next = j + 1 < n;
-        ok = mbar_wait(BAR(V_FULL + j % VST), (j / VST) & 1, abort_flag);
-        if (ok && j == clean_j) ok = mbar_wait(BAR(V_CLEAN), 0, abort_flag);
-        if (ok && have_next) ok = mbar_wait(BAR(K_FULL + (j + 1) % KST), ((j + 1) / KST) & 1, abort_flag);
+        ok = mbar_wait_all(BAR(V_FULL + j % VST), (j / VST) & 1, abort_flag);
+        if (ok && j == clean_j) ok = mbar_wait_all(BAR(V_CLEAN), 0, abort_flag);
+        if (ok && have_next) ok = mbar_wait_all(BAR(K_FULL + (j + 1) % KST), ((j + 1) / KST) & 1, abort_flag);
         if (!ok) break;
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
           if (j < n_t[t]) {
             PJX_TRACE_AT(2, j, 4 * t + 0);
-            ok = mbar_wait(BAR(P_FULL + t), j & 1, abort_flag);
+            ok = mbar_wait_all(BAR(P_FULL + t), j & 1, abort_flag);
             if (!ok) break;
             tc_fence_after();
             PJX_TRACE_AT(2, j, 4 * t + 1);
             issue_pv(t, j);
             PJX_TRACE_AT(2, j, 4 * t + 2);
-            if (j == n_t[t] - 1) mma_commit(BAR(O_FULL + t));
+            if (j == n_t[t] - 1) mma_commit(BAR(O_FULL + t), leader);
           }
           if (j + 1 < n_t[t]) {
             issue_s(t, j + 1);
-            mma_commit(BAR(S_FULL + t));
+            mma_commit(BAR(S_FULL + t), leader);
             PJX_TRACE_AT(2, j, 4 * t + 3);
           }
         }
         if (!ok) break;
-        mma_commit(BAR(V_EMPTY + j % VST));
-        if (have_next) mma_commit(BAR(K_EMPTY + (j + 1) % KST));
+        mma_commit(BAR(V_EMPTY + j % VST), leader);
+        if (have_next) mma_commit(BAR(K_EMPTY + (j + 1) % KST), leader);
       }
       PJX_CTA_AT(3);
     }

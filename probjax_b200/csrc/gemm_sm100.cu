@@ -76,12 +76,12 @@ gemm_tn_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
   constexpr int ST = GC::ST, G_OFF_BAR = GC::OFF_BAR, G_NBAR = GC::NBAR, G_OFF_STAGE = GC::OFF_STAGE;
   extern __shared__ unsigned char smem_unaligned[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~uintptr_t(1023));
-  const uint32_t sbase = smem_u32(smem);
+  const uint32_t sbase = uniform(smem_u32(smem));
   auto BAR = [&](int i) { return sbase + G_OFF_BAR + 8u * i; };
   const int FULL = 0, EMPTY = ST, ACC_FULL = 2 * ST, ACC_EMPTY = 2 * ST + 2, OUT_STAGED = 2 * ST + 4, OUT_FREE = 2 * ST + 5;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + G_OFF_BAR + G_NBAR * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform(static_cast<int>(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   const int nk = (g.K + TK - 1) / TK;
   const int mt = (int)((g.M + TM - 1) / TM);
   const int nt0 = (g.n0 + TN - 1) / TN, nt1 = (g.n1 + TN - 1) / TN;
@@ -116,7 +116,7 @@ gemm_tn_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = uniform(*tmem_slot);
 
   if (warp == 0) {
     if (lane == 0) {
@@ -143,28 +143,29 @@ gemm_tn_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      const uint32_t leader = elect_leader();
       constexpr uint32_t idesc = make_idesc(TM, TN, BF16, false, false);
       int it = 0, local = 0;
       bool ok = true;
       for (int tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x, ++local) {
         const int acc = local & 1;
-        ok = mbar_wait(BAR(ACC_EMPTY + acc), ((local >> 1) & 1) ^ 1, abort_flag);
+        ok = mbar_wait_all(BAR(ACC_EMPTY + acc), ((local >> 1) & 1) ^ 1, abort_flag);
         if (!ok) break;
         tc_fence_after();
         for (int k = 0; k < nk; ++k, ++it) {
           const int s = it % ST;
-          ok = mbar_wait(BAR(FULL + s), (it / ST) & 1, abort_flag);
+          ok = mbar_wait_all(BAR(FULL + s), (it / ST) & 1, abort_flag);
           if (!ok) break;
           tc_fence_after();
           const uint32_t a = sbase + s * (A_BYTES + B_BYTES), bb = a + A_BYTES;
 #pragma unroll
           for (int kk = 0; kk < TK / 16; ++kk)
             mma_ss(tmem + acc * TN, make_smem_desc(a + kk * 32, 16, 1024), make_smem_desc(bb + kk * 32, 16, 1024),
-                   idesc, (k | kk) != 0);
-          mma_commit(BAR(EMPTY + s));
+                   idesc, (k | kk) != 0, leader);
+          mma_commit(BAR(EMPTY + s), leader);
         }
-        if (ok) mma_commit(BAR(ACC_FULL + acc));
+        if (ok) mma_commit(BAR(ACC_FULL + acc), leader);
       }
     }
   } else {
@@ -307,12 +308,12 @@ linear_grad_sm100_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid
   constexpr int ST = GC::ST, STAGE = A_BYTES + GC::BBYTES;
   extern __shared__ unsigned char smem_unaligned[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~uintptr_t(1023));
-  const uint32_t sbase = smem_u32(smem);
+  const uint32_t sbase = uniform(smem_u32(smem));
   auto BAR = [&](int i) { return sbase + GC::OFF_BAR + 8u * i; };
   const int FULL = 0, EMPTY = ST, ACC_FULL = 2 * ST, ACC_EMPTY = 2 * ST + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + GC::OFF_BAR + GC::NBAR * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform(static_cast<int>(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   const int nt = (g.n + TN_ - 1) / TN_;
   const int mt0 = (int)((g.m[0] + TM - 1) / TM), mt1 = (!CHAIN && g.pairs > 1) ? (int)((g.m[1] + TM - 1) / TM) : 0;
   const int ntiles = (mt0 + mt1) * nt;
@@ -338,7 +339,7 @@ linear_grad_sm100_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = uniform(*tmem_slot);
 
   if (warp == 0) {
     if (lane == 0) {
@@ -372,7 +373,8 @@ linear_grad_sm100_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      const uint32_t leader = elect_leader();
       constexpr uint32_t idesc = make_idesc(TM, TN_, BF16, !CHAIN, true);
       int it = 0, local = 0;
       bool ok = true;
@@ -380,22 +382,22 @@ linear_grad_sm100_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid
         int which, m_idx, n_idx;
         decode(tile, which, m_idx, n_idx);
         const int nk = steps(which), acc = local & 1;
-        ok = mbar_wait(BAR(ACC_EMPTY + acc), ((local >> 1) & 1) ^ 1, abort_flag);
+        ok = mbar_wait_all(BAR(ACC_EMPTY + acc), ((local >> 1) & 1) ^ 1, abort_flag);
         if (!ok) break;
         tc_fence_after();
         for (int k = 0; k < nk; ++k, ++it) {
           const int s = it % ST;
-          ok = mbar_wait(BAR(FULL + s), (it / ST) & 1, abort_flag);
+          ok = mbar_wait_all(BAR(FULL + s), (it / ST) & 1, abort_flag);
           if (!ok) break;
           tc_fence_after();
           const uint32_t a = sbase + s * STAGE, bb = a + A_BYTES;
 #pragma unroll
           for (int kk = 0; kk < TK / 16; ++kk)
             mma_ss(tmem + acc * 256, CHAIN ? make_smem_desc(a + kk * 32, 16, 1024) : make_smem_desc(a + kk * 2048, TK * 128, 1024),
-                   make_smem_desc(bb + kk * 2048, TK * 128, 1024), idesc, (k | kk) != 0);
-          mma_commit(BAR(EMPTY + s));
+                   make_smem_desc(bb + kk * 2048, TK * 128, 1024), idesc, (k | kk) != 0, leader);
+          mma_commit(BAR(EMPTY + s), leader);
         }
-        if (ok) mma_commit(BAR(ACC_FULL + acc));
+        if (ok) mma_commit(BAR(ACC_FULL + acc), leader);
       }
     }
   } else {

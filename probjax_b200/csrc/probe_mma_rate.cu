@@ -44,22 +44,22 @@ __global__ void __launch_bounds__(128, 1) rate_kernel(long long* out, int tiles,
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
             mma_ss(d, make_smem_desc(a_addr + s * 128 * 128 + kk * 32, 16, 1024),
-                   make_smem_desc(b_addr + s * N * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0);
+                   make_smem_desc(b_addr + s * N * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0, 1u);
       }
       if (MODE == 1) {
 #pragma unroll
         for (int s = 0; s < 2; ++s)
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
-            mma_ts(d, tmem + 256 + (s * 4 + kk) * 8, make_smem_desc(b_addr + s * N * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0);
+            mma_ts(d, tmem + 256 + (s * 4 + kk) * 8, make_smem_desc(b_addr + s * N * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0, 1u);
       }
       if (MODE == 2 || MODE == 3) {
 #pragma unroll
         for (int kk = 0; kk < N / 16; ++kk)
-          mma_ts(tmem + 384 + (t & 1) * 0, tmem + 256 + kk * 8, make_smem_desc(v_addr + kk * 2048, 128 * 128, 1024), idesc_o, kk != 0);
+          mma_ts(tmem + 384 + (t & 1) * 0, tmem + 256 + kk * 8, make_smem_desc(v_addr + kk * 2048, 128 * 128, 1024), idesc_o, kk != 0, 1u);
       }
     }
-    mma_commit(bar);
+    mma_commit(bar, 1u);
     const bool ok = mbar_wait(bar, 0, &abort_flag);
     const long long t1 = clock64();
     if (!ok) atomicExch(status, 1);

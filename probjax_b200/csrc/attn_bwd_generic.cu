@@ -115,29 +115,62 @@ int launch_delta(const BwdParams& p, cudaStream_t stream) {
   return check_cuda(cudaGetLastError(), "backward delta launch");
 }
 
-// Shared-memory views of one tile step.
+// Shared-memory views of one tile step.  Rows are padded to whole float4 units plus one: every inner loop reads 16 bytes
+// per load (4 columns of a row), and the rows of a quarter warp start in different banks.
 struct Tiles {
   float *Qs, *dOs, *Ks, *Vs, *Ps, *dSs, *lse_s, *delta_s;
   int Dp, Dvp;
 };
+constexpr int SP = T + 4;  // pitch of the P and dS tiles
+
+__host__ __device__ inline int pitch4(int d) { return (d + 3) / 4 * 4 + 4; }
 
 __device__ __forceinline__ Tiles carve(float* smem, int D, int Dv) {
   Tiles t;
-  t.Dp = D | 1;
-  t.Dvp = Dv | 1;
+  t.Dp = pitch4(D);
+  t.Dvp = pitch4(Dv);
   t.Qs = smem;
   t.dOs = t.Qs + T * t.Dp;
   t.Ks = t.dOs + T * t.Dvp;
   t.Vs = t.Ks + T * t.Dp;
   t.Ps = t.Vs + T * t.Dvp;
-  t.dSs = t.Ps + T * (T + 1);
-  t.lse_s = t.dSs + T * (T + 1);
+  t.dSs = t.Ps + T * SP;
+  t.lse_s = t.dSs + T * SP;
   t.delta_s = t.lse_s + T;
   return t;
 }
 inline size_t bwd_smem_bytes(int D, int Dv) {
-  return sizeof(float) * ((size_t)2 * T * (D | 1) + (size_t)2 * T * (Dv | 1) + 2 * T * (T + 1) + 2 * T);
+  return sizeof(float) * ((size_t)2 * T * pitch4(D) + (size_t)2 * T * pitch4(Dv) + 2 * T * SP + 2 * T);
 }
+
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float dot4(float4 a, float4 b, float s) {
+  return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, s))));
+}
+__device__ __forceinline__ void axpy4(float4& s, float a, float4 x) {
+  s.x = fmaf(a, x.x, s.x);
+  s.y = fmaf(a, x.y, s.y);
+  s.z = fmaf(a, x.z, s.z);
+  s.w = fmaf(a, x.w, s.w);
+}
+
+// 32 rows of `width` elements into a tile of pitch4(width), rows at or past `limit` and the padding up to the next
+// multiple of 4 as zeros; 8 threads per row.  fp32 rows of whole aligned 16-byte units are copied as such.
+template <typename T_>
+__device__ __forceinline__ void load_tile(float* dst, int pitch, const T_* src, int64_t row_stride, int first, int limit, int width,
+                                          bool vec) {
+  const int r = threadIdx.x >> 3, u = threadIdx.x & 7, g = first + r;
+  const T_* row = src + (int64_t)g * row_stride;
+  if (sizeof(T_) == 4 && vec) {
+    for (int d = u * 4; d < width; d += 32)
+      *reinterpret_cast<float4*>(dst + r * pitch + d) =
+          g < limit ? __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(row) + d)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  } else {
+    for (int d = u; d < (width + 3) / 4 * 4; d += 8) dst[r * pitch + d] = g < limit && d < width ? Elem<T_>::to_f(row[d]) : 0.f;
+  }
+}
+// Whether fp32 rows can be read in 16-byte units.
+__device__ __forceinline__ bool rows_vec(const void* p, int width) { return width % 4 == 0 && (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 template <typename T_>
 __device__ __forceinline__ void load_rows(float* dst, int pitch, const T_* src, int64_t row_stride, int first, int limit,
@@ -154,21 +187,25 @@ __device__ __forceinline__ void load_rows(float* dst, int pitch, const T_* src, 
 __device__ __forceinline__ void tile_p_ds(const BwdParams& p, const Tiles& t, int b, int h, int q0, int k0, int kv_len) {
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   float s[2][2] = {}, dp[2][2] = {};
-  for (int d = 0; d < p.D; ++d) {
-    const float q0v = t.Qs[(ty * 2) * t.Dp + d], q1v = t.Qs[(ty * 2 + 1) * t.Dp + d];
-    const float k0v = t.Ks[tx * t.Dp + d], k1v = t.Ks[(tx + 16) * t.Dp + d];
-    s[0][0] = fmaf(q0v, k0v, s[0][0]);
-    s[0][1] = fmaf(q0v, k1v, s[0][1]);
-    s[1][0] = fmaf(q1v, k0v, s[1][0]);
-    s[1][1] = fmaf(q1v, k1v, s[1][1]);
+  const float* qr = t.Qs + (ty * 2) * t.Dp;
+  const float* kr = t.Ks + tx * t.Dp;
+#pragma unroll 4
+  for (int d = 0; d < p.D; d += 4) {
+    const float4 q0v = ld4(qr + d), q1v = ld4(qr + t.Dp + d), k0v = ld4(kr + d), k1v = ld4(kr + 16 * t.Dp + d);
+    s[0][0] = dot4(q0v, k0v, s[0][0]);
+    s[0][1] = dot4(q0v, k1v, s[0][1]);
+    s[1][0] = dot4(q1v, k0v, s[1][0]);
+    s[1][1] = dot4(q1v, k1v, s[1][1]);
   }
-  for (int d = 0; d < p.Dv; ++d) {
-    const float a0 = t.dOs[(ty * 2) * t.Dvp + d], a1 = t.dOs[(ty * 2 + 1) * t.Dvp + d];
-    const float v0 = t.Vs[tx * t.Dvp + d], v1 = t.Vs[(tx + 16) * t.Dvp + d];
-    dp[0][0] = fmaf(a0, v0, dp[0][0]);
-    dp[0][1] = fmaf(a0, v1, dp[0][1]);
-    dp[1][0] = fmaf(a1, v0, dp[1][0]);
-    dp[1][1] = fmaf(a1, v1, dp[1][1]);
+  const float* gr = t.dOs + (ty * 2) * t.Dvp;
+  const float* vr = t.Vs + tx * t.Dvp;
+#pragma unroll 4
+  for (int d = 0; d < p.Dv; d += 4) {
+    const float4 a0 = ld4(gr + d), a1 = ld4(gr + t.Dvp + d), v0 = ld4(vr + d), v1 = ld4(vr + 16 * t.Dvp + d);
+    dp[0][0] = dot4(a0, v0, dp[0][0]);
+    dp[0][1] = dot4(a0, v1, dp[0][1]);
+    dp[1][0] = dot4(a1, v0, dp[1][0]);
+    dp[1][1] = dot4(a1, v1, dp[1][1]);
   }
   const float* bias = p.bias ? p.bias + (int64_t)b * p.bias_bs + (int64_t)h * p.bias_hs : nullptr;
   const bool has_mod = p.mod.on != 0;
@@ -194,13 +231,22 @@ __device__ __forceinline__ void tile_p_ds(const BwdParams& p, const Tiles& t, in
       // dropout: dV sees the dropped, rescaled probabilities and dP is dropped the same way
       // (kernels/attention.py:1038-1039); delta = rowsum(o * do) already includes it
       const float dm = (has_mod && keep) ? mod_dropout(mv, qi, kj) : 1.f;
-      t.Ps[r * (T + 1) + col] = pr * dm;
-      t.dSs[r * (T + 1) + col] = pr * (dp[i][c] * dm - delta) * dsds;
+      t.Ps[r * SP + col] = pr * dm;
+      t.dSs[r * SP + col] = pr * (dp[i][c] * dm - delta) * dsds;
     }
   }
 }
 
-template <typename T_, int NC>  // NC: per-thread columns = ceil(D / 16)
+// Columns d .. d + 3 of a gradient row of `width` elements.
+template <typename T_>
+__device__ __forceinline__ void store4(T_* row, int d, int width, float4 x, float scale) {
+  const float v[4] = {x.x * scale, x.y * scale, x.z * scale, x.w * scale};
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if (d + i < width) row[d + i] = Elem<T_>::from_f(v[i]);
+}
+
+template <typename T_, int NC>  // NC: groups of four columns per thread = ceil(D / 64)
 __global__ void __launch_bounds__(NT) bwd_dq_kernel(const BwdParams p) {
   extern __shared__ float smem[];
   const Tiles t = carve(smem, p.D, p.Dv);
@@ -218,23 +264,24 @@ __global__ void __launch_bounds__(NT) bwd_dq_kernel(const BwdParams p) {
   const T_* d_o = static_cast<const T_*>(p.d_o) + ((int64_t)b * p.Lq * p.Hq + h) * p.Dv;
   const T_* k = static_cast<const T_*>(p.k) + ((int64_t)b * p.Lkv * p.Hkv + hk) * p.D;
   const T_* v = static_cast<const T_*>(p.v) + ((int64_t)b * p.Lkv * p.Hkv + hk) * p.Dv;
-  load_rows<T_>(t.Qs, t.Dp, q, qstride, q0, p.Lq, p.D);
-  load_rows<T_>(t.dOs, t.Dvp, d_o, ostride, q0, p.Lq, p.Dv);
+  const bool vec = rows_vec(p.q, p.D) && rows_vec(p.k, p.D), vec_v = rows_vec(p.d_o, p.Dv) && rows_vec(p.v, p.Dv);
+  load_tile<T_>(t.Qs, t.Dp, q, qstride, q0, p.Lq, p.D, vec);
+  load_tile<T_>(t.dOs, t.Dvp, d_o, ostride, q0, p.Lq, p.Dv, vec_v);
   if (threadIdx.x < T) {
     const int qi = q0 + threadIdx.x;
     const int64_t at = ((int64_t)b * p.Hq + h) * p.Lq + qi;
     t.lse_s[threadIdx.x] = qi < p.Lq ? p.lse[at] : INFINITY;
     t.delta_s[threadIdx.x] = qi < p.Lq ? p.delta[((int64_t)b * p.Hq + h) * p.Lq_pad + qi] : 0.f;
   }
-  float acc[2][NC];
+  float4 acc[2][NC];
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int c = 0; c < NC; ++c) acc[i][c] = 0.f;
+    for (int c = 0; c < NC; ++c) acc[i][c] = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int k0 = kv_begin; k0 < kv_end; k0 += T) {
     __syncthreads();
-    load_rows<T_>(t.Ks, t.Dp, k, kstride, k0, kv_len, p.D);
-    load_rows<T_>(t.Vs, t.Dvp, v, vstride, k0, kv_len, p.Dv);
+    load_tile<T_>(t.Ks, t.Dp, k, kstride, k0, kv_len, p.D, vec);
+    load_tile<T_>(t.Vs, t.Dvp, v, vstride, k0, kv_len, p.Dv, vec_v);
     __syncthreads();
     tile_p_ds(p, t, b, h, q0, k0, kv_len);
     __syncthreads();
@@ -247,20 +294,23 @@ __global__ void __launch_bounds__(NT) bwd_dq_kernel(const BwdParams p) {
           const int r = ty * 2 + i, col = tx + 16 * c;
           const int qi = q0 + r, kj = k0 + col;
           if (qi < p.Lq && kj < p.Lkv) {
-            const float g = t.dSs[r * (T + 1) + col];
+            const float g = t.dSs[r * SP + col];
             if (p.dbias_atomic) atomicAdd(&db[(int64_t)qi * p.Lkv + kj], g);
             else db[(int64_t)qi * p.Lkv + kj] = g;
           }
         }
     }
-    for (int c = 0; c < T; ++c) {
-      const float d0 = t.dSs[(ty * 2) * (T + 1) + c], d1 = t.dSs[(ty * 2 + 1) * (T + 1) + c];
+#pragma unroll 2
+    for (int c = 0; c < T; c += 4) {
+      const float4 d0 = ld4(t.dSs + (ty * 2) * SP + c), d1 = ld4(t.dSs + (ty * 2 + 1) * SP + c);
 #pragma unroll
       for (int cc = 0; cc < NC; ++cc) {
-        const int d = tx + 16 * cc;
-        const float kv = d < p.D ? t.Ks[c * t.Dp + d] : 0.f;
-        acc[0][cc] = fmaf(d0, kv, acc[0][cc]);
-        acc[1][cc] = fmaf(d1, kv, acc[1][cc]);
+        const int d = tx * 4 + 64 * cc;
+        if (d >= p.D) break;
+        const float* kc = t.Ks + c * t.Dp + d;
+        const float4 k0v = ld4(kc), k1v = ld4(kc + t.Dp), k2v = ld4(kc + 2 * t.Dp), k3v = ld4(kc + 3 * t.Dp);
+        axpy4(acc[0][cc], d0.x, k0v); axpy4(acc[0][cc], d0.y, k1v); axpy4(acc[0][cc], d0.z, k2v); axpy4(acc[0][cc], d0.w, k3v);
+        axpy4(acc[1][cc], d1.x, k0v); axpy4(acc[1][cc], d1.y, k1v); axpy4(acc[1][cc], d1.z, k2v); axpy4(acc[1][cc], d1.w, k3v);
       }
     }
   }
@@ -270,14 +320,11 @@ __global__ void __launch_bounds__(NT) bwd_dq_kernel(const BwdParams p) {
     const int qi = q0 + ty * 2 + i;
     if (qi >= p.Lq) continue;
 #pragma unroll
-    for (int cc = 0; cc < NC; ++cc) {
-      const int d = tx + 16 * cc;
-      if (d < p.D) dq[(int64_t)qi * qstride + d] = Elem<T_>::from_f(acc[i][cc] * p.sm_scale);
-    }
+    for (int cc = 0; cc < NC; ++cc) store4<T_>(dq + (int64_t)qi * qstride, tx * 4 + 64 * cc, p.D, acc[i][cc], p.sm_scale);
   }
 }
 
-template <typename T_, int NCK, int NCV>  // per-thread columns of dK (D) and dV (Dv)
+template <typename T_, int NCK, int NCV>  // groups of four columns per thread of dK (D) and dV (Dv)
 __global__ void __launch_bounds__(NT) bwd_dkdv_kernel(const BwdParams p) {
   extern __shared__ float smem[];
   const Tiles t = carve(smem, p.D, p.Dv);
@@ -290,17 +337,18 @@ __global__ void __launch_bounds__(NT) bwd_dkdv_kernel(const BwdParams p) {
   const int64_t kstride = (int64_t)p.Hkv * p.D, vstride = (int64_t)p.Hkv * p.Dv;
   const T_* k = static_cast<const T_*>(p.k) + ((int64_t)b * p.Lkv * p.Hkv + hk) * p.D;
   const T_* v = static_cast<const T_*>(p.v) + ((int64_t)b * p.Lkv * p.Hkv + hk) * p.Dv;
-  float acck[2][NCK], accv[2][NCV];
+  float4 acck[2][NCK], accv[2][NCV];
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
 #pragma unroll
-    for (int c = 0; c < NCK; ++c) acck[i][c] = 0.f;
+    for (int c = 0; c < NCK; ++c) acck[i][c] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int c = 0; c < NCV; ++c) accv[i][c] = 0.f;
+    for (int c = 0; c < NCV; ++c) accv[i][c] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   if (k0 < kv_len) {  // keys past the valid length get zero gradients
-    load_rows<T_>(t.Ks, t.Dp, k, kstride, k0, kv_len, p.D);
-    load_rows<T_>(t.Vs, t.Dvp, v, vstride, k0, kv_len, p.Dv);
+    const bool vec = rows_vec(p.q, p.D) && rows_vec(p.k, p.D), vec_v = rows_vec(p.d_o, p.Dv) && rows_vec(p.v, p.Dv);
+    load_tile<T_>(t.Ks, t.Dp, k, kstride, k0, kv_len, p.D, vec);
+    load_tile<T_>(t.Vs, t.Dvp, v, vstride, k0, kv_len, p.Dv, vec_v);
     // queries outside [first key - band_hi, last key - band_lo] never see a key of this tile
     int q_first = (max(0, k0 - p.band_hi) / T) * T;
     const int q_end = min(p.Lq, k0 + T - p.band_lo);
@@ -311,8 +359,8 @@ __global__ void __launch_bounds__(NT) bwd_dkdv_kernel(const BwdParams p) {
       const T_* d_o = static_cast<const T_*>(p.d_o) + ((int64_t)b * p.Lq * p.Hq + h) * p.Dv;
       for (int q0 = q_first; q0 < q_end; q0 += T) {
         __syncthreads();
-        load_rows<T_>(t.Qs, t.Dp, q, qstride, q0, p.Lq, p.D);
-        load_rows<T_>(t.dOs, t.Dvp, d_o, ostride, q0, p.Lq, p.Dv);
+        load_tile<T_>(t.Qs, t.Dp, q, qstride, q0, p.Lq, p.D, vec);
+        load_tile<T_>(t.dOs, t.Dvp, d_o, ostride, q0, p.Lq, p.Dv, vec_v);
         if (threadIdx.x < T) {
           const int qi = q0 + threadIdx.x;
           const int64_t at = ((int64_t)b * p.Hq + h) * p.Lq + qi;
@@ -322,22 +370,25 @@ __global__ void __launch_bounds__(NT) bwd_dkdv_kernel(const BwdParams p) {
         __syncthreads();
         tile_p_ds(p, t, b, h, q0, k0, kv_len);
         __syncthreads();
+#pragma unroll 4
         for (int r = 0; r < T; ++r) {
-          const float p0 = t.Ps[r * (T + 1) + ty * 2], p1 = t.Ps[r * (T + 1) + ty * 2 + 1];
-          const float s0 = t.dSs[r * (T + 1) + ty * 2], s1 = t.dSs[r * (T + 1) + ty * 2 + 1];
+          const float2 pv = *reinterpret_cast<const float2*>(t.Ps + r * SP + ty * 2);
+          const float2 sv = *reinterpret_cast<const float2*>(t.dSs + r * SP + ty * 2);
 #pragma unroll
           for (int cc = 0; cc < NCV; ++cc) {
-            const int d = tx + 16 * cc;
-            const float g_o = d < p.Dv ? t.dOs[r * t.Dvp + d] : 0.f;
-            accv[0][cc] = fmaf(p0, g_o, accv[0][cc]);
-            accv[1][cc] = fmaf(p1, g_o, accv[1][cc]);
+            const int d = tx * 4 + 64 * cc;
+            if (d >= p.Dv) break;
+            const float4 g_o = ld4(t.dOs + r * t.Dvp + d);
+            axpy4(accv[0][cc], pv.x, g_o);
+            axpy4(accv[1][cc], pv.y, g_o);
           }
 #pragma unroll
           for (int cc = 0; cc < NCK; ++cc) {
-            const int d = tx + 16 * cc;
-            const float qv = d < p.D ? t.Qs[r * t.Dp + d] : 0.f;
-            acck[0][cc] = fmaf(s0, qv, acck[0][cc]);
-            acck[1][cc] = fmaf(s1, qv, acck[1][cc]);
+            const int d = tx * 4 + 64 * cc;
+            if (d >= p.D) break;
+            const float4 qv = ld4(t.Qs + r * t.Dp + d);
+            axpy4(acck[0][cc], sv.x, qv);
+            axpy4(acck[1][cc], sv.y, qv);
           }
         }
       }
@@ -350,15 +401,9 @@ __global__ void __launch_bounds__(NT) bwd_dkdv_kernel(const BwdParams p) {
     const int kj = k0 + ty * 2 + i;
     if (kj >= p.Lkv) continue;
 #pragma unroll
-    for (int cc = 0; cc < NCK; ++cc) {
-      const int d = tx + 16 * cc;
-      if (d < p.D) dk[(int64_t)kj * kstride + d] = Elem<T_>::from_f(acck[i][cc] * p.sm_scale);
-    }
+    for (int cc = 0; cc < NCK; ++cc) store4<T_>(dk + (int64_t)kj * kstride, tx * 4 + 64 * cc, p.D, acck[i][cc], p.sm_scale);
 #pragma unroll
-    for (int cc = 0; cc < NCV; ++cc) {
-      const int d = tx + 16 * cc;
-      if (d < p.Dv) dv[(int64_t)kj * vstride + d] = Elem<T_>::from_f(accv[i][cc]);
-    }
+    for (int cc = 0; cc < NCV; ++cc) store4<T_>(dv + (int64_t)kj * vstride, tx * 4 + 64 * cc, p.Dv, accv[i][cc], 1.f);
   }
 }
 
@@ -394,18 +439,18 @@ int launch_dtype(const BwdParams& p, BwdRoute route, void* scratch, cudaStream_t
   if (rc) return rc;
   if (route == BwdRoute::Sm100) return launch_bwd_sm100(p, stream);
   if (route == BwdRoute::Sm100Exact) return launch_bwd_exact_sm100(p, scratch, stream);
-  const int nk = p.D <= 64 ? 4 : (p.D <= 128 ? 8 : 16);
-  const int nv = p.Dv <= 64 ? 4 : (p.Dv <= 128 ? 8 : 16);
-  switch (nk * 100 + nv) {
-    case 404: return launch_widths<T_, 4, 4>(p, stream);
-    case 408: return launch_widths<T_, 4, 8>(p, stream);
-    case 416: return launch_widths<T_, 4, 16>(p, stream);
-    case 804: return launch_widths<T_, 8, 4>(p, stream);
-    case 808: return launch_widths<T_, 8, 8>(p, stream);
-    case 816: return launch_widths<T_, 8, 16>(p, stream);
-    case 1604: return launch_widths<T_, 16, 4>(p, stream);
-    case 1608: return launch_widths<T_, 16, 8>(p, stream);
-    default: return launch_widths<T_, 16, 16>(p, stream);
+  const int nk = p.D <= 64 ? 1 : (p.D <= 128 ? 2 : 4);
+  const int nv = p.Dv <= 64 ? 1 : (p.Dv <= 128 ? 2 : 4);
+  switch (nk * 10 + nv) {
+    case 11: return launch_widths<T_, 1, 1>(p, stream);
+    case 12: return launch_widths<T_, 1, 2>(p, stream);
+    case 14: return launch_widths<T_, 1, 4>(p, stream);
+    case 21: return launch_widths<T_, 2, 1>(p, stream);
+    case 22: return launch_widths<T_, 2, 2>(p, stream);
+    case 24: return launch_widths<T_, 2, 4>(p, stream);
+    case 41: return launch_widths<T_, 4, 1>(p, stream);
+    case 42: return launch_widths<T_, 4, 2>(p, stream);
+    default: return launch_widths<T_, 4, 4>(p, stream);
   }
 }
 

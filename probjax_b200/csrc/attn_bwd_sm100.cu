@@ -89,11 +89,15 @@ struct DqCfg {
   static constexpr int TILE = SUB * 128 * 128;     // bytes of a 128-row tile
   static constexpr int OFF_Q = 0;
   static constexpr int OFF_DO = TILE;
-  static constexpr int OFF_K = 2 * TILE;           // 2 stages
-  static constexpr int OFF_V = 4 * TILE;           // 2 stages
-  static constexpr int OFF_BAR = 6 * TILE;
-  // barriers: QDO_FULL, K_FULL[2], K_EMPTY[2], V_FULL[2], V_EMPTY[2], SP_FULL[2], DS_FULL[2], DQ_FULL, K_CLEAN
-  static constexpr int N_BAR = 15;
+  // K is held from the score products of a tile to its accumulation one step later, and the next tile is wanted half a
+  // step after that: with two stages a load has half a step (about 1000 cycles) and the issuer waited 450-1000 cycles
+  // per step for it.  V is free after the score products, two stages do.
+  static constexpr int KST = 3;
+  static constexpr int OFF_K = 2 * TILE;
+  static constexpr int OFF_V = OFF_K + KST * TILE;  // 2 stages
+  static constexpr int OFF_BAR = OFF_V + 2 * TILE;
+  // barriers: QDO_FULL, K_FULL[3], K_EMPTY[3], V_FULL[2], V_EMPTY[2], SP_FULL[2], DS_FULL[2], DQ_FULL, K_CLEAN
+  static constexpr int N_BAR = 17;
   static constexpr int SMEM_BYTES = OFF_BAR + N_BAR * 8 + 16 + 1024;
   static constexpr int TMEM_COLS = 512;            // S 128 | dP 128 | dQ D
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
@@ -110,8 +114,9 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   const uint32_t sbase = uniform(smem_u32(smem));
   const uint32_t bar0 = sbase + C::OFF_BAR;
   auto BAR = [&](int i) { return bar0 + 8u * i; };
-  const int QDO_FULL = 0, K_FULL = 1, K_EMPTY = 3, V_FULL = 5, V_EMPTY = 7, SP_FULL = 9, DS_FULL = 11, DQ_FULL = 13,
-            K_CLEAN = 14;
+  constexpr int KST = C::KST;
+  const int QDO_FULL = 0, K_FULL = 1, K_EMPTY = K_FULL + KST, V_FULL = K_EMPTY + KST, V_EMPTY = V_FULL + 2, SP_FULL = V_EMPTY + 2,
+            DS_FULL = SP_FULL + 2, DQ_FULL = DS_FULL + 2, K_CLEAN = DQ_FULL + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::OFF_BAR + C::N_BAR * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -166,12 +171,12 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         tma_load_4d(sbase + C::OFF_DO + s * BM * 128, &tm_do, BAR(QDO_FULL), s * 64, h, q0, b);
       }
       for (int j = 0; j < n; ++j) {
-        const int st = j & 1;
-        if (!mbar_wait(BAR(K_EMPTY + st), ((j >> 1) & 1) ^ 1, abort_flag)) break;
-        mbar_arrive_expect_tx(BAR(K_FULL + st), C::TILE);
+        const int st = j & 1, ks = j % KST;
+        if (!mbar_wait(BAR(K_EMPTY + ks), ((j / KST) & 1) ^ 1, abort_flag)) break;
+        mbar_arrive_expect_tx(BAR(K_FULL + ks), C::TILE);
 #pragma unroll
         for (int s = 0; s < C::SUB; ++s)
-          tma_load_4d(sbase + C::OFF_K + st * C::TILE + s * BN * 128, &tm_k, BAR(K_FULL + st), s * 64, hk,
+          tma_load_4d(sbase + C::OFF_K + ks * C::TILE + s * BN * 128, &tm_k, BAR(K_FULL + ks), s * 64, hk,
                       (j_lo + j) * BN, b);
         if (!mbar_wait(BAR(V_EMPTY + st), ((j >> 1) & 1) ^ 1, abort_flag)) break;
         mbar_arrive_expect_tx(BAR(V_FULL + st), C::TILE);
@@ -183,8 +188,8 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     }
     __syncwarp();
     if (clean_j >= 0) {
-      const int st = clean_j & 1;
-      if (mbar_wait(BAR(K_FULL + st), (clean_j >> 1) & 1, abort_flag)) {
+      const int st = clean_j % KST;
+      if (mbar_wait(BAR(K_FULL + st), (clean_j / KST) & 1, abort_flag)) {
         for (int r = kv_len - (j_lo + clean_j) * BN + lane; r < BN; r += 32) {
           const uint32_t krow = sbase + C::OFF_K + st * C::TILE + r * 128;
 #pragma unroll
@@ -206,7 +211,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       const uint32_t qa = sbase + C::OFF_Q, doa = sbase + C::OFF_DO;
       // S and dP of one half (64 keys) of KV tile j: the B operands start 64 rows into the tiles
       auto issue_sdp = [&](int half, int j) {
-        const uint32_t ka = sbase + C::OFF_K + (j & 1) * C::TILE + half * 64 * 128;
+        const uint32_t ka = sbase + C::OFF_K + (j % KST) * C::TILE + half * 64 * 128;
         const uint32_t va = sbase + C::OFF_V + (j & 1) * C::TILE + half * 64 * 128;
 #pragma unroll
         for (int s = 0; s < C::SUB; ++s)
@@ -225,7 +230,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       // dQ += dS.K over one half: A = dS (16-bit pairs at the first 32 columns of the half of S),
       // B = the K tile read MN-major
       auto issue_acc = [&](int half, int j) {
-        const uint32_t ka = sbase + C::OFF_K + (j & 1) * C::TILE;
+        const uint32_t ka = sbase + C::OFF_K + (j % KST) * C::TILE;
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
           mma_ts(T_DQ, T_S + half * 64 + kk * 8, make_smem_desc(ka + (half * 4 + kk) * 2048, BN * 128, 1024), idesc_q,
@@ -251,7 +256,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         PJX_BTRACE(0, j, 1);
         issue_acc(0, j);
         if (next) {
-          ok = mbar_wait_all(BAR(K_FULL + (st ^ 1)), ((j + 1) >> 1) & 1, abort_flag);
+          ok = mbar_wait_all(BAR(K_FULL + (j + 1) % KST), ((j + 1) / KST) & 1, abort_flag);
           if (ok && j + 1 == clean_j) ok = mbar_wait_all(BAR(K_CLEAN), 0, abort_flag);
           if (ok) ok = mbar_wait_all(BAR(V_FULL + (st ^ 1)), ((j + 1) >> 1) & 1, abort_flag);
           if (!ok) break;
@@ -263,7 +268,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         if (!ok) break;
         tc_fence_after();
         issue_acc(1, j);
-        mma_commit(BAR(K_EMPTY + st), leader);
+        mma_commit(BAR(K_EMPTY + j % KST), leader);
         if (next) {
           issue_sdp(1, j + 1);
           mma_commit(BAR(V_EMPTY + (st ^ 1)), leader);
@@ -355,13 +360,21 @@ struct DkvCfg {
   static constexpr int TILE = SUB * 128 * 128;
   static constexpr int OFF_K = 0;
   static constexpr int OFF_V = TILE;
-  static constexpr int OFF_Q = 2 * TILE;            // 2 stages
-  static constexpr int OFF_DO = 4 * TILE;           // 2 stages
-  static constexpr int OFF_ROW = 6 * TILE;          // 2 stages x { float lse2[128]; float delta[128]; }
-  static constexpr int OFF_BAR = OFF_ROW + 2 * 2 * BM * 4;
-  // barriers: KV_FULL, QDO_FULL[2], QDO_EMPTY[2], SP_FULL[2], PDS_FULL[2], ACC_FULL
-  static constexpr int N_BAR = 10;
-  static constexpr int SMEM_BYTES = OFF_BAR + N_BAR * 8 + 16 + 1024;
+  // Q and dO travel as half tiles of 64 rows (a slot: Q | dO | lse2 | delta), the unit the issuer works in.  A slot is
+  // free as soon as its half has been accumulated, so that a load has a step and a half before it is wanted; two whole
+  // tiles gave it half a step, and the issuer waited for it.
+  static constexpr int HTILE = TILE / 2;
+  static constexpr int NS = D > 64 ? 5 : 6;
+  static constexpr int OFF_Q = 2 * TILE;
+  static constexpr int SLOT = 2 * HTILE;
+  static constexpr int OFF_ROW = OFF_Q + NS * SLOT;  // NS x { float lse2[64]; float delta[64]; }
+  static constexpr int OFF_BAR = OFF_ROW + NS * 2 * 64 * 4;
+  // barriers: KV_FULL, QDO_FULL[NS], QDO_EMPTY[NS], SP_FULL[2], PDS_FULL[2], ACC_FULL
+  static constexpr int N_BAR = 2 * NS + 6;
+  // alignment slack: the dynamic shared memory of a kernel without static one starts at a multiple of 1024; the kernel
+  // reports an error instead of running should it ever not
+  static constexpr int SLACK = 256;
+  static constexpr int SMEM_BYTES = OFF_BAR + N_BAR * 8 + 16 + SLACK;
   static constexpr int TMEM_COLS = 512;             // S^T 128 | dP^T 128 | dV D | dK D
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
   static_assert(2 * BM + 2 * D <= 512, "tensor memory has 512 columns");
@@ -373,12 +386,18 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                       const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                       const BwdParams p, const int order_w) {
   using C = DkvCfg<D>;
-  extern __shared__ unsigned char smem_unaligned[];
+  extern __shared__ __align__(1024) unsigned char smem_unaligned[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~uintptr_t(1023));
   const uint32_t sbase = uniform(smem_u32(smem));
   const uint32_t bar0 = sbase + C::OFF_BAR;
   auto BAR = [&](int i) { return bar0 + 8u * i; };
-  const int KV_FULL = 0, QDO_FULL = 1, QDO_EMPTY = 3, SP_FULL = 5, PDS_FULL = 7, ACC_FULL = 9;
+  constexpr int NS = C::NS;
+  const int KV_FULL = 0, QDO_FULL = 1, QDO_EMPTY = QDO_FULL + NS, SP_FULL = QDO_EMPTY + NS, PDS_FULL = SP_FULL + 2,
+            ACC_FULL = PDS_FULL + 2;
+  if (smem - smem_unaligned > C::SLACK) {
+    if (threadIdx.x == 0 && p.status) atomicExch(p.status, (int)PJX_ERR_CUDA);
+    return;
+  }
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::OFF_BAR + C::N_BAR * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* row_s = reinterpret_cast<float*>(smem + C::OFF_ROW);
@@ -428,21 +447,22 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         tma_load_4d(sbase + C::OFF_K + s * BN * 128, &tm_k, BAR(KV_FULL), s * 64, hk, k0, b);
         tma_load_4d(sbase + C::OFF_V + s * BN * 128, &tm_v, BAR(KV_FULL), s * 64, hk, k0, b);
       }
-      for (int it = 0; it < n; ++it) {
-        const int st = it & 1;
+      for (int hh = 0; hh < 2 * n; ++hh) {  // half tiles: step hh / 2, rows 64 (hh & 1) ..
+        const int st = hh % NS, it = hh >> 1;
         const int h = hk * G + it / n_t;
-        const int q0 = (t_lo + it % n_t) * BM;
-        if (!mbar_wait(BAR(QDO_EMPTY + st), ((it >> 1) & 1) ^ 1, abort_flag)) break;
-        mbar_arrive_expect_tx(BAR(QDO_FULL + st), 2 * C::TILE + 2 * BM * 4);
+        const int q0 = (t_lo + it % n_t) * BM + (hh & 1) * 64;
+        const uint32_t slot = sbase + C::OFF_Q + st * C::SLOT;
+        if (!mbar_wait(BAR(QDO_EMPTY + st), ((hh / NS) & 1) ^ 1, abort_flag)) break;
+        mbar_arrive_expect_tx(BAR(QDO_FULL + st), C::SLOT + 2 * 64 * 4);
 #pragma unroll
         for (int s = 0; s < C::SUB; ++s) {
-          tma_load_4d(sbase + C::OFF_Q + st * C::TILE + s * BM * 128, &tm_q, BAR(QDO_FULL + st), s * 64, h, q0, b);
-          tma_load_4d(sbase + C::OFF_DO + st * C::TILE + s * BM * 128, &tm_do, BAR(QDO_FULL + st), s * 64, h, q0, b);
+          tma_load_4d(slot + s * 64 * 128, &tm_q, BAR(QDO_FULL + st), s * 64, h, q0, b);
+          tma_load_4d(slot + C::HTILE + s * 64 * 128, &tm_do, BAR(QDO_FULL + st), s * 64, h, q0, b);
         }
-        // the 128 query rows' log-sum-exp (base 2) and delta out of the padded workspace arrays
+        // the query rows' log-sum-exp (base 2) and delta out of the padded workspace arrays
         const int64_t at = ((int64_t)b * p.Hq + h) * p.Lq_pad + q0;
-        bulk_load(sbase + C::OFF_ROW + st * 2 * BM * 4, p.lse2 + at, BM * 4, BAR(QDO_FULL + st));
-        bulk_load(sbase + C::OFF_ROW + st * 2 * BM * 4 + BM * 4, p.delta + at, BM * 4, BAR(QDO_FULL + st));
+        bulk_load(sbase + C::OFF_ROW + st * 512, p.lse2 + at, 256, BAR(QDO_FULL + st));
+        bulk_load(sbase + C::OFF_ROW + st * 512 + 256, p.delta + at, 256, BAR(QDO_FULL + st));
       }
     }
   } else if (warp == 1) {
@@ -455,44 +475,46 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       // S^T and dP^T of one half (64 query rows) of step `it`: keys on the lanes, query rows on
       // the columns; the B operands start 64 rows into the Q / dO tiles
       auto issue_sdp = [&](int half, int it) {
-        const uint32_t qa = sbase + C::OFF_Q + (it & 1) * C::TILE + half * 64 * 128;
-        const uint32_t doa = sbase + C::OFF_DO + (it & 1) * C::TILE + half * 64 * 128;
+        const uint32_t qa = sbase + C::OFF_Q + (2 * it + half) % NS * C::SLOT, doa = qa + C::HTILE;
 #pragma unroll
         for (int s = 0; s < C::SUB; ++s)
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
             mma_ss(T_S + half * 64, make_smem_desc(ka + s * BN * 128 + kk * 32, 16, 1024),
-                   make_smem_desc(qa + s * BM * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0, leader);
+                   make_smem_desc(qa + s * 64 * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0, leader);
 #pragma unroll
         for (int s = 0; s < C::SUB; ++s)
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
             mma_ss(T_DP + half * 64, make_smem_desc(va + s * BN * 128 + kk * 32, 16, 1024),
-                   make_smem_desc(doa + s * BM * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0, leader);
+                   make_smem_desc(doa + s * 64 * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0, leader);
         mma_commit(BAR(SP_FULL + half), leader);
       };
       // dV += P^T.dO and dK += dS^T.Q over one half: A from tensor memory (16-bit pairs at the
       // first 32 columns of the half), dO / Q tiles read MN-major
       auto issue_acc = [&](int half, int it) {
-        const uint32_t qa = sbase + C::OFF_Q + (it & 1) * C::TILE, doa = sbase + C::OFF_DO + (it & 1) * C::TILE;
+        const uint32_t qa = sbase + C::OFF_Q + (2 * it + half) % NS * C::SLOT, doa = qa + C::HTILE;
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
-          mma_ts(T_DV, T_S + half * 64 + kk * 8, make_smem_desc(doa + (half * 4 + kk) * 2048, BM * 128, 1024), idesc_acc,
+          mma_ts(T_DV, T_S + half * 64 + kk * 8, make_smem_desc(doa + kk * 2048, 64 * 128, 1024), idesc_acc,
                  (it | half | kk) != 0, leader);
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
-          mma_ts(T_DK, T_DP + half * 64 + kk * 8, make_smem_desc(qa + (half * 4 + kk) * 2048, BM * 128, 1024), idesc_acc,
+          mma_ts(T_DK, T_DP + half * 64 + kk * 8, make_smem_desc(qa + kk * 2048, 64 * 128, 1024), idesc_acc,
                  (it | half | kk) != 0, leader);
+        mma_commit(BAR(QDO_EMPTY + (2 * it + half) % NS), leader);
       };
+      auto half_landed = [&](int hh) { return mbar_wait_all(BAR(QDO_FULL + hh % NS), (hh / NS) & 1, abort_flag); };
       bool ok = mbar_wait_all(BAR(KV_FULL), 0, abort_flag);
-      if (ok) ok = mbar_wait_all(BAR(QDO_FULL), 0, abort_flag);
-      if (ok) {
-        tc_fence_after();
-        issue_sdp(0, 0);
-        issue_sdp(1, 0);
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        if (ok) ok = half_landed(half);
+        if (ok) {
+          tc_fence_after();
+          issue_sdp(half, 0);
+        }
       }
       for (int it = 0; ok && it < n; ++it) {
-        const int st = it & 1;
         const bool next = it + 1 < n;
         PJX_KTRACE(0, it, 0);
         ok = mbar_wait_all(BAR(PDS_FULL + 0), it & 1, abort_flag);
@@ -501,7 +523,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         PJX_KTRACE(0, it, 1);
         issue_acc(0, it);
         if (next) {
-          ok = mbar_wait_all(BAR(QDO_FULL + (st ^ 1)), ((it + 1) >> 1) & 1, abort_flag);
+          ok = half_landed(2 * it + 2);
           if (!ok) break;
           tc_fence_after();
           issue_sdp(0, it + 1);  // over P^T / dS^T of half 0, which the MMAs just issued consume first
@@ -511,8 +533,12 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         if (!ok) break;
         tc_fence_after();
         issue_acc(1, it);
-        mma_commit(BAR(QDO_EMPTY + st), leader);
-        if (next) issue_sdp(1, it + 1);
+        if (next) {
+          ok = half_landed(2 * it + 3);
+          if (!ok) break;
+          tc_fence_after();
+          issue_sdp(1, it + 1);
+        }
         PJX_KTRACE(0, it, 3);
       }
       if (ok) mma_commit(BAR(ACC_FULL), leader);
@@ -530,18 +556,18 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     const uint32_t s_addr = T_S + lane_sel + grp * 64, dp_addr = T_DP + lane_sel + grp * 64;
     bool ok = true;
     for (int it = 0; it < n; ++it) {
-      const int st = it & 1;
+      const int st = (2 * it + grp) % NS;
       const int q0 = (t_lo + it % n_t) * BM + grp * 64;  // first query row of this group's columns
       if (r_in == 64 && grp == 0) PJX_KTRACE(1, it, 0);
       ok = mbar_wait(BAR(SP_FULL + grp), it & 1, abort_flag);
       if (r_in == 64 && grp == 0) PJX_KTRACE(1, it, 1);
-      if (ok) ok = mbar_wait(BAR(QDO_FULL + st), (it >> 1) & 1, abort_flag);  // the row vectors landed with Q and dO
+      if (ok) ok = mbar_wait(BAR(QDO_FULL + st), ((2 * it + grp) / NS) & 1, abort_flag);  // the row vectors landed with Q and dO
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
       if (r_in == 64 && grp == 0) PJX_KTRACE(1, it, 2);
-      const float* lse2_s = row_s + st * 2 * BM + grp * 64;
-      const float* delta_s = lse2_s + BM;
+      const float* lse2_s = row_s + st * 128;
+      const float* delta_s = lse2_s + 64;
       // this key row against query rows q0 .. q0+63: visible iff q + band_lo <= key <= q + band_hi
       const bool need_mask = !key_ok || (key > q0 + p.band_hi) || (key < q0 + 63 + p.band_lo);
 #pragma unroll
@@ -633,6 +659,9 @@ int launch_both(const BwdParams& p, cudaStream_t stream) {
   kq<<<dim3((unsigned)n_dq), NTHREADS, DqCfg<D>::SMEM_BYTES, stream>>>(tq, tdo, tk, tv, p, order_w);
   count_launch();
   if ((rc = check_cuda(cudaGetLastError(), "sm100 dq launch"))) return rc;
+  // the dK/dV kernel takes Q and dO in halves of a tile
+  if ((rc = make_tmap_blhd(&tq, p.q, p.dtype, p.B, p.Lq, p.Hq, D, BM / 2))) return rc;
+  if ((rc = make_tmap_blhd(&tdo, p.d_o, p.dtype, p.B, p.Lq, p.Hq, D, BM / 2))) return rc;
   auto kk = bwd_dkdv_sm100_kernel<D, BF16>;
   if ((rc = check_cuda(cudaFuncSetAttribute(kk, cudaFuncAttributeMaxDynamicSharedMemorySize, DkvCfg<D>::SMEM_BYTES),
                        "cudaFuncSetAttribute(sm100 dk/dv)")))

@@ -339,24 +339,27 @@ template <int D, int DV, int FEAT>
 struct DqCfg {
   static constexpr int SUBQ = D / 64, SUBV = DV / 64;  // 64-element (128-byte) column blocks of a row
   static constexpr int TQ = SUBQ * 128 * 128, TV = SUBV * 128 * 128;  // bytes of a 128-row tile
-  static constexpr int KST = 2, VST = D > 128 ? 1 : 2;
+  // A K tile is held from its score products to its accumulation one step later and the next one is wanted half a step
+  // after that: three stages.  dO, the other operand that stays for the whole loop, sits in tensor memory (DV / 2
+  // columns, written once by the compute warps), which makes the room.
+  static constexpr int KST = 3, VST = D > 128 ? 1 : 2;
   static constexpr int OFF_Q = 0;
-  static constexpr int OFF_DO = TQ;
-  static constexpr int OFF_K = OFF_DO + TV;
+  static constexpr int OFF_K = TQ;
   static constexpr int OFF_V = OFF_K + KST * TQ;
   static constexpr int OFF_BIAS = OFF_V + VST * TV;                    // dense bias: a ring per compute warp
   static constexpr int OFF_BAR = OFF_BIAS + ((FEAT & 2) ? 8 * BIAS_RING<D> * BIAS_SLOT : 0);
-  // barriers: QDO_FULL, K_FULL[2], K_EMPTY[2], V_FULL[2], V_EMPTY[2], SP_FULL[2], DS_FULL[2], DQ_FULL, K_CLEAN
-  static constexpr int N_BAR = 15;
+  // barriers: Q_FULL, K_FULL[3], K_EMPTY[3], V_FULL[2], V_EMPTY[2], SP_FULL[2], DS_FULL[2], DQ_FULL, K_CLEAN, DO_READY
+  static constexpr int N_BAR = 18;
   static constexpr int SMEM_BYTES = OFF_BAR + N_BAR * 8 + 16 + 1024;
-  static constexpr int TMEM_COLS = 512;  // S 128 | dP 128 | dQ D
+  static constexpr int TMEM_COLS = 512;  // S 128 | dP 128 | dQ D | dO DV / 2
+  static_assert(2 * BN + D + DV / 2 <= 512, "tensor memory has 512 columns");
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
 };
 
 template <int D, int DV, bool BF16, int FEAT>
 __global__ void __launch_bounds__(NTHREADS, 1)
-bwd_dq_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
-                          const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
+bwd_dq_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                          const __grid_constant__ CUtensorMap tm_v,
                           const __grid_constant__ BwdParams p, const __grid_constant__ ExactArgs a) {
   using C = DqCfg<D, DV, FEAT>;
   extern __shared__ unsigned char smem_unaligned[];
@@ -364,8 +367,8 @@ bwd_dq_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
   const uint32_t sbase = uniform(smem_u32(smem));
   const uint32_t bar0 = sbase + C::OFF_BAR;
   auto BAR = [&](int i) { return bar0 + 8u * i; };
-  const int QDO_FULL = 0, K_FULL = 1, K_EMPTY = 3, V_FULL = 5, V_EMPTY = 7, SP_FULL = 9, DS_FULL = 11, DQ_FULL = 13,
-            K_CLEAN = 14;
+  const int Q_FULL = 0, K_FULL = 1, K_EMPTY = 4, V_FULL = 7, V_EMPTY = 9, SP_FULL = 11, DS_FULL = 13, DQ_FULL = 15, K_CLEAN = 16,
+            DO_READY = 17;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::OFF_BAR + C::N_BAR * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -403,7 +406,7 @@ bwd_dq_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < C::N_BAR; ++i)
-      mbar_init(BAR(i), i == K_CLEAN ? 32u : ((i == DS_FULL || i == DS_FULL + 1) ? 128u : 1u));
+      mbar_init(BAR(i), i == K_CLEAN ? 32u : ((i == DS_FULL || i == DS_FULL + 1) ? 128u : i == DO_READY ? 256u : 1u));
     *abort_flag = 0;
     fence_barrier_init();
   }
@@ -415,20 +418,17 @@ bwd_dq_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = uniform(*tmem_slot);
-  const uint32_t T_S = tmem, T_DP = tmem + BN, T_DQ = tmem + 2 * BN;
+  const uint32_t T_S = tmem, T_DP = tmem + BN, T_DQ = tmem + 2 * BN, T_DO = T_DQ + D;
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer
     if (lane == 0 && n > 0) {
       prefetch_tmap(&tm_q);
-      prefetch_tmap(&tm_do);
       prefetch_tmap(&tm_k);
       prefetch_tmap(&tm_v);
-      mbar_arrive_expect_tx(BAR(QDO_FULL), C::TQ + C::TV);
+      mbar_arrive_expect_tx(BAR(Q_FULL), C::TQ);
 #pragma unroll
-      for (int s = 0; s < C::SUBQ; ++s) tma_load_4d(sbase + C::OFF_Q + s * BM * 128, &tm_q, BAR(QDO_FULL), s * 64, h, q0, b);
-#pragma unroll
-      for (int s = 0; s < C::SUBV; ++s) tma_load_4d(sbase + C::OFF_DO + s * BM * 128, &tm_do, BAR(QDO_FULL), s * 64, h, q0, b);
+      for (int s = 0; s < C::SUBQ; ++s) tma_load_4d(sbase + C::OFF_Q + s * BM * 128, &tm_q, BAR(Q_FULL), s * 64, h, q0, b);
       for (int j = 0; j < n; ++j) {
         const int ks = j % C::KST, vs = j % C::VST;
         if (!mbar_wait(BAR(K_EMPTY + ks), ((j / C::KST) & 1) ^ 1, abort_flag)) break;
@@ -458,7 +458,7 @@ bwd_dq_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
       const uint32_t leader = elect_leader();
       constexpr uint32_t idesc_s = make_idesc(BM, BN / 2, BF16, false, false);
       constexpr uint32_t idesc_q = make_idesc(BM, D, BF16, false, true);
-      const uint32_t qa = sbase + C::OFF_Q, doa = sbase + C::OFF_DO;
+      const uint32_t qa = sbase + C::OFF_Q;
       // S and dP of one half (64 keys) of KV tile j
       auto issue_sdp = [&](int half, int j) {
         const uint32_t ka = sbase + C::OFF_K + (j % C::KST) * C::TQ + half * 64 * 128;
@@ -473,8 +473,8 @@ bwd_dq_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
         for (int s = 0; s < C::SUBV; ++s)
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
-            mma_ss(T_DP + half * 64, make_smem_desc(doa + s * BM * 128 + kk * 32, 16, 1024),
-                   make_smem_desc(va + s * BN * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0, leader);
+            mma_ts(T_DP + half * 64, T_DO + (s * 4 + kk) * 8, make_smem_desc(va + s * BN * 128 + kk * 32, 16, 1024), idesc_s,
+                   (s | kk) != 0, leader);
         mma_commit(BAR(SP_FULL + half), leader);
       };
       // dQ += (hi + lo of dS).K over one half, the K tile read MN-major
@@ -487,7 +487,8 @@ bwd_dq_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
           mma_ts(T_DQ, T_S + half * 64 + kk * CH + CH / 2, kd, idesc_q, true, leader);
         }
       };
-      bool ok = mbar_wait_all(BAR(QDO_FULL), 0, abort_flag);
+      bool ok = mbar_wait_all(BAR(Q_FULL), 0, abort_flag);
+      if (ok) ok = mbar_wait_all(BAR(DO_READY), 0, abort_flag);
       if (ok) ok = mbar_wait_all(BAR(K_FULL), 0, abort_flag);
       if (ok && clean_j == 0) ok = mbar_wait_all(BAR(K_CLEAN), 0, abort_flag);
       if (ok) ok = mbar_wait_all(BAR(V_FULL), 0, abort_flag);
@@ -531,6 +532,26 @@ bwd_dq_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     const int row = q0 + r_in;
     const bool row_ok = row < p.Lq;
     const uint32_t lane_sel = static_cast<uint32_t>(quarter * 32) << 16;
+    if (n > 0) {  // this group's half of the row's dO into tensor memory: the A operand of dP
+      const uint4* src = reinterpret_cast<const uint4*>(static_cast<const unsigned char*>(p.d_o) +
+                                                        (((int64_t)b * p.Lq + min(row, p.Lq - 1)) * p.Hq + h) * DV * 2) + grp * (DV / 16);
+#pragma unroll
+      for (int u = 0; u < DV / 64; ++u) {  // 16 columns (32 elements) at a time
+        uint32_t r[16];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint4 w = row_ok ? __ldg(src + u * 4 + i) : make_uint4(0u, 0u, 0u, 0u);
+          r[4 * i] = w.x;
+          r[4 * i + 1] = w.y;
+          r[4 * i + 2] = w.z;
+          r[4 * i + 3] = w.w;
+        }
+        tmem_st16(T_DO + lane_sel + grp * (DV / 4) + u * 16, r);
+      }
+      tmem_wait_st();
+      tc_fence_before();
+      mbar_arrive(BAR(DO_READY));
+    }
     const float c = p.sm_scale;
     const float pack = ds_pack_scale<DV, BF16>(a, p.mod);
     // padded per-row vectors: +inf / 0 for rows past Lq and +inf for rows without keys, so P = 0 there
@@ -636,17 +657,22 @@ struct DkvCfg {
   static constexpr int QT = D > 128 ? 96 : 128;      // query rows per step: S^T | dP^T | dV | dK fill tensor memory
   static constexpr int HALF = QT / 2;
   static constexpr int TK = SUBQ * BN * 128, TV = SUBV * BN * 128;
-  static constexpr int TQ = SUBQ * QT * 128, TDO = SUBV * QT * 128;
+  // Q and dO travel as half tiles (a slot: HALF rows of Q | of dO), the unit the issuer works in; a slot is free as soon
+  // as its half has been accumulated.
+  static constexpr int HQ = SUBQ * HALF * 128, HDO = SUBV * HALF * 128, SLOT = HQ + HDO;
+  static constexpr int NS = D > 128 || (D > 64 && (FEAT & 2)) ? 4 : D > 64 ? 5 : 6;
   static constexpr int OFF_K = 0;
   static constexpr int OFF_V = TK;
-  static constexpr int OFF_Q = OFF_V + TV;           // 2 stages
-  static constexpr int OFF_DO = OFF_Q + 2 * TQ;      // 2 stages
-  static constexpr int OFF_ROW = OFF_DO + 2 * TDO;   // 2 stages x { float lse[QT]; float delta[QT]; }
-  static constexpr int OFF_BIAS = OFF_ROW + 2 * 2 * QT * 4;
+  static constexpr int OFF_Q = OFF_V + TV;
+  static constexpr int OFF_ROW = OFF_Q + NS * SLOT;  // NS x { float lse[HALF]; float delta[HALF]; }
+  static constexpr int OFF_BIAS = OFF_ROW + NS * 2 * HALF * 4;
   static constexpr int OFF_BAR = OFF_BIAS + ((FEAT & 2) ? 8 * BIAS_RING<D> * BIAS_SLOT : 0);
-  // barriers: KV_FULL, QDO_FULL[2], QDO_EMPTY[2], SP_FULL[2], PDS_FULL[2], ACC_FULL
-  static constexpr int N_BAR = 10;
-  static constexpr int SMEM_BYTES = OFF_BAR + N_BAR * 8 + 16 + 896;  // 1024-byte alignment from a 128-byte one
+  // barriers: KV_FULL, QDO_FULL[NS], QDO_EMPTY[NS], SP_FULL[2], PDS_FULL[2], ACC_FULL
+  static constexpr int N_BAR = 2 * NS + 6;
+  // alignment slack: the dynamic shared memory of a kernel without static one starts at a multiple of 1024; the kernel
+  // reports an error instead of running should it ever not
+  static constexpr int SLACK = 256;
+  static constexpr int SMEM_BYTES = OFF_BAR + N_BAR * 8 + 16 + SLACK;
   static constexpr int TMEM_COLS = 512;              // S^T QT | dP^T QT | dV DV | dK D
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
   static_assert(2 * QT + DV + D <= 512, "tensor memory has 512 columns");
@@ -660,12 +686,18 @@ bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
                             const __grid_constant__ BwdParams p, const __grid_constant__ ExactArgs a) {
   using C = DkvCfg<D, DV, FEAT>;
   constexpr int QT = C::QT, HALF = C::HALF, NCH = HALF / CH;
-  extern __shared__ __align__(128) unsigned char smem_unaligned[];
+  extern __shared__ __align__(1024) unsigned char smem_unaligned[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~uintptr_t(1023));
   const uint32_t sbase = uniform(smem_u32(smem));
   const uint32_t bar0 = sbase + C::OFF_BAR;
   auto BAR = [&](int i) { return bar0 + 8u * i; };
-  const int KV_FULL = 0, QDO_FULL = 1, QDO_EMPTY = 3, SP_FULL = 5, PDS_FULL = 7, ACC_FULL = 9;
+  constexpr int NS = C::NS;
+  const int KV_FULL = 0, QDO_FULL = 1, QDO_EMPTY = QDO_FULL + NS, SP_FULL = QDO_EMPTY + NS, PDS_FULL = SP_FULL + 2,
+            ACC_FULL = PDS_FULL + 2;
+  if (smem - smem_unaligned > C::SLACK) {
+    if (threadIdx.x == 0 && p.status) atomicExch(p.status, (int)PJX_ERR_CUDA);
+    return;
+  }
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::OFF_BAR + C::N_BAR * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* row_s = reinterpret_cast<float*>(smem + C::OFF_ROW);
@@ -725,24 +757,25 @@ bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
       for (int s = 0; s < C::SUBQ; ++s) tma_load_4d(sbase + C::OFF_K + s * BN * 128, &tm_k, BAR(KV_FULL), s * 64, hk, k0, b);
 #pragma unroll
       for (int s = 0; s < C::SUBV; ++s) tma_load_4d(sbase + C::OFF_V + s * BN * 128, &tm_v, BAR(KV_FULL), s * 64, hk, k0, b);
-      for (int it = 0; it < n; ++it) {
-        const int st = it & 1;
+      for (int hh = 0; hh < 2 * n; ++hh) {  // half tiles: step hh / 2, rows HALF (hh & 1) ..
+        const int st = hh % NS, it = hh >> 1;
         const int h = hk * G + it / n_t;
-        const int q0 = (t_lo + it % n_t) * QT;
-        // the rows' log-sum-exp and delta out of the padded workspace arrays (a 96-row tile may reach past their
-        // padding: a multiple of 4 floats either way)
-        const int rows = QT == 128 ? 128 : min(QT, p.Lq_pad - q0);
-        if (!mbar_wait(BAR(QDO_EMPTY + st), ((it >> 1) & 1) ^ 1, abort_flag)) break;
-        mbar_arrive_expect_tx(BAR(QDO_FULL + st), C::TQ + C::TDO + 2 * rows * 4);
+        const int q0 = (t_lo + it % n_t) * QT + (hh & 1) * HALF;
+        const uint32_t slot = sbase + C::OFF_Q + st * C::SLOT, rows_at = sbase + C::OFF_ROW + st * 2 * HALF * 4;
+        // the rows' log-sum-exp and delta out of the padded workspace arrays (a 96-row tile may reach past their padding,
+        // or lie past it with its second half: a multiple of 4 floats either way)
+        const int rows = QT == 128 ? HALF : max(0, min(HALF, p.Lq_pad - q0));
+        if (!mbar_wait(BAR(QDO_EMPTY + st), ((hh / NS) & 1) ^ 1, abort_flag)) break;
+        mbar_arrive_expect_tx(BAR(QDO_FULL + st), C::SLOT + 2 * rows * 4);
 #pragma unroll
-        for (int s = 0; s < C::SUBQ; ++s)
-          tma_load_4d(sbase + C::OFF_Q + st * C::TQ + s * QT * 128, &tm_q, BAR(QDO_FULL + st), s * 64, h, q0, b);
+        for (int s = 0; s < C::SUBQ; ++s) tma_load_4d(slot + s * HALF * 128, &tm_q, BAR(QDO_FULL + st), s * 64, h, q0, b);
 #pragma unroll
-        for (int s = 0; s < C::SUBV; ++s)
-          tma_load_4d(sbase + C::OFF_DO + st * C::TDO + s * QT * 128, &tm_do, BAR(QDO_FULL + st), s * 64, h, q0, b);
-        const int64_t at = ((int64_t)b * p.Hq + h) * p.Lq_pad + q0;
-        bulk_load(sbase + C::OFF_ROW + st * 2 * QT * 4, p.lse2 + at, rows * 4, BAR(QDO_FULL + st));
-        bulk_load(sbase + C::OFF_ROW + st * 2 * QT * 4 + QT * 4, p.delta + at, rows * 4, BAR(QDO_FULL + st));
+        for (int s = 0; s < C::SUBV; ++s) tma_load_4d(slot + C::HQ + s * HALF * 128, &tm_do, BAR(QDO_FULL + st), s * 64, h, q0, b);
+        if (rows > 0) {
+          const int64_t at = ((int64_t)b * p.Hq + h) * p.Lq_pad + q0;
+          bulk_load(rows_at, p.lse2 + at, rows * 4, BAR(QDO_FULL + st));
+          bulk_load(rows_at + HALF * 4, p.delta + at, rows * 4, BAR(QDO_FULL + st));
+        }
       }
     }
   } else if (warp == 1) {
@@ -755,54 +788,56 @@ bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
       const uint32_t ka = sbase + C::OFF_K, va = sbase + C::OFF_V;
       // S^T and dP^T of one half of step `it`: keys on the lanes, query rows on the columns
       auto issue_sdp = [&](int half, int it) {
-        const uint32_t qa = sbase + C::OFF_Q + (it & 1) * C::TQ + half * HALF * 128;
-        const uint32_t doa = sbase + C::OFF_DO + (it & 1) * C::TDO + half * HALF * 128;
+        const uint32_t qa = sbase + C::OFF_Q + (2 * it + half) % NS * C::SLOT, doa = qa + C::HQ;
 #pragma unroll
         for (int s = 0; s < C::SUBQ; ++s)
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
             mma_ss(T_S + half * HALF, make_smem_desc(ka + s * BN * 128 + kk * 32, 16, 1024),
-                   make_smem_desc(qa + s * QT * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0, leader);
+                   make_smem_desc(qa + s * HALF * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0, leader);
 #pragma unroll
         for (int s = 0; s < C::SUBV; ++s)
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
             mma_ss(T_DP + half * HALF, make_smem_desc(va + s * BN * 128 + kk * 32, 16, 1024),
-                   make_smem_desc(doa + s * QT * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0, leader);
+                   make_smem_desc(doa + s * HALF * 128 + kk * 32, 16, 1024), idesc_s, (s | kk) != 0, leader);
         mma_commit(BAR(SP_FULL + half), leader);
       };
       // dV += (hi + lo of P^T).dO and dK += (hi + lo of dS^T).Q over one half, dO / Q tiles read MN-major
       auto issue_acc = [&](int half, int it) {
-        const uint32_t qa = sbase + C::OFF_Q + (it & 1) * C::TQ, doa = sbase + C::OFF_DO + (it & 1) * C::TDO;
+        const uint32_t qa = sbase + C::OFF_Q + (2 * it + half) % NS * C::SLOT, doa = qa + C::HQ;
 #pragma unroll
         for (int kk = 0; kk < NCH; ++kk) {
-          const uint64_t dd = make_smem_desc(doa + (half * NCH + kk) * 2048, QT * 128, 1024);
+          const uint64_t dd = make_smem_desc(doa + kk * 2048, HALF * 128, 1024);
           mma_ts(T_DV, T_S + half * HALF + kk * CH, dd, idesc_v, (it | half | kk) != 0, leader);
           mma_ts(T_DV, T_S + half * HALF + kk * CH + CH / 2, dd, idesc_v, true, leader);
         }
 #pragma unroll
         for (int kk = 0; kk < NCH; ++kk) {
-          const uint64_t qd = make_smem_desc(qa + (half * NCH + kk) * 2048, QT * 128, 1024);
+          const uint64_t qd = make_smem_desc(qa + kk * 2048, HALF * 128, 1024);
           mma_ts(T_DK, T_DP + half * HALF + kk * CH, qd, idesc_k, (it | half | kk) != 0, leader);
           mma_ts(T_DK, T_DP + half * HALF + kk * CH + CH / 2, qd, idesc_k, true, leader);
         }
+        mma_commit(BAR(QDO_EMPTY + (2 * it + half) % NS), leader);
       };
+      auto half_landed = [&](int hh) { return mbar_wait_all(BAR(QDO_FULL + hh % NS), (hh / NS) & 1, abort_flag); };
       bool ok = mbar_wait_all(BAR(KV_FULL), 0, abort_flag);
-      if (ok) ok = mbar_wait_all(BAR(QDO_FULL), 0, abort_flag);
-      if (ok) {
-        tc_fence_after();
-        issue_sdp(0, 0);
-        issue_sdp(1, 0);
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        if (ok) ok = half_landed(half);
+        if (ok) {
+          tc_fence_after();
+          issue_sdp(half, 0);
+        }
       }
       for (int it = 0; ok && it < n; ++it) {
-        const int st = it & 1;
         const bool next = it + 1 < n;
         ok = mbar_wait_all(BAR(PDS_FULL + 0), it & 1, abort_flag);
         if (!ok) break;
         tc_fence_after();
         issue_acc(0, it);
         if (next) {
-          ok = mbar_wait_all(BAR(QDO_FULL + (st ^ 1)), ((it + 1) >> 1) & 1, abort_flag);
+          ok = half_landed(2 * it + 2);
           if (!ok) break;
           tc_fence_after();
           issue_sdp(0, it + 1);  // over P^T / dS^T of half 0, which the MMAs just issued consume first
@@ -811,8 +846,12 @@ bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
         if (!ok) break;
         tc_fence_after();
         issue_acc(1, it);
-        mma_commit(BAR(QDO_EMPTY + st), leader);
-        if (next) issue_sdp(1, it + 1);
+        if (next) {
+          ok = half_landed(2 * it + 3);
+          if (!ok) break;
+          tc_fence_after();
+          issue_sdp(1, it + 1);
+        }
       }
       if (ok) mma_commit(BAR(ACC_FULL), leader);
     }
@@ -854,7 +893,7 @@ bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
     }
     bool ok = true;
     for (int it = 0; it < n; ++it) {
-      const int st = it & 1;
+      const int st = (2 * it + grp) % NS;
       const int q0 = (t_lo + it % n_t) * QT + grp * HALF;  // first query row of this group's columns
       bool mixed = false;
       if (it % n_t == 0) {  // the next query head of the group
@@ -868,12 +907,12 @@ bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
         if (mv.seg_q) mixed = segments_mixed(mv.seg_q, q0, HALF, p.Lq, own_seg, lane);
       }
       ok = mbar_wait(BAR(SP_FULL + grp), it & 1, abort_flag);
-      if (ok) ok = mbar_wait(BAR(QDO_FULL + st), (it >> 1) & 1, abort_flag);  // the row vectors landed with Q and dO
+      if (ok) ok = mbar_wait(BAR(QDO_FULL + st), ((2 * it + grp) / NS) & 1, abort_flag);  // the row vectors landed with Q and dO
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      const float* lse_s = row_s + st * 2 * QT + grp * HALF;
-      const float* delta_s = lse_s + QT;
+      const float* lse_s = row_s + st * 2 * HALF;
+      const float* delta_s = lse_s + HALF;
       float s_next[CH], dp_next[CH];
       tmem_ld16f(s_addr, s_next);
       tmem_ld16f(dp_addr, dp_next);
@@ -1208,15 +1247,11 @@ int launch_feat(const BwdParams& p, const ExactArgs& a, cudaStream_t stream) {
   if ((rc = make_tmap_blhd(&tdo, p.d_o, p.dtype, p.B, p.Lq, p.Hq, DV, BM))) return rc;
   if ((rc = make_tmap_blhd(&tk, p.k, p.dtype, p.B, p.Lkv, p.Hkv, D, BN))) return rc;
   if ((rc = make_tmap_blhd(&tv, p.v, p.dtype, p.B, p.Lkv, p.Hkv, DV, BN))) return rc;
-  tq2 = tq;
-  tdo2 = tdo;
-  if constexpr (KV::QT != BM) {
-    if ((rc = make_tmap_blhd(&tq2, p.q, p.dtype, p.B, p.Lq, p.Hq, D, KV::QT))) return rc;
-    if ((rc = make_tmap_blhd(&tdo2, p.d_o, p.dtype, p.B, p.Lq, p.Hq, DV, KV::QT))) return rc;
-  }
+  if ((rc = make_tmap_blhd(&tq2, p.q, p.dtype, p.B, p.Lq, p.Hq, D, KV::HALF))) return rc;
+  if ((rc = make_tmap_blhd(&tdo2, p.d_o, p.dtype, p.B, p.Lq, p.Hq, DV, KV::HALF))) return rc;
   const int64_t n_q = (p.Lq + BM - 1) / BM, n_k = (p.Lkv + BN - 1) / BN;
   if ((rc = launch_kernel(bwd_dq_exact_sm100_kernel<D, DV, BF16, FEAT>, n_q * p.Hq * p.B, Q::SMEM_BYTES, stream,
-                          "sm100 exact dq launch", tq, tdo, tk, tv, p, a)))
+                          "sm100 exact dq launch", tq, tk, tv, p, a)))
     return rc;
   if ((rc = launch_kernel(bwd_dkdv_exact_sm100_kernel<D, DV, BF16, FEAT>, n_k * p.Hkv * p.B, KV::SMEM_BYTES, stream,
                           "sm100 exact dk/dv launch", tq2, tdo2, tk, tv, p, a)))

@@ -40,14 +40,17 @@ def _ptr(t) -> Optional[int]:
 
 
 def _stream(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    """Handle of the current CUDA stream of ``device`` (the raw accessor: no Stream object per call)."""
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
 def _status_word(device) -> torch.Tensor:
-    key = torch.device(device).index or 0
-    if key not in _status_words:
-        _status_words[key] = torch.zeros(1, dtype=torch.int32, device=device)
-    return _status_words[key]
+    key = device.index or 0
+    word = _status_words.get(key)
+    if word is None:
+        word = _status_words[key] = torch.zeros(1, dtype=torch.int32, device=device)
+    return word
 
 
 def check_status(device=None) -> None:
@@ -65,7 +68,6 @@ def _scratch_bytes(device, tag: str, nbytes: int) -> torch.Tensor:
     (device, CUDA stream, purpose): calls issued on different streams never share scratch, and a
     buffer that is outgrown is only dropped by the stream that owns it, whose earlier kernels
     are ordered before anything that reuses the memory."""
-    device = torch.device(device)
     key = (device.index or 0, _stream(device), tag)
     buf = _scratch.get(key)
     if buf is None or buf.numel() < nbytes:
@@ -127,10 +129,16 @@ def _result(given, shape, dtype, device, pin=False):
     return torch.empty(shape, dtype=dtype, device=device)
 
 
+_gpu_seen = False  # a CUDA device was there once: the query (a driver call) is not repeated per call
+
+
 def _require_gpu():
+    global _gpu_seen
     _lib.lib()  # raises when the library is not built
-    if not torch.cuda.is_available():
-        raise RuntimeError("probjax_b200 needs a CUDA device (sm_100a); there is no CPU path")
+    if not _gpu_seen:
+        if not torch.cuda.is_available():
+            raise RuntimeError("probjax_b200 needs a CUDA device (sm_100a); there is no CPU path")
+        _gpu_seen = True
 
 
 def _gqa_group(hq: int, hkv: int) -> int:
@@ -379,6 +387,7 @@ class _AttentionFunction(torch.autograd.Function):
         ctx.save_for_forward(q, k, v, lse)
         ctx.args = (band, kv_lengths, bias, sm_scale, impl, mods)
         ctx.mark_non_differentiable(lse)
+        ctx.set_materialize_grads(False)  # no zero-filled gradient of the log-sum-exp per call
         return o, lse
 
     @staticmethod
@@ -392,6 +401,8 @@ class _AttentionFunction(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, d_o, _d_lse):
+        if d_o is None:
+            return (None,) * 9
         q, k, v, o, lse = ctx.saved_tensors
         band, kv_lengths, bias, sm_scale, impl, mods = ctx.args
         want_dbias = bias is not None and ctx.needs_input_grad[5]

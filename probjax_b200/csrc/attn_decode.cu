@@ -455,6 +455,68 @@ __global__ void combine_splits_kernel(const DecodeParams p) {
     p.lse[decode_lse_index(p, sq, h, t)] = denom > 0.f ? (msafe + log2f(denom)) * kLn2 : INFINITY;
 }
 
+// The same for a balanced latent decode: the splits of a sequence are numbered by the device-side plan.  Their weights are
+// computed once, one split per thread, and the rows are read four splits at a time.
+template <typename TO>
+__global__ void __launch_bounds__(128) combine_balanced_kernel(const DecodeParams p) {
+  __shared__ float w_s[kBalancedMaxItems];
+  __shared__ float red[4];
+  const int r = blockIdx.x, hk = blockIdx.y, b = blockIdx.z, tid = threadIdx.x;
+  const BalancedPlan plan = balanced_plan(p);  // (reads the lengths only: before the wait for the split kernel)
+  int ns = 0, first = 0;
+#pragma unroll
+  for (int i = 0; i < kBalancedMaxSeqs / 32; ++i)
+    if (b / 32 == i) {
+      ns = __shfl_sync(0xffffffffu, plan.n[i], b % 32);
+      first = __shfl_sync(0xffffffffu, plan.first[i], b % 32);
+    }
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  const int64_t base = (int64_t)hk * p.balanced + first;
+  auto reduce = [&](float x, bool maximum) {
+#pragma unroll
+    for (int o = 16; o > 0; o /= 2) {
+      const float y = __shfl_xor_sync(0xffffffffu, x, o);
+      x = maximum ? fmaxf(x, y) : x + y;
+    }
+    __syncthreads();
+    if ((tid & 31) == 0) red[tid >> 5] = x;
+    __syncthreads();
+    return maximum ? fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3])) : (red[0] + red[1]) + (red[2] + red[3]);
+  };
+  float m = -INFINITY;
+  for (int s = tid; s < ns; s += 128) {
+    const float l = p.lse_part[(base + s) * p.rows + r];
+    w_s[s] = l;
+    m = fmaxf(m, l);
+  }
+  m = reduce(m, true);
+  const float msafe = (m == -INFINITY) ? 0.f : m;
+  float denom = 0.f;
+  for (int s = tid; s < ns; s += 128) {
+    const float w = exp2f(w_s[s] - msafe);
+    w_s[s] = w;
+    denom += w;
+  }
+  denom = reduce(denom, false);  // (its barriers also publish the weights)
+  const float inv = denom > 0.f ? 1.f / denom : 0.f;
+  const int G = p.Hq / p.Hkv;
+  const int h = hk * G + r / p.Lq, t = r % p.Lq;
+  TO* o = static_cast<TO*>(p.o) + (((int64_t)b * p.Lq + t) * p.Hq + h) * p.Dv;
+  const float* part = p.o_part + (base * p.rows + r) * p.Dv;
+  const int64_t step = (int64_t)p.rows * p.Dv;
+  for (int d = tid; d < p.Dv; d += 128) {
+    float acc = 0.f;
+    int s = 0;
+    for (; s + 4 <= ns; s += 4) {
+      const float x0 = part[s * step + d], x1 = part[(s + 1) * step + d], x2 = part[(s + 2) * step + d], x3 = part[(s + 3) * step + d];
+      acc = fmaf(w_s[s + 3], x3, fmaf(w_s[s + 2], x2, fmaf(w_s[s + 1], x1, fmaf(w_s[s], x0, acc))));
+    }
+    for (; s < ns; ++s) acc = fmaf(w_s[s], part[s * step + d], acc);
+    o[d] = Elem<TO>::from_f(acc * inv);
+  }
+  if (p.lse && tid == 0) p.lse[((int64_t)b * p.Hq + h) * p.Lq + t] = denom > 0.f ? (msafe + log2f(denom)) * kLn2 : INFINITY;
+}
+
 // Combine of n_parts partials laid out [n_parts, n_rows, Dv] with natural-log LSEs.
 template <typename TO>
 __global__ void combine_parts_kernel(const float* __restrict__ o_parts, const float* __restrict__ lse_parts,
@@ -604,7 +666,7 @@ template <typename TO>
 cudaError_t launch_combine_splits(const DecodeParams& p, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(p.rows, p.Hkv, p.B);
-  cfg.blockDim = dim3(p.Dv >= 128 ? 128 : 64);
+  cfg.blockDim = dim3(p.balanced || p.Dv >= 128 ? 128 : 64);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
@@ -612,6 +674,7 @@ cudaError_t launch_combine_splits(const DecodeParams& p, cudaStream_t stream) {
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  if (p.balanced) return cudaLaunchKernelEx(&cfg, combine_balanced_kernel<TO>, p);
   return cudaLaunchKernelEx(&cfg, combine_splits_kernel<TO>, p);
 }
 

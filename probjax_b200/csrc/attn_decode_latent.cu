@@ -60,12 +60,10 @@ __global__ void __launch_bounds__(LTHR, 1) decode_latent_kernel(const DecodePara
   const uint32_t sbase = smem_u32(smem_raw);
   float* red = reinterpret_cast<float*>(smem_raw + C::OFF_RED);
 
-  const int split = blockIdx.x, grp = blockIdx.y;
-  const DecodeSeq sq = decode_seq(p, blockIdx.z);
-  const int b = sq.cache_b, len = sq.len;
-  const int start = split * p.split_len;
-  if (start >= len) return;  // the combine never reads this split
-  const int end = min(len, start + p.split_len);
+  const int grp = blockIdx.y;
+  LatentItem item;
+  if (!latent_item(p, item)) return;
+  const int b = item.b, start = item.start, end = item.end;
   // the combine of the splits, next on the stream, may become resident as SM slots free up (it waits
   // for this grid before it reads a partial)
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
@@ -108,7 +106,7 @@ __global__ void __launch_bounds__(LTHR, 1) decode_latent_kernel(const DecodePara
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
       if (r < p.rows) {
         const int g = r / p.Lq, t = r % p.Lq;
-        v = *reinterpret_cast<const uint4*>(q + ((sq.q_b * p.Lq + t) * p.Hq + grp * G + g) * R + c * 8);
+        v = *reinterpret_cast<const uint4*>(q + ((item.q_b * p.Lq + t) * p.Hq + grp * G + g) * R + c * 8);
       }
       *reinterpret_cast<uint4*>(smem_raw + C::OFF_Q + lswz(r, c, C::ROW_BYTES)) = v;
     }
@@ -255,7 +253,7 @@ __global__ void __launch_bounds__(LTHR, 1) decode_latent_kernel(const DecodePara
     lsum[0] += red[LWARPS * 16 + w * 16 + row_lo];
     lsum[1] += red[LWARPS * 16 + w * 16 + row_lo + 8];
   }
-  const int64_t part = (((int64_t)blockIdx.z * p.Hkv + grp) * p.num_splits + split) * p.rows;
+  const int64_t part = item.part;
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const int r = row_lo + 8 * h;
@@ -278,7 +276,7 @@ int launch_latent_t(const DecodeParams& p, cudaStream_t stream) {
   int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM),
                       "cudaFuncSetAttribute(latent decode)");
   if (rc) return rc;
-  kern<<<dim3(p.num_splits, p.Hkv, p.B), LTHR, C::SMEM, stream>>>(p);
+  kern<<<latent_grid(p), LTHR, C::SMEM, stream>>>(p);
   count_launch();
   return check_cuda(cudaGetLastError(), "latent decode launch");
 }

@@ -154,12 +154,10 @@ decode_latent_tc_kernel(const __grid_constant__ CUtensorMap tm_c, const DecodePa
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* red = reinterpret_cast<float*>(smem + C::OFF_RED);
 
-  const int split = blockIdx.x, grp = blockIdx.y;
-  const DecodeSeq sq = decode_seq(p, blockIdx.z);
-  const int b = sq.cache_b, len = sq.len;
-  const int start = split * p.split_len;
-  if (start >= len) return;  // the combine never reads this split
-  const int end = min(len, start + p.split_len);
+  const int grp = blockIdx.y;
+  LatentItem item;
+  if (!latent_item(p, item)) return;
+  const int b = item.b, start = item.start, end = item.end;
   // the combine of the splits, next on the stream, may become resident as SM slots free up (it waits
   // for this grid before it reads a partial)
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
@@ -187,7 +185,7 @@ decode_latent_tc_kernel(const __grid_constant__ CUtensorMap tm_c, const DecodePa
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
       if (r < p.rows) {
         const int g = r / p.Lq, t = r % p.Lq;
-        v = *reinterpret_cast<const uint4*>(q + ((sq.q_b * p.Lq + t) * p.Hq + grp * G + g) * R + c * 8);
+        v = *reinterpret_cast<const uint4*>(q + ((item.q_b * p.Lq + t) * p.Hq + grp * G + g) * R + c * 8);
       }
       const int sub = c >> 3, ch = c & 7;
       *reinterpret_cast<uint4*>(smem + C::OFF_Q + sub * 2048 + r * 128 + ((ch ^ (r & 7)) << 4)) = v;
@@ -423,7 +421,7 @@ decode_latent_tc_kernel(const __grid_constant__ CUtensorMap tm_c, const DecodePa
           inv[h] = ls > 0.f ? 1.f / ls : 0.f;
           if (h == kl) lsum_mine = ls;
         }
-        const int64_t part = (((int64_t)blockIdx.z * p.Hkv + grp) * p.num_splits + split) * p.rows;
+        const int64_t part = item.part;
 #pragma unroll
         for (int m = 0; m < NBLK; ++m) {
           float o[NROW];
@@ -463,7 +461,7 @@ int launch_tc_t(const DecodeParams& p, int dtype, cudaStream_t stream) {
   rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM),
                   "cudaFuncSetAttribute(latent decode, tcgen05)");
   if (rc) return rc;
-  kern<<<dim3(p.num_splits, p.Hkv, p.B), TC_THREADS, C::SMEM, stream>>>(tm, p);
+  kern<<<latent_grid(p), TC_THREADS, C::SMEM, stream>>>(tm, p);
   count_launch();
   return check_cuda(cudaGetLastError(), "latent decode (tcgen05) launch");
 }

@@ -552,6 +552,11 @@ int pjx_mla_decode_absorbed_impl(const void* q, const void* cache, const int32_t
   if (p.split_len < 64 || p.split_len % 64 != 0)
     return fail(PJX_ERR_BAD_ARG, "split_len must be a positive multiple of 64 (got %d)", p.split_len);
   p.num_splits = (capacity + p.split_len - 1) / p.split_len;
+  // Lengths given and no split length asked for: as many splits in all as equal ones over the capacity would be (about
+  // one per SM), cut on the device from the valid lengths.  Equal splits of the capacity leave the CTAs past a sequence's
+  // end without work: with lengths of 2k to 32k keys 83 of 144 had any, 115 us; balanced 79 us (B16 H16 R576).
+  if (split_len == 0 && kv_lengths && p.num_splits > 1 && B <= kBalancedMaxSeqs && B * p.num_splits <= kBalancedMaxItems)
+    p.balanced = B * p.num_splits;
   const size_t need = pjx_mla_decode_workspace_bytes(B, Lq, H, R, capacity, p.split_len);
   if (!workspace || workspace_bytes < need)
     return fail(PJX_ERR_WORKSPACE, "mla decode workspace: need %zu bytes, got %zu", need, workspace ? workspace_bytes : (size_t)0);

@@ -113,7 +113,12 @@ struct DecodeParams {
   // t = seq_first + z % seq_tokens of seq_total, and sees the keys below t + seq_visible (and below
   // the cache row's valid length); its partials are indexed by z, its output by (cache row, t).
   int seq_tokens = 0, seq_first = 0, seq_total = 0, seq_visible = 0;
+  // Latent decode over ragged sequences (balanced > 0): the split length is chosen on the device from the valid lengths
+  // (balanced_plan below) so that `balanced` splits in all cover the batch; grid x walks them, partials are indexed by it.
+  int balanced = 0;
 };
+constexpr int kBalancedMaxSeqs = 128;   // sequences the device-side plan takes (4 per lane)
+constexpr int kBalancedMaxItems = 256;  // splits of one row group
 
 // What grid index z of a decode launch stands for (see DecodeParams::seq_tokens).
 struct DecodeSeq {
@@ -139,6 +144,93 @@ __device__ __forceinline__ DecodeSeq decode_seq(const DecodeParams& p, int z) {
   }
   s.len = p.kv_lengths ? max(0, min(lim, p.kv_lengths[s.cache_b])) : lim;
   return s;
+}
+
+// Plan of a balanced decode, computed by every warp that needs it (all 32 lanes): the smallest split length, a multiple
+// of 128 keys, with which the batch has at most p.balanced splits.  Splits are numbered through the batch.
+struct BalancedPlan {
+  int split_len;
+  int n[kBalancedMaxSeqs / 32];      // splits of sequence lane + 32 i
+  int first[kBalancedMaxSeqs / 32];  // number of its first split
+};
+__device__ __forceinline__ BalancedPlan balanced_plan(const DecodeParams& p) {
+  constexpr int PER = kBalancedMaxSeqs / 32;
+  const int lane = threadIdx.x & 31;
+  BalancedPlan r;
+  int len[PER], total = 0;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int b = lane + 32 * i;
+    len[i] = b < p.B ? max(0, min(p.capacity, p.kv_lengths[b])) : 0;
+    total += (len[i] + 127) / 128;
+  }
+  total = __reduce_add_sync(0xffffffffu, total);  // blocks of 128 keys
+  int unit = max(2, (total + p.balanced - 1) / p.balanced);
+  while (true) {  // ends: p.balanced >= B, and a split length of the longest sequence gives one split each
+    int cnt = 0;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      r.n[i] = (len[i] + unit * 128 - 1) / (unit * 128);
+      cnt += r.n[i];
+    }
+    if (static_cast<int>(__reduce_add_sync(0xffffffffu, cnt)) <= p.balanced) break;
+    unit += max(1, unit / 16);
+  }
+  r.split_len = unit * 128;
+  int before = 0;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    int incl = r.n[i];
+#pragma unroll
+    for (int o = 1; o < 32; o *= 2) {
+      const int up = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += up;
+    }
+    r.first[i] = before + incl - r.n[i];
+    before += __shfl_sync(0xffffffffu, incl, 31);
+  }
+  return r;
+}
+
+// What CTA (x, y, z) of a latent split kernel does.  False: nothing (a split past the sequence's end).
+struct LatentItem {
+  int b;          // batch row of the cache
+  int64_t q_b;    // row of q / o
+  int start, end; // keys
+  int64_t part;   // row of its first partial
+};
+__device__ __forceinline__ bool latent_item(const DecodeParams& p, LatentItem& it) {
+  if (p.balanced) {
+    const BalancedPlan plan = balanced_plan(p);
+    const int x = blockIdx.x;
+    int b = -1, first = 0;
+#pragma unroll
+    for (int i = 0; i < kBalancedMaxSeqs / 32; ++i) {
+      const unsigned mine = __ballot_sync(0xffffffffu, x >= plan.first[i] && x < plan.first[i] + plan.n[i]);
+      if (mine) {
+        b = __ffs(mine) - 1 + 32 * i;
+        first = __shfl_sync(0xffffffffu, plan.first[i], __ffs(mine) - 1);
+      }
+    }
+    if (b < 0) return false;
+    it.b = b;
+    it.q_b = b;
+    it.start = (x - first) * plan.split_len;
+    it.end = min(max(0, min(p.capacity, p.kv_lengths[b])), it.start + plan.split_len);
+    it.part = ((int64_t)blockIdx.y * p.balanced + x) * p.rows;
+    return true;
+  }
+  const DecodeSeq sq = decode_seq(p, blockIdx.z);
+  it.b = sq.cache_b;
+  it.q_b = sq.q_b;
+  it.start = blockIdx.x * p.split_len;
+  if (it.start >= sq.len) return false;  // the combine never reads this split
+  it.end = min(sq.len, it.start + p.split_len);
+  it.part = (((int64_t)blockIdx.z * p.Hkv + blockIdx.y) * p.num_splits + blockIdx.x) * p.rows;
+  return true;
+}
+inline dim3 latent_grid(const DecodeParams& p) {
+  return p.balanced ? dim3(p.balanced, p.Hkv, 1) : dim3(p.num_splits, p.Hkv, p.B);
 }
 
 // Index of the LSE of (sequence, head, token of the launch) in the caller's [B, Hq, Lq] array.

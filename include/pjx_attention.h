@@ -180,11 +180,12 @@ int pjx_attn_bwd(const void* q, const void* k, const void* v, const void* o, con
                  int Lkv, int Hq, int Hkv, int D, int Dv, int dtype, int causal, float sm_scale,
                  void* workspace, size_t workspace_bytes, void* stream);
 /* The same for the band form of the mask (see pjx_attn_fwd_band).  `impl` picks the
- * kernels as in the forward: AUTO runs the tcgen05 dQ and dK/dV kernels for 16-bit
- * inputs with D = Dv in {64, 128} and no bias, the CUDA-core kernels otherwise;
+ * kernels as in the forward: AUTO runs tcgen05 kernels for 16-bit inputs with D = Dv in
+ * {64, 128} (with a dense bias too) or (D, Dv) = (192, 128) without one, the CUDA-core kernels
+ * otherwise; SM100 forces the plain tcgen05 kernels (D = Dv in {64, 128}, no bias).
  * `status` as in pjx_attn_fwd.  `dbias` (float32, shape and strides of `bias`, or NULL) receives
- * the gradient of a learnable dense bias, summed over the axes the bias broadcasts (with
- * atomic adds there, so that sum is not bit-repeatable). */
+ * the gradient of a learnable dense bias, summed over the axes the bias broadcasts: in a fixed order
+ * by the tcgen05 kernels, with atomic adds (not bit-repeatable) by the CUDA-core ones. */
 int pjx_attn_bwd_band(const void* q, const void* k, const void* v, const void* o, const float* lse,
                       const void* d_o, void* dq, void* dk, void* dv, const int32_t* kv_lengths,
                       const float* bias, int64_t bias_batch_stride, int64_t bias_head_stride,

@@ -17,7 +17,7 @@
 //   tiles of 96 rows (two halves of 48: 2 x 96 + 320 = 512 columns) instead of 128.
 // * a segment mask cuts the tile loops to the ranges that can match (one range per 128 rows, both ways).
 // * a dense bias is read with keys on the lanes (coalesced) in the dK/dV and dbias kernels; the dQ kernel,
-//   whose threads own query rows, transposes it through a per-warp window in shared memory.
+//   whose threads own query rows, transposes it through its ring in shared memory.
 // * the gradient of the bias is a kernel of its own: one CTA per 128 x 128 tile of the bias, walking the
 //   (batch, head) pairs that share it and summing dS in registers in a fixed order (no atomics).
 //
@@ -28,11 +28,12 @@
 // the natural log-sum-exp, subtracted before the change of base, so that an entry of the type's lowest value
 // cannot overflow to inf - inf.
 //
-// Bound by the MMA issue stream at D = 128 and by the element work of the compute warps at D = 64.
+// Bound by the element work of the compute warps at D = 64 and with modifiers (20 to 30 issue slots per score), by the
+// chain of MMAs, element work and barrier round trips at D = 128 and 192 without.
 // Measured (forward + backward, against the CUDA-core kernels these calls ran on before; B200):
-//   packed documents + ALiBi, B1 S4096 Hq32 Hkv8 D128 bf16     41.9 ms -> 0.52 ms
-//   dense bias with gradient, B8 S1024 H16 D64 bf16            6.26 ms -> 0.59 ms
-//   latent training step, B2 S2048 H16 (192,128) bf16          16.6 ms -> 0.65 ms
+//   packed documents + ALiBi, B1 S4096 Hq32 Hkv8 D128 bf16     41.9 ms -> 0.48 ms
+//   dense bias with gradient, B8 S1024 H16 D64 bf16            6.26 ms -> 0.49 ms
+//   latent training step, B2 S2048 H16 (192,128) bf16          16.6 ms -> 0.42 ms
 #include "attn_bwd_sm100.cuh"
 
 namespace pjx {
@@ -56,6 +57,7 @@ struct ExactArgs {
   const int32_t* k_range;  // [nb, ceil(Lkv/128), 2]: query rows a key tile is seen by, or null
   int64_t q_range_bs, k_range_bs;  // batch strides in tiles (0 = shared)
   const uint32_t* amax;    // fp16: bit patterns of max|dO|, max|V|, max|head_scale|
+  bool bias_vec;           // rows of the dense bias are whole aligned 16-byte units
   float p_scale;           // fp16: factor P is packed with (a power of two); 1 for bf16
 };
 
@@ -93,10 +95,11 @@ __device__ __forceinline__ void split_pack(const float2 (&x)[CH / 2], float scal
   }
 }
 
-// Dense bias: a ring of CH-column chunks per compute warp (2 KB each: 32 lanes x 16 values), filled by 4-byte
-// asynchronous copies (rows of the bias may start at any element) a half step (D = 64) or two chunks (D = 128, where the
-// tiles leave no more room) ahead of their use.  Loads into registers one chunk ahead did not cover the L2 latency:
-// 600 to 1900 cycles per chunk against 350 without a bias.
+// Dense bias: a ring of CH-column chunks per compute warp (2 KB each: 32 lanes x 16 values), filled by asynchronous copies
+// a half step (D = 64) or two chunks (D = 128, where the tiles leave no more room) ahead of their use.  Loads into
+// registers one chunk ahead did not cover the L2 latency: 600 to 1900 cycles per chunk against 350 without a bias.  Rows
+// of whole aligned 16-byte units are copied in such units, four copies per lane and chunk; others (an odd number of keys)
+// 4 bytes at a time, sixteen.
 template <int D>
 constexpr int BIAS_RING = D > 64 ? 2 : 4;
 constexpr int BIAS_SLOT = 32 * CH * 4;
@@ -115,32 +118,61 @@ __device__ __forceinline__ float lds(uint32_t addr) {
   return x;
 }
 
-// Keys on the lanes: this lane's key (`src` is at its column), rows i0 .. i0 + CH - 1, clamped to the tensor.
-__device__ __forceinline__ void fetch_bias_column(uint32_t slot, const float* src, int i0, int Lq, int Lkv, int lane) {
-  const float* ptr = src + (int64_t)min(i0, Lq - 1) * Lkv;
+__device__ __forceinline__ void copy16_async(uint32_t dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+}
+
+// Keys on the lanes: keys key0 .. key0 + 31, rows i0 .. i0 + CH - 1 of a plane, rows and keys past the tensor clamped (their
+// values are masked).  Slot layout [CH rows][32 keys].
+__device__ __forceinline__ void fetch_bias_column(uint32_t slot, const float* plane, int key0, int i0, int Lq, int Lkv, bool vec, int lane) {
+  if (vec) {
+    const float* src = plane + min(key0 + 4 * (lane & 7), Lkv - 4);
 #pragma unroll
-  for (int e = 0; e < CH; ++e) {
-    copy4_async(slot + (e * 32 + lane) * 4, ptr);
-    ptr += i0 + e + 1 < Lq ? Lkv : 0;
+    for (int e = 0; e < 4; ++e) {
+      const int row = 4 * e + (lane >> 3);
+      copy16_async(slot + row * 128 + (lane & 7) * 16, src + (int64_t)min(i0 + row, Lq - 1) * Lkv);
+    }
+  } else {
+    const float* ptr = plane + min(key0 + lane, Lkv - 1) + (int64_t)min(i0, Lq - 1) * Lkv;
+#pragma unroll
+    for (int e = 0; e < CH; ++e) {
+      copy4_async(slot + (e * 32 + lane) * 4, ptr);
+      ptr += i0 + e + 1 < Lq ? Lkv : 0;
+    }
   }
 }
 __device__ __forceinline__ void read_bias_column(uint32_t slot, int lane, float (&out)[CH]) {
 #pragma unroll
   for (int e = 0; e < CH; ++e) out[e] = lds(slot + (e * 32 + lane) * 4);
 }
-// Rows on the lanes: rows r0 .. r0 + 31 of keys j0 .. j0 + CH - 1, copied two rows at a time (64 contiguous bytes each)
-// and read a row per lane; element (r, k) is stored at column k ^ (r / 2), which keeps both free of bank conflicts.
-__device__ __forceinline__ void fetch_bias_rows(uint32_t slot, const float* plane, int r0, int j0, int Lq, int Lkv, int lane) {
-  const int k = lane & 15, key = min(j0 + k, Lkv - 1);
+// Rows on the lanes: rows r0 .. r0 + 31 of keys j0 .. j0 + CH - 1, read a row per lane.  Slot layout [32 rows][4 units of 16
+// bytes], unit c of row r at c ^ (r / 2 % 4): free of bank conflicts both ways.
+__device__ __forceinline__ void fetch_bias_rows(uint32_t slot, const float* plane, int r0, int j0, int Lq, int Lkv, bool vec, int lane) {
+  if (vec) {
+    const int c = lane & 3;
+    const float* src = plane + min(j0 + 4 * c, Lkv - 4);
 #pragma unroll
-  for (int e = 0; e < CH; ++e) {
-    const int r = 2 * e + (lane >> 4);
-    copy4_async(slot + (r * CH + (k ^ e)) * 4, plane + (int64_t)min(r0 + r, Lq - 1) * Lkv + key);
+    for (int e = 0; e < 4; ++e) {
+      const int r = 8 * e + (lane >> 2);
+      copy16_async(slot + r * 64 + (c ^ ((r >> 1) & 3)) * 16, src + (int64_t)min(r0 + r, Lq - 1) * Lkv);
+    }
+  } else {
+    const int k = lane & 15;
+    const float* src = plane + min(j0 + k, Lkv - 1);
+#pragma unroll
+    for (int e = 0; e < CH; ++e) {
+      const int r = 2 * e + (lane >> 4);
+      copy4_async(slot + r * 64 + ((k >> 2) ^ ((r >> 1) & 3)) * 16 + (k & 3) * 4, src + (int64_t)min(r0 + r, Lq - 1) * Lkv);
+    }
   }
 }
 __device__ __forceinline__ void read_bias_row(uint32_t slot, int lane, float (&out)[CH]) {
 #pragma unroll
-  for (int e = 0; e < CH; ++e) out[e] = lds(slot + (lane * CH + (e ^ (lane >> 1))) * 4);
+  for (int c = 0; c < 4; ++c)
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(out[4 * c]), "=f"(out[4 * c + 1]), "=f"(out[4 * c + 2]), "=f"(out[4 * c + 3])
+                 : "r"(slot + lane * 64 + (c ^ ((lane >> 1) & 3)) * 16)
+                 : "memory");
 }
 
 // Chunks of a half step in straight line; with modifiers as a loop, whose code stays in the instruction cache.
@@ -571,7 +603,7 @@ bwd_dq_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     auto fetch_bias = [&](int t) {  // chunk t of this warp: CH keys, four chunks per tile
       if (t < 4 * n)
         fetch_bias_rows(ring + (t % NB) * BIAS_SLOT, bsrc, q0 + quarter * 32, (j_lo + t / 4) * BN + grp * 64 + (t % 4) * CH, p.Lq,
-                        p.Lkv, lane);
+                        p.Lkv, a.bias_vec, lane);
       copy_commit();
     };
     if constexpr ((FEAT & 2) != 0) {
@@ -873,11 +905,11 @@ bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
     // dense bias: position of the next chunk to fetch (chunk of the half, query tile, head of the group)
     [[maybe_unused]] int f_cc = 0, f_t = 0, f_g = 0;
     [[maybe_unused]] const float* bsrc =
-        (FEAT & 2) ? p.bias + (int64_t)b * p.bias_bs + (int64_t)hk * G * p.bias_hs + min(key, p.Lkv - 1) : nullptr;
+        (FEAT & 2) ? p.bias + (int64_t)b * p.bias_bs + (int64_t)hk * G * p.bias_hs : nullptr;
     auto fetch_bias = [&](int slot) {
       if (f_g < G && n > 0)
-        fetch_bias_column(ring + slot * BIAS_SLOT, bsrc + (int64_t)f_g * p.bias_hs, (t_lo + f_t) * QT + grp * HALF + f_cc * CH, p.Lq,
-                          p.Lkv, lane);
+        fetch_bias_column(ring + slot * BIAS_SLOT, bsrc + (int64_t)f_g * p.bias_hs, k0 + quarter * 32,
+                          (t_lo + f_t) * QT + grp * HALF + f_cc * CH, p.Lq, p.Lkv, a.bias_vec, lane);
       copy_commit();
       if (++f_cc == NCH) {
         f_cc = 0;
@@ -927,7 +959,9 @@ bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
         }
         if constexpr ((FEAT & 2) != 0) {
           copy_wait<NB - 1>();
-          read_bias_column(ring + (cc % NB) * BIAS_SLOT, lane, bias);  // this lane's own copies
+          __syncwarp();
+          read_bias_column(ring + (cc % NB) * BIAS_SLOT, lane, bias);
+          __syncwarp();  // the slot has been read by all lanes
           fetch_bias(cc % NB);
         }
         tmem_wait_ld();
@@ -1302,6 +1336,7 @@ int launch_bwd_exact_sm100(const BwdParams& p, void* scratch, cudaStream_t strea
   ExactArgs a = {};
   a.order_w = (p.band_hi < PJX_BAND_NO_UPPER && p.band_lo == PJX_BAND_NO_LOWER) ? 16 : 1;
   a.p_scale = 1.f;
+  a.bias_vec = p.bias && p.Lkv % 4 == 0 && p.bias_bs % 4 == 0 && p.bias_hs % 4 == 0 && (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0;
   uint32_t* amax = static_cast<uint32_t*>(scratch);
   int rc;
   if (p.dtype == PJX_F16) {

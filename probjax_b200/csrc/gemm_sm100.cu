@@ -279,7 +279,7 @@ gemm_tn_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
 //   else:   dw_p [n_p, K] = dy_p [M, n_p]^T . x [M, K]          the tiles of both products in one launch
 // Persistent CTAs over 128 x TN output tiles, a TMA lane, an MMA lane and four epilogue warps with the accumulator
 // double buffered, as above.  Tiles of 192 columns where they cover the width with less padding (576 = 3 x 192).
-// Measured there (both layers): dx 51 -> @DX@ us, dw 61 -> @DW@ us, and no copies.
+// Measured there (both layers): dx 51 -> 33 us, dw 61 -> 30 us, and no copies.
 // ---------------------------------------------------------------------------------------------
 struct GradArgs {
   void* c[2];      // CHAIN: c[0] only

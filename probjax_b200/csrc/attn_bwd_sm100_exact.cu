@@ -3,10 +3,10 @@
 // latent head shape (192, 128).  Same two-kernel split, warp roles and half-step issue order as
 // attn_bwd_sm100.cu (dQ owns query tiles, dK/dV owns key tiles, no atomics); what differs:
 //
-// * P and dS enter the accumulating products as a sum of two 16-bit numbers, x = hi + lo with
-//   hi = round16(x) and lo = round16(x - hi): two MMAs against the same B descriptor instead of one.  The
-//   calls that arrive here ran on CUDA cores with P and dS in fp32 before, and 16 + 16 bits keep what that
-//   gave (2^-17 relative in bf16 against the 2^-9 of the stored gradients).  Per 128 x 128 tile that is 10
+// * P and dS enter the accumulating products as a sum of two 16-bit numbers, x = hi + lo with hi the upper 16
+//   bits of x (bf16) or its rounding (fp16) and lo = round16(x - hi): two MMAs against the same B descriptor
+//   instead of one.  The calls that arrive here ran on CUDA cores with P and dS in fp32 before, and 16 + 16 bits
+//   keep what that gave (2^-16 relative in bf16 against the 2^-9 of the stored gradients).  Per 128 x 128 tile that is 10
 //   products of 128 x 128 x D for both kernels instead of 7.  A 16-column chunk of scores (16 columns of
 //   tensor memory) is overwritten by its own 8 columns of hi and 8 of lo pairs, so the split costs no
 //   tensor memory.

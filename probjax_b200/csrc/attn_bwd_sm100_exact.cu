@@ -10,9 +10,13 @@
 //   products of 128 x 128 x D for both kernels instead of 7.  A 16-column chunk of scores (16 columns of
 //   tensor memory) is overwritten by its own 8 columns of hi and 8 of lo pairs, so the split costs no
 //   tensor memory.
-// * fp16 has no exponent range to spare for lo: P is packed scaled by a power of two (`p_scale`), dS by one
-//   derived from max|dO| and max|V| (`bwd_amax_kernel`), and the accumulators are scaled back when they
-//   leave tensor memory.
+// * fp16 has no exponent range to spare for lo (its lowest step is 2^-24): what a thread packs belongs to one row of
+//   the accumulator it feeds, so every row has a power of two of its own, undone when the accumulators leave tensor
+//   memory.  dQ: from the row's |dO|, its delta and the longest V row of the key tiles it walks (`v_norm_kernel`).  dK
+//   and dV: from the largest P and the largest term of dS of the key over all rows and heads that see it, which the dQ
+//   kernel collects on its way (`add_col_max`).  One power of two for the whole call, from the largest |dO| and |V|,
+//   took the bits of every row far below the largest: beside a row of dO 1e6 times larger the others' dQ was off by 40
+//   to 120 times its rounding.
 // * head shape (192, 128): dV and dK take 320 columns of tensor memory, so the dK/dV kernel walks query
 //   tiles of 96 rows (two halves of 48: 2 x 96 + 320 = 512 columns) instead of 128.
 // * a segment mask cuts the tile loops to the ranges that can match (one range per 128 rows, both ways).
@@ -56,22 +60,45 @@ struct ExactArgs {
   const int32_t* q_range;  // [nb, ceil(Lq/128), 2]: keys a query tile can see (segments), or null
   const int32_t* k_range;  // [nb, ceil(Lkv/128), 2]: query rows a key tile is seen by, or null
   int64_t q_range_bs, k_range_bs;  // batch strides in tiles (0 = shared)
-  const uint32_t* amax;    // fp16: bit patterns of max|dO|, max|V|, max|head_scale|
+  const float* v_norm;     // fp16: longest finite V row of each key tile, [B, Hkv, ceil(Lkv/128)]
+  uint32_t* col_max;       // fp16: per key the largest term of dS and the largest P, bit patterns, [B, Hkv, 2, Lkv]
   bool bias_vec;           // rows of the dense bias are whole aligned 16-byte units
-  float p_scale;           // fp16: factor P is packed with (a power of two); 1 for bf16
 };
 
-// fp16: the power of two dS is packed with.  |dS| <= P (|dP| + |delta|) |ds'/ds| and both |dP| and |delta| are at
-// most keep * Dv * max|dO| * max|V|, so the packed values stay below 2^15.
-template <int DV, bool BF16>
-__device__ __forceinline__ float ds_pack_scale(const ExactArgs& a, const ScoreMod& m) {
-  if constexpr (BF16) return 1.f;
-  const float keep = m.dropout_rate > 0.f ? 1.f / (1.f - m.dropout_rate) : 1.f;
-  const float bound = 2.f * keep * DV * __uint_as_float(a.amax[0]) * __uint_as_float(a.amax[1]) *
-                      (1.f + __uint_as_float(a.amax[2]));
-  if (!(bound > 0.f)) return 1.f;
-  const int e = (int)((__float_as_uint(bound) >> 23) & 255u) - 127;  // bound in [2^e, 2^(e+1))
-  return exp2f((float)max(-100, min(100, 14 - e)));
+// fp16: the power of two that takes `bound` into [2^top, 2^(top+1)); 1 where there is no positive finite bound.
+__device__ __forceinline__ float pack_scale(float bound, int top) {
+  const int e = (int)(__float_as_uint(bound) >> 23);  // (never negative: 255 is inf or NaN)
+  if (!(bound > 0.f) || e == 255) return 1.f;
+  return __uint_as_float((uint32_t)(127 + max(-126, min(126, top + 127 - e))) << 23);
+}
+
+// fp16: largest magnitudes of a chunk's CH keys over the warp's 32 query rows, added to those of the keys: of dS (together
+// with P dP, the term its difference is formed from: where the two cancel the result is rounding noise of that
+// size, another one in the dK/dV kernel) and of P.  The upper halves of the fp32 words order like the values; both are
+// reduced at once, each step leaving a lane half of the columns.  `out` points at the chunk's first key.
+__device__ __forceinline__ void add_col_max(const float2 (&pr)[CH / 2], const float2 (&ds)[CH / 2], const float (&dp)[CH],
+                                            uint32_t* out, int n_cols, int Lkv, int lane) {
+  uint32_t v[CH];
+#pragma unroll
+  for (int i = 0; i < CH / 2; ++i) {
+    // (fmaxf drops a NaN: of a masked entry, 0 times a dP that may be anything)
+    const float x = fmaxf(fabsf(ds[i].x), fabsf(pr[i].x * dp[2 * i])), y = fmaxf(fabsf(ds[i].y), fabsf(pr[i].y * dp[2 * i + 1]));
+    v[2 * i] = __byte_perm(__float_as_uint(pr[i].x), __float_as_uint(x), 0x7632) & 0x7fff7fffu;
+    v[2 * i + 1] = __byte_perm(__float_as_uint(pr[i].y), __float_as_uint(y), 0x7632) & 0x7fff7fffu;
+  }
+#pragma unroll
+  for (int w = CH / 2; w >= 1; w /= 2) {
+    const bool upper = lane & w;
+#pragma unroll
+    for (int i = 0; i < w; ++i) {
+      const uint32_t other = __shfl_xor_sync(0xffffffffu, upper ? v[i] : v[i + w], w);
+      v[i] = __vmaxu2(upper ? v[i + w] : v[i], other);
+    }
+  }
+  const uint32_t m = __vmaxu2(v[0], __shfl_xor_sync(0xffffffffu, v[0], CH));  // of key lane % CH
+  const uint32_t mine = lane < CH ? m & 0xffff0000u : m << 16;                // dS in the lower lanes, P in the upper
+  const int col = lane % CH;
+  if (mine && col < n_cols) atomicMax(out + (lane < CH ? 0 : Lkv) + col, mine);
 }
 
 // A chunk of CH fp32 values as hi pairs (8 registers) and lo pairs (8 registers).  bf16 truncates hi (the upper half of
@@ -564,31 +591,62 @@ bwd_dq_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     const int row = q0 + r_in;
     const bool row_ok = row < p.Lq;
     const uint32_t lane_sel = static_cast<uint32_t>(quarter * 32) << 16;
+    [[maybe_unused]] float do_sq[2] = {0.f, 0.f};  // fp16: sum of squares of this group's half of the row's dO, of the other's
     if (n > 0) {  // this group's half of the row's dO into tensor memory: the A operand of dP
       const uint4* src = reinterpret_cast<const uint4*>(static_cast<const unsigned char*>(p.d_o) +
-                                                        (((int64_t)b * p.Lq + min(row, p.Lq - 1)) * p.Hq + h) * DV * 2) + grp * (DV / 16);
+                                                        (((int64_t)b * p.Lq + min(row, p.Lq - 1)) * p.Hq + h) * DV * 2);
 #pragma unroll
-      for (int u = 0; u < DV / 64; ++u) {  // 16 columns (32 elements) at a time
-        uint32_t r[16];
+      for (int side = 0; side < (BF16 ? 1 : 2); ++side) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const uint4 w = row_ok ? __ldg(src + u * 4 + i) : make_uint4(0u, 0u, 0u, 0u);
-          r[4 * i] = w.x;
-          r[4 * i + 1] = w.y;
-          r[4 * i + 2] = w.z;
-          r[4 * i + 3] = w.w;
+        for (int u = 0; u < DV / 64; ++u) {  // 16 columns (32 elements) at a time
+          uint32_t r[16];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const uint4 w = row_ok ? __ldg(src + (side ? 1 - grp : grp) * (DV / 16) + u * 4 + i) : make_uint4(0u, 0u, 0u, 0u);
+            r[4 * i] = w.x;
+            r[4 * i + 1] = w.y;
+            r[4 * i + 2] = w.z;
+            r[4 * i + 3] = w.w;
+          }
+          if (side == 0) tmem_st16(T_DO + lane_sel + grp * (DV / 4) + u * 16, r);
+          if constexpr (!BF16) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&r[i]));
+              do_sq[side] = fmaf(f.x, f.x, fmaf(f.y, f.y, do_sq[side]));
+            }
+          }
         }
-        tmem_st16(T_DO + lane_sel + grp * (DV / 4) + u * 16, r);
       }
       tmem_wait_st();
       tc_fence_before();
       mbar_arrive(BAR(DO_READY));
     }
     const float c = p.sm_scale;
-    const float pack = ds_pack_scale<DV, BF16>(a, p.mod);
     // padded per-row vectors: +inf / 0 for rows past Lq and +inf for rows without keys, so P = 0 there
     const int64_t at = ((int64_t)b * p.Hq + h) * p.Lq_pad + row;
     const float lse = p.lse2[at], delta = p.delta[at];
+    // fp16: |dS| <= P (keep |dO||v_j| + |delta|) |ds'/ds|, packed below 2^15; the two groups, which share the row of the
+    // accumulator, arrive at the same value (the sum of the halves does not depend on their order)
+    float pack = 1.f;
+    [[maybe_unused]] uint32_t* col_max = nullptr;
+    if constexpr (!BF16) {
+      col_max = a.col_max + ((int64_t)b * p.Hkv + hk) * 2 * p.Lkv;
+      const float* norms = a.v_norm + ((int64_t)b * p.Hkv + hk) * ((p.Lkv + BN - 1) / BN) + j_lo;
+      float v_max = 0.f;
+      for (int t = lane; t < n; t += 32) v_max = fmaxf(v_max, __ldg(norms + t));
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v_max = fmaxf(v_max, __shfl_xor_sync(0xffffffffu, v_max, o));
+      float bound = sqrtf(do_sq[0] + do_sq[1]) * v_max;
+      if constexpr ((FEAT & 4) != 0) {
+        if (p.mod.dropout_rate > 0.f) bound /= 1.f - p.mod.dropout_rate;
+      }
+      bound += fabsf(delta);
+      if constexpr ((FEAT & 4) != 0) {  // ds'/ds is head_scale, or under a cap between head_scale - 1 and head_scale
+        if (p.mod.head_scale) bound *= 1.f + fabsf(p.mod.head_scale[h]);
+      }
+      pack = pack_scale(bound, 14);
+    }
     const uint32_t s_addr = T_S + lane_sel + grp * 64, dp_addr = T_DP + lane_sel + grp * 64;
     const Place pl = {kv_len, p.Lq, p.Lkv, p.band_lo, p.band_hi};
     ScoreModView mv = {};
@@ -648,6 +706,7 @@ bwd_dq_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
         const int j0 = k0 + cc * CH;
         const uint32_t keep = keep_bits<FEAT, true>(pl, mv, mixed, own_seg, row, j0);
         chunk_p_ds<FEAT, true>(s, dp, c, pl, mv, keep, row, j0, &lse, &delta, bias, pr, ds);
+        if constexpr (!BF16) add_col_max(pr, ds, dp, col_max + j0, p.Lkv - j0, p.Lkv, lane);
         uint32_t pk[CH];
         split_pack<BF16>(ds, pack, pk);
         tmem_st16(s_addr + cc * CH, pk);  // over the chunk's own scores, which were read already
@@ -895,7 +954,13 @@ bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
     const int key = k0 + r_in;
     const uint32_t lane_sel = static_cast<uint32_t>(quarter * 32) << 16;
     const float c = p.sm_scale;
-    const float pack = ds_pack_scale<DV, BF16>(a, p.mod);
+    // fp16: the key's own scales; two bits more room than the dQ kernel's maxima, whose products summed in another order
+    float pack = 1.f, pack_p = 1.f;
+    if constexpr (!BF16) {
+      const uint32_t* col_max = a.col_max + ((int64_t)b * p.Hkv + hk) * 2 * p.Lkv + min(key, p.Lkv - 1);
+      pack = pack_scale(__uint_as_float(col_max[0]), 12);
+      pack_p = pack_scale(__uint_as_float(col_max[p.Lkv]), 12);
+    }
     const uint32_t s_addr = T_S + lane_sel + grp * HALF, dp_addr = T_DP + lane_sel + grp * HALF;
     const Place pl = {kv_len, p.Lq, p.Lkv, p.band_lo, p.band_hi};
     ScoreModView mv = {};
@@ -979,7 +1044,7 @@ bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
         const uint32_t keep = keep_bits<FEAT, false>(pl, mv, mixed, own_seg, i0, key);
         chunk_p_ds<FEAT, false>(s, dp, c, pl, mv, keep, i0, key, lse, delta, bias, pr, ds);
         uint32_t pk[CH];
-        split_pack<BF16>(pr, a.p_scale, pk);
+        split_pack<BF16>(pr, pack_p, pk);
         tmem_st16(s_addr + cc * CH, pk);  // over the chunk's own scores, which were read already
         split_pack<BF16>(ds, pack, pk);
         tmem_st16(dp_addr + cc * CH, pk);
@@ -999,7 +1064,7 @@ bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
         const bool row_ok = key < p.Lkv;
         const int64_t at = ((int64_t)b * p.Lkv + key) * p.Hkv + hk;
         // group 0 stores the dV row, group 1 the dK row
-        if (grp == 0) store_row<DV, BF16>(T_DV + lane_sel, static_cast<unsigned char*>(p.dv) + at * DV * 2, 1.f / a.p_scale, n > 0, row_ok);
+        if (grp == 0) store_row<DV, BF16>(T_DV + lane_sel, static_cast<unsigned char*>(p.dv) + at * DV * 2, 1.f / pack_p, n > 0, row_ok);
         else store_row<D, BF16>(T_DK + lane_sel, static_cast<unsigned char*>(p.dk) + at * D * 2, p.sm_scale / pack, n > 0, row_ok);
       }
     }
@@ -1228,37 +1293,42 @@ bwd_dbias_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
 }
 
 // ---------------------------------------------------------------------------------------------
-// fp16: largest finite |dO|, |V| (valid keys only) and |head_scale|, as bit patterns (non-negative
-// floats order like their bits)
+// fp16: the longest V row (2-norm) of each key tile, rows past the valid length and rows that are not finite left out
 // ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ float amax8(uint4 w, float m) {
-  const uint32_t r[4] = {w.x, w.y, w.z, w.w};
+template <int DV>
+__global__ void __launch_bounds__(256) v_norm_kernel(const BwdParams p, float* out) {
+  constexpr int LPR = DV / 8, ROWS = 256 / LPR;  // lanes per row (16 bytes each), rows at a time
+  __shared__ float warp_max[8];
+  const int n_kt = (p.Lkv + BN - 1) / BN;
+  const int k0 = (int)(blockIdx.x % n_kt) * BN, pair = blockIdx.x / n_kt;
+  const int hk = pair % p.Hkv, b = pair / p.Hkv;
+  const int u = threadIdx.x % LPR;
+  const int k_end = min(min(k0 + BN, p.Lkv), p.kv_lengths ? p.kv_lengths[b] : p.Lkv);
+  float m = 0.f;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&r[i]));
-    const float x = fabsf(f.x), y = fabsf(f.y);
-    if (x < INFINITY) m = fmaxf(m, x);  // not for inf, nor for NaN
-    if (y < INFINITY) m = fmaxf(m, y);
+  for (int r = 0; r < BN / ROWS; ++r) {
+    const int j = k0 + r * ROWS + (int)threadIdx.x / LPR;
+    float sq = 0.f;
+    if (j < k_end) {
+      const uint4 w = __ldg(static_cast<const uint4*>(p.v) + (((int64_t)b * p.Lkv + j) * p.Hkv + hk) * LPR + u);
+      const uint32_t x[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&x[i]));
+        sq = fmaf(f.x, f.x, fmaf(f.y, f.y, sq));
+      }
+    }
+#pragma unroll
+    for (int o = LPR / 2; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+    if (sq < INFINITY) m = fmaxf(m, sq);  // not for inf, nor for NaN
   }
-  return m;
-}
-
-__global__ void __launch_bounds__(256) bwd_amax_kernel(const BwdParams p, uint32_t* out) {
-  const int64_t step = (int64_t)gridDim.x * blockDim.x, first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t n_o = (int64_t)p.B * p.Lq * p.Hq * p.Dv / 8, row_v = (int64_t)p.Hkv * p.Dv / 8, n_v = (int64_t)p.B * p.Lkv * row_v;
-  float m[3] = {0.f, 0.f, 0.f};
-  for (int64_t i = first; i < n_o; i += step) m[0] = amax8(static_cast<const uint4*>(p.d_o)[i], m[0]);
-  for (int64_t i = first; i < n_v; i += step) {
-    const int64_t t = i / row_v;
-    if (p.kv_lengths && (int)(t % p.Lkv) >= p.kv_lengths[t / p.Lkv]) continue;
-    m[1] = amax8(static_cast<const uint4*>(p.v)[i], m[1]);
-  }
-  if (p.mod.head_scale && first < p.Hq && fabsf(p.mod.head_scale[first]) < INFINITY) m[2] = fabsf(p.mod.head_scale[first]);
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m[k] = fmaxf(m[k], __shfl_xor_sync(0xffffffffu, m[k], o));
-    if ((threadIdx.x & 31) == 0 && m[k] > 0.f) atomicMax(out + k, __float_as_uint(m[k]));
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if (threadIdx.x % 32 == 0) warp_max[threadIdx.x / 32] = m;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int i = 1; i < 8; ++i) m = fmaxf(m, warp_max[i]);
+    out[blockIdx.x] = sqrtf(m);
   }
 }
 
@@ -1331,28 +1401,31 @@ bool bwd_exact_sm100_supported(const BwdParams& p) {
   return true;
 }
 
-// Bytes of stream-ordered scratch: segment ranges both ways and the three fp16 maxima.
+// Scratch: [fp16: longest V rows | maxima of the keys] [segment ranges both ways], 4-byte words.
+static size_t fp16_words(const BwdParams& p) {
+  return p.dtype == PJX_F16 ? (size_t)p.B * p.Hkv * ((p.Lkv + BN - 1) / BN + 2 * (size_t)p.Lkv) : 0;
+}
+
 int launch_bwd_exact_sm100(const BwdParams& p, void* scratch, cudaStream_t stream) {
   ExactArgs a = {};
   a.order_w = (p.band_hi < PJX_BAND_NO_UPPER && p.band_lo == PJX_BAND_NO_LOWER) ? 16 : 1;
-  a.p_scale = 1.f;
   a.bias_vec = p.bias && p.Lkv % 4 == 0 && p.bias_bs % 4 == 0 && p.bias_hs % 4 == 0 && (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0;
-  uint32_t* amax = static_cast<uint32_t*>(scratch);
   int rc;
   if (p.dtype == PJX_F16) {
-    if ((rc = check_cuda(cudaMemsetAsync(amax, 0, 16, stream), "clear maxima"))) return rc;
-    const int64_t n = ((int64_t)p.B * p.Lq * p.Hq * p.Dv / 8 + 255) / 256;
-    bwd_amax_kernel<<<(unsigned)(n < 592 ? n : 592), 256, 0, stream>>>(p, amax);
+    const size_t tiles = (size_t)p.B * p.Hkv * ((p.Lkv + BN - 1) / BN);
+    float* norms = static_cast<float*>(scratch);
+    a.v_norm = norms;
+    a.col_max = static_cast<uint32_t*>(scratch) + tiles;
+    if ((rc = check_cuda(cudaMemsetAsync(a.col_max, 0, (fp16_words(p) - tiles) * 4, stream), "clear maxima"))) return rc;
+    if (p.Dv == 64) v_norm_kernel<64><<<(unsigned)tiles, 256, 0, stream>>>(p, norms);
+    else v_norm_kernel<128><<<(unsigned)tiles, 256, 0, stream>>>(p, norms);
     count_launch();
-    if ((rc = check_cuda(cudaGetLastError(), "backward amax launch"))) return rc;
-    a.amax = amax;
-    a.p_scale = 16384.f;  // P <= 1 / (1 - rate): below 2^15 once scaled
-    for (float keep = 1.f / (1.f - p.mod.dropout_rate); keep > 1.f && a.p_scale > 0x1p-14f; keep *= 0.5f) a.p_scale *= 0.5f;
+    if ((rc = check_cuda(cudaGetLastError(), "backward V norm launch"))) return rc;
   }
   if (bwd_exact_uses_ranges(p)) {
     const int n_q = (p.Lq + BM - 1) / BM, n_k = (p.Lkv + BN - 1) / BN;
     const int nb = (p.mod.seg_q_bs == 0 && p.mod.seg_k_bs == 0) ? 1 : p.B;
-    int32_t* qr = static_cast<int32_t*>(scratch) + 4;
+    int32_t* qr = static_cast<int32_t*>(scratch) + fp16_words(p);
     int32_t* kr = qr + (int64_t)nb * n_q * 2;
     launch_seg_tile_range(p.mod.seg_q, p.mod.seg_k, p.mod.seg_q_bs, p.mod.seg_k_bs, p.Lq, p.Lkv, n_q, nb, qr, stream);
     launch_seg_tile_range(p.mod.seg_k, p.mod.seg_q, p.mod.seg_k_bs, p.mod.seg_q_bs, p.Lkv, p.Lq, n_k, nb, kr, stream);
@@ -1371,8 +1444,7 @@ bool bwd_exact_uses_ranges(const BwdParams& p) {
 }
 
 size_t bwd_exact_scratch_bytes(const BwdParams& p) {
-  if (p.dtype != PJX_F16 && !bwd_exact_uses_ranges(p)) return 0;
-  size_t n = 16;
+  size_t n = fp16_words(p) * 4;
   if (bwd_exact_uses_ranges(p)) n += (size_t)p.B * ((p.Lq + BM - 1) / BM + (p.Lkv + BN - 1) / BN) * 2 * sizeof(int32_t);
   return n;
 }

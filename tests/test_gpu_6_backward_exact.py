@@ -139,3 +139,97 @@ def test_fp16_gradients_far_from_one():
     """fp16 packs P and dS scaled: output gradients of 1e-3 and of 100 keep what fp32 arithmetic gave."""
     for scale in (1e-3, 1.0, 100.0):
         _compare(2, 200, 300, 4, 2, 64, 64, torch.float16, bias=M.SymmetricAlibiBias(), grad_scale=scale)
+
+
+# ------------------------------------------------------------------------------------------- against float64
+
+
+def _float64_backward(q, k, v, o, lse, g, keep, sm_scale, bias=None):
+    """Gradients in float64 from the residuals the kernels get, ``keep [B, 1|H, Lq, Lkv]``, and for each of dq, dk, dv
+    what fp32 arithmetic may add to it: 2^-20 (sums of D <= 192 products, the exponential, and sums over the keys, a
+    dozen roundings of 2^-24) of the sum of the magnitudes of its terms, P |dP| and P |delta| before they cancel."""
+    G = q.shape[2] // k.shape[2]
+    qd, od, gd = (t.double().transpose(1, 2) for t in (q, o, g))
+    kd, vd = (t.double().transpose(1, 2).repeat_interleave(G, 1) for t in (k, v))
+    s = qd @ kd.transpose(2, 3) * sm_scale
+    if bias is not None:
+        s = s + bias.double()
+    p = torch.where(keep, torch.exp(s - lse.double()[..., None]), 0.0)
+    dp, delta = gd @ vd.transpose(2, 3), (od * gd).sum(3, keepdim=True)
+    ds, mag = p * (dp - delta), p * (dp.abs() + delta.abs())
+
+    def per_key_head(x):
+        return x.unflatten(1, (-1, G)).sum(2).transpose(1, 2)
+
+    want = [(ds @ kd * sm_scale).transpose(1, 2), per_key_head(ds.transpose(2, 3) @ qd * sm_scale), per_key_head(p.transpose(2, 3) @ gd)]
+    noise = [(mag @ kd.abs() * sm_scale).transpose(1, 2), per_key_head(mag.transpose(2, 3) @ qd.abs() * sm_scale),
+             per_key_head(p.transpose(2, 3) @ gd.abs())]
+    return want, [2.0**-20 * n for n in noise]
+
+
+def _segment_ids(lengths):
+    return torch.repeat_interleave(torch.arange(len(lengths), dtype=torch.int32), torch.tensor(lengths))[None].repeat(2, 1)
+
+
+@pytest.mark.parametrize("d,dv", [(64, 64), (128, 128), (192, 128)])
+@pytest.mark.parametrize("spread", [1e3, 1e6])
+@pytest.mark.parametrize("where", ["row", "head", "sequence", "value", "uniform"])
+def test_fp16_rows_keep_their_bits_beside_much_larger_ones(where, spread, d, dv):
+    """fp16 has no range to spare for the low parts: a row of dO (of one head, of one sequence), or of V, far above the
+    rest must not take bits from the others.  Every row of every gradient is held to its own magnitude: the rounding
+    to fp16 (2^-11 of an element, 2^-25 below the normal range) and the fp32 term of ``_float64_backward``."""
+    b, l, hq, hkv = 2, 200, 4, 2
+    dvc, dtype = dev(), torch.float16
+    q, k, v = randn((b, l, hq, d), dtype, 1), randn((b, l, hkv, d), dtype, 2), randn((b, l, hkv, dv), dtype, 3)
+    g = randn((b, l, hq, dv), torch.float32, 4)
+    low = min(1.0, 5e4 / (4 * spread))  # the large entries stay finite in fp16
+    if where == "value":  # 5e3 above the rest at most, in a document of its own: P dP of the others does not feel it
+        v[0, 150, 1] *= min(spread, 5e3)
+    elif where == "uniform":
+        g = g * low
+    else:
+        big = torch.zeros(b, l, hq, 1)
+        big[{"row": (0, 7, 1), "head": (slice(None), slice(None), 2), "sequence": (1,)}[where]] = 1.0
+        g = g * torch.where(big > 0, low * spread, low)
+    q, k, v, g = (t.to(dvc) for t in (q, k, v, g.clamp(-6e4, 6e4).to(dtype)))
+    mask = M.BlockDiagonalMask(_segment_ids([60, 71, 69]))
+    mods = A.ScoreMods(M.split_mask(mask, b, l, l)[0], M.lower_bias_structured(None, b, hq, l, l), dvc, 0.0, 0)
+    kw = dict(sm_scale=1 / math.sqrt(d), mods=mods)
+    o, lse = A.attention_forward(q, k, v, return_lse=True, **kw)
+    got = A.attention_backward(q, k, v, o, lse, g, **kw)
+    A.check_status(dvc)
+    keep = mask.dense(l, l, batch_size=b, num_heads=1).to(dvc).reshape(b, 1, l, l)
+    want, noise = _float64_backward(q, k, v, o, lse, g, keep, kw["sm_scale"])
+    for name, x, w, n in zip(("dq", "dk", "dv"), got, want, noise):
+        fits = w.abs() < 6.5e4
+        bound = (2.0**-11 * w.abs() + 2.0**-25 + n).norm(dim=3)
+        err = torch.where(fits, x.double() - w, 0.0).norm(dim=3)
+        worst = float((err / bound).max())
+        assert worst <= 1.0, f"{name}: a row is off by {worst:.3g} of its bound"
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("kind", ["latent", "packed", "dense", "dense_128"])
+def test_only_the_rounding_of_the_result_is_left(kind, dtype):
+    """Against float64 the error is that of rounding the result to 16 bits, as with fp32 arithmetic throughout.  P and dS
+    without their low parts add 2^-9 (bf16) or 2^-12 (fp16) of each term and raise it by half."""
+    b, l, hq = 2, 515, 4
+    d, dv = {"latent": (192, 128), "packed": (128, 128), "dense": (64, 64), "dense_128": (128, 128)}[kind]
+    dvc = dev()
+    q, k, v = randn((b, l, hq, d), dtype, 1).to(dvc), randn((b, l, 2, d), dtype, 2).to(dvc), randn((b, l, 2, dv), dtype, 3).to(dvc)
+    g = randn((b, l, hq, dv), dtype, 4).to(dvc)
+    keep, dense, kw = torch.ones(b, 1, l, l, dtype=torch.bool, device=dvc), None, dict(sm_scale=1 / math.sqrt(d))
+    if kind == "packed":
+        mask = M.BlockDiagonalMask(_segment_ids([200, 115, 200]))
+        keep = mask.dense(l, l, batch_size=b, num_heads=1).to(dvc).reshape(b, 1, l, l)
+        kw["mods"] = A.ScoreMods(M.split_mask(mask, b, l, l)[0], M.lower_bias_structured(None, b, hq, l, l), dvc, 0.0, 0)
+    elif kind != "latent":
+        dense = kw["bias"] = randn((1, hq, l, l), torch.float32, 7).to(dvc)
+    o, lse = A.attention_forward(q, k, v, return_lse=True, **kw)
+    got = A.attention_backward(q, k, v, o, lse, g, **kw)
+    A.check_status(dvc)
+    want, noise = _float64_backward(q, k, v, o, lse, g, keep, kw["sm_scale"], dense)
+    for name, x, w, n in zip(("dq", "dk", "dv"), got, want, noise):
+        rounding = float((w.to(dtype).double() - w).norm())
+        err = float((x.double() - w).norm())
+        assert err <= 1.001 * rounding + float(n.norm()), f"{name}: {err / rounding:.5f} of the rounding error"

@@ -113,13 +113,17 @@ def rope_interleaved(x: torch.Tensor, positions=None, *, base: float = 10_000.0,
     return y
 
 
+def _check_layers(x, *weights) -> None:
+    if not x.is_cuda or any(x.dtype != w.dtype or x.shape[-1] != w.shape[-1] or w.dim() != 2 for w in weights):
+        raise ValueError("linear takes CUDA tensors x [..., K] and weight [N, K] of one dtype")
+
+
 def linear(x: torch.Tensor, weight: torch.Tensor, *, implementation: str | None = None) -> torch.Tensor:
     """``x [..., K] @ weight[N, K]^T`` on the device (``pjx_linear``): the bias-free query / key /
     value / output projections around the attention call (layers/attention.py:591-594).  A fused
     QKV projection is one call with the three weights concatenated along ``N``."""
     _require_gpu()
-    if not x.is_cuda or x.dtype != weight.dtype or x.shape[-1] != weight.shape[-1] or weight.dim() != 2:
-        raise ValueError("linear takes CUDA tensors x [..., K] and weight [N, K] of one dtype")
+    _check_layers(x, weight)
     if implementation not in _IMPL:
         raise ValueError(f"implementation must be None or one of {sorted(k for k in _IMPL if k)}")
     x2 = x.contiguous().view(-1, x.shape[-1])
@@ -177,7 +181,9 @@ class _LinearFunction(torch.autograd.Function):
 
 def linear_autograd(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     """:func:`linear` that records itself for reverse-mode differentiation."""
-    return _LinearFunction.apply(x, weight)
+    _require_gpu()
+    _check_layers(x, weight)
+    return _LinearFunction.apply(x, weight.to(x.device))  # (a gradient goes back to the weight's device)
 
 
 class _LinearPairFunction(torch.autograd.Function):
@@ -208,9 +214,9 @@ class _LinearPairFunction(torch.autograd.Function):
 
 def linear_pair_autograd(x: torch.Tensor, w0: torch.Tensor, w1: torch.Tensor):
     """``(linear(x, w0), linear(x, w1))``, recorded for reverse-mode differentiation."""
-    if not x.is_cuda or x.shape[-1] != w0.shape[-1] or x.shape[-1] != w1.shape[-1] or not x.dtype == w0.dtype == w1.dtype:
-        raise ValueError("linear takes CUDA tensors x [..., K] and weight [N, K] of one dtype")
-    return _LinearPairFunction.apply(x, w0, w1)
+    _require_gpu()
+    _check_layers(x, w0, w1)
+    return _LinearPairFunction.apply(x, w0.to(x.device), w1.to(x.device))
 
 
 def decode_paged(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, block_table: torch.Tensor, kv_lengths,

@@ -42,3 +42,20 @@ def test_pair_against_float64(m, k, n0, n1, dtype):
     w3 = w1.clone().requires_grad_(True)
     y0, y1 = C.linear_pair_autograd(x, w0, w3)
     check("dw1 alone", torch.autograd.grad(y1, w3, g1)[0], g1.double().T @ x.double())
+
+
+def test_weights_elsewhere_and_of_another_rank():
+    """As in ``linear``: weights are moved to the device of ``x`` (their gradients come back), other ranks are refused."""
+    d = dev()
+    x = randn((70, 64), torch.bfloat16, 1).to(d).requires_grad_(True)
+    ws = [randn((n, 64), torch.bfloat16, n).requires_grad_(True) for n in (72, 80)]  # on the host
+    gs = [randn((70, n), torch.bfloat16, 3).to(d) for n in (72, 80)]
+    ons = [w.detach().to(d).requires_grad_(True) for w in ws]
+    got = torch.autograd.grad(C.linear_pair_autograd(x, *ws), [x, *ws], gs)
+    want = torch.autograd.grad(C.linear_pair_autograd(x, *ons), [x, *ons], gs)
+    assert all(not g.is_cuda for g in got[1:]) and all(torch.equal(a.to(d), b) for a, b in zip(got, want))
+    one = torch.autograd.grad(C.linear_autograd(x, ws[0]), [x, ws[0]], gs[0])
+    assert torch.equal(one[1], got[1])
+    with pytest.raises(ValueError, match="weight"):
+        C.linear_pair_autograd(x, ons[0], ons[1].view(2, 40, 64))
+

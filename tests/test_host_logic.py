@@ -544,3 +544,20 @@ def test_latent_layer_dropout_resolution():
     with pytest.raises(ValueError, match="keep_rngs=True"):
         lay._resolve_dropout(None, None)
     assert lay._resolve_dropout(None, [1, 2]) == (0.1, [1, 2])
+
+
+def test_layers_of_another_shape_or_type_are_refused():
+    """What ``linear`` refuses, ``linear_autograd`` and ``linear_pair_autograd`` refuse before a pointer is taken."""
+    from types import SimpleNamespace
+
+    from probjax_b200 import cache
+
+    x = SimpleNamespace(is_cuda=True, dtype=torch.bfloat16, shape=(3, 64))
+    good, deep, narrow = (torch.zeros(s, dtype=torch.bfloat16) for s in ((72, 64), (2, 36, 64), (72, 32)))
+    cache._check_layers(x, good, good)
+    for bad in (deep, narrow, good.float()):
+        with pytest.raises(ValueError, match="weight"):
+            cache._check_layers(x, good, bad)
+    with pytest.raises(ValueError, match="CUDA"):
+        cache._check_layers(good, good)
+

@@ -46,15 +46,17 @@ int validate_common(const void* q, const void* k, const void* v, const void* o, 
 
 }  // namespace
 
-// Validates a caller's pjx_score_mod and converts it to the kernels' form (null: no modifiers).
 int bind_context() {
-  static thread_local bool bound = false;
-  if (bound) return PJX_OK;
-  const int rc = check_cuda(cudaFree(nullptr), "initialise the device context");
-  bound = rc == PJX_OK;
+  // (cudaSetDevice makes the primary context current; unlike the cudaFree family it is open to a thread that captures)
+  static thread_local int bound = -1;
+  int dev = -1, rc = check_cuda(cudaGetDevice(&dev), "query the current device");
+  if (rc || dev == bound) return rc;
+  rc = check_cuda(cudaSetDevice(dev), "initialise the device context");
+  if (!rc) bound = dev;
   return rc;
 }
 
+// Validates a caller's pjx_score_mod and converts it to the kernels' form (null: no modifiers).
 int convert_score_mod(const pjx_score_mod* m, ScoreMod* out) {
   *out = ScoreMod();
   if (!m) return PJX_OK;

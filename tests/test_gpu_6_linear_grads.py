@@ -4,6 +4,8 @@ Against float64 products of the same 16-bit operands: fp32 accumulation over n t
 so at most one unit in the last place (2^-8 in bf16, 2^-11 in fp16) of the norm.
 """
 
+import threading
+
 import pytest
 import torch
 
@@ -59,3 +61,25 @@ def test_weights_elsewhere_and_of_another_rank():
     with pytest.raises(ValueError, match="weight"):
         C.linear_pair_autograd(x, ons[0], ons[1].view(2, 40, 64))
 
+
+def test_first_call_of_a_thread_inside_a_capture():
+    """The device context is bound on a thread's first tensor-core call by a means that stream capture allows."""
+    d = dev()
+    x, w = randn((128, 64), torch.bfloat16, 1).to(d), randn((64, 64), torch.bfloat16, 2).to(d)
+    want = C.linear(x, w)  # (the status word exists from here on)
+    graph, out = torch.cuda.CUDAGraph(), []
+
+    def capture():
+        try:
+            with torch.cuda.device(d), torch.cuda.graph(graph, stream=torch.cuda.Stream(d)):
+                out.append(C.linear(x, w))
+        except Exception as e:
+            out.append(e)
+
+    thread = threading.Thread(target=capture)
+    thread.start()
+    thread.join()
+    assert isinstance(out[0], torch.Tensor), out
+    graph.replay()
+    torch.cuda.synchronize(d)
+    assert torch.equal(out[0], want)

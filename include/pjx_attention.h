@@ -3,7 +3,9 @@
  *
  * Everything probjax.nn's attention hot path lowers to on a GPU, as plain
  * `extern "C"` entry points: caller-owned device buffers, sizes, a CUDA stream.
- * No entry point allocates or frees device memory, synchronises the device
+ * No entry point allocates or frees device memory (two forms of the tcgen05
+ * forward take stream-ordered scratch for the length of the call, see
+ * pjx_attn_fwd), synchronises the device
  * (except the *_host and pjx_read_status helpers, which say so) or throws.
  * All tensors are row-major and dense, laid out exactly as the reference
  * passes them to its kernels (no transposes):
@@ -68,6 +70,10 @@ const char* pjx_last_error(void);
  *   causal       nonzero: key j is valid for query i iff j <= i.
  *   status       int32 device word or NULL; a kernel writes a nonzero pjx_status
  *                there if a bounded wait expires. Read it with pjx_read_status.
+ *
+ * Stream-ordered scratch (cudaMallocAsync / cudaFreeAsync within the call, capturable): the tcgen05 forward takes
+ * some for an unmasked grid whose last wave is partly filled (partials of the two key halves of its items, at most
+ * 40 MB) and for segment ids (8 bytes per 128 query rows).  Where it cannot be had the call runs without.
  */
 int pjx_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse,
                  const int32_t* kv_lengths, const float* bias, int64_t bias_batch_stride,
@@ -163,7 +169,7 @@ int pjx_attn_fwd_mod(const void* q, const void* k, const void* v, void* o, float
 /*
  * Backward of pjx_attn_fwd: dq, dk, dv from q, k, v, o, d_o and the forward's
  * natural-log lse, for the same masks and bias (the bias itself gets no gradient
- * here).  First correct path: exact fp32 arithmetic on CUDA cores for every dtype.
+ * here).  Runs the kernels pjx_attn_bwd_band picks under AUTO.
  *
  * Replaces the `mha_bwd` primitive (probjax/nn/pallas_kernels/kernels/
  * attention.py:2509-2534; kernels `_preprocess_backward_kernel` 853-906,
@@ -195,7 +201,13 @@ int pjx_attn_bwd_band(const void* q, const void* k, const void* v, const void* o
 size_t pjx_attn_bwd_workspace_bytes(int B, int Lq, int Hq);
 /* pjx_attn_bwd_band with score modifiers (mod may be NULL).  16-bit calls with modifiers run on the
  * tensor cores as well (head shapes (64, 64), (128, 128), (192, 128)) unless `impl` forces a kernel;
- * `dbias` cannot be combined with head_scale / softcap. */
+ * `dbias` cannot be combined with head_scale / softcap.
+ *
+ * All forms of the backward take pjx_attn_bwd_workspace_bytes or more.  With
+ * pjx_attn_bwd_mod_workspace_bytes, and 16-byte aligned, every 16-bit call of those head shapes runs on
+ * the tensor cores.  With less, fp16 calls that carry modifiers, a dense bias or the head shape (192, 128) run
+ * on the CUDA cores, and bf16 calls with segment ids visit all tiles instead of those that can match. */
+size_t pjx_attn_bwd_mod_workspace_bytes(int B, int Lq, int Lkv, int Hq, int Hkv, int dtype);
 int pjx_attn_bwd_mod(const void* q, const void* k, const void* v, const void* o, const float* lse,
                      const void* d_o, void* dq, void* dk, void* dv, const int32_t* kv_lengths,
                      const float* bias, int64_t bias_batch_stride, int64_t bias_head_stride,

@@ -332,7 +332,7 @@ def attention_backward(q, k, v, o, lse, d_o, *, causal=False, band=None, kv_leng
             raise ValueError("bias_grad needs a bias")
         dbias = torch.empty_like(bt)
     L = _lib.lib()
-    ws = _scratch_bytes(dev, "bwd", L.pjx_attn_bwd_workspace_bytes(B, Lq, Hq))
+    ws = _scratch_bytes(dev, "bwd", L.pjx_attn_bwd_mod_workspace_bytes(B, Lq, Lkv, Hq, Hkv, _DTYPES[q.dtype]))
     with torch.cuda.device(dev):
         rc = L.pjx_attn_bwd_mod(_ptr(q), _ptr(k), _ptr(v), _ptr(o), _ptr(lse), _ptr(d_o), _ptr(dq), _ptr(dk),
                                 _ptr(dv), _ptr(kvl), _ptr(bt), bs, hs, _ptr(dbias), B, Lq, Lkv, Hq, Hkv, D, Dv,

@@ -434,11 +434,11 @@ int launch_widths(const BwdParams& p, cudaStream_t stream) {
 enum class BwdRoute { CudaCores, Sm100, Sm100Exact };
 
 template <typename T_>
-int launch_dtype(const BwdParams& p, BwdRoute route, void* scratch, cudaStream_t stream) {
+int launch_dtype(const BwdParams& p, BwdRoute route, void* scratch, size_t scratch_bytes, cudaStream_t stream) {
   const int rc = launch_delta<T_>(p, stream);
   if (rc) return rc;
   if (route == BwdRoute::Sm100) return launch_bwd_sm100(p, stream);
-  if (route == BwdRoute::Sm100Exact) return launch_bwd_exact_sm100(p, scratch, stream);
+  if (route == BwdRoute::Sm100Exact) return launch_bwd_exact_sm100(p, scratch, scratch_bytes, stream);
   const int nk = p.D <= 64 ? 1 : (p.D <= 128 ? 2 : 4);
   const int nv = p.Dv <= 64 ? 1 : (p.Dv <= 128 ? 2 : 4);
   switch (nk * 10 + nv) {
@@ -649,6 +649,16 @@ size_t pjx_attn_bwd_workspace_bytes(int B, int Lq, int Hq) {
   return 2 * (size_t)B * Hq * lq_pad * sizeof(float);
 }
 
+size_t pjx_attn_bwd_mod_workspace_bytes(int B, int Lq, int Lkv, int Hq, int Hkv, int dtype) {
+  if (B < 0 || Lq < 0 || Lkv < 0 || Hq < 1 || Hkv < 1) return 0;
+  BwdParams p;
+  static const int32_t ids = 0;
+  p.B = B; p.Lq = Lq; p.Lkv = Lkv; p.Hq = Hq; p.Hkv = Hkv;
+  p.dtype = dtype;
+  p.mod.seg_q = p.mod.seg_k = &ids;  // as with segment ids
+  return pjx_attn_bwd_workspace_bytes(B, Lq, Hq) + bwd_exact_scratch_bytes(p);
+}
+
 int pjx_attn_bwd_band(const void* q, const void* k, const void* v, const void* o, const float* lse, const void* d_o,
                       void* dq, void* dk, void* dv, const int32_t* kv_lengths, const float* bias,
                       int64_t bias_batch_stride, int64_t bias_head_stride, float* dbias, int B, int Lq, int Lkv, int Hq,
@@ -715,8 +725,8 @@ int pjx_attn_bwd_mod(const void* q, const void* k, const void* v, const void* o,
     p.dbias_atomic = (bias_batch_stride == 0 && B > 1) || (bias_head_stride == 0 && Hq > 1);
   }
   // 16-bit calls that the plain tcgen05 kernels do not take (score modifiers, dense bias, the latent head shape) run
-  // on the tensor cores with P and dS as 16 + 16 bits; what is left there (fp32 inputs, other head widths) and calls
-  // whose scratch cannot be had run on the CUDA cores.  A forced tcgen05 backward means the plain kernels.
+  // on the tensor cores with P and dS as 16 + 16 bits; what is left there (fp32 inputs, other head widths) and fp16
+  // calls whose workspace stops at the row vectors run on the CUDA cores.  A forced tcgen05 backward means the plain kernels.
   const char* why = nullptr;
   bool tc_ok = bwd_sm100_supported(p, &why);
   if (tc_ok && smod.on) {
@@ -725,19 +735,10 @@ int pjx_attn_bwd_mod(const void* q, const void* k, const void* v, const void* o,
   }
   if (impl == PJX_IMPL_SM100 && !tc_ok && Lq > 0) return fail(PJX_ERR_UNSUPPORTED, "tcgen05 backward: %s", why);
   BwdRoute route = impl != PJX_IMPL_GENERIC && tc_ok ? BwdRoute::Sm100 : BwdRoute::CudaCores;
-  void* scratch = nullptr;
-  if (impl == PJX_IMPL_AUTO && !tc_ok && bwd_exact_sm100_supported(p)) {
+  void* scratch = static_cast<char*>(workspace) + need;
+  const size_t scratch_bytes = workspace_bytes > need ? workspace_bytes - need : 0;
+  if (impl == PJX_IMPL_AUTO && !tc_ok && bwd_exact_sm100_supported(p) && scratch_bytes >= bwd_exact_scratch_bytes_needed(p))
     route = BwdRoute::Sm100Exact;
-    const size_t bytes = bwd_exact_scratch_bytes(p);
-    if (bytes > 0) {
-      keep_pool_memory();
-      if (cudaMallocAsync(&scratch, bytes, st) != cudaSuccess) {
-        (void)cudaGetLastError();
-        scratch = nullptr;
-        route = BwdRoute::CudaCores;
-      }
-    }
-  }
   p.lse_natural = route == BwdRoute::Sm100Exact && (smod.rel_bias || bias);
   if (dbias_bytes > 0 && route == BwdRoute::CudaCores) {  // (the tcgen05 kernel writes every entry)
     const int rc0 = check_cuda(cudaMemsetAsync(dbias, 0, dbias_bytes, st), "clear dbias");
@@ -748,14 +749,11 @@ int pjx_attn_bwd_mod(const void* q, const void* k, const void* v, const void* o,
     if (rc) return rc;
     return check_cuda(cudaMemsetAsync(dv, 0, (size_t)B * Lkv * Hkv * Dv * dtype_size(dtype), st), "clear dv");
   }
-  int rc;
   switch (dtype) {
-    case PJX_F32: rc = launch_dtype<float>(p, route, scratch, st); break;
-    case PJX_BF16: rc = launch_dtype<__nv_bfloat16>(p, route, scratch, st); break;
-    default: rc = launch_dtype<__half>(p, route, scratch, st);
+    case PJX_F32: return launch_dtype<float>(p, route, scratch, scratch_bytes, st);
+    case PJX_BF16: return launch_dtype<__nv_bfloat16>(p, route, scratch, scratch_bytes, st);
+    default: return launch_dtype<__half>(p, route, scratch, scratch_bytes, st);
   }
-  if (scratch) cudaFreeAsync(scratch, st);
-  return rc;
 }
 
 int pjx_attn_bwd(const void* q, const void* k, const void* v, const void* o, const float* lse, const void* d_o,

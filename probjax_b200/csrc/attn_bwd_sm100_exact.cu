@@ -43,7 +43,6 @@
 namespace pjx {
 
 int make_tmap_blhd(CUtensorMap* m, const void* base, int dtype, int B, int L, int H, int Dim, int rows);
-bool bwd_exact_uses_ranges(const BwdParams& p);
 
 namespace {
 
@@ -1401,12 +1400,13 @@ bool bwd_exact_sm100_supported(const BwdParams& p) {
   return true;
 }
 
-// Scratch: [fp16: longest V rows | maxima of the keys] [segment ranges both ways], 4-byte words.
+// Scratch: [fp16: longest V rows | maxima of the keys] [segment ranges both ways], 4-byte words.  fp16 needs its part; the
+// ranges only spare work and are left out where there is no room for them.
 static size_t fp16_words(const BwdParams& p) {
   return p.dtype == PJX_F16 ? (size_t)p.B * p.Hkv * ((p.Lkv + BN - 1) / BN + 2 * (size_t)p.Lkv) : 0;
 }
 
-int launch_bwd_exact_sm100(const BwdParams& p, void* scratch, cudaStream_t stream) {
+int launch_bwd_exact_sm100(const BwdParams& p, void* scratch, size_t scratch_bytes, cudaStream_t stream) {
   ExactArgs a = {};
   a.order_w = (p.band_hi < PJX_BAND_NO_UPPER && p.band_lo == PJX_BAND_NO_LOWER) ? 16 : 1;
   a.bias_vec = p.bias && p.Lkv % 4 == 0 && p.bias_bs % 4 == 0 && p.bias_hs % 4 == 0 && (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0;
@@ -1422,7 +1422,7 @@ int launch_bwd_exact_sm100(const BwdParams& p, void* scratch, cudaStream_t strea
     count_launch();
     if ((rc = check_cuda(cudaGetLastError(), "backward V norm launch"))) return rc;
   }
-  if (bwd_exact_uses_ranges(p)) {
+  if (bwd_exact_uses_ranges(p) && scratch_bytes >= bwd_exact_scratch_bytes(p)) {
     const int n_q = (p.Lq + BM - 1) / BM, n_k = (p.Lkv + BN - 1) / BN;
     const int nb = (p.mod.seg_q_bs == 0 && p.mod.seg_k_bs == 0) ? 1 : p.B;
     int32_t* qr = static_cast<int32_t*>(scratch) + fp16_words(p);
@@ -1448,5 +1448,7 @@ size_t bwd_exact_scratch_bytes(const BwdParams& p) {
   if (bwd_exact_uses_ranges(p)) n += (size_t)p.B * ((p.Lq + BM - 1) / BM + (p.Lkv + BN - 1) / BN) * 2 * sizeof(int32_t);
   return n;
 }
+
+size_t bwd_exact_scratch_bytes_needed(const BwdParams& p) { return fp16_words(p) * 4; }
 
 }  // namespace pjx

@@ -1013,6 +1013,8 @@ int make_tmap_blhd(CUtensorMap* m, const void* base, int dtype, int B, int L, in
   return PJX_OK;
 }
 
+namespace {
+
 // Scratch of a call (partials of the KV halves, segment ranges) comes from the stream-ordered allocator.  Its default pool hands freed memory
 // back to the driver at every synchronisation, which would make each call pay for a fresh mapping: keep it.
 void keep_pool_memory() {
@@ -1027,8 +1029,6 @@ void keep_pool_memory() {
       cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
   }
 }
-
-namespace {
 
 // fp32 bias [Bb, Hb, Lq, Lkv] (strides in elements, 0 = broadcast): box = 32 keys x 128 rows.
 int make_tmap_bias(CUtensorMap* m, const FwdParams& p) {

@@ -308,14 +308,16 @@ int launch_fwd_sm100(const FwdParams& p, int dtype, cudaStream_t stream);
 bool bwd_sm100_supported(const BwdParams& p, const char** why);
 int launch_bwd_sm100(const BwdParams& p, cudaStream_t stream);
 // tcgen05 backward with P and dS as 16 + 16 bits: score modifiers, dense bias, head shape (192, 128)
-// (attn_bwd_sm100_exact.cu); expects p.delta filled and `scratch` of bwd_exact_scratch_bytes (0: may be null).
+// (attn_bwd_sm100_exact.cu); expects p.delta filled and `scratch` of bwd_exact_scratch_bytes, at least
+// bwd_exact_scratch_bytes_needed (with segment ids and less than the former, every tile is visited).
 bool bwd_exact_sm100_supported(const BwdParams& p);
+bool bwd_exact_uses_ranges(const BwdParams& p);
 size_t bwd_exact_scratch_bytes(const BwdParams& p);
-int launch_bwd_exact_sm100(const BwdParams& p, void* scratch, cudaStream_t stream);
+size_t bwd_exact_scratch_bytes_needed(const BwdParams& p);
+int launch_bwd_exact_sm100(const BwdParams& p, void* scratch, size_t scratch_bytes, cudaStream_t stream);
 // Range of keys per tile of 128 query rows that can share a segment with the tile (attn_fwd_sm100.cu).
 void launch_seg_tile_range(const int32_t* seg_q, const int32_t* seg_k, int64_t sq_bs, int64_t sk_bs, int Lq, int Lkv, int tiles,
                            int nb, int32_t* out, cudaStream_t stream);
-void keep_pool_memory();
 bool decode_fast_supported(const DecodeParams& p, int dtype);
 int launch_decode(const DecodeParams& p, int dtype, cudaStream_t stream);
 // Split length chosen for split_len = 0; `ragged`: per-sequence lengths are given (see pjx_api.cu).

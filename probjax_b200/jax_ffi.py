@@ -96,6 +96,10 @@ def mha_fwd_impl(q, k, v, rng_seed=None, b_data=None, q_id=None, k_id=None, drop
     return (o, lse) if return_residuals else o
 
 
+def _dtype_code(dtype) -> int:
+    return {"float32": _lib.PJX_F32, "bfloat16": _lib.PJX_BF16, "float16": _lib.PJX_F16}[str(dtype)]
+
+
 def mha_bwd_impl(q, k, v, o, lse, d_o, b_data=None, *, kv_lengths=None, bias_grad=False, **static):
     """``impl`` for the ``mha_bwd`` spec (kernels/attention.py:2509-2534).  ``lse`` is the natural-log
     residual of :func:`mha_fwd_impl`, not the base-2 residual of the Triton kernels."""
@@ -105,7 +109,8 @@ def mha_bwd_impl(q, k, v, o, lse, d_o, b_data=None, *, kv_lengths=None, bias_gra
     register()
     B, Lq, Hq, _ = q.shape
     lo, hi = _band(static)
-    ws = int(_lib.lib().pjx_attn_bwd_workspace_bytes(B, Lq, Hq))
+    _, Lkv, Hkv, _ = k.shape
+    ws = int(_lib.lib().pjx_attn_bwd_mod_workspace_bytes(B, Lq, Lkv, Hq, Hkv, _dtype_code(q.dtype)))
     out_types = (jax.ShapeDtypeStruct(q.shape, q.dtype), jax.ShapeDtypeStruct(k.shape, k.dtype),
                  jax.ShapeDtypeStruct(v.shape, v.dtype),
                  jax.ShapeDtypeStruct(b_data.shape if (bias_grad and b_data is not None) else (0,), jnp.float32),
@@ -168,7 +173,7 @@ def mla_fwd_impl(q, cache, wk=None, wv=None, rng_seed=None, b_data=None, q_id=No
     B, Lq, H, Dqk = q.shape
     S, R = cache.shape[1], cache.shape[2]
     Dv = R if wv is None else wv.shape[1]
-    code = {jnp.dtype("float32"): 0, jnp.dtype("bfloat16"): 1, jnp.dtype("float16"): 2}[jnp.dtype(q.dtype)]
+    code = _dtype_code(q.dtype)
     ws = int(_lib.lib().pjx_mla_workspace_bytes(B, S, H, Dqk, Dv, R, code, int(wk is not None)))
     z = _absent(q.dtype)
     out_types = (jax.ShapeDtypeStruct((B, Lq, H, Dv), q.dtype),

@@ -561,3 +561,15 @@ def test_layers_of_another_shape_or_type_are_refused():
     with pytest.raises(ValueError, match="CUDA"):
         cache._check_layers(good, good)
 
+
+def test_backward_workspace_sizes(built_lib):
+    """The sized query adds, behind the row vectors, two ints per tile of 128 rows and keys (segment ranges) and for fp16 per
+    (sequence, key head) a float per key tile and two words per key."""
+    from probjax_b200 import _lib
+
+    L = _lib.lib()
+    base = L.pjx_attn_bwd_workspace_bytes(2, 130, 8)
+    assert L.pjx_attn_bwd_mod_workspace_bytes(2, 130, 300, 8, 4, _lib.PJX_BF16) == base + 2 * (2 + 3) * 8
+    assert L.pjx_attn_bwd_mod_workspace_bytes(2, 130, 300, 8, 4, _lib.PJX_F16) == base + 2 * (2 + 3) * 8 + 2 * 4 * (3 + 600) * 4
+    assert L.pjx_attn_bwd_mod_workspace_bytes(2, 0, 0, 8, 4, _lib.PJX_F16) == 0
+    assert L.pjx_attn_bwd_mod_workspace_bytes(2, -1, 300, 8, 4, _lib.PJX_BF16) == 0

@@ -122,3 +122,55 @@ def test_static_scratch_decode_rejects_what_it_cannot_hold():
     rc = L.pjx_attn_decode_splitkv_static(_ptr(q), _ptr(q), _ptr(q), None, _ptr(o), None,
                                           1, 1, Hq, Hkv, D, D, 64, _lib.PJX_F32, 0.1, 64, stream)
     assert rc == _lib.PJX_ERR_UNSUPPORTED
+
+
+def _pool_high_water(dev, reset=False):
+    """Most bytes the device's stream-ordered pool had in use at a time (since the last reset)."""
+    rt = C.CDLL("libcudart.so.12")
+    pool, value = C.c_void_p(), C.c_uint64(0)
+    assert rt.cudaDeviceGetDefaultMemPool(C.byref(pool), dev.index) == 0
+    if reset:
+        assert rt.cudaMemPoolSetAttribute(pool, 8, C.byref(value)) == 0  # cudaMemPoolAttrUsedMemHigh
+    assert rt.cudaMemPoolGetAttribute(pool, 8, C.byref(value)) == 0
+    return value.value
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("kind", ["segments", "latent"])
+def test_backward_keeps_its_scratch_in_the_workspace(kind, dtype):
+    """With the sized workspace the call takes nothing from the stream-ordered pool.  With the one of the row vectors alone
+    it is still accepted: bf16 visits every tile (those that cannot match add exact zeros), fp16 runs on the CUDA cores."""
+    from _gpu_util import dev, randn
+    from probjax_b200 import _lib
+    from probjax_b200 import attention as A
+    from probjax_b200 import masks as M
+
+    b, l, h, d, dv = 2, 300, 4, *((192, 128) if kind == "latent" else (128, 128))
+    dvc, L = dev(), _lib.lib()
+    q, k, v, g = (randn((b, l, h, n), dtype, i).to(dvc) for i, n in enumerate((d, d, dv, dv)))
+    mods = None
+    if kind == "segments":
+        ids = torch.repeat_interleave(torch.arange(3, dtype=torch.int32), torch.tensor([140, 100, 60]))[None].repeat(b, 1)
+        mods = A.ScoreMods(M.split_mask(M.SameSegmentMask(ids), b, l, l)[0], M.lower_bias_structured(None, b, h, l, l), dvc, 0.0, 0)
+    kw = dict(sm_scale=1 / math.sqrt(d), mods=mods)
+    o, lse = A.attention_forward(q, k, v, return_lse=True, **kw)
+    want = A.attention_backward(q, k, v, o, lse, g, **kw)
+    slow = A.attention_backward(q, k, v, o, lse, g, impl="b200:generic", **kw)
+    torch.cuda.synchronize(dvc)
+    held = _pool_high_water(dvc, reset=True)
+    again = A.attention_backward(q, k, v, o, lse, g, **kw)
+    torch.cuda.synchronize(dvc)
+    assert _pool_high_water(dvc) == held
+    assert all(torch.equal(x, y) for x, y in zip(again, want))
+
+    code = A._DTYPES[dtype]
+    need = L.pjx_attn_bwd_workspace_bytes(b, l, h)
+    assert need < L.pjx_attn_bwd_mod_workspace_bytes(b, l, l, h, h, code)
+    ws = torch.empty(need, dtype=torch.uint8, device=dvc)
+    got = [torch.empty_like(t) for t in (q, k, v)]
+    rc = L.pjx_attn_bwd_mod(*(A._ptr(t) for t in (q, k, v, o, lse, g, *got)), None, None, 0, 0, None, b, l, l, h, h, d, dv, code,
+                            -(1 << 30), 1 << 30, kw["sm_scale"], A.ScoreMods.arg(mods), 0, A._ptr(ws), need,
+                            A._ptr(A._status_word(dvc)), A._stream(dvc))
+    _lib.check(rc)
+    A.check_status(dvc)
+    assert all(torch.equal(x, y) for x, y in zip(got, want if dtype == torch.bfloat16 else slow))

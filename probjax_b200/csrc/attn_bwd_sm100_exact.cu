@@ -3,10 +3,10 @@
 // latent head shape (192, 128).  Same two-kernel split, warp roles and half-step issue order as
 // attn_bwd_sm100.cu (dQ owns query tiles, dK/dV owns key tiles, no atomics); what differs:
 //
-// * P and dS enter the accumulating products as a sum of two 16-bit numbers, x = hi + lo with hi the upper 16
-//   bits of x (bf16) or its rounding (fp16) and lo = round16(x - hi): two MMAs against the same B descriptor
+// * P and dS enter the accumulating products as a sum of two 16-bit numbers, x = hi + lo with hi = round16(x)
+//   and lo = round16(x - hi): two MMAs against the same B descriptor
 //   instead of one.  The calls that arrive here ran on CUDA cores with P and dS in fp32 before, and 16 + 16 bits
-//   keep what that gave (2^-16 relative in bf16 against the 2^-9 of the stored gradients).  Per 128 x 128 tile that is 10
+//   keep what that gave (2^-18 relative in bf16 against the 2^-9 of the stored gradients).  Per 128 x 128 tile that is 10
 //   products of 128 x 128 x D for both kernels instead of 7.  A 16-column chunk of scores (16 columns of
 //   tensor memory) is overwritten by its own 8 columns of hi and 8 of lo pairs, so the split costs no
 //   tensor memory.
@@ -100,16 +100,16 @@ __device__ __forceinline__ void add_col_max(const float2 (&pr)[CH / 2], const fl
   if (mine && col < n_cols) atomicMax(out + (lane < CH ? 0 : Lkv) + col, mine);
 }
 
-// A chunk of CH fp32 values as hi pairs (8 registers) and lo pairs (8 registers).  bf16 truncates hi (the upper half of
-// the fp32 word: one byte permute packs a pair, one AND gives its value back) and rounds lo: 2^-16 of x at most.
+// A chunk of CH fp32 values as hi pairs (8 registers) and lo pairs (8 registers), both rounded: 2^-18 of x at most in
+// bf16.  (hi cut off instead, one byte permute per pair, left 2^-16.)
 template <bool BF16>
 __device__ __forceinline__ void split_pack(const float2 (&x)[CH / 2], float scale, uint32_t (&r)[CH]) {
 #pragma unroll
   for (int i = 0; i < CH / 2; ++i) {
     if constexpr (BF16) {
-      const uint32_t u = __float_as_uint(x[i].x), v = __float_as_uint(x[i].y);
-      r[i] = __byte_perm(u, v, 0x7632);
-      const float2 lo = __fadd2_rn(x[i], make_float2(-__uint_as_float(u & 0xffff0000u), -__uint_as_float(v & 0xffff0000u)));
+      const uint32_t hi = pack16<true>(x[i].x, x[i].y);
+      const float2 lo = __fadd2_rn(x[i], make_float2(-__uint_as_float(hi << 16), -__uint_as_float(hi & 0xffff0000u)));
+      r[i] = hi;
       r[CH / 2 + i] = pack16<true>(lo.x, lo.y);
     } else {
       const float2 y = __fmul2_rn(x[i], make_float2(scale, scale));

@@ -295,8 +295,7 @@ def main():
                          "the staircase of waves and what cutting the last wave into KV halves buys "
                          "(PJX_FWD_SPLIT_TAIL=0 switches the halves off)")
     ap.add_argument("--only-prefill", action="store_true",
-                    help="time only the headline forward, non-causal and causal, without checking the result "
-                         "(what-if builds of the forward kernel, whose outputs are wrong on purpose)")
+                    help="time only the headline forward, non-causal and causal, without checking the result")
     ap.add_argument("--only-latent", action="store_true",
                     help="time only the latent-attention configuration on --batch batch rows (profiling captures)")
     ap.add_argument("--only-modifier", default=None,
@@ -743,9 +742,7 @@ def only_waves(args, dev, pk):
 
 
 def only_prefill(args, dev, pk):
-    """The headline forward on `--batch` batch rows, non-causal and causal, timing only: the command the
-    what-if builds of the forward kernel (`python -m probjax_b200.build --what-if N`, loaded through
-    PJX_ATTENTION_LIB) are timed with."""
+    """The headline forward on `--batch` batch rows, non-causal and causal, timing only."""
     import oracle
     import probjax_b200 as pj
 

@@ -40,24 +40,6 @@ constexpr int BM = 128;        // query rows per tile
 constexpr int BN = 128;        // keys per tile
 constexpr int NTHREADS = 320;  // 10 warps
 
-// Optional phase timeline of one CTA of the dQ kernel (debug builds only, -DPJX_TRACE).
-#ifdef PJX_TRACE
-__device__ long long g_btrace[4][64][8];
-#define PJX_BTRACE(r, j, pt)                                                                     \
-  do {                                                                                           \
-    if (blockIdx.x == gridDim.x / 2 && (j) < 64)                                                 \
-      g_btrace[(r)][(j)][(pt)] = clock64();                                                      \
-  } while (0)
-#define PJX_KTRACE(r, j, pt)                                                                     \
-  do {                                                                                           \
-    if (blockIdx.x == gridDim.x / 2 && (j) < 64)                                                 \
-      g_btrace[2 + (r)][(j)][(pt)] = clock64();                                                  \
-  } while (0)
-#else
-#define PJX_BTRACE(r, j, pt) do {} while (0)
-#define PJX_KTRACE(r, j, pt) do {} while (0)
-#endif
-
 // dS of 32 score columns of one query row: p = exp2(s c1 - lse2), dS = p (dP - delta), packed to
 // 16 bits.  Straight-line over independent elements so that the scheduler can overlap them.
 template <bool BF16>
@@ -249,11 +231,9 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       for (int j = 0; ok && j < n; ++j) {
         const int st = j & 1;
         const bool next = j + 1 < n;
-        PJX_BTRACE(0, j, 0);
         ok = mbar_wait_all(BAR(DS_FULL + 0), j & 1, abort_flag);
         if (!ok) break;
         tc_fence_after();
-        PJX_BTRACE(0, j, 1);
         issue_acc(0, j);
         if (next) {
           ok = mbar_wait_all(BAR(K_FULL + (j + 1) % KST), ((j + 1) / KST) & 1, abort_flag);
@@ -263,7 +243,6 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           tc_fence_after();
           issue_sdp(0, j + 1);  // over dS of half 0, which the MMAs just issued consume first
         }
-        PJX_BTRACE(0, j, 2);
         ok = mbar_wait_all(BAR(DS_FULL + 1), j & 1, abort_flag);
         if (!ok) break;
         tc_fence_after();
@@ -273,7 +252,6 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           issue_sdp(1, j + 1);
           mma_commit(BAR(V_EMPTY + (st ^ 1)), leader);
         }
-        PJX_BTRACE(0, j, 3);
       }
       if (ok) mma_commit(BAR(DQ_FULL), leader);
     }
@@ -292,12 +270,10 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     const uint32_t s_addr = T_S + lane_sel + grp * 64, dp_addr = T_DP + lane_sel + grp * 64;
     bool ok = true;
     for (int j = 0; j < n; ++j) {
-      if (r_in == 64 && grp == 0) PJX_BTRACE(1, j, 0);
       ok = mbar_wait(BAR(SP_FULL + grp), j & 1, abort_flag);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      if (r_in == 64 && grp == 0) PJX_BTRACE(1, j, 1);
       const int k0 = (j_lo + j) * BN + grp * 64;  // first key of this group's columns
       const bool need_mask = (k0 + 64 > kv_len) || (k0 + 63 > q0 + p.band_hi) || (k0 < q0 + BM - 1 + p.band_lo);
 #pragma unroll
@@ -306,7 +282,6 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         tmem_ld32f(s_addr + c * 32, s);
         tmem_ld32f(dp_addr + c * 32, dp);
         tmem_wait_ld();
-        if (r_in == 64 && grp == 0) PJX_BTRACE(1, j, 2 + 2 * c);
         ds_row_chunk<BF16>(s, dp, c1, -lse2, -delta, d);
         if (need_mask) {  // selects, not products: masked scores may be anything
 #pragma unroll
@@ -321,12 +296,10 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         for (int i = 0; i < 16; ++i) pk[i] = pack16<BF16>(d[2 * i], d[2 * i + 1]);
         // over columns of this group's half that were read already (chunk 0: 0-15, chunk 1: 16-31)
         tmem_st16(s_addr + c * 16, pk);
-        if (r_in == 64 && grp == 0) PJX_BTRACE(1, j, 3 + 2 * c);
       }
       tmem_wait_st();
       tc_fence_before();
       mbar_arrive(BAR(DS_FULL + grp));
-      if (r_in == 64 && grp == 0) PJX_BTRACE(1, j, 6);
     }
     if (ok && q0 < p.Lq) {
       if (n > 0) {
@@ -516,11 +489,9 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       }
       for (int it = 0; ok && it < n; ++it) {
         const bool next = it + 1 < n;
-        PJX_KTRACE(0, it, 0);
         ok = mbar_wait_all(BAR(PDS_FULL + 0), it & 1, abort_flag);
         if (!ok) break;
         tc_fence_after();
-        PJX_KTRACE(0, it, 1);
         issue_acc(0, it);
         if (next) {
           ok = half_landed(2 * it + 2);
@@ -528,7 +499,6 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
           tc_fence_after();
           issue_sdp(0, it + 1);  // over P^T / dS^T of half 0, which the MMAs just issued consume first
         }
-        PJX_KTRACE(0, it, 2);
         ok = mbar_wait_all(BAR(PDS_FULL + 1), it & 1, abort_flag);
         if (!ok) break;
         tc_fence_after();
@@ -539,7 +509,6 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
           tc_fence_after();
           issue_sdp(1, it + 1);
         }
-        PJX_KTRACE(0, it, 3);
       }
       if (ok) mma_commit(BAR(ACC_FULL), leader);
     }
@@ -558,14 +527,11 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     for (int it = 0; it < n; ++it) {
       const int st = (2 * it + grp) % NS;
       const int q0 = (t_lo + it % n_t) * BM + grp * 64;  // first query row of this group's columns
-      if (r_in == 64 && grp == 0) PJX_KTRACE(1, it, 0);
       ok = mbar_wait(BAR(SP_FULL + grp), it & 1, abort_flag);
-      if (r_in == 64 && grp == 0) PJX_KTRACE(1, it, 1);
       if (ok) ok = mbar_wait(BAR(QDO_FULL + st), ((2 * it + grp) / NS) & 1, abort_flag);  // the row vectors landed with Q and dO
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      if (r_in == 64 && grp == 0) PJX_KTRACE(1, it, 2);
       const float* lse2_s = row_s + st * 128;
       const float* delta_s = lse2_s + 64;
       // this key row against query rows q0 .. q0+63: visible iff q + band_lo <= key <= q + band_hi
@@ -609,12 +575,10 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         // over columns of this group's half that were read already (chunk 0: 0-15, chunk 1: 16-31)
         tmem_st16(s_addr + c * 16, pkp);
         tmem_st16(dp_addr + c * 16, pkd);
-        if (r_in == 64 && grp == 0) PJX_KTRACE(1, it, 3 + c);
       }
       tmem_wait_st();
       tc_fence_before();
       mbar_arrive(BAR(PDS_FULL + grp));
-      if (r_in == 64 && grp == 0) PJX_KTRACE(1, it, 5);
     }
     if (ok && k0 < p.Lkv) {
       if (n > 0) {
@@ -692,11 +656,6 @@ bool bwd_sm100_supported(const BwdParams& p, const char** why) {
   return w == nullptr;
 }
 
-#ifdef PJX_TRACE
-extern "C" int pjx_debug_read_bwd_trace(long long* host_out) {
-  return (int)cudaMemcpyFromSymbol(host_out, g_btrace, sizeof(long long) * 4 * 64 * 8);
-}
-#endif
 
 int launch_bwd_sm100(const BwdParams& p, cudaStream_t stream) {
   const char* why = nullptr;

@@ -40,36 +40,8 @@ namespace {
 
 using namespace sm100;
 
-// Timing experiments (python -m probjax_b200.build --what-if N): 0 = the shipped kernel.
-#ifndef PJX_EXP_VARIANT
-#define PJX_EXP_VARIANT 0
-#endif
-
 constexpr int BM = 128;          // rows per query tile (= tensor-memory lanes)
 constexpr int NTHREADS = 320;    // 10 warps
-
-// Optional phase timeline of one CTA (debug builds only, -DPJX_TRACE): role r
-// (0/1 = softmax of tile 0/1, 2 = MMA issuer) stamps clock64() at point `pt` of KV
-// iteration j.
-#ifdef PJX_TRACE
-__device__ long long g_trace[3][64][8];
-#define PJX_TRACE_AT(r, j, pt)                                                                   \
-  do {                                                                                           \
-    if (blockIdx.x == gridDim.x / 2 && (j) < 64 &&                                               \
-        ((r) == 2 || (threadIdx.x & 127) == 64))                                                 \
-      g_trace[(r)][(j)][(pt)] = clock64();                                                       \
-  } while (0)
-// Per-CTA timeline: [0] SM id, then clock64 at [1] entry, [2] first S MMA issued, [3] last MMA
-// issued, [4] epilogue of tile 1 begins, [5] exit; [6] globaltimer at entry.
-__device__ long long g_cta[8192][8];
-#define PJX_CTA_AT(slot)                                                        \
-  do {                                                                          \
-    if (blockIdx.x < 8192) g_cta[blockIdx.x][(slot)] = clock64();               \
-  } while (0)
-#else
-#define PJX_TRACE_AT(r, j, pt) do {} while (0)
-#define PJX_CTA_AT(slot) do {} while (0)
-#endif
 
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
@@ -138,52 +110,6 @@ __device__ __forceinline__ void exp_pack_store(const float (&s)[BN], float2 cs2,
     sum1 = __fadd2_rn(sum1, p1);
     pk[i] = pack16<BF16>(p0.x, p0.y);
     pk[i + 1] = pack16<BF16>(p1.x, p1.y);
-  }
-#if PJX_EXP_VARIANT == 11
-#pragma unroll
-  for (int i = 0; i < BN / 2; ++i) asm volatile("" ::"r"(pk[i]));
-#else
-#pragma unroll
-  for (int c = 0; c < BN / 64; ++c) tmem_st32(s_addr + c * 32, *reinterpret_cast<const uint32_t(*)[32]>(&pk[c * 32]));
-#endif
-}
-
-// The same with EMU of every 4 score pairs exponentiated on the FMA pipe instead of the
-// special-function unit: x = n + f with n = round(x), f in [-0.5, 0.5]; 2^f as a degree-3
-// polynomial (max relative error 7.5e-5, far below the 16-bit rounding of P); n is added to the
-// exponent field.  x is clamped at -126, so the result is never exactly 0: only for tiles that
-// need no mask (a masked score must give exactly 0).
-template <int BN, bool BF16, int EMU>
-__device__ __forceinline__ void exp_pack_store_emu(const float (&s)[BN], float2 cs2, float2 nm2, float2& sum0,
-                                                   float2& sum1, uint32_t s_addr) {
-  uint32_t pk[BN / 2];
-  const float2 magic = make_float2(12582912.f, 12582912.f), nmagic = make_float2(-12582912.f, -12582912.f);
-  const float2 neg1 = make_float2(-1.f, -1.f);
-  const float2 c0 = make_float2(0.9999280572f, 0.9999280572f), c1 = make_float2(0.6932609677f, 0.6932609677f);
-  const float2 c2 = make_float2(0.2426111251f, 0.2426111251f), c3 = make_float2(0.0551716648f, 0.0551716648f);
-#pragma unroll
-  for (int i = 0; i < BN / 2; ++i) {
-    float2 x = __ffma2_rn(make_float2(s[2 * i], s[2 * i + 1]), cs2, nm2);
-    float2 p;
-    if ((i & 3) < EMU) {
-      x.x = fmaxf(x.x, -126.f);
-      x.y = fmaxf(x.y, -126.f);
-      const float2 r = __fadd2_rn(x, magic);
-      const float2 f = __ffma2_rn(__fadd2_rn(r, nmagic), neg1, x);
-      float2 q = __ffma2_rn(f, c3, c2);
-      q = __ffma2_rn(q, f, c1);
-      q = __ffma2_rn(q, f, c0);
-      p.x = __uint_as_float(__float_as_uint(q.x) + (__float_as_uint(r.x) << 23));
-      p.y = __uint_as_float(__float_as_uint(q.y) + (__float_as_uint(r.y) << 23));
-    } else {
-#if PJX_EXP_VARIANT == 9
-      p = x;
-#else
-      p = make_float2(ex2_approx(x.x), ex2_approx(x.y));
-#endif
-    }
-    if (i & 1) sum1 = __fadd2_rn(sum1, p); else sum0 = __fadd2_rn(sum0, p);
-    pk[i] = pack16<BF16>(p.x, p.y);
   }
 #pragma unroll
   for (int c = 0; c < BN / 64; ++c) tmem_st32(s_addr + c * 32, *reinterpret_cast<const uint32_t(*)[32]>(&pk[c * 32]));
@@ -354,17 +280,6 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   const int clean_j = (n > 0 && (j_base + n) * BN > kv_len) ? n - 1 : -1;
 
   if (threadIdx.x == 0) {
-#ifdef PJX_TRACE
-    if (blockIdx.x < 8192) {
-      unsigned smid;
-      unsigned long long gt;
-      asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
-      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(gt));
-      g_cta[blockIdx.x][0] = smid;
-      g_cta[blockIdx.x][6] = (long long)gt;
-    }
-#endif
-    PJX_CTA_AT(1);
     for (int i = 0; i < C::N_BAR; ++i)
       mbar_init(BAR(i), i == V_CLEAN ? 32u : (((i >= P_FULL && i < P_FULL + 2) || i >= B_EMPTY) ? 128u : 1u));
     *abort_flag = 0;
@@ -479,7 +394,6 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             mma_commit(BAR(S_FULL + t), leader);
           }
         mma_commit(BAR(K_EMPTY + 0), leader);
-        PJX_CTA_AT(2);
       }
       for (int j = 0; ok && j < n; ++j) {
         const bool have_next = j + 1 < n;
@@ -490,26 +404,21 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
           if (j < n_t[t]) {
-            PJX_TRACE_AT(2, j, 4 * t + 0);
             ok = mbar_wait_all(BAR(P_FULL + t), j & 1, abort_flag);
             if (!ok) break;
             tc_fence_after();
-            PJX_TRACE_AT(2, j, 4 * t + 1);
             issue_pv(t, j);
-            PJX_TRACE_AT(2, j, 4 * t + 2);
             if (j == n_t[t] - 1) mma_commit(BAR(O_FULL + t), leader);
           }
           if (j + 1 < n_t[t]) {
             issue_s(t, j + 1);
             mma_commit(BAR(S_FULL + t), leader);
-            PJX_TRACE_AT(2, j, 4 * t + 3);
           }
         }
         if (!ok) break;
         mma_commit(BAR(V_EMPTY + j % VST), leader);
         if (have_next) mma_commit(BAR(K_EMPTY + (j + 1) % KST), leader);
       }
-      PJX_CTA_AT(3);
     }
   } else {
     // ------------------------------------------------------------ softmax warps
@@ -550,18 +459,10 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     float m_ref = -INFINITY, l = 0.f;
     bool ok = true;
     for (int j = 0; j < my_n; ++j) {
-      PJX_TRACE_AT(t, j, 0);
       ok = mbar_wait(BAR(S_FULL + t), j & 1, abort_flag);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      PJX_TRACE_AT(t, j, 1);
-#if PJX_EXP_VARIANT == 12
-      l = 1.f;
-      tc_fence_before();
-      mbar_arrive(BAR(P_FULL + t));
-      continue;
-#endif
       constexpr int NCH = BN / 32;
       const int k0 = (j_base + j) * BN;
       bool need_mask;
@@ -578,15 +479,9 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 
       // The whole row of scores in registers: all loads in flight at once.
       float s[BN];
-#if PJX_EXP_VARIANT == 10
-#pragma unroll
-      for (int i = 0; i < BN; ++i) s[i] = __int_as_float(0x3c000000 + ((i * 37 + j * 11 + lane) & 0xffff));
-#else
 #pragma unroll
       for (int c = 0; c < NCH; ++c) tmem_ld32f(s_addr + c * 32, &s[c * 32]);
       tmem_wait_ld();
-#endif
-      PJX_TRACE_AT(t, j, 2);
 
       if (MOD == 2 && mod_terms) {
         // scaled score -> modifiers -> exp2 domain; a dense bias (BIAS == 1) is added below on top.
@@ -778,9 +673,6 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         mx = fmaxf(fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3])), fmaxf(fmaxf(m[4], m[5]), fmaxf(m[6], m[7])));
       }
       mx *= cs;  // cs > 0
-#if PJX_EXP_VARIANT == 13
-      mx = 4.f;
-#endif
 
       // lazy running maximum: advance only when it grew by more than 8 (base 2)
       const bool need = (mx > m_ref + 8.f) || (m_ref == -INFINITY && mx > -INFINITY);
@@ -797,25 +689,14 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       const float neg_m = (m_ref == -INFINITY) ? 0.f : -m_ref;
       const float2 cs2 = make_float2(cs, cs), nm2 = make_float2(neg_m, neg_m);
       float2 sum0 = make_float2(0.f, 0.f), sum1 = make_float2(0.f, 0.f);
-      PJX_TRACE_AT(t, j, 3);
       if constexpr (MOD == 2) {
         if (mv.drop_rate > 0.f)
           exp_pack_store_scaled<BN, BF16>(s, cs2, nm2, sum0, sum1, s_addr, [&](int i) { return mod_dropout(mv, row, k0 + i); });
         else
           exp_pack_store<BN, BF16>(s, cs2, nm2, sum0, sum1, s_addr);
       } else {
-#if PJX_EXP_VARIANT == 0 || PJX_EXP_VARIANT >= 10
         exp_pack_store<BN, BF16>(s, cs2, nm2, sum0, sum1, s_addr);
-#elif PJX_EXP_VARIANT == 9
-        exp_pack_store_emu<BN, BF16, 0>(s, cs2, nm2, sum0, sum1, s_addr);
-#else
-        if (need_mask)
-          exp_pack_store<BN, BF16>(s, cs2, nm2, sum0, sum1, s_addr);
-        else
-          exp_pack_store_emu<BN, BF16, PJX_EXP_VARIANT>(s, cs2, nm2, sum0, sum1, s_addr);
-#endif
       }
-      PJX_TRACE_AT(t, j, 4);
       const float lsum = (sum0.x + sum0.y) + (sum1.x + sum1.y);
 
       // rescale O only now: the score registers are free again (the previous P.V of this
@@ -835,7 +716,6 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       tmem_wait_st();
       tc_fence_before();
       mbar_arrive(BAR(P_FULL + t));
-      PJX_TRACE_AT(t, j, 5);
     }
 
     if (ok && (q0 + t * BM) < p.Lq) {
@@ -901,7 +781,6 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         // first half to arrive: nothing more to do
       } else if (ok) {
         tc_fence_after();
-        if (threadIdx.x == 320 - 128) PJX_CTA_AT(4);
         // O leaves through shared memory: every thread writes its row (16-bit, 128-byte-swizzled
         // like the tensor map expects) over the query tile, which the MMAs no longer read, and one
         // thread hands the tile to a TMA store, which clips rows past Lq. Stores straight from the
@@ -970,7 +849,6 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   if (warp == 0) {
     __syncwarp();
     tmem_dealloc(tmem, C::TMEM_COLS);
-    if (lane == 0) PJX_CTA_AT(5);
     if (lane == 0 && *abort_flag && p.status) atomicExch(p.status, (int)PJX_ERR_DEVICE_TIMEOUT);
   }
 }
@@ -1310,14 +1188,6 @@ bool fwd_sm100_supported(const FwdParams& p, int dtype, const char** why) {
   return w == nullptr;
 }
 
-#ifdef PJX_TRACE
-extern "C" int pjx_debug_read_trace(long long* host_out) {
-  return (int)cudaMemcpyFromSymbol(host_out, g_trace, sizeof(long long) * 3 * 64 * 8);
-}
-extern "C" int pjx_debug_read_cta(long long* host_out) {
-  return (int)cudaMemcpyFromSymbol(host_out, g_cta, sizeof(long long) * 8192 * 8);
-}
-#endif
 
 int launch_fwd_sm100(const FwdParams& p, int dtype, cudaStream_t stream) {
   const char* why = nullptr;

@@ -149,7 +149,9 @@ __device__ __forceinline__ void copy16_async(uint32_t dst, const float* src) {
 }
 
 // Keys on the lanes: keys key0 .. key0 + 31, rows i0 .. i0 + CH - 1 of a plane, rows and keys past the tensor clamped (their
-// values are masked).  Slot layout [CH rows][32 keys].
+// values are masked).  Slot layout [CH rows][32 keys].  Callers leave out chunks wholly past the tensor: clamped, they read
+// the last row or key only, and with short sequences that share a plane every SM hit those few lines of the L2 (backward at
+// B64 L64 H16 D64: 482 us with one plane, 107 with a plane per head; now 98 with either).
 __device__ __forceinline__ void fetch_bias_column(uint32_t slot, const float* plane, int key0, int i0, int Lq, int Lkv, bool vec, int lane) {
   if (vec) {
     const float* src = plane + min(key0 + 4 * (lane & 7), Lkv - 4);
@@ -657,8 +659,12 @@ bwd_dq_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     constexpr int NB = BIAS_RING<D>;
     [[maybe_unused]] const uint32_t ring = sbase + C::OFF_BIAS + (warp - 2) * NB * BIAS_SLOT;
     [[maybe_unused]] const float* bsrc = (FEAT & 2) ? p.bias + (int64_t)b * p.bias_bs + (int64_t)h * p.bias_hs : nullptr;
-    auto fetch_bias = [&](int t) {  // chunk t of this warp: CH keys, four chunks per tile
-      if (t < 4 * n)
+    // chunk t of this warp: CH keys, four chunks per tile; the chunks before t_end have a row and a key within the tensor
+    const int keys = p.Lkv - j_lo * BN - grp * 64;
+    [[maybe_unused]] const int t_end =
+        q0 + quarter * 32 < p.Lq && keys > 0 ? min(4 * n, keys / BN * 4 + min(4, (keys % BN + CH - 1) / CH)) : 0;
+    auto fetch_bias = [&](int t) {
+      if (t < t_end)
         fetch_bias_rows(ring + (t % NB) * BIAS_SLOT, bsrc, q0 + quarter * 32, (j_lo + t / 4) * BN + grp * 64 + (t % 4) * CH, p.Lq,
                         p.Lkv, a.bias_vec, lane);
       copy_commit();
@@ -967,13 +973,13 @@ bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
     constexpr int NB = BIAS_RING<D>;
     [[maybe_unused]] const uint32_t ring = sbase + C::OFF_BIAS + (warp - 2) * NB * BIAS_SLOT;
     // dense bias: position of the next chunk to fetch (chunk of the half, query tile, head of the group)
-    [[maybe_unused]] int f_cc = 0, f_t = 0, f_g = 0;
+    [[maybe_unused]] int f_cc = 0, f_t = 0, f_g = n > 0 && k0 + quarter * 32 < p.Lkv ? 0 : G;
     [[maybe_unused]] const float* bsrc =
         (FEAT & 2) ? p.bias + (int64_t)b * p.bias_bs + (int64_t)hk * G * p.bias_hs : nullptr;
     auto fetch_bias = [&](int slot) {
-      if (f_g < G && n > 0)
-        fetch_bias_column(ring + slot * BIAS_SLOT, bsrc + (int64_t)f_g * p.bias_hs, k0 + quarter * 32,
-                          (t_lo + f_t) * QT + grp * HALF + f_cc * CH, p.Lq, p.Lkv, a.bias_vec, lane);
+      const int i0 = (t_lo + f_t) * QT + grp * HALF + f_cc * CH;
+      if (f_g < G && i0 < p.Lq)
+        fetch_bias_column(ring + slot * BIAS_SLOT, bsrc + (int64_t)f_g * p.bias_hs, k0 + quarter * 32, i0, p.Lq, p.Lkv, a.bias_vec, lane);
       copy_commit();
       if (++f_cc == NCH) {
         f_cc = 0;

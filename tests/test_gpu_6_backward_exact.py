@@ -233,3 +233,34 @@ def test_only_the_rounding_of_the_result_is_left(kind, dtype):
         rounding = float((w.to(dtype).double() - w).norm())
         err = float((x.double() - w).norm())
         assert err <= 1.001 * rounding + float(n.norm()), f"{name}: {err / rounding:.5f} of the rounding error"
+
+
+# ------------------------------------------------------------------------------------------- many short sequences
+
+
+def _time_us(fn):
+    start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+    best = math.inf
+    for _ in range(6):
+        torch.cuda._sleep(1_000_000)
+        start.record()
+        for _ in range(5):
+            fn()
+        end.record()
+        end.synchronize()
+        best = min(best, start.elapsed_time(end) * 200)
+    return best
+
+
+@pytest.mark.parametrize("b,n,h,planes,bias_grad", [(64, 64, 16, 1, False)])
+def test_many_short_sequences_are_not_slower_than_on_cuda_cores(b, n, h, planes, bias_grad):
+    """Short sequences that share a bias: the default route takes at most 1.3 times as long as the CUDA-core kernels (every SM
+    reading the last line of the bias: 1.4 times)."""
+    dvc = dev()
+    q, k, v, g = (randn((b, n, h, 64), torch.bfloat16, i).to(dvc) for i in range(4))
+    kw = dict(sm_scale=0.125, bias=randn((1, planes, n, n), torch.float32, 5).to(dvc))
+    o, lse = A.attention_forward(q, k, v, return_lse=True, **kw)
+    kw["bias_grad"] = bias_grad
+    got = _time_us(lambda: A.attention_backward(q, k, v, o, lse, g, **kw))
+    base = _time_us(lambda: A.attention_backward(q, k, v, o, lse, g, impl="b200:generic", **kw))
+    assert got <= 1.3 * base, f"{got:.1f} us against {base:.1f}"

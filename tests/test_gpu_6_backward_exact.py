@@ -238,6 +238,23 @@ def test_only_the_rounding_of_the_result_is_left(kind, dtype):
 # ------------------------------------------------------------------------------------------- many short sequences
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("b,lq,lkv,hq,hkv,planes,d", [
+    (8, 64, 64, 4, 4, (1, 1), 64),      # one tile, 32 pairs: clusters of four
+    (33, 40, 72, 2, 2, (1, 1), 128),    # 66 pairs over eight CTAs, slices of unequal length
+    (64, 130, 33, 2, 1, (1, 2), 64),    # two query tiles, an odd number of keys
+    (2, 260, 200, 16, 4, (2, 1), 64),   # three by two tiles per sequence, 16 heads each
+])
+def test_bias_gradient_shared_by_many_pairs(b, lq, lkv, hq, hkv, planes, d, dtype):
+    """A bias that many (sequence, head) pairs share: its gradient is summed by clusters of CTAs, among them slices of pairs
+    whose keys are all past the valid length.  The order of the sum differs from the oracle route's by the pairs: 2^-24
+    sqrt(pairs) of the magnitudes, far inside ``_compare``'s bound."""
+    dense = randn((*planes, lq, lkv), torch.float32, 7).to(dev())
+    lens = torch.tensor([(i * 29) % (lkv + 1) for i in range(b)], dtype=torch.int32)
+    _compare(b, lq, lkv, hq, hkv, d, d, dtype, mask=M.KVLenMask(lens), dense=dense, poison=True)
+    _compare(b, lq, lkv, hq, hkv, d, d, dtype, mask=M.LocalWindowMask(20, 9), bias=M.CausalAlibiBias(), dense=dense)
+
+
 def _time_us(fn):
     start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
     best = math.inf
@@ -252,10 +269,10 @@ def _time_us(fn):
     return best
 
 
-@pytest.mark.parametrize("b,n,h,planes,bias_grad", [(64, 64, 16, 1, False)])
+@pytest.mark.parametrize("b,n,h,planes,bias_grad", [(64, 64, 16, 1, False), (64, 64, 16, 1, True)])
 def test_many_short_sequences_are_not_slower_than_on_cuda_cores(b, n, h, planes, bias_grad):
     """Short sequences that share a bias: the default route takes at most 1.3 times as long as the CUDA-core kernels (every SM
-    reading the last line of the bias: 1.4 times)."""
+    reading the last line of the bias: 1.4 times; one CTA walking all pairs of a tile: 5.4 times)."""
     dvc = dev()
     q, k, v, g = (randn((b, n, h, 64), torch.bfloat16, i).to(dvc) for i in range(4))
     kw = dict(sm_scale=0.125, bias=randn((1, planes, n, n), torch.float32, 5).to(dvc))

@@ -206,7 +206,10 @@ size_t pjx_attn_bwd_workspace_bytes(int B, int Lq, int Hq);
  * All forms of the backward take pjx_attn_bwd_workspace_bytes or more.  With
  * pjx_attn_bwd_mod_workspace_bytes, and 16-byte aligned, every 16-bit call of those head shapes runs on
  * the tensor cores.  With less, fp16 calls that carry modifiers, a dense bias or the head shape (192, 128) run
- * on the CUDA cores, and bf16 calls with segment ids visit all tiles instead of those that can match. */
+ * on the CUDA cores, and bf16 calls with segment ids visit all tiles instead of those that can match.
+ * Except: calls with modifiers or a dense bias of at most 32 queries and 32 keys run on the CUDA cores where that is
+ * faster (D = 64, fp16, or `dbias` asked for); a shared bias' gradient is then summed over the pairs in a fixed order
+ * from dS in the workspace (with less room, on the tensor cores). */
 size_t pjx_attn_bwd_mod_workspace_bytes(int B, int Lq, int Lkv, int Hq, int Hkv, int dtype);
 int pjx_attn_bwd_mod(const void* q, const void* k, const void* v, const void* o, const float* lse,
                      const void* d_o, void* dq, void* dk, void* dv, const int32_t* kv_lengths,

@@ -17,6 +17,8 @@
 // tiles); dK/dV (one CTA per 32-key tile of a KV head, walking the group's query heads
 // and their query tiles).  Threads form a 16 x 16 grid with 2 x 2 micro-tiles of the
 // 32 x 32 score tile.
+#include <algorithm>
+
 #include "pjx_common.cuh"
 
 namespace pjx {
@@ -286,7 +288,7 @@ __global__ void __launch_bounds__(NT) bwd_dq_kernel(const BwdParams p) {
     tile_p_ds(p, t, b, h, q0, k0, kv_len);
     __syncthreads();
     if (p.dbias) {  // d(loss)/d(bias_ij) = dS_ij (the bias enters the score unscaled)
-      float* db = p.dbias + (int64_t)b * p.bias_bs + (int64_t)h * p.bias_hs;
+      float* db = p.dbias + (int64_t)b * p.dbias_bs + (int64_t)h * p.dbias_hs;
 #pragma unroll
       for (int i = 0; i < 2; ++i)
 #pragma unroll
@@ -432,6 +434,53 @@ int launch_widths(const BwdParams& p, cudaStream_t stream) {
 
 // The kernels behind one backward call, picked by pjx_attn_bwd_mod.
 enum class BwdRoute { CudaCores, Sm100, Sm100Exact };
+
+// Calls of at most 32 queries and keys: one tile of the CUDA-core kernels, of which an SM runs several CTAs at a time, and a
+// 128 x 128 tile of the tcgen05 ones that is filled to a sixteenth.  Measured (backward at L = 16, us, tcgen05 / CUDA cores):
+//   ALiBi, 1024 (sequence, head) pairs: D64 bf16 117 / 88, fp16 134 / 88; D128 bf16 137 / 143, fp16 158 / 143; (192, 128) 155 / 168
+//          64 pairs (less than a wave of CTAs): D64 bf16 24 / 27, fp16 31 / 27; D128 bf16 27 / 35
+//   gradient of a shared bias, a product more per pair: 1024 pairs D64 195 / 99, D128 344 / 159; 64 pairs D64 39 / 34
+// From 33 rows on, four tiles of the CUDA-core kernels, the tensor cores are the faster ones.  The heads of a group are
+// walked by one CTA in both, with longer steps here: groups count only where the key heads fill the SMs.
+bool one_tile_on_cuda_cores(const BwdParams& p) {
+  if (p.Lq > T || p.Lkv > T || p.B > 65535 || p.Hq > 65535) return false;  // (their grids have B and Hq as axes)
+  const bool filled = (int64_t)p.B * p.Hkv > 148, fp16 = p.dtype == PJX_F16;
+  return filled ? p.dbias || p.D == 64 || (fp16 && p.D == 128) : p.Hq == p.Hkv && (p.dbias || (fp16 && p.D == 64));
+}
+
+// Bytes for dS of every (sequence, head) pair of such a call.
+size_t one_tile_ds_bytes(const BwdParams& p) {
+  return p.dtype != PJX_F32 && p.Lq <= T && p.Lkv <= T ? (size_t)p.B * p.Hq * p.Lq * p.Lkv * sizeof(float) : 0;
+}
+
+// Gradient of a bias from dS [B, Hq, n] of its pairs, summed in a fixed order: 32 threads take 32 entries of a plane, 32 warps
+// every 32nd pair each.
+__global__ void __launch_bounds__(1024) sum_pairs_kernel(const float* ds, float* dbias, int64_t bs, int64_t hs, int B, int Hq, int n) {
+  __shared__ float part[32][33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + lane, plane = blockIdx.y;
+  const int nhb = hs ? Hq : 1;
+  const int h0 = hs ? plane % nhb : 0, nh = hs ? 1 : Hq;
+  const int b0 = bs ? plane / nhb : 0, nb = bs ? 1 : B;
+  float sum = 0.f;
+  if (i < n) {
+#pragma unroll 8
+    for (int pi = warp; pi < nb * nh; pi += 32) sum += __ldg(ds + ((int64_t)(b0 + pi / nh) * Hq + h0 + pi % nh) * n + i);
+  }
+  part[warp][lane] = sum;
+  __syncthreads();
+  if (warp == 0 && i < n) {
+    for (int w = 1; w < 32; ++w) sum += part[w][lane];
+    dbias[b0 * bs + h0 * hs + i] = sum;
+  }
+}
+
+int launch_sum_pairs(const BwdParams& p, const float* ds, float* dbias, cudaStream_t stream) {
+  const int n = p.Lq * p.Lkv, planes = (p.bias_bs ? p.B : 1) * (p.bias_hs ? p.Hq : 1);
+  sum_pairs_kernel<<<dim3((n + 31) / 32, planes), 1024, 0, stream>>>(ds, dbias, p.bias_bs, p.bias_hs, p.B, p.Hq, n);
+  count_launch();
+  return check_cuda(cudaGetLastError(), "bias gradient sum launch");
+}
 
 template <typename T_>
 int launch_dtype(const BwdParams& p, BwdRoute route, void* scratch, size_t scratch_bytes, cudaStream_t stream) {
@@ -656,7 +705,7 @@ size_t pjx_attn_bwd_mod_workspace_bytes(int B, int Lq, int Lkv, int Hq, int Hkv,
   p.B = B; p.Lq = Lq; p.Lkv = Lkv; p.Hq = Hq; p.Hkv = Hkv;
   p.dtype = dtype;
   p.mod.seg_q = p.mod.seg_k = &ids;  // as with segment ids
-  return pjx_attn_bwd_workspace_bytes(B, Lq, Hq) + bwd_exact_scratch_bytes(p);
+  return pjx_attn_bwd_workspace_bytes(B, Lq, Hq) + std::max(bwd_exact_scratch_bytes(p), one_tile_ds_bytes(p));
 }
 
 int pjx_attn_bwd_band(const void* q, const void* k, const void* v, const void* o, const float* lse, const void* d_o,
@@ -722,6 +771,8 @@ int pjx_attn_bwd_mod(const void* q, const void* k, const void* v, const void* o,
     const int64_t hb = bias_head_stride ? Hq : 1, bbn = bias_batch_stride ? B : 1;
     dbias_bytes = (size_t)bbn * hb * Lq * Lkv * sizeof(float);
     p.dbias = dbias;
+    p.dbias_bs = bias_batch_stride;
+    p.dbias_hs = bias_head_stride;
     p.dbias_atomic = (bias_batch_stride == 0 && B > 1) || (bias_head_stride == 0 && Hq > 1);
   }
   // 16-bit calls that the plain tcgen05 kernels do not take (score modifiers, dense bias, the latent head shape) run
@@ -737,11 +788,24 @@ int pjx_attn_bwd_mod(const void* q, const void* k, const void* v, const void* o,
   BwdRoute route = impl != PJX_IMPL_GENERIC && tc_ok ? BwdRoute::Sm100 : BwdRoute::CudaCores;
   void* scratch = static_cast<char*>(workspace) + need;
   const size_t scratch_bytes = workspace_bytes > need ? workspace_bytes - need : 0;
-  if (impl == PJX_IMPL_AUTO && !tc_ok && bwd_exact_sm100_supported(p) && scratch_bytes >= bwd_exact_scratch_bytes_needed(p))
-    route = BwdRoute::Sm100Exact;
+  float* pair_ds = nullptr;  // dS of every pair, where the gradient of the bias sums it over several
+  if (impl == PJX_IMPL_AUTO && !tc_ok && bwd_exact_sm100_supported(p)) {
+    const bool shared = p.dbias && p.dbias_atomic;
+    if (one_tile_on_cuda_cores(p) && (!shared || scratch_bytes >= one_tile_ds_bytes(p))) {
+      if (shared) {
+        pair_ds = p.dbias = static_cast<float*>(scratch);
+        p.dbias_hs = (int64_t)Lq * Lkv;
+        p.dbias_bs = Hq * p.dbias_hs;
+        p.dbias_atomic = false;
+        dbias_bytes = one_tile_ds_bytes(p);
+      }
+    } else if (scratch_bytes >= bwd_exact_scratch_bytes_needed(p)) {
+      route = BwdRoute::Sm100Exact;
+    }
+  }
   p.lse_natural = route == BwdRoute::Sm100Exact && (smod.rel_bias || bias);
   if (dbias_bytes > 0 && route == BwdRoute::CudaCores) {  // (the tcgen05 kernel writes every entry)
-    const int rc0 = check_cuda(cudaMemsetAsync(dbias, 0, dbias_bytes, st), "clear dbias");
+    const int rc0 = check_cuda(cudaMemsetAsync(p.dbias, 0, dbias_bytes, st), "clear dbias");
     if (rc0) return rc0;
   }
   if (Lq == 0) {  // no queries: the key-side gradients are zero
@@ -749,11 +813,14 @@ int pjx_attn_bwd_mod(const void* q, const void* k, const void* v, const void* o,
     if (rc) return rc;
     return check_cuda(cudaMemsetAsync(dv, 0, (size_t)B * Lkv * Hkv * Dv * dtype_size(dtype), st), "clear dv");
   }
+  int rc;
   switch (dtype) {
-    case PJX_F32: return launch_dtype<float>(p, route, scratch, scratch_bytes, st);
-    case PJX_BF16: return launch_dtype<__nv_bfloat16>(p, route, scratch, scratch_bytes, st);
-    default: return launch_dtype<__half>(p, route, scratch, scratch_bytes, st);
+    case PJX_F32: rc = launch_dtype<float>(p, route, scratch, scratch_bytes, st); break;
+    case PJX_BF16: rc = launch_dtype<__nv_bfloat16>(p, route, scratch, scratch_bytes, st); break;
+    default: rc = launch_dtype<__half>(p, route, scratch, scratch_bytes, st);
   }
+  if (rc || !pair_ds) return rc;
+  return launch_sum_pairs(p, pair_ds, dbias, st);
 }
 
 int pjx_attn_bwd(const void* q, const void* k, const void* v, const void* o, const float* lse, const void* d_o,

@@ -571,5 +571,10 @@ def test_backward_workspace_sizes(built_lib):
     base = L.pjx_attn_bwd_workspace_bytes(2, 130, 8)
     assert L.pjx_attn_bwd_mod_workspace_bytes(2, 130, 300, 8, 4, _lib.PJX_BF16) == base + 2 * (2 + 3) * 8
     assert L.pjx_attn_bwd_mod_workspace_bytes(2, 130, 300, 8, 4, _lib.PJX_F16) == base + 2 * (2 + 3) * 8 + 2 * 4 * (3 + 600) * 4
+    # calls of one 32 x 32 tile: dS of every (sequence, head) pair, where that is more
+    small = L.pjx_attn_bwd_workspace_bytes(3, 20, 8)
+    assert L.pjx_attn_bwd_mod_workspace_bytes(3, 20, 32, 8, 4, _lib.PJX_BF16) == small + 3 * 8 * 20 * 32 * 4
+    assert L.pjx_attn_bwd_mod_workspace_bytes(3, 20, 33, 8, 4, _lib.PJX_BF16) == small + 3 * (1 + 1) * 8
+    assert L.pjx_attn_bwd_mod_workspace_bytes(3, 20, 32, 8, 4, _lib.PJX_F32) == small + 3 * (1 + 1) * 8
     assert L.pjx_attn_bwd_mod_workspace_bytes(2, 0, 0, 8, 4, _lib.PJX_F16) == 0
     assert L.pjx_attn_bwd_mod_workspace_bytes(2, -1, 300, 8, 4, _lib.PJX_BF16) == 0

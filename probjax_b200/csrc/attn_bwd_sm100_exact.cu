@@ -144,7 +144,7 @@ __device__ __forceinline__ float lds(uint32_t addr) {
   return x;
 }
 
-// Thread-block clusters (1 and 0 in a launch without them): shared memory of CTA `rank`, and a barrier of all threads.
+// Thread-block clusters: shared memory of CTA `rank`, and a barrier of all threads.
 __device__ __forceinline__ int cluster_size() {
   uint32_t n;
   asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(n));
@@ -1136,7 +1136,7 @@ struct DbCfg {
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
 };
 
-template <int D, int DV, bool BF16, int FEAT>
+template <int D, int DV, bool BF16, int FEAT, bool CLUSTER>
 __global__ void __launch_bounds__(NTHREADS, 1)
 bwd_dbias_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                        const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
@@ -1154,7 +1154,9 @@ bwd_dbias_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
 
   const int warp = uniform(static_cast<int>(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   const int n_kt = (p.Lkv + BN - 1) / BN, n_qt = (p.Lq + BM - 1) / BM;
-  const int item = blockIdx.x / cluster_size();
+  auto n_ranks = [] { return CLUSTER ? cluster_size() : 1; };  // (read where they are needed: nothing held over the loop)
+  auto rank = [] { return CLUSTER ? cluster_rank() : 0; };
+  const int item = blockIdx.x / n_ranks();
   const int k0 = item % n_kt * BN, q0 = item / n_kt % n_qt * BM;
   const int plane = item / (n_kt * n_qt);  // (batch, head) plane of the bias
   const int nhb = p.bias_hs ? p.Hq : 1;
@@ -1164,7 +1166,7 @@ bwd_dbias_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
   const bool in_band = p.mod.prefix_len || (k0 <= min(q0 + BM, p.Lq) - 1 + p.band_hi && min(k0 + BN, p.Lkv) - 1 >= q0 + p.band_lo);
   // this CTA's slice of them
   const int64_t n_all = in_band ? (int64_t)nb * nh : 0;
-  const int pi_begin = (int)(n_all * cluster_rank() / cluster_size()), pi_end = (int)(n_all * (cluster_rank() + 1) / cluster_size());
+  const int pi_begin = (int)(n_all * rank() / n_ranks()), pi_end = (int)(n_all * (rank() + 1) / n_ranks());
   const int G = p.Hq / p.Hkv;
   auto len_of = [&](int b) { return p.kv_lengths ? max(0, min(p.Lkv, p.kv_lengths[b])) : p.Lkv; };
 
@@ -1314,7 +1316,7 @@ bwd_dbias_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
       mbar_arrive(BAR(T_FREE + buf));
       ++it;
     }
-    if (cluster_size() > 1) {
+    if constexpr (CLUSTER) {
 #pragma unroll
       for (int e = 0; e < 64; ++e)
         asm volatile("st.shared.f32 [%0], %1;" ::"r"(btile + e * BN * 4), "f"(e % 2 ? acc[e / 2].y : acc[e / 2].x) : "memory");
@@ -1326,17 +1328,16 @@ bwd_dbias_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     }
   }
 
-  if (cluster_size() > 1) {
-    const int n_ranks = cluster_size(), rank = cluster_rank();  // (read again: nothing held over the loop)
+  if constexpr (CLUSTER) {
     // (after a wait that expired in one of the CTAs the sum means nothing: the status word says so)
     cluster_sync();
-    const int rows = BM / n_ranks, row0 = rank * rows;
+    const int rows = BM / n_ranks(), row0 = rank() * rows, n = n_ranks();
     const int64_t plane_at = (int64_t)b0 * p.bias_bs + (int64_t)h0 * p.bias_hs;
     for (int u = threadIdx.x; u < rows * BN; u += NTHREADS) {
       const int i = q0 + row0 + u / BN, j = k0 + u % BN;
       const uint32_t mine = sbase + C::OFF_BIAS + (row0 * BN + u) * 4;
       float sum = 0.f;
-      for (int r = 0; r < n_ranks; ++r) sum += lds_cluster(mine, r);
+      for (int r = 0; r < n; ++r) sum += lds_cluster(mine, r);
       if (i < p.Lq && j < p.Lkv) p.dbias[plane_at + (int64_t)i * p.Lkv + j] = sum;
     }
     cluster_sync();  // a CTA's shared memory outlives the reads of the others
@@ -1443,7 +1444,8 @@ int launch_feat(const BwdParams& p, const ExactArgs& a, cudaStream_t stream) {
     if (p.dbias) {
       const int64_t planes = (int64_t)(p.bias_bs ? p.B : 1) * (p.bias_hs ? p.Hq : 1), tiles = planes * n_q * n_k;
       const int cluster = dbias_cluster(tiles, (int64_t)p.B * p.Hq / planes);
-      return launch_kernel(bwd_dbias_sm100_kernel<D, DV, BF16, FEAT>, tiles * cluster, DbCfg<D, DV>::SMEM_BYTES, cluster, stream,
+      auto kern = cluster > 1 ? bwd_dbias_sm100_kernel<D, DV, BF16, FEAT, true> : bwd_dbias_sm100_kernel<D, DV, BF16, FEAT, false>;
+      return launch_kernel(kern, tiles * cluster, DbCfg<D, DV>::SMEM_BYTES, cluster, stream,
                            "sm100 dbias launch", tq, tdo, tk, tv, p);
     }
   }

@@ -295,3 +295,28 @@ def test_many_short_sequences_are_not_slower_than_on_cuda_cores(b, n, h, planes,
     got = _time_us(lambda: A.attention_backward(q, k, v, o, lse, g, **kw))
     base = _time_us(lambda: A.attention_backward(q, k, v, o, lse, g, impl="b200:generic", **kw))
     assert got <= 1.3 * base, f"{got:.1f} us against {base:.1f}"
+
+
+@pytest.mark.parametrize("b,n", [(32, 64), (40, 16)])
+def test_shared_bias_gradient_under_capture(b, n):
+    """The cluster launch and the sum over pairs replay from a graph, on new inputs in the captured buffers."""
+    dvc = dev()
+    q, k, v, g = (randn((b, n, 4, 64), torch.bfloat16, i).to(dvc) for i in range(4))
+    kw = dict(sm_scale=0.125, bias=randn((1, 1, n, n), torch.float32, 5).to(dvc))
+
+    def step():
+        o, lse = A.attention_forward(q, k, v, return_lse=True, **kw)
+        return A.attention_backward(q, k, v, o, lse, g, bias_grad=True, **kw)
+
+    side = torch.cuda.Stream(dvc)
+    with torch.cuda.stream(side):
+        step()
+    side.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        got = step()
+    for t in (q, k, v, g):
+        t.copy_(t.flip(0) * 0.5)
+    graph.replay()
+    torch.cuda.synchronize(dvc)
+    assert all(torch.equal(x, y) for x, y in zip(got, step()))

@@ -191,7 +191,8 @@ int pjx_attn_bwd(const void* q, const void* k, const void* v, const void* o, con
  * otherwise; SM100 forces the plain tcgen05 kernels (D = Dv in {64, 128}, no bias).
  * `status` as in pjx_attn_fwd.  `dbias` (float32, shape and strides of `bias`, or NULL) receives
  * the gradient of a learnable dense bias, summed over the axes the bias broadcasts: in a fixed order
- * by the tcgen05 kernels, with atomic adds (not bit-repeatable) by the CUDA-core ones. */
+ * by the tcgen05 kernels and for one-tile calls (see pjx_attn_bwd_mod), with atomic adds (not bit-repeatable) by
+ * the CUDA-core ones otherwise. */
 int pjx_attn_bwd_band(const void* q, const void* k, const void* v, const void* o, const float* lse,
                       const void* d_o, void* dq, void* dk, void* dv, const int32_t* kv_lengths,
                       const float* bias, int64_t bias_batch_stride, int64_t bias_head_stride,

@@ -18,7 +18,7 @@
 // to the input dtype before those products, as the reference does.  Scaling by sm_scale is
 // applied once, when dQ and dK leave tensor memory.
 //
-// Warps: 0 = TMA producer, 1 = MMA issuer (one lane), 2-5 and 6-9 = two compute groups; a group
+// Warps: 0 = TMA producer, 1 = MMA issuer (converged), 2-5 and 6-9 = two compute groups; a group
 // has one thread per tensor-memory lane (query row, or key row in the dK/dV kernel) and takes
 // one half of the 128 score columns, so that every scheduler has two compute warps to
 // interleave.  A group writes its 16-bit results over the first 32 columns of its own half,
@@ -642,7 +642,7 @@ bool bwd_sm100_supported(const BwdParams& p, const char** why) {
   const char* w = nullptr;
   if (p.dtype != PJX_BF16 && p.dtype != PJX_F16) w = "dtype must be bf16 or fp16";
   else if (!(p.D == p.Dv && (p.D == 64 || p.D == 128))) w = "head dims must be (64,64) or (128,128)";
-  else if (p.bias) w = "a dense bias is taken by the CUDA-core kernels only";
+  else if (p.bias) w = "the plain kernels take no dense bias (AUTO runs others on it)";
   else if (p.B < 1 || p.Lq < 1 || p.Lkv < 1) w = "empty problem";
   else if ((int64_t)((p.Lq + BM - 1) / BM) * p.Hq * p.B > 0x7fffffffLL ||
            (int64_t)((p.Lkv + BN - 1) / BN) * p.Hkv * p.B > 0x7fffffffLL)

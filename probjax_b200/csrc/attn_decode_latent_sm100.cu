@@ -20,9 +20,9 @@
 //   warp 0      TMA producer of the score ring (one lane)
 //   warp 6      TMA producer of the output ring (one lane); the whole warp clears the rows past the valid
 //               length in the pairs of a split's last tile (0 x NaN is not 0 inside the second product)
-//   warp 1      MMA issuer of the scores (one lane): S^T(0), S^T(1), then S^T(t+2) once P(t) has been written
+//   warp 1      MMA issuer of the scores (converged, one elected lane): S^T(0), S^T(1), then S^T(t+2) once P(t) has been written
 //               (the softmax has then read S^T[t % 2])
-//   warp 7      MMA issuer of the output (one lane): the pairs of P(t).C(t).  Two issuers, because an N = 16
+//   warp 7      MMA issuer of the output (likewise): the pairs of P(t).C(t).  Two issuers, because an N = 16
 //               MMA takes 32 cycles and one thread cannot issue them that fast, and because either ring
 //               would otherwise wait for the other's data
 //   warps 2-5   softmax: one thread per key (= tensor-memory lane).  The maximum over the keys of a

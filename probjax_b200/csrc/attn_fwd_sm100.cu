@@ -7,7 +7,7 @@
 // CTA and used by both query tiles.
 //
 //   warp 0      TMA producer (one lane): Q tiles, then a K ring and a V ring
-//   warp 1      MMA issuer (one lane): S_t = Q_t.K^T (both operands in shared
+//   warp 1      MMA issuer (converged, one elected lane): S_t = Q_t.K^T (both operands in shared
 //               memory), O_t += P_t.V (P_t read from tensor memory, V in shared
 //               memory, MN-major)
 //   warps 2-5   softmax of tile 0: one thread per query row, the row's scores held

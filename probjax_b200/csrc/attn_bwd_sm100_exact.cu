@@ -34,9 +34,9 @@
 //
 // Bound by the element work of the compute warps at D = 64 and with modifiers (20 to 30 issue slots per score), by the
 // chain of MMAs, element work and barrier round trips at D = 128 and 192 without.
-// Spills (bytes stored / loaded, -Xptxas -v): dK/dV with modifiers 48 / 112 in bf16, with a dense bias beside them 168 to 200 /
-// 180 to 236; the bias gradient with modifiers 312 / 328; the others 44 / 40 at most.  The two compute groups leave 168 to 200
-// registers to a thread.
+// Spills (bytes stored / loaded, -Xptxas -v; 320 threads leave 204 registers to each): dK/dV with modifiers 44 to 68 / 76 to
+// 112, with a dense bias beside them 168 to 200 / 180 to 236; the bias gradient 16 to 24 / 16 to 44, with modifiers 312 / 328;
+// the other kernels 52 / 60 at most.
 // Measured (forward + backward, against the CUDA-core kernels these calls ran on before; B200):
 //   packed documents + ALiBi, B1 S4096 Hq32 Hkv8 D128 bf16     41.9 ms -> 0.48 ms
 //   dense bias with gradient, B8 S1024 H16 D64 bf16            6.26 ms -> 0.49 ms

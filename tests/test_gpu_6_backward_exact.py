@@ -4,7 +4,8 @@ Its P and dS enter the products as 16 + 16 bits, so its 16-bit gradients may dif
 CUDA-core kernels (same inputs, same saved o and lse) by the rounding of the result only: one unit in the last
 place of an element, 2^-8 (bf16) or 2^-11 (fp16) of it, hence at most that of the norm.  The bias gradient is fp32;
 its error is that of the scores and of dP, sums of D products (2^-24 sqrt(D) each, doubled for the unit's
-truncation), times the cancellation in dP - delta: 1e-4 of the norm leaves a factor of ten.
+truncation), times the cancellation in dP - delta: 1e-4 of the norm leaves a factor of ten.  That bound is one unit of the
+whole norm and does not show whether the low halves are there: the comparisons with float64 further down do, row by row.
 """
 
 import math
@@ -122,6 +123,14 @@ def test_dense_bias_and_its_gradient(shape, d, dtype):
         lens = torch.tensor([lkv, lkv // 2], dtype=torch.int32)
         _compare(2, lq, lkv, 4, 2, d, d, dtype, mask=M.KVLenMask(lens), dense=dense, poison=True)
         _compare(2, lq, lkv, 4, 2, d, d, dtype, mask=M.CausalMask(), bias=M.CausalAlibiBias(), dense=dense, dropout=0.1)
+
+
+def test_large_grids():
+    """More CTAs than SMs in both kernels, 19 tiles along both axes, a last tile of 5 rows."""
+    n = 18 * 128 + 5
+    _compare(1, n, n, 16, 4, 128, 128, torch.bfloat16, mask=M.BlockDiagonalCausalMask(_segments(1, n, 5)), bias=M.CausalAlibiBias())
+    _compare(2, n, n, 8, 8, 192, 128, torch.float16, mask=M.CausalMask())
+    _compare(3, n, 1025, 8, 8, 64, 64, torch.float16, dense=randn((1, 8, n, 1025), torch.float32, 7).to(dev()))
 
 
 @pytest.mark.parametrize("fill", [-math.inf, torch.finfo(torch.float32).min, -1e9])

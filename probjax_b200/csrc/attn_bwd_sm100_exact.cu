@@ -41,6 +41,8 @@
 //   packed documents + ALiBi, B1 S4096 Hq32 Hkv8 D128 bf16     41.9 ms -> 0.48 ms
 //   dense bias with gradient, B8 S1024 H16 D64 bf16            6.26 ms -> 0.49 ms
 //   latent training step, B2 S2048 H16 (192,128) bf16          16.6 ms -> 0.42 ms
+#include <atomic>
+
 #include "attn_bwd_sm100.cuh"
 
 namespace pjx {
@@ -1120,9 +1122,10 @@ bwd_dkdv_exact_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
 // costs two products per pair and no memory traffic; adding dS into memory from the dQ kernel instead would move
 // 4 bytes per score through the L2's atomic units (537 MB at B8 S1024 H16) in an order that changes per run.
 // Where the tiles leave SMs idle and many pairs share them (short sequences, a bias shared by the heads) a cluster of up to
-// eight CTAs shares a tile: each walks a slice of the pairs and keeps its sum in shared memory, then each adds up a slice of
+// sixteen CTAs shares a tile: each walks a slice of the pairs and keeps its sum in shared memory, then each adds up a slice of
 // the rows over the cluster in rank order.  One CTA per tile took 1.4 us per pair: B64 L64 H16 D64 with one plane (1024
-// pairs, one tile) 1474 us for the whole backward, against 344 on the CUDA cores; now 238.
+// pairs, one tile) 1474 us for the whole backward, against 344 on the CUDA cores; with up
+// to eight 236, with up to sixteen 172.
 template <int D, int DV>
 struct DbCfg {
   static constexpr int SUBQ = D / 64, SUBV = DV / 64;
@@ -1286,6 +1289,14 @@ bwd_dbias_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
           mixed = segments_mixed(mv.seg_q, i_first, 64, p.Lq, own_seg, lane);
         }
       }
+      // with modifiers the mask of all chunks ahead of the wait and out of the straight line below, whose code and registers
+      // it fills otherwise
+      [[maybe_unused]] uint64_t visible = 0;
+      if constexpr ((FEAT & 1) != 0) {
+#pragma unroll 1
+        for (int cc = 0; cc < 64 / CH; ++cc)
+          visible |= (uint64_t)keep_bits<FEAT, false>(pl, mv, mixed, own_seg, i_first + cc * CH, key) << (CH * cc);
+      }
       const uint32_t s_addr = tmem + buf * 256 + lane_sel + grp * 64, dp_addr = s_addr + 128;
       ok = mbar_wait(BAR(SP_FULL + buf), (it >> 1) & 1, abort_flag);
       if (ok) ok = mbar_wait(BAR(ROW_FULL + buf), (it >> 1) & 1, abort_flag);
@@ -1310,7 +1321,8 @@ bwd_dbias_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         tmem_wait_ld();
         int i0 = i_first + cc * CH;
         asm volatile("" : "+r"(i0));  // the tests below do not change over the pairs: not all of them ahead of the loop
-        const uint32_t keep = keep_bits<FEAT, false>(pl, mv, mixed, own_seg, i0, key);
+        const uint32_t keep = (FEAT & 1) ? (uint32_t)(visible >> (CH * cc)) & ((1u << CH) - 1)
+                                         : keep_bits<FEAT, false>(pl, mv, mixed, own_seg, i0, key);
         chunk_p_ds<FEAT, false, false>(s, dp, p.sm_scale, pl, mv, keep, i0, key, lse, delta, bias, pr, ds);
 #pragma unroll
         for (int i = 0; i < CH / 2; ++i) acc[cc * CH / 2 + i] = __fadd2_rn(acc[cc * CH / 2 + i], ds[i]);
@@ -1398,6 +1410,7 @@ template <typename... Params, typename... Args>
 int launch_kernel(void (*kern)(Params...), int64_t grid, int smem, int cluster, cudaStream_t stream, const char* what,
                   const Args&... args) {
   int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), what);
+  if (!rc && cluster > 8) rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1), what);
   if (rc) return rc;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
@@ -1416,12 +1429,48 @@ int launch_kernel(void (*kern)(Params...), int64_t grid, int smem, int cluster, 
 }
 
 // CTAs that share a tile of the bias gradient: as many as the SMs take, each with four pairs or more (below that the exchange
-// costs what the shorter walk saves).
-int dbias_cluster(int64_t tiles, int64_t pairs) {
+// costs what the shorter walk saves).  Sixteen, for a tile or a few that thousands of pairs share, is past the portable size:
+// only where the device says that such a cluster finds its SMs.
+template <typename K>
+int dbias_cluster(K kern, int smem, int64_t tiles, int64_t pairs) {
+  static std::atomic<signed char> sixteen[64];  // per device: 0 not asked yet, 1 yes, -1 no
   int dev = 0, sms = 148, n = 1;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  while (n < 8 && 2 * n * tiles <= sms && pairs >= 8 * n) n *= 2;
-  return n;
+  while (n < 16 && 2 * n * tiles <= sms && pairs >= 8 * n) n *= 2;
+  if (n < 16) return n;
+  if (dev < 0 || dev >= 64) return 8;
+  if (sixteen[dev] == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(16);
+    cfg.blockDim = dim3(NTHREADS);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 16;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int fit = 0;
+    const bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
+                    cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&fit, kern, &cfg) == cudaSuccess && fit > 0;
+    if (!ok) (void)cudaGetLastError();
+    sixteen[dev] = ok ? 1 : -1;
+  }
+  return sixteen[dev] > 0 ? 16 : 8;
+}
+
+template <int D, int DV, bool BF16, int FEAT>
+int launch_dbias(const BwdParams& p, const CUtensorMap& tq, const CUtensorMap& tdo, const CUtensorMap& tk, const CUtensorMap& tv,
+                 cudaStream_t stream) {
+  constexpr int SMEM = DbCfg<D, DV>::SMEM_BYTES;
+  const char* what = "sm100 dbias launch";
+  const int64_t planes = (int64_t)(p.bias_bs ? p.B : 1) * (p.bias_hs ? p.Hq : 1);
+  const int64_t tiles = planes * ((p.Lq + BM - 1) / BM) * ((p.Lkv + BN - 1) / BN);
+  auto shared = bwd_dbias_sm100_kernel<D, DV, BF16, FEAT, true>;
+  const int cluster = dbias_cluster(shared, SMEM, tiles, (int64_t)p.B * p.Hq / planes);
+  if (cluster > 1) return launch_kernel(shared, tiles * cluster, SMEM, cluster, stream, what, tq, tdo, tk, tv, p);
+  return launch_kernel(bwd_dbias_sm100_kernel<D, DV, BF16, FEAT, false>, tiles, SMEM, 1, stream, what, tq, tdo, tk, tv, p);
 }
 
 template <int D, int DV, bool BF16, int FEAT>
@@ -1445,11 +1494,9 @@ int launch_feat(const BwdParams& p, const ExactArgs& a, cudaStream_t stream) {
     return rc;
   if constexpr ((FEAT & 2) != 0) {
     if (p.dbias) {
-      const int64_t planes = (int64_t)(p.bias_bs ? p.B : 1) * (p.bias_hs ? p.Hq : 1), tiles = planes * n_q * n_k;
-      const int cluster = dbias_cluster(tiles, (int64_t)p.B * p.Hq / planes);
-      auto kern = cluster > 1 ? bwd_dbias_sm100_kernel<D, DV, BF16, FEAT, true> : bwd_dbias_sm100_kernel<D, DV, BF16, FEAT, false>;
-      return launch_kernel(kern, tiles * cluster, DbCfg<D, DV>::SMEM_BYTES, cluster, stream,
-                           "sm100 dbias launch", tq, tdo, tk, tv, p);
+      // of head scale, soft cap and dropout only dropout comes with the gradient of a bias
+      return p.mod.dropout_rate > 0.f ? launch_dbias<D, DV, BF16, FEAT>(p, tq, tdo, tk, tv, stream)
+                                      : launch_dbias<D, DV, BF16, FEAT & 3>(p, tq, tdo, tk, tv, stream);
     }
   }
   return PJX_OK;

@@ -249,10 +249,10 @@ def test_only_the_rounding_of_the_result_is_left(kind, dtype):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("b,lq,lkv,hq,hkv,planes,d", [
-    (8, 64, 64, 4, 4, (1, 1), 64),      # one tile, 32 pairs: clusters of four
-    (33, 40, 72, 2, 2, (1, 1), 128),    # 66 pairs over eight CTAs, slices of unequal length
-    (64, 130, 33, 2, 1, (1, 2), 64),    # two query tiles, an odd number of keys
-    (2, 260, 200, 16, 4, (2, 1), 64),   # three by two tiles per sequence, 16 heads each
+    (8, 64, 64, 4, 4, (1, 1), 64),      # one tile, 32 pairs: a cluster of eight
+    (33, 40, 72, 2, 2, (1, 1), 128),    # one tile, 66 pairs: sixteen CTAs, slices of unequal length
+    (64, 130, 33, 2, 1, (1, 2), 64),    # four tiles, an odd number of keys, 64 pairs each
+    (2, 260, 200, 16, 4, (2, 1), 64),   # three by two tiles per sequence, 16 heads each: clusters of four
 ])
 def test_bias_gradient_shared_by_many_pairs(b, lq, lkv, hq, hkv, planes, d, dtype):
     """A bias that many (sequence, head) pairs share: its gradient is summed by clusters of CTAs, among them slices of pairs
@@ -291,14 +291,17 @@ def _time_us(fn):
     return best
 
 
+@pytest.mark.parametrize("alibi", [False, True])
 @pytest.mark.parametrize("b,n,h,planes,bias_grad", [(64, 64, 16, 1, False), (64, 64, 16, 1, True), (256, 16, 8, 1, True), (256, 16, 8, 8, False)])
-def test_many_short_sequences_are_not_slower_than_on_cuda_cores(b, n, h, planes, bias_grad):
+def test_many_short_sequences_are_not_slower_than_on_cuda_cores(b, n, h, planes, bias_grad, alibi):
     """Short sequences that share a bias: the default route takes at most 1.3 times as long as the CUDA-core kernels (every SM
     reading the last line of the bias: 1.4 times; one CTA walking all pairs of a tile: 5.4 times; tcgen05 tiles filled to a
     sixteenth: 3.2 times)."""
     dvc = dev()
     q, k, v, g = (randn((b, n, h, 64), torch.bfloat16, i).to(dvc) for i in range(4))
     kw = dict(sm_scale=0.125, bias=randn((1, planes, n, n), torch.float32, 5).to(dvc))
+    if alibi:
+        kw["mods"] = A.ScoreMods(M.split_mask(None, b, n, n)[0], M.lower_bias_structured(M.CausalAlibiBias(), b, h, n, n), dvc, 0.0, 0)
     o, lse = A.attention_forward(q, k, v, return_lse=True, **kw)
     kw["bias_grad"] = bias_grad
     got = _time_us(lambda: A.attention_backward(q, k, v, o, lse, g, **kw))

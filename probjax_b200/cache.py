@@ -114,8 +114,15 @@ def rope_interleaved(x: torch.Tensor, positions=None, *, base: float = 10_000.0,
 
 
 def _check_layers(x, *weights) -> None:
-    if not x.is_cuda or any(x.dtype != w.dtype or x.shape[-1] != w.shape[-1] or w.dim() != 2 for w in weights):
+    ok, k, dtype = x.is_cuda, x.shape[-1], x.dtype
+    for w in weights:
+        ok = ok and w.dim() == 2 and w.shape[-1] == k and w.dtype == dtype
+    if not ok:
         raise ValueError("linear takes CUDA tensors x [..., K] and weight [N, K] of one dtype")
+
+
+def _on(device, w):
+    return w if w.device == device else w.to(device)
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, *, implementation: str | None = None) -> torch.Tensor:
@@ -183,7 +190,7 @@ def linear_autograd(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     """:func:`linear` that records itself for reverse-mode differentiation."""
     _require_gpu()
     _check_layers(x, weight)
-    return _LinearFunction.apply(x, weight.to(x.device))  # (a gradient goes back to the weight's device)
+    return _LinearFunction.apply(x, _on(x.device, weight))  # (a gradient goes back to the weight's device)
 
 
 class _LinearPairFunction(torch.autograd.Function):
@@ -216,7 +223,7 @@ def linear_pair_autograd(x: torch.Tensor, w0: torch.Tensor, w1: torch.Tensor):
     """``(linear(x, w0), linear(x, w1))``, recorded for reverse-mode differentiation."""
     _require_gpu()
     _check_layers(x, w0, w1)
-    return _LinearPairFunction.apply(x, w0.to(x.device), w1.to(x.device))
+    return _LinearPairFunction.apply(x, _on(x.device, w0), _on(x.device, w1))
 
 
 def decode_paged(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, block_table: torch.Tensor, kv_lengths,

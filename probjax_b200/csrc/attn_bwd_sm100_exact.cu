@@ -34,9 +34,9 @@
 //
 // Bound by the element work of the compute warps at D = 64 and with modifiers (20 to 30 issue slots per score), by the
 // chain of MMAs, element work and barrier round trips at D = 128 and 192 without.
-// Spills (bytes stored / loaded, -Xptxas -v; 320 threads leave 204 registers to each): dK/dV with modifiers 44 to 68 / 76 to
-// 112, with a dense bias beside them 168 to 200 / 180 to 236; the bias gradient 16 to 24 / 16 to 44, with modifiers 312 / 328;
-// the other kernels 52 / 60 at most.
+// Spills (bytes stored / loaded, -Xptxas -v; a thread has 168 registers): dK/dV with modifiers 24 to 68 / 32 to 112, with a
+// dense bias beside them 168 to 200 / 180 to 236; the bias gradient 4 to 24 / 4 to 44, with modifiers 304 to 340 / 304 to 360;
+// the other kernels 28 / 60 at most.
 // Measured (forward + backward, against the CUDA-core kernels these calls ran on before; B200):
 //   packed documents + ALiBi, B1 S4096 Hq32 Hkv8 D128 bf16     41.9 ms -> 0.48 ms
 //   dense bias with gradient, B8 S1024 H16 D64 bf16            6.26 ms -> 0.49 ms
@@ -1430,10 +1430,11 @@ int launch_kernel(void (*kern)(Params...), int64_t grid, int smem, int cluster, 
 
 // CTAs that share a tile of the bias gradient: as many as the SMs take, each with four pairs or more (below that the exchange
 // costs what the shorter walk saves).  Sixteen, for a tile or a few that thousands of pairs share, is past the portable size:
-// only where the device says that such a cluster finds its SMs.
+// only as many such clusters as the device says find their SMs at a time (seven on this part; with eight planes of B1024 L64 H8
+// a second wave of one cluster took as long as clusters of eight).
 template <typename K>
 int dbias_cluster(K kern, int smem, int64_t tiles, int64_t pairs) {
-  static std::atomic<signed char> sixteen[64];  // per device: 0 not asked yet, 1 yes, -1 no
+  static std::atomic<int> sixteen[64];  // clusters of sixteen at a time on each device: 0 not asked yet, -1 none
   int dev = 0, sms = 148, n = 1;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   while (n < 16 && 2 * n * tiles <= sms && pairs >= 8 * n) n *= 2;
@@ -1455,9 +1456,9 @@ int dbias_cluster(K kern, int smem, int64_t tiles, int64_t pairs) {
                     cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
                     cudaOccupancyMaxActiveClusters(&fit, kern, &cfg) == cudaSuccess && fit > 0;
     if (!ok) (void)cudaGetLastError();
-    sixteen[dev] = ok ? 1 : -1;
+    sixteen[dev] = ok ? fit : -1;
   }
-  return sixteen[dev] > 0 ? 16 : 8;
+  return tiles <= sixteen[dev] ? 16 : 8;
 }
 
 template <int D, int DV, bool BF16, int FEAT>
